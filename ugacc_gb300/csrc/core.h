@@ -305,22 +305,12 @@ struct GemmPtrs {
   double* C;
 };
 
-// C = alpha * op(A) op(B) + beta * C, row-major; op(A)[m][k] = ta ? A[k*lda+m] : A[m*lda+k];
-// op(B)[k][n] = tb ? B[n*ldb+k] : B[k*ldb+n].  Batched over `batch` with either strides
-// or a device array of pointer triples.
-void dgemm(Ctx& c, bool ta, bool tb, int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t lda,
-           const double* B, int64_t ldb, double beta, double* C, const GemmEpilogue& epi, int batch = 1,
-           int64_t sA = 0, int64_t sB = 0, int64_t sC = 0, const GemmPtrs* ptrs = nullptr);
-
-// Same with arbitrary operand strides: op(A)[m][k] = A[m*sAm + k*sAk], op(B)[k][n] = B[k*sBk + n*sBn].
 // Status of the tensor-core launches since the last check (pipeline-wait timeout, sliced
 // operand out of range), read after synchronising the stream; throws on either.
 void tc_check(Ctx& c);
-// FP64 GEMM for a small output (M, N <= 256, M N <= 4096) and a long K (>= 8192): K chunks
-// per block and a fixed-order reduce.  False when the shape does not qualify.
-bool dgemm_small_output(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t sAm,
-                        int64_t sAk, const double* B, int64_t sBk, int64_t sBn, double beta, double* C,
-                        const GemmEpilogue& epi);
+// C = alpha * A B + beta * C with arbitrary operand strides: element (m, k) of A at A[m*sAm + k*sAk],
+// (k, n) of B at B[k*sBk + n*sBn].  Batched over `batch` with either strides or a device
+// array of pointer triples.
 void dgemm_strided(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t sAm, int64_t sAk,
                    const double* B, int64_t sBk, int64_t sBn, double beta, double* C, const GemmEpilogue& epi,
                    int batch, int64_t bA, int64_t bB, int64_t bC, const GemmPtrs* ptrs);

@@ -521,6 +521,7 @@ void contract(Ctx& c, const std::string& spec, double alpha, const Tensor& A, co
   bool done = false;
   const bool mixed = c.opt.precision == UCC_MIXED;
   const bool anchored = c.anchors.mode != 0 && mixed && (double)M * N * K >= kAnchorMinWork && tc_eligible(M, N, K);
+  // a reduction rather than a GEMM: mostly padding on the tensor tiles, FP64 in every precision
   const bool small_out = M <= 256 && N <= 256 && M * N <= 4096 && K >= 8192;
   // the tensor-core paths read operands whose index groups are two strided runs directly:
   // no gather
@@ -573,16 +574,9 @@ void contract(Ctx& c, const std::string& spec, double alpha, const Tensor& A, co
   }
   if (!done && c.opt.precision == UCC_MIXED && !c.force_fp64)
     done = mixed_gemm(c, M, N, K, ga, a.p, sAm, sAk, b.p, sBk, sBn, gb, ct.p, sCm, sCn);
-  if (!done) {  // small output, long K: a reduction rather than a GEMM (every precision)
-    GemmEpilogue epi;
-    epi.msplit = 0;
-    epi.s_mhi = sCm;
-    epi.s_n = sCn;
-    done = dgemm_small_output(c, M, N, K, ga, a.p, sAm, sAk, b.p, sBk, sBn, gb, ct.p, epi);
-  }
   // the FP64 work of the MIXED form (refinement sweeps, one-shot builds): sliced operands
   // on the tensor cores, FP64-accurate
-  if (!done && c.opt.precision == UCC_MIXED && !recorder()) {
+  if (!done && c.opt.precision == UCC_MIXED && !recorder() && !small_out) {
     const double t0 = c.stats.sliced_gemm_ms;
     done = sliced_gemm(c, M, N, K, ga, a.p, sAm, sAk, b.p, sBk, sBn, gb, ct.p, sCm, sCn);
     if (done && c.opt.print >= 3)  // PRINT >= 3: every sliced FP64 GEMM with its shape and time

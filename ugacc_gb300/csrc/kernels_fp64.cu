@@ -1,8 +1,6 @@
 // FP64 kernels for the plain form of the RHF-CC solver (sm_103a).
 //
-//  * dgemm_kernel      -- register-blocked DFMA GEMM over arbitrarily strided operands,
-//                         with a permuting epilogue so that a contraction result lands
-//                         directly in its tensor layout (no separate transpose pass)
+//  (the GEMM itself is dgemm.cu)
 //  * permute_kernel_*  -- tensor transposition with alpha/beta through a 32x33 shared tile
 //  * reductions        -- compensated (Neumaier) FP64 sums in two deterministic passes
 //  * amplitude kernels -- tau/ttau, Jacobi update with on-the-fly denominators, DIIS
@@ -28,116 +26,7 @@ static void check_launch(const char* what) {
   if (e != cudaSuccess) throw Error(UCC_CUDA_ERROR, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// ------------------------------------------------------------------------------------
-// GEMM
-// ------------------------------------------------------------------------------------
 namespace {
-constexpr int BM = 64, BN = 64, BK = 16, GT = 256;
-
-struct GemmArgs {
-  int64_t M, N, K;
-  int64_t kchunk;  // > 0: split-K, blockIdx.z selects K range [z*kchunk, min(K,(z+1)*kchunk)) and the
-                   // tile goes to C + z*M*N as a plain row-major partial (alpha = 1, beta = 0)
-  double alpha, beta;
-  const double* A;
-  int64_t sAm, sAk, bA;
-  const double* B;
-  int64_t sBk, sBn, bB;
-  double* C;
-  int64_t bC;
-  GemmEpilogue epi;
-  const GemmPtrs* ptrs;
-};
-
-template <bool AK, bool BN_>
-__global__ void __launch_bounds__(GT) dgemm_kernel(GemmArgs g) {
-  __shared__ double As[BK][BM + 1];
-  __shared__ double Bs[BK][BN + 1];
-  const int tid = threadIdx.x;
-  const int tx = tid % 16, ty = tid / 16;
-  const int64_t m0 = (int64_t)blockIdx.y * BM, n0 = (int64_t)blockIdx.x * BN;
-  const double* A;
-  const double* B;
-  double* C;
-  int64_t kbeg = 0, kend = g.K;
-  if (g.ptrs) {
-    A = g.ptrs[blockIdx.z].A;
-    B = g.ptrs[blockIdx.z].B;
-    C = g.ptrs[blockIdx.z].C;
-  } else if (g.kchunk > 0) {
-    A = g.A;
-    B = g.B;
-    C = g.C + (int64_t)blockIdx.z * g.M * g.N;
-    kbeg = (int64_t)blockIdx.z * g.kchunk;
-    kend = min(g.K, kbeg + g.kchunk);
-  } else {
-    A = g.A + (int64_t)blockIdx.z * g.bA;
-    B = g.B + (int64_t)blockIdx.z * g.bB;
-    C = g.C + (int64_t)blockIdx.z * g.bC;
-  }
-  double acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
-
-  for (int64_t k0 = kbeg; k0 < kend; k0 += BK) {
-#pragma unroll
-    for (int r = 0; r < (BM * BK) / GT; r++) {
-      const int e = tid + r * GT;
-      int mm, kk;
-      if (AK) { mm = e / BK; kk = e % BK; } else { kk = e / BM; mm = e % BM; }
-      const int64_t m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < g.M && k < kend) ? A[m * g.sAm + k * g.sAk] : 0.0;
-    }
-#pragma unroll
-    for (int r = 0; r < (BN * BK) / GT; r++) {
-      const int e = tid + r * GT;
-      int nn, kk;
-      if (BN_) { kk = e / BN; nn = e % BN; } else { nn = e / BK; kk = e % BK; }
-      const int64_t n = n0 + nn, k = k0 + kk;
-      Bs[kk][nn] = (n < g.N && k < kend) ? B[k * g.sBk + n * g.sBn] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; kk++) {
-      double a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  GemmEpilogue ep = g.epi;
-  double alpha = g.alpha, beta = g.beta;
-  if (g.kchunk > 0) {
-    ep.msplit = 0;
-    ep.s_mhi = g.N;
-    ep.s_n = 1;
-    alpha = 1.0;
-    beta = 0.0;
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int64_t m = m0 + ty + 16 * i;
-    if (m >= g.M) continue;
-    const int64_t mo = ep.msplit ? (m / ep.msplit) * ep.s_mhi + (m % ep.msplit) * ep.s_mlo : m * ep.s_mhi;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int64_t n = n0 + tx + 16 * j;
-      if (n >= g.N) continue;
-      double* cp = C + mo + n * ep.s_n;
-      const double v = alpha * acc[i][j];
-      *cp = (beta == 0.0) ? v : fma(beta, *cp, v);
-    }
-  }
-}
-
 // alpha * x + beta * y with the common coefficients taken off the FP64 pipe (GB300 issues
 // about two FP64 operations per SM clock, so a multiply per element already competes with
 // HBM): alpha = +-1 is exact (a sign flip), beta = 0 stores, beta = 1 adds once.  The
@@ -160,7 +49,15 @@ __global__ void splitk_reduce_kernel(int64_t M, int64_t N, int nsplit, const dou
   const int64_t MN = M * N;
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < MN; x += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int z = 0; z < nsplit; z++) s += P[(int64_t)z * MN + x];
+    int z = 0;
+    for (; z + 8 <= nsplit; z += 8) {  // eight loads in flight, added in order
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = P[(int64_t)(z + u) * MN + x];
+#pragma unroll
+      for (int u = 0; u < 8; u++) s += v[u];
+    }
+    for (; z < nsplit; z++) s += P[(int64_t)z * MN + x];
     const int64_t m = x / N, n = x - m * N;
     const int64_t mo = ep.msplit ? (m / ep.msplit) * ep.s_mhi + (m % ep.msplit) * ep.s_mlo : m * ep.s_mhi;
     double* cp = C + mo + n * ep.s_n;
@@ -171,149 +68,12 @@ __global__ void splitk_reduce_kernel(int64_t M, int64_t N, int nsplit, const dou
 }  // namespace
 
 void splitk_reduce(Ctx& c, int64_t M, int64_t N, int nsplit, const double* P, double alpha, double beta, double* C,
-                   const GemmEpilogue& epi);
-
-void dgemm_strided(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t sAm, int64_t sAk,
-                   const double* B, int64_t sBk, int64_t sBn, double beta, double* C, const GemmEpilogue& epi,
-                   int batch, int64_t bA, int64_t bB, int64_t bC, const GemmPtrs* ptrs) {
-  if (M <= 0 || N <= 0 || batch <= 0) return;
-  if (Recorder* r = recorder()) {
-    UCC_REQUIRE(batch == 1 && !ptrs && epi.msplit == 0, UCC_UNSUPPORTED, "dgemm: form not recordable");
-    RecordedOp o;
-    o.kind = RecordedOp::kGemm;
-    o.M = M, o.N = N, o.K = K, o.sAm = sAm, o.sAk = sAk, o.sBk = sBk, o.sBn = sBn, o.sCm = epi.s_mhi, o.sCn = epi.s_n;
-    o.A = A, o.B = B, o.C = C, o.alpha = alpha, o.beta = beta;
-    r->ops.push_back(o);
-    return;
-  }
-  UCC_REQUIRE(batch <= 65535, UCC_BAD_ARGS, "dgemm: batch too large");
-  GemmArgs g{M, N, K, 0, alpha, beta, A, sAm, sAk, bA, B, sBk, sBn, bB, C, bC, epi, ptrs};
-  dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)((M + BM - 1) / BM), (unsigned)batch);
-  UCC_REQUIRE(grid.y <= 65535, UCC_BAD_ARGS, "dgemm: M too large");
-  // Too few output tiles to fill the GPU and a long K: split K over blockIdx.z into
-  // partial tiles, then reduce them in a fixed order (deterministic).
-  const int64_t tiles = (int64_t)grid.x * grid.y;
-  std::unique_ptr<Scratch> part;
-  int nsplit = 1;
-  if (batch == 1 && !ptrs && tiles < 2 * 152 && K >= 4 * 64) {
-    nsplit = (int)std::min<int64_t>({(2 * 152 + tiles - 1) / tiles, K / 64, 512});
-    const int64_t kchunk = ((K + nsplit - 1) / nsplit + BK - 1) / BK * BK;
-    nsplit = (int)((K + kchunk - 1) / kchunk);
-    if (nsplit > 1) {
-      part = std::make_unique<Scratch>(c, sizeof(double) * M * N * nsplit);
-      g.kchunk = kchunk;
-      g.C = part->d();
-      grid.z = (unsigned)nsplit;
-    }
-  }
-  const bool ak = (sAk == 1) || (sAm != 1 && sAk < sAm);
-  const bool bn = (sBn == 1) || (sBk != 1 && sBn < sBk);
-  cudaEvent_t ev0 = c.take_event(), ev1 = c.take_event();
-  cudaEventRecord(ev0, c.stream);
-  if (ak && bn)
-    dgemm_kernel<true, true><<<grid, GT, 0, c.stream>>>(g);
-  else if (ak)
-    dgemm_kernel<true, false><<<grid, GT, 0, c.stream>>>(g);
-  else if (bn)
-    dgemm_kernel<false, true><<<grid, GT, 0, c.stream>>>(g);
-  else
-    dgemm_kernel<false, false><<<grid, GT, 0, c.stream>>>(g);
-  count_launch();
-  check_launch("dgemm");
-  if (part) splitk_reduce(c, M, N, nsplit, part->d(), alpha, beta, C, epi);
-  cudaEventRecord(ev1, c.stream);
-  c.gemm_timers.push_back({ev0, ev1, 2.0 * (double)M * (double)N * (double)K * (double)batch});
-  if (c.gemm_timers.size() >= 4096) c.resolve_timers();
-}
-
-void splitk_reduce(Ctx& c, int64_t M, int64_t N, int nsplit, const double* P, double alpha, double beta, double* C,
                    const GemmEpilogue& epi) {
   const int64_t MN = M * N;
   const unsigned blocks = (unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 16);
   splitk_reduce_kernel<<<blocks, 256, 0, c.stream>>>(M, N, nsplit, P, alpha, beta, C, epi);
   count_launch();
   check_launch("split-K reduce");
-}
-
-// ------------------------------------------------------------------------------------
-// GEMM with a small output (M, N <= 256, M N <= 4096) and a long K (reductions such as
-// sum_nef t_inef L_mnef): block z sums the K chunk [z kc, (z+1) kc) for every output into
-// P[z][m][n]; splitk_reduce adds the chunks in a fixed order.  A 64 x 64 tile would leave
-// most of its multiply-adds idle on such shapes.
-// ------------------------------------------------------------------------------------
-namespace {
-constexpr int SMT = 256, SMK = 16;  // threads, K rows staged per step
-__global__ void __launch_bounds__(SMT) dgemm_smallmn_kernel(int M, int N, int64_t K, int64_t kc,
-                                                           const double* __restrict__ A, int64_t sAm, int64_t sAk,
-                                                           const double* __restrict__ B, int64_t sBk, int64_t sBn,
-                                                           double* P) {
-  extern __shared__ double sm[];
-  double* As = sm;                   // [SMK][M]
-  double* Bs = sm + (size_t)SMK * M;  // [SMK][N]
-  const int MN = M * N, t = threadIdx.x;
-  const int64_t k0 = (int64_t)blockIdx.x * kc, k1 = min(K, k0 + kc);
-  double acc[16];
-#pragma unroll
-  for (int j = 0; j < 16; j++) acc[j] = 0.0;
-  for (int64_t kb = k0; kb < k1; kb += SMK) {
-    const int kn = (int)(k1 - kb < SMK ? k1 - kb : SMK);
-    __syncthreads();
-    for (int e = t; e < SMK * M; e += SMT) {  // A tile, k fastest when A is K-contiguous
-      const int kk = sAk == 1 ? e % SMK : e / M, m = sAk == 1 ? e / SMK : e % M;
-      As[kk * M + m] = kk < kn ? A[(int64_t)m * sAm + (kb + kk) * sAk] : 0.0;
-    }
-    for (int e = t; e < SMK * N; e += SMT) {
-      const int kk = sBk == 1 ? e % SMK : e / N, n = sBk == 1 ? e / SMK : e % N;
-      Bs[kk * N + n] = kk < kn ? B[(kb + kk) * sBk + (int64_t)n * sBn] : 0.0;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-      const int o = t + j * SMT;
-      if (o < MN) {
-        const int m = o / N, n = o - m * N;
-        double s = acc[j];
-#pragma unroll
-        for (int kk = 0; kk < SMK; kk++) s = fma(As[kk * M + m], Bs[kk * N + n], s);
-        acc[j] = s;
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < 16; j++) {
-    const int o = t + j * SMT;
-    if (o < MN) P[(int64_t)blockIdx.x * MN + o] = acc[j];
-  }
-}
-}  // namespace
-
-bool dgemm_small_output(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t sAm,
-                        int64_t sAk, const double* B, int64_t sBk, int64_t sBn, double beta, double* C,
-                        const GemmEpilogue& epi) {
-  if (recorder() || M > 256 || N > 256 || M * N > 16 * SMT || K < 8192) return false;
-  int64_t nblk = std::min<int64_t>((K + 511) / 512, 4 * 152);
-  const int64_t kc = ((K + nblk - 1) / nblk + SMK - 1) / SMK * SMK;
-  nblk = (K + kc - 1) / kc;
-  Scratch part(c, sizeof(double) * M * N * nblk);
-  cudaEvent_t ev0 = c.take_event(), ev1 = c.take_event();
-  cudaEventRecord(ev0, c.stream);
-  dgemm_smallmn_kernel<<<(unsigned)nblk, SMT, sizeof(double) * SMK * (M + N), c.stream>>>(
-      (int)M, (int)N, K, kc, A, sAm, sAk, B, sBk, sBn, part.d());
-  count_launch();
-  check_launch("dgemm_smallmn");
-  splitk_reduce(c, M, N, (int)nblk, part.d(), alpha, beta, C, epi);
-  cudaEventRecord(ev1, c.stream);
-  c.gemm_timers.push_back({ev0, ev1, 2.0 * (double)M * N * K});
-  if (c.gemm_timers.size() >= 4096) c.resolve_timers();
-  return true;
-}
-
-void dgemm(Ctx& c, bool ta, bool tb, int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t lda,
-           const double* B, int64_t ldb, double beta, double* C, const GemmEpilogue& epi, int batch, int64_t sA,
-           int64_t sB, int64_t sC, const GemmPtrs* ptrs) {
-  const int64_t sAm = ta ? 1 : lda, sAk = ta ? lda : 1;
-  const int64_t sBk = tb ? 1 : ldb, sBn = tb ? ldb : 1;
-  dgemm_strided(c, M, N, K, alpha, A, sAm, sAk, B, sBk, sBn, beta, C, epi, batch, sA, sB, sC, ptrs);
 }
 
 // ------------------------------------------------------------------------------------
