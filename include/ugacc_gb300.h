@@ -234,7 +234,7 @@ typedef struct ucc_batch_info {
   int sweeps;              /* sweeps of the last solve (all of them inside one graph launch) */
   int grouped_ops;         /* recorded residual operations, each one grouped launch per sweep */
   int graph_kernels;       /* kernel nodes in the sweep graph */
-  int shape_choice[4];     /* GEMM operations given tile 64x64, 32x32, 64x32, 32x64 by the autotuner */
+  int shape_choice[4];     /* GEMM operations on 16x16 and on 32x32 tiles (the other two entries are 0) */
   double solve_ms;         /* device time of the last solve (CUDA events) */
   double flops;            /* algorithmic CCSD FLOPs of the last solve, summed over members' iterations */
   double arena_bytes;      /* recorded scratch held for the members */

@@ -7,10 +7,11 @@
 // scratch placed in a per-member arena.  Operation k of all members then becomes ONE
 // grouped launch:
 //
-//   grouped_gemm<BM,BN>  -- FP64 DFMA tiles of every member's GEMM k, a flat tile space
-//                           (prefix sums over members), the tile shape chosen per
-//                           operation by timing the candidates on the real operands;
-//   grouped_perm         -- every member's permute / axpby / fill k, in 2048-element chunks.
+//   grouped_gemm  -- FP64 DFMA tiles of every member's GEMM k, a flat tile space (prefix
+//                    sums over members), tile shape and K split chosen per operation by
+//                    dgemm_plan;
+//   grouped_perm  -- every member's permute / axpby / fill k, in 2048-element chunks;
+//   grouped_pack_tau, grouped_unpack -- the two ends of the packed particle ladder.
 //
 // The rest of a sweep (Jacobi update, residual norm, convergence mask, DIIS with its
 // B-matrix rows, subspace solve and extrapolation, tau/ttau, energy) is written directly
@@ -30,7 +31,9 @@
 #include <vector>
 
 #include "cc.h"
+#include "dgemm_tile.h"
 #include "engine.h"
+#include "pairs.h"
 #include "pert.h"
 
 namespace ucc {
@@ -48,12 +51,13 @@ struct GemmDesc {
   const double* A;
   const double* B;
   double* C;
+  double* part;  // partial products [zg][M][N] of a split operation
   double alpha, beta;
   int prob;
 };
 
 struct PermDesc {
-  int rank, prob, fill;
+  int rank, prob, fill, narrow;
   int64_t total;
   int64_t d[kMaxRank], si[kMaxRank], so[kMaxRank];
   const double* in;
@@ -124,78 +128,116 @@ __device__ __forceinline__ int find_item(const int64_t* __restrict__ prefix, int
 }
 
 // ---------------------------------------------------------------------------------------
-// Grouped GEMM: 16x16 threads, each (BM/16) x (BN/16) outputs, K in steps of 16 through
-// shared memory; operand loads follow whichever index is contiguous.
+// Grouped GEMM: the tiles of dgemm_tile.h over a flat tile space of all members, one CTA (or
+// one cluster of zc CTAs that share K) per tile, zg K shares per tile as partial products.
+// The members come longest K share first and every tile is its own CTA, so the hardware's
+// dispatch evens out the SMs; the FP64 pipe bounds the launch.  16 members of the
+// no <= 12 / nv <= 96 family, per solve of 8 sweeps: 1111 ms with padded 32 x 32 tiles on a
+// fixed grid, one CTA per tile whatever its K and the unpacked ladder, 354 ms now.
 // ---------------------------------------------------------------------------------------
-template <int BM_, int BN_>
-__global__ void __launch_bounds__(256) grouped_gemm(const GemmDesc* __restrict__ desc,
-                                                    const int64_t* __restrict__ prefix, int nd, int64_t total,
-                                                    const int* __restrict__ active) {
-  constexpr int TM = BM_ / 16, TN = BN_ / 16, BK = 16;
-  __shared__ double As[BK][BM_ + 1];
-  __shared__ double Bs[BK][BN_ + 1];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+template <class T, bool CLUSTER>
+__global__ void __launch_bounds__(T::THREADS) grouped_gemm(const GemmDesc* __restrict__ desc,
+                                                           const int64_t* __restrict__ prefix, int nd, int64_t total,
+                                                           int zc, int zg, const int* __restrict__ active) {
+  __shared__ double smem[T::SMEM];
+  const int rank = CLUSTER ? (int)dgemm_cluster_rank() : 0;
+  const int64_t u = CLUSTER ? blockIdx.x / zc : blockIdx.x;
+  // K share zi of tile t: the shares of one member's tiles are neighbours, its longest first
+  const int64_t t = u / zg;
+  const int zi = (int)(u - t * zg);
+  const int di = find_item(prefix, nd, t);
+  const GemmDesc g = desc[di];
+  if (!active[g.prob]) return;  // the whole cluster
+  const int64_t local = t - prefix[di], ntn = (g.N + T::BN - 1) / T::BN;
+  const int64_t z = (int64_t)zc * zg, kchunk = (g.K + z - 1) / z;
+  const int64_t m0 = local / ntn * T::BM, n0 = local % ntn * T::BN, k0 = ((int64_t)zi * zc + rank) * kchunk;
+  const GemmEpilogue direct{0, g.sCm, 0, g.sCn}, partial{0, g.N, 0, 1};
+  dgemm_cta<T, CLUSTER>(smem, rank, zc, g.M, g.N, g.K, m0, n0, k0, kchunk, g.A, g.sAm, g.sAk, g.B, g.sBk, g.sBn,
+                        zg > 1 ? 1.0 : g.alpha, zg > 1 ? 0.0 : g.beta, zg > 1 ? g.part + (int64_t)zi * g.M * g.N : g.C,
+                        zg > 1 ? partial : direct);
+}
+
+// C = alpha * (the zg partial products, in order) + beta * C, kChunk outputs per work item
+__global__ void grouped_splitk_reduce(const GemmDesc* __restrict__ desc, const int64_t* __restrict__ prefix, int nd,
+                                      int64_t total, int zg, const int* __restrict__ active) {
   for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
     const int di = find_item(prefix, nd, t);
-    const GemmDesc g = desc[di];
+    const GemmDesc& g = desc[di];
     if (!active[g.prob]) continue;
-    const int64_t local = t - prefix[di];
-    const int64_t ntn = (g.N + BN_ - 1) / BN_;
-    const int64_t m0 = local / ntn * BM_, n0 = local % ntn * BN_;
-    double acc[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; i++)
-#pragma unroll
-      for (int j = 0; j < TN; j++) acc[i][j] = 0.0;
-    const bool a_kfast = g.sAk == 1, b_nfast = g.sBn == 1;
-    for (int64_t k0 = 0; k0 < g.K; k0 += BK) {
-      for (int e = tid; e < BM_ * BK; e += 256) {
-        const int mm = a_kfast ? e / BK : e % BM_, kk = a_kfast ? e % BK : e / BM_;
-        const int64_t m = m0 + mm, k = k0 + kk;
-        As[kk][mm] = (m < g.M && k < g.K) ? g.A[m * g.sAm + k * g.sAk] : 0.0;
-      }
-      for (int e = tid; e < BN_ * BK; e += 256) {
-        const int nn = b_nfast ? e % BN_ : e / BK, kk = b_nfast ? e / BN_ : e % BK;
-        const int64_t n = n0 + nn, k = k0 + kk;
-        Bs[kk][nn] = (n < g.N && k < g.K) ? g.B[k * g.sBk + n * g.sBn] : 0.0;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < BK; kk++) {
-        double a[TM], b[TN];
-#pragma unroll
-        for (int i = 0; i < TM; i++) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-        for (int j = 0; j < TN; j++) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-        for (int i = 0; i < TM; i++)
-#pragma unroll
-          for (int j = 0; j < TN; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < TM; i++) {
-      const int64_t m = m0 + ty + 16 * i;
-      if (m >= g.M) continue;
-#pragma unroll
-      for (int j = 0; j < TN; j++) {
-        const int64_t n = n0 + tx + 16 * j;
-        if (n >= g.N) continue;
-        double* c = g.C + m * g.sCm + n * g.sCn;
-        const double v = g.alpha * acc[i][j];
-        *c = (g.beta == 0.0) ? v : fma(g.beta, *c, v);
-      }
+    const int64_t mn = g.M * g.N, e0 = (t - prefix[di]) * kChunk, e1 = min(e0 + kChunk, mn);
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
+      double s = 0.0;
+#pragma unroll 8
+      for (int q = 0; q < zg; q++) s += g.part[(int64_t)q * mn + e];
+      const int64_t m = e / g.N, n = e - m * g.N;
+      double* c = g.C + m * g.sCm + n * g.sCn;
+      const double v = g.alpha * s;
+      *c = (g.beta == 0.0) ? v : fma(g.beta, *c, v);
     }
   }
 }
 
-struct TileShape {
-  int bm, bn;
+// The packed ladder's operations (pairs.h) of all members: tau into Tp / Tm, one block per
+// (tile pair, i <= j) item; S and A into R2, kChunk elements per item.
+struct LadderDesc {
+  int no, nv, prob;
+  double alpha;
+  const double* in;   // tau, or S
+  const double* in2;  // A
+  double* out;        // Tp, or R2
+  double* out2;       // Tm
 };
-constexpr TileShape kShapes[] = {{64, 64}, {32, 32}, {64, 32}, {32, 64}};
-constexpr int kNumShapes = 4;
+__global__ void grouped_pack_tau(const LadderDesc* __restrict__ desc, const int64_t* __restrict__ prefix, int nd,
+                                 int64_t total, const int* __restrict__ active) {
+  for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+    const int di = find_item(prefix, nd, t);
+    const LadderDesc& p = desc[di];
+    if (!active[p.prob]) continue;
+    const int nt = (p.nv + 31) / 32, tiles = nt * (nt + 1) / 2;
+    const int64_t local = t - prefix[di];
+    pack_pairs_tile(p.no, p.nv, 0.5, p.in, p.out, p.out2, (int)(local % tiles), local / tiles);
+    __syncthreads();  // the tile's shared memory is reused
+  }
+}
+__global__ void grouped_unpack(const LadderDesc* __restrict__ desc, const int64_t* __restrict__ prefix, int nd,
+                               int64_t total, const int* __restrict__ active) {
+  for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
+    const int di = find_item(prefix, nd, t);
+    const LadderDesc& p = desc[di];
+    if (!active[p.prob]) continue;
+    const int64_t n = (int64_t)p.no * p.no * p.nv * p.nv;
+    const int64_t e0 = (t - prefix[di]) * kChunk, e1 = min(e0 + kChunk, n);
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x)  // n < 2^31 (build)
+      p.out[e] += p.alpha * unpack_pair<uint32_t>(p.no, p.nv, p.in, p.in2, (uint32_t)e);
+  }
+}
 
+template <class I>
+__device__ __forceinline__ void perm_chunk(const PermDesc& p, int64_t e0, int64_t e1) {
+  I d[kMaxRank], si[kMaxRank], so[kMaxRank];
+  const int r = p.rank;
+  for (int k = 0; k < r; k++) d[k] = (I)p.d[k], si[k] = (I)p.si[k], so[k] = (I)p.so[k];
+  const bool scale = p.alpha != 1.0;  // one FP64 operation less per element on GB300's narrow pipe
+  for (I e = (I)e0 + threadIdx.x; e < (I)e1; e += blockDim.x) {
+    I rem = e, oi = 0, oo = 0;
+    for (int k = r - 1; k > 0; k--) {
+      const I q = rem / d[k], x = rem - q * d[k];
+      rem = q;
+      oi += x * si[k];
+      oo += x * so[k];
+    }
+    oi += rem * si[0];
+    oo += rem * so[0];
+    if (p.fill) {
+      p.out[oo] = p.alpha;
+    } else {
+      const double x = p.in[oi], v = scale ? p.alpha * x : x;
+      p.out[oo] = (p.beta == 0.0) ? v : fma(p.beta, p.out[oo], v);
+    }
+  }
+}
+// The axes come merged where both sides are contiguous (build): most operations are one or
+// two axes long; 32-bit indices where every offset fits.
 __global__ void grouped_perm(const PermDesc* __restrict__ desc, const int64_t* __restrict__ prefix, int nd,
                              int64_t total, const int* __restrict__ active) {
   for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
@@ -203,21 +245,10 @@ __global__ void grouped_perm(const PermDesc* __restrict__ desc, const int64_t* _
     const PermDesc& p = desc[di];
     if (!active[p.prob]) continue;
     const int64_t e0 = (t - prefix[di]) * kChunk, e1 = min(e0 + kChunk, p.total);
-    for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-      int64_t r = e, oi = 0, oo = 0;
-      for (int k = p.rank - 1; k >= 0; k--) {
-        const int64_t x = r % p.d[k];
-        r /= p.d[k];
-        oi += x * p.si[k];
-        oo += x * p.so[k];
-      }
-      if (p.fill) {
-        p.out[oo] = p.alpha;
-      } else {
-        const double v = p.alpha * p.in[oi];
-        p.out[oo] = (p.beta == 0.0) ? v : fma(p.beta, p.out[oo], v);
-      }
-    }
+    if (p.narrow)
+      perm_chunk<uint32_t>(p, e0, e1);
+    else
+      perm_chunk<int64_t>(p, e0, e1);
   }
 }
 
@@ -539,11 +570,12 @@ struct DevArray {
 
 struct GroupOp {
   int kind = 0;  // RecordedOp::Kind (fill is a permute descriptor with fill = 1)
-  int shape = 0;  // GEMM tile shape (index into kShapes)
+  DgemmPlan plan{1, 1, 1};  // GEMM: tile shape and K split
   DevArray<GemmDesc> gdesc;
   DevArray<PermDesc> pdesc;
-  DevArray<int64_t> prefix[kNumShapes];
-  int64_t total[kNumShapes] = {};
+  DevArray<LadderDesc> ldesc;
+  DevArray<int64_t> prefix, rprefix;  // work items; of a split GEMM's reduction
+  int64_t total = 0, rtotal = 0;
   int nd = 0;
   double flops = 0.0;
 };
@@ -569,6 +601,7 @@ struct ucc_batch {
   int64_t total_np = 0, total_t2 = 0;
   DevArray<int> active, iterations, converged, status;
   DevArray<double> partial, dpartial, sumsq, rms, energy, Bmat, coef, epartial;
+  DevArray<double> splitk;  // partial products of the split GEMMs (one operation at a time)
   DevArray<SweepState> state;
   std::vector<std::unique_ptr<DeviceBuffer>> diis_store;
   cudaGraph_t graph = nullptr;
@@ -609,37 +642,113 @@ ucc_status bguard(ucc_batch* b, F&& f) {
 
 unsigned grid_for(int64_t items) { return (unsigned)std::max<int64_t>(1, std::min<int64_t>(items, 152 * 8)); }
 
-void launch_gemm(ucc_batch& B, GroupOp& op, int shape) {
-  const int64_t total = op.total[shape];
-  if (total == 0) return;
-  const unsigned grid = grid_for(total);
-  const GemmDesc* d = op.gdesc.p;
-  const int64_t* pf = op.prefix[shape].p;
-  switch (shape) {
-    case 0:
-      grouped_gemm<64, 64><<<grid, 256, 0, B.stream>>>(d, pf, op.nd, total, B.active.p);
-      break;
-    case 1:
-      grouped_gemm<32, 32><<<grid, 256, 0, B.stream>>>(d, pf, op.nd, total, B.active.p);
-      break;
-    case 2:
-      grouped_gemm<64, 32><<<grid, 256, 0, B.stream>>>(d, pf, op.nd, total, B.active.p);
-      break;
-    default:
-      grouped_gemm<32, 64><<<grid, 256, 0, B.stream>>>(d, pf, op.nd, total, B.active.p);
-      break;
+template <class T>
+void launch_tiles(ucc_batch& B, GroupOp& op) {
+  const DgemmPlan& p = op.plan;
+  const unsigned grid = (unsigned)(op.total * p.zc * p.zg);
+  if (p.zc == 1) {
+    grouped_gemm<T, false><<<grid, T::THREADS, 0, B.stream>>>(op.gdesc.p, op.prefix.p, op.nd, op.total, 1, p.zg,
+                                                              B.active.p);
+    return;
   }
-  UCC_CUDA(cudaGetLastError());
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(T::THREADS);
+  cfg.stream = B.stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)p.zc;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const GemmDesc* d = op.gdesc.p;
+  const int64_t* pf = op.prefix.p;
+  const int* act = B.active.p;
+  UCC_CUDA(cudaLaunchKernelEx(&cfg, grouped_gemm<T, true>, d, pf, op.nd, op.total, p.zc, p.zg, act));
 }
 
-void launch_op(ucc_batch& B, GroupOp& op) {
-  if (op.kind == RecordedOp::kGemm) {
-    launch_gemm(B, op, op.shape);
-  } else if (op.total[0] > 0) {
-    grouped_perm<<<grid_for(op.total[0]), 256, 0, B.stream>>>(op.pdesc.p, op.prefix[0].p, op.nd, op.total[0],
-                                                              B.active.p);
+// launches one operation of all members; the number of kernels
+int launch_op(ucc_batch& B, GroupOp& op) {
+  int k = 0;
+  if (op.total > 0) {
+    const unsigned grid = grid_for(op.total);
+    k++;
+    switch (op.kind) {
+      case RecordedOp::kGemm:
+        if (op.plan.shape == 0)
+          launch_tiles<DTile16>(B, op);
+        else
+          launch_tiles<DTile32>(B, op);
+        if (op.plan.zg > 1) {
+          grouped_splitk_reduce<<<grid_for(op.rtotal), 256, 0, B.stream>>>(op.gdesc.p, op.rprefix.p, op.nd, op.rtotal,
+                                                                           op.plan.zg, B.active.p);
+          k++;
+        }
+        break;
+      case RecordedOp::kPackTau:
+        grouped_pack_tau<<<grid, dim3(32, 8), 0, B.stream>>>(op.ldesc.p, op.prefix.p, op.nd, op.total, B.active.p);
+        break;
+      case RecordedOp::kUnpack:
+        grouped_unpack<<<grid, 256, 0, B.stream>>>(op.ldesc.p, op.prefix.p, op.nd, op.total, B.active.p);
+        break;
+      default:
+        grouped_perm<<<grid, 256, 0, B.stream>>>(op.pdesc.p, op.prefix.p, op.nd, op.total, B.active.p);
+    }
     UCC_CUDA(cudaGetLastError());
   }
+  return k;
+}
+
+// neighbouring axes that are contiguous on both sides become one, unit axes go
+void merge_axes(PermDesc& p) {
+  int r = 0;
+  int64_t mi = 0, mo = 0;
+  for (int k = 0; k < p.rank; k++) {
+    if (p.d[k] == 1) continue;
+    mi += (p.d[k] - 1) * p.si[k];
+    mo += (p.d[k] - 1) * p.so[k];
+    if (r > 0 && p.si[r - 1] == p.si[k] * p.d[k] && p.so[r - 1] == p.so[k] * p.d[k]) {
+      p.d[r - 1] *= p.d[k];
+      p.si[r - 1] = p.si[k];
+      p.so[r - 1] = p.so[k];
+      continue;
+    }
+    p.d[r] = p.d[k], p.si[r] = p.si[k], p.so[r] = p.so[k];
+    r++;
+  }
+  if (r == 0) p.d[0] = 1, p.si[0] = p.so[0] = 1, r = 1;
+  p.rank = r;
+  const int64_t lim = (int64_t)1 << 31;
+  p.narrow = p.total + 256 < lim && mi < lim && mo < lim;
+}
+
+// a GEMM operation of all members: its plan, and the members longest K share first
+void group_gemm(ucc_batch& B, GroupOp& g, const std::vector<std::vector<RecordedOp>>& traces, size_t k,
+                std::vector<GemmDesc>& d) {
+  const int nm = (int)traces.size();
+  std::vector<GemmShape> shapes;
+  for (int b = 0; b < nm; b++) {
+    const RecordedOp& o = traces[b][k];
+    d.push_back(GemmDesc{o.M, o.N, o.K, o.sAm, o.sAk, o.sBk, o.sBn, o.sCm, o.sCn, o.A, o.B, o.C, nullptr, o.alpha,
+                         o.beta, b});
+    shapes.push_back({o.M, o.N, o.K, 1});
+    g.flops += 2.0 * (double)o.M * (double)o.N * (double)o.K;
+  }
+  g.plan = dgemm_plan(shapes, true);
+  std::stable_sort(d.begin(), d.end(), [](const GemmDesc& x, const GemmDesc& y) { return x.K > y.K; });
+  const int bm = g.plan.shape == 0 ? DTile16::BM : DTile32::BM, bn = g.plan.shape == 0 ? DTile16::BN : DTile32::BN;
+  std::vector<int64_t> pf(nm), rpf(nm);
+  for (int b = 0; b < nm; b++) {
+    pf[b] = g.total;
+    g.total += ((d[b].M + bm - 1) / bm) * ((d[b].N + bn - 1) / bn);
+    rpf[b] = g.rtotal;
+    g.rtotal += (d[b].M * d[b].N + kChunk - 1) / kChunk;
+  }
+  UCC_REQUIRE(g.total * g.plan.zc * g.plan.zg < ((int64_t)1 << 31), UCC_UNSUPPORTED, "batch: too many output tiles");
+  g.prefix.upload(pf, B.stream);
+  if (g.plan.zg > 1) g.rprefix.upload(rpf, B.stream);
+  B.info.shape_choice[g.plan.shape]++;
 }
 
 // record every member's residual build and group the operations
@@ -651,14 +760,28 @@ void build(ucc_batch& B) {
   B.arenas.clear();
   B.diis_store.clear();
   double arena_bytes = 0.0;
+  // the ladder runs on packed pairs when every member has pairs on both sides (all members
+  // record the same operations) and its amplitudes fit the 32-bit unpacking
+  // and the packed operators (half of <ab|ef> again) leave half of the free memory
+  bool packed = true;
+  double operator_bytes = 0.0;
+  for (const auto& m : B.members) {
+    packed = packed && m->no > 1 && m->nv > 1 && (int64_t)m->no * m->no * m->nv * m->nv + 256 < ((int64_t)1 << 31);
+    if (!m->has("Vpp")) operator_bytes += 4.0 * std::pow((double)m->nv, 4);
+  }
+  size_t free_b = 0, total_b = 0;
+  UCC_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  packed = packed && operator_bytes < 0.5 * (double)free_b;
   for (int b = 0; b < nm; b++) {
     Ctx& c = *B.members[b];
     ccsd_alloc(c);
+    if (packed) ladder_operator(c, "Vvvvv", 0, "Vpp", "Vmm");
     const double* to = c.get("Told").p;
     double* r = c.get("R").p;
     size_t need = 0;
     for (int pass = 0; pass < 2; pass++) {
       Recorder rec;
+      rec.packed_ladder = packed;
       const bool first = b == 0 && pass == 0;
       if (!first) {
         rec.tape = tape;
@@ -694,28 +817,31 @@ void build(ucc_batch& B) {
   }
   B.ops.clear();
   B.ops.resize(nops);
+  for (int& n : B.info.shape_choice) n = 0;
+  std::vector<std::vector<GemmDesc>> gemms(nops);
+  int64_t split_size = 0;
   for (size_t k = 0; k < nops; k++) {
     GroupOp& g = B.ops[k];
     g.kind = traces[0][k].kind;
     g.nd = nm;
     if (g.kind == RecordedOp::kGemm) {
-      std::vector<GemmDesc> d(nm);
+      group_gemm(B, g, traces, k, gemms[k]);
+      int64_t part = 0;
+      for (const GemmDesc& d : gemms[k]) part += d.M * d.N * g.plan.zg;
+      if (g.plan.zg > 1) split_size = std::max(split_size, part);
+    } else if (g.kind == RecordedOp::kPackTau || g.kind == RecordedOp::kUnpack) {
+      std::vector<LadderDesc> d(nm);
+      std::vector<int64_t> pf(nm);
       for (int b = 0; b < nm; b++) {
         const RecordedOp& o = traces[b][k];
-        d[b] = GemmDesc{o.M, o.N, o.K, o.sAm, o.sAk, o.sBk, o.sBn, o.sCm, o.sCn, o.A, o.B, o.C, o.alpha, o.beta, b};
-        g.flops += 2.0 * (double)o.M * (double)o.N * (double)o.K;
+        const int no = (int)o.d[0], nv = (int)o.d[1];
+        const int64_t nt = (nv + 31) / 32, n = (int64_t)no * no * nv * nv;
+        d[b] = LadderDesc{no, nv, b, o.alpha, o.in, o.in2, o.out, o.out2};
+        pf[b] = g.total;
+        g.total += g.kind == RecordedOp::kPackTau ? nt * (nt + 1) / 2 * no * (no + 1) / 2 : (n + kChunk - 1) / kChunk;
       }
-      g.gdesc.upload(d, B.stream);
-      for (int s = 0; s < kNumShapes; s++) {
-        std::vector<int64_t> pf(nm);
-        int64_t run = 0;
-        for (int b = 0; b < nm; b++) {
-          pf[b] = run;
-          run += ((d[b].M + kShapes[s].bm - 1) / kShapes[s].bm) * ((d[b].N + kShapes[s].bn - 1) / kShapes[s].bn);
-        }
-        g.total[s] = run;
-        g.prefix[s].upload(pf, B.stream);
-      }
+      g.ldesc.upload(d, B.stream);
+      g.prefix.upload(pf, B.stream);
     } else {
       std::vector<PermDesc> d(nm);
       std::vector<int64_t> pf(nm);
@@ -738,13 +864,25 @@ void build(ucc_batch& B) {
         p.out = o.out;
         p.alpha = o.alpha;
         p.beta = o.beta;
+        merge_axes(p);
         pf[b] = run;
         run += (p.total + kChunk - 1) / kChunk;
       }
-      g.total[0] = run;
+      g.total = run;
       g.pdesc.upload(d, B.stream);
-      g.prefix[0].upload(pf, B.stream);
+      g.prefix.upload(pf, B.stream);
     }
+  }
+  // the split operations run one after the other and share one array of partial products
+  B.splitk.zeros((size_t)split_size, B.stream);
+  for (size_t k = 0; k < nops; k++) {
+    if (gemms[k].empty()) continue;
+    double* part = B.splitk.p;
+    for (GemmDesc& d : gemms[k]) {
+      d.part = part;
+      if (B.ops[k].plan.zg > 1) part += d.M * d.N * B.ops[k].plan.zg;
+    }
+    B.ops[k].gdesc.upload(gemms[k], B.stream);
   }
   // sweep tables
   std::vector<Member> mh(nm);
@@ -799,51 +937,13 @@ void set_all_active(ucc_batch& B) {
   B.active.upload(one, B.stream);
 }
 
-// one residual build with the default shapes (valid data in every buffer), then each
-// GEMM operation timed with every tile shape; the fastest is kept
-void autotune(ucc_batch& B) {
-  set_all_active(B);
-  for (auto& op : B.ops) launch_op(B, op);
-  UCC_CUDA(cudaStreamSynchronize(B.stream));
-  cudaEvent_t e0, e1;
-  UCC_CUDA(cudaEventCreate(&e0));
-  UCC_CUDA(cudaEventCreate(&e1));
-  for (int s = 0; s < kNumShapes; s++) B.info.shape_choice[s] = 0;
-  for (auto& op : B.ops) {
-    if (op.kind != RecordedOp::kGemm) continue;
-    float best = 1e30f;
-    int pick = 0;
-    for (int s = 0; s < kNumShapes; s++) {
-      if (op.total[s] == 0) continue;
-      launch_gemm(B, op, s);  // warm
-      cudaEventRecord(e0, B.stream);
-      launch_gemm(B, op, s);
-      cudaEventRecord(e1, B.stream);
-      UCC_CUDA(cudaEventSynchronize(e1));
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, e0, e1);
-      if (ms < best) {
-        best = ms;
-        pick = s;
-      }
-    }
-    op.shape = pick;
-    B.info.shape_choice[pick]++;
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-}
-
 // the kernels of one sweep, in order (captured into the sweep graph)
 int enqueue_sweep(ucc_batch& B) {
   const int nm = (int)B.members.size();
   int k = 0;
   save_kernel<<<grid_for(B.total_np), 256, 0, B.stream>>>(B.mem.p, B.prefix_np.p, nm, B.total_np, B.active.p);
   k++;
-  for (auto& op : B.ops) {
-    launch_op(B, op);
-    k++;
-  }
+  for (auto& op : B.ops) k += launch_op(B, op);
   jacobi_kernel<<<grid_for(B.total_np), 256, 0, B.stream>>>(B.mem.p, B.prefix_np.p, nm, B.total_np, B.active.p,
                                                             B.partial.p);
   reduce_kernel<<<nm, 256, 0, B.stream>>>(B.prefix_np.p, nm, B.total_np, B.active.p, B.partial.p, B.sumsq.p);
@@ -1010,10 +1110,7 @@ ucc_status ucc_batch_ccsd(ucc_batch* b, const ucc_options* opt, double* e_ccsd, 
     UCC_REQUIRE(opt->maxiter >= 1 && opt->r_convergence > 0, UCC_BAD_ARGS, "bad maxiter or r_convergence");
     const int nm = (int)B.members.size();
     UCC_REQUIRE(nm >= 1, UCC_BAD_STATE, "empty batch");
-    if (!B.built) {
-      build(B);
-      autotune(B);
-    }
+    if (!B.built) build(B);
     capture(B, opt->diis != 0);
     start_members(B);
     set_all_active(B);

@@ -101,7 +101,9 @@ double run_triples(Ctx& c);
 // mode (0: H_abef, 1: H_efab + H_feba, 2: H_abef + H_bafe)
 void packed_ladder(Ctx& c, double alpha, const Tensor& amp, const char* src, int mode, const char* vp_name,
                    const char* vm_name, double* R2);
-// the packed form needs pairs on both sides and runs eagerly (it is not part of a recorded sweep)
+// the packed operator of a ladder, built from block src once per Hamiltonian or HBAR
+void ladder_operator(Ctx& c, const char* src, int mode, const char* vp_name, const char* vm_name);
+// the packed HBAR ladders need pairs on both sides and run eagerly (not part of a recorded sweep)
 inline bool hbar_ladder_packed(Ctx& c) { return !recorder() && c.no > 1 && c.nv > 1; }
 void run_triples_gradient(Ctx& c);  // tgrad.cu
 void run_hbar(Ctx& c);

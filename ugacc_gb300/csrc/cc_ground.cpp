@@ -324,6 +324,13 @@ void build_t1(Ctx& c, const Tensor& t1, const Tensor& t2, Tensor R1) {
 //
 }  // namespace
 
+void ladder_operator(Ctx& c, const char* src, int mode, const char* vp_name, const char* vm_name) {
+  const int64_t nv = c.nv, vp = nv * (nv + 1) / 2, vm = nv * (nv - 1) / 2;
+  if (c.has(vp_name)) return;
+  Tensor Vp = c.alloc(vp_name, {vp, vp}, false), Vm = c.alloc(vm_name, {vm, vm}, false);
+  pack_vvvv(c, c.nv, mode, c.get(src).p, Vp.p, Vm.p);
+}
+
 // R2 += alpha sum_ef W_abef amp_ijef on packed pairs (kernels_fp64.cu): S = Tp Vp^T over
 // (i<=j, a<=b, e<=f), A = Tm Vm^T over strict pairs, a quarter of the multiply-adds of the
 // plain contraction; amp must be invariant under (i,j,e,f) -> (j,i,f,e).  The packed
@@ -333,10 +340,7 @@ void packed_ladder(Ctx& c, double alpha, const Tensor& amp, const char* src, int
   const int no = c.no, nv = c.nv;
   const int64_t op = (int64_t)no * (no + 1) / 2, om = (int64_t)no * (no - 1) / 2;
   const int64_t vp = (int64_t)nv * (nv + 1) / 2, vm = (int64_t)nv * (nv - 1) / 2;
-  if (!c.has(vp_name)) {
-    Tensor Vp = c.alloc(vp_name, {vp, vp}, false), Vm = c.alloc(vm_name, {vm, vm}, false);
-    pack_vvvv(c, nv, mode, c.get(src).p, Vp.p, Vm.p);
-  }
+  if (!recorder()) ladder_operator(c, src, mode, vp_name, vm_name);
   UCC_REQUIRE(amp.dense(), UCC_BAD_ARGS, "packed ladder: dense amplitudes");
   Temp Tp(c, {op, vp}), Tm(c, {om, vm}), S(c, {op, vp}), A(c, {om, vm});
   pack_tau(c, no, nv, amp.p, Tp->p, Tm->p);
@@ -347,12 +351,12 @@ void packed_ladder(Ctx& c, double alpha, const Tensor& amp, const char* src, int
 
 namespace {
 
-// particle ladder sum_ef <ab|ef> tau_ijef, ccwfn.cc:508-510.  Outside a recorded batch it
-// runs on packed pairs: S = Tp Vp^T over (i<=j, a<=b, e<=f) and A = Tm Vm^T over strict
-// pairs, a quarter of the multiply-adds (the result is symmetric under the simultaneous
-// swap (i,j,a,b) -> (j,i,b,a) and the integrals under (a,b,e,f) -> (b,a,f,e))
+// particle ladder sum_ef <ab|ef> tau_ijef, ccwfn.cc:508-510, on packed pairs where there are
+// pairs: S = Tp Vp^T over (i<=j, a<=b, e<=f) and A = Tm Vm^T over strict pairs, a quarter of
+// the multiply-adds (the result is symmetric under the simultaneous swap
+// (i,j,a,b) -> (j,i,b,a) and the integrals under (a,b,e,f) -> (b,a,f,e))
 void ladder(Ctx& c, const Tensor& tau, const Tensor& R2) {
-  if (recorder() || c.no < 2 || c.nv < 2) {
+  if (recorder() ? !recorder()->packed_ladder : c.no < 2 || c.nv < 2) {
     contract(c, "ijef,abef->ijab", 1.0, tau, V(c, "vvvv"), 1.0, R2);
     return;
   }

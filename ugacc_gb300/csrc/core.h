@@ -250,7 +250,7 @@ struct Ctx {
 // so that every problem yields the same operation sequence.
 // ----------------------------------------------------------------------------------
 struct RecordedOp {
-  enum Kind { kGemm = 0, kPermute = 1, kFill = 2 } kind = kGemm;
+  enum Kind { kGemm = 0, kPermute = 1, kFill = 2, kPackTau = 3, kUnpack = 4 } kind = kGemm;
   // GEMM: C[m*sCm + n*sCn] = alpha * sum_k A[m*sAm + k*sAk] B[k*sBk + n*sBn] + beta * C
   int64_t M = 0, N = 0, K = 0, sAm = 0, sAk = 0, sBk = 0, sBn = 0, sCm = 0, sCn = 0;
   const double* A = nullptr;
@@ -260,8 +260,11 @@ struct RecordedOp {
   // permute: out = alpha * in + beta * out over out's dims; fill: out = alpha
   int rank = 0;
   int64_t d[kMaxRank] = {}, si[kMaxRank] = {}, so[kMaxRank] = {};
+  // pack tau (in) into Tp, Tm (out, out2); unpack S, A (in, in2) into R2 (out): d = {no, nv}
   const double* in = nullptr;
   double* out = nullptr;
+  const double* in2 = nullptr;
+  double* out2 = nullptr;
 };
 
 struct Recorder {
@@ -276,6 +279,7 @@ struct Recorder {
   std::vector<std::string> tape;
   size_t tape_pos = 0;
   bool replay_tape = false;
+  bool packed_ladder = false;  // particle ladder on packed pairs (the operator built beforehand)
   void* alloc(size_t bytes);
   void release(void* p);
 };

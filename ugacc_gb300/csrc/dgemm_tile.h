@@ -17,6 +17,8 @@
 
 #include <cstdint>
 
+#include "core.h"
+
 namespace ucc {
 
 __device__ __forceinline__ void cp_async8(double* dst, const double* src, bool valid) {
@@ -139,5 +141,94 @@ struct DTile {
 // 768^3 -> 761 us (floor 753), 102400 x 160 x 16 616 -> 490 us on 32 x 32 (floor 436).
 using DTile32 = DTile<2, 2, 2, 4, 16>;
 using DTile16 = DTile<2, 2, 1, 2, 32>;
+
+__device__ __forceinline__ uint32_t dgemm_cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void dgemm_cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// element of CTA `rank`'s copy of this shared-memory address
+__device__ __forceinline__ double ld_cluster(const double* p, uint32_t rank) {
+  const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(r) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ int64_t dgemm_c_offset(const GemmEpilogue& ep, int64_t m, int64_t n) {
+  return (ep.msplit ? (m / ep.msplit) * ep.s_mhi + (m % ep.msplit) * ep.s_mlo : m * ep.s_mhi) + n * ep.s_n;
+}
+
+// One CTA's share of C = alpha A B + beta C: the tile at (m0, n0), K from k0 over at most kchunk
+// steps.  CLUSTER: the zc CTAs of a cluster hold the same tile's K shares, and their partial
+// tiles are added through distributed shared memory in rank order, so a split costs no second
+// launch and no trip through device memory.
+template <class T, bool CLUSTER>
+__device__ __forceinline__ void dgemm_cta(double* smem, int rank, int zc, int64_t M, int64_t N, int64_t K, int64_t m0,
+                                          int64_t n0, int64_t k0, int64_t kchunk, const double* A, int64_t sAm,
+                                          int64_t sAk, const double* B, int64_t sBk, int64_t sBn, double alpha,
+                                          double beta, double* C, const GemmEpilogue& epi) {
+  const int64_t kn = k0 < K ? (K - k0 < kchunk ? K - k0 : kchunk) : 0;
+  double acc[T::PM][T::PN], old[T::PM][T::PN];
+  if (!CLUSTER && beta != 0.0) {  // the old values travel while the product runs
+#pragma unroll
+    for (int i = 0; i < T::PM; i++)
+#pragma unroll
+      for (int j = 0; j < T::PN; j++) {
+        const int64_t m = m0 + T::row(i), n = n0 + T::col(j);
+        old[i][j] = m < M && n < N ? C[dgemm_c_offset(epi, m, n)] : 0.0;
+      }
+  }
+  T::product(smem, A + m0 * sAm + k0 * sAk, sAm, sAk, B + k0 * sBk + n0 * sBn, sBk, sBn, M - m0, N - n0, kn, acc);
+  if (!CLUSTER) {
+#pragma unroll
+    for (int i = 0; i < T::PM; i++)
+#pragma unroll
+      for (int j = 0; j < T::PN; j++) {
+        const int64_t m = m0 + T::row(i), n = n0 + T::col(j);
+        if (m < M && n < N) {
+          const double v = alpha * acc[i][j];
+          C[dgemm_c_offset(epi, m, n)] = beta == 0.0 ? v : fma(beta, old[i][j], v);
+        }
+      }
+    return;
+  }
+  // product() ended with a barrier: its stages are free for the partial tile, [m][n] or
+  // [n][m] so that consecutive elements are consecutive in C where one of its indices allows
+  const bool mfast = epi.s_n != 1 && !epi.msplit && epi.s_mhi == 1;
+#pragma unroll
+  for (int i = 0; i < T::PM; i++)
+#pragma unroll
+    for (int j = 0; j < T::PN; j++)
+      smem[mfast ? T::col(j) * T::BM + T::row(i) : T::row(i) * T::BN + T::col(j)] = acc[i][j];
+  dgemm_cluster_barrier();
+  for (int e = rank * T::THREADS + (int)threadIdx.x; e < T::BM * T::BN; e += zc * T::THREADS) {
+    const int64_t m = m0 + (mfast ? e % T::BM : e / T::BN), n = n0 + (mfast ? e / T::BM : e % T::BN);
+    if (m >= M || n >= N) continue;
+    double* cp = C + dgemm_c_offset(epi, m, n);
+    const double o = beta != 0.0 ? *cp : 0.0;
+    double s = 0.0;
+    for (int q = 0; q < zc; q++) s += ld_cluster(smem + e, (uint32_t)q);
+    const double v = alpha * s;
+    *cp = beta == 0.0 ? v : fma(beta, o, v);
+  }
+  dgemm_cluster_barrier();  // no CTA leaves while another still reads its partial tile
+}
+
+// `count` products of one shape in a launch
+struct GemmShape {
+  int64_t M, N, K;
+  int count;
+};
+struct DgemmPlan {
+  int shape;   // 0: DTile16, 1: DTile32
+  int zc, zg;  // K over the zc CTAs of a cluster, times zg partial products in device memory
+};
+DgemmPlan dgemm_plan(const std::vector<GemmShape>& probs, bool may_split);
 
 }  // namespace ucc
