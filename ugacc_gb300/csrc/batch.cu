@@ -11,7 +11,7 @@
 //                    sums over members), tile shape and K split chosen per operation by
 //                    dgemm_plan;
 //   grouped_perm  -- every member's permute / axpby / fill k, in 2048-element chunks;
-//   grouped_pack_tau, grouped_unpack -- the two ends of the packed particle ladder.
+//   grouped_pairs -- every member's amplitude pass (pairs.h).
 //
 // The rest of a sweep (Jacobi update, residual norm, convergence mask, DIIS with its
 // B-matrix rows, subspace solve and extrapolation, tau/ttau, energy) is written directly
@@ -177,38 +177,36 @@ __global__ void grouped_splitk_reduce(const GemmDesc* __restrict__ desc, const i
   }
 }
 
-// The packed ladder's operations (pairs.h) of all members: tau into Tp / Tm, one block per
-// (tile pair, i <= j) item; S and A into R2, kChunk elements per item.
-struct LadderDesc {
+// The amplitude passes of pairs.h for all members: a work item is one (tile or tile pair, slice
+// or row pair) of a member, or kChunk elements of Z.
+struct PairDesc {
   int no, nv, prob;
-  double alpha;
-  const double* in;   // tau, or S
-  const double* in2;  // A
-  double* out;        // Tp, or R2
-  double* out2;       // Tm
+  int64_t tiles;  // tile pairs or tiles per slice
+  const double* src[5];
+  double* dst[3];
 };
-__global__ void grouped_pack_tau(const LadderDesc* __restrict__ desc, const int64_t* __restrict__ prefix, int nd,
-                                 int64_t total, const int* __restrict__ active) {
+template <int KIND>
+__global__ void grouped_pairs(const PairDesc* __restrict__ desc, const int64_t* __restrict__ prefix, int nd,
+                              int64_t total, const int* __restrict__ active) {
+  __shared__ TileBuf s;
   for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
     const int di = find_item(prefix, nd, t);
-    const LadderDesc& p = desc[di];
-    if (!active[p.prob]) continue;
-    const int nt = (p.nv + 31) / 32, tiles = nt * (nt + 1) / 2;
-    const int64_t local = t - prefix[di];
-    pack_pairs_tile(p.no, p.nv, 0.5, p.in, p.out, p.out2, (int)(local % tiles), local / tiles);
-    __syncthreads();  // the tile's shared memory is reused
-  }
-}
-__global__ void grouped_unpack(const LadderDesc* __restrict__ desc, const int64_t* __restrict__ prefix, int nd,
-                               int64_t total, const int* __restrict__ active) {
-  for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
-    const int di = find_item(prefix, nd, t);
-    const LadderDesc& p = desc[di];
-    if (!active[p.prob]) continue;
-    const int64_t n = (int64_t)p.no * p.no * p.nv * p.nv;
-    const int64_t e0 = (t - prefix[di]) * kChunk, e1 = min(e0 + kChunk, n);
-    for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x)  // n < 2^31 (build)
-      p.out[e] += p.alpha * unpack_pair<uint32_t>(p.no, p.nv, p.in, p.in2, (uint32_t)e);
+    const PairDesc& p = desc[di];
+    if (!active[p.prob]) continue;  // the whole block
+    const int64_t local = t - prefix[di], row = local / p.tiles;
+    const int tile = (int)(local - row * p.tiles);
+    const PairLd ld(p.no, p.nv);
+    if (KIND == RecordedOp::kPackTau) {
+      pack_tau_tile(s, p.no, p.nv, p.src[0], p.dst[0], p.dst[1], tile, row);
+    } else if (KIND == RecordedOp::kRing) {
+      ring_tile(s, p.no, p.nv, p.src[0], p.src[1], p.dst[0], p.dst[1], p.dst[2], tile, row);
+    } else if (KIND == RecordedOp::kAssemble) {
+      assemble_tile(s, p.no, p.nv, p.src[0], p.src[1], ld.s, p.src[2], ld.a, p.src[3], p.src[4], p.dst[0], tile, row);
+    } else {
+      const int64_t n = (int64_t)p.no * p.no * p.no * p.nv, e1 = min((local + 1) * kChunk, n);
+      for (int64_t e = local * kChunk + threadIdx.y * 32 + threadIdx.x; e < e1; e += 256)
+        p.dst[0][e] = z_element(p.no, p.nv, p.src[0], ld.s, p.src[1], ld.a, e);
+    }
   }
 }
 
@@ -573,7 +571,7 @@ struct GroupOp {
   DgemmPlan plan{1, 1, 1};  // GEMM: tile shape and K split
   DevArray<GemmDesc> gdesc;
   DevArray<PermDesc> pdesc;
-  DevArray<LadderDesc> ldesc;
+  DevArray<PairDesc> pairs;
   DevArray<int64_t> prefix, rprefix;  // work items; of a split GEMM's reduction
   int64_t total = 0, rtotal = 0;
   int nd = 0;
@@ -668,6 +666,12 @@ void launch_tiles(ucc_batch& B, GroupOp& op) {
   UCC_CUDA(cudaLaunchKernelEx(&cfg, grouped_gemm<T, true>, d, pf, op.nd, op.total, p.zc, p.zg, act));
 }
 
+template <int KIND>
+void launch_pairs(ucc_batch& B, GroupOp& op) {
+  grouped_pairs<KIND><<<grid_for(op.total), dim3(32, 8), 0, B.stream>>>(op.pairs.p, op.prefix.p, op.nd, op.total,
+                                                                        B.active.p);
+}
+
 // launches one operation of all members; the number of kernels
 int launch_op(ucc_batch& B, GroupOp& op) {
   int k = 0;
@@ -686,12 +690,10 @@ int launch_op(ucc_batch& B, GroupOp& op) {
           k++;
         }
         break;
-      case RecordedOp::kPackTau:
-        grouped_pack_tau<<<grid, dim3(32, 8), 0, B.stream>>>(op.ldesc.p, op.prefix.p, op.nd, op.total, B.active.p);
-        break;
-      case RecordedOp::kUnpack:
-        grouped_unpack<<<grid, 256, 0, B.stream>>>(op.ldesc.p, op.prefix.p, op.nd, op.total, B.active.p);
-        break;
+      case RecordedOp::kPackTau: launch_pairs<RecordedOp::kPackTau>(B, op); break;
+      case RecordedOp::kRing: launch_pairs<RecordedOp::kRing>(B, op); break;
+      case RecordedOp::kAssemble: launch_pairs<RecordedOp::kAssemble>(B, op); break;
+      case RecordedOp::kUnpackZ: launch_pairs<RecordedOp::kUnpackZ>(B, op); break;
       default:
         grouped_perm<<<grid, 256, 0, B.stream>>>(op.pdesc.p, op.prefix.p, op.nd, op.total, B.active.p);
     }
@@ -760,28 +762,24 @@ void build(ucc_batch& B) {
   B.arenas.clear();
   B.diis_store.clear();
   double arena_bytes = 0.0;
-  // the ladder runs on packed pairs when every member has pairs on both sides (all members
-  // record the same operations) and its amplitudes fit the 32-bit unpacking
-  // and the packed operators (half of <ab|ef> again) leave half of the free memory
-  bool packed = true;
+  // the packed operators (half of <ab|ef> again, and <ma|ef>) as long as they leave half of the
+  // free memory to the amplitudes, the scratch and the DIIS vectors
   double operator_bytes = 0.0;
-  for (const auto& m : B.members) {
-    packed = packed && m->no > 1 && m->nv > 1 && (int64_t)m->no * m->no * m->nv * m->nv + 256 < ((int64_t)1 << 31);
-    if (!m->has("Vpp")) operator_bytes += 4.0 * std::pow((double)m->nv, 4);
-  }
+  for (const auto& m : B.members)
+    if (!m->has("Vpp")) operator_bytes += 4.0 * std::pow((double)m->nv, 3) * (m->nv + 2.0 * m->no);
   size_t free_b = 0, total_b = 0;
   UCC_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  packed = packed && operator_bytes < 0.5 * (double)free_b;
+  const bool packed = operator_bytes < 0.5 * (double)free_b;
   for (int b = 0; b < nm; b++) {
     Ctx& c = *B.members[b];
     ccsd_alloc(c);
-    if (packed) ladder_operator(c, "Vvvvv", 0, "Vpp", "Vmm");
+    if (packed) pair_operator(c);
     const double* to = c.get("Told").p;
     double* r = c.get("R").p;
     size_t need = 0;
     for (int pass = 0; pass < 2; pass++) {
       Recorder rec;
-      rec.packed_ladder = packed;
+      rec.packed = packed;
       const bool first = b == 0 && pass == 0;
       if (!first) {
         rec.tape = tape;
@@ -829,18 +827,22 @@ void build(ucc_batch& B) {
       int64_t part = 0;
       for (const GemmDesc& d : gemms[k]) part += d.M * d.N * g.plan.zg;
       if (g.plan.zg > 1) split_size = std::max(split_size, part);
-    } else if (g.kind == RecordedOp::kPackTau || g.kind == RecordedOp::kUnpack) {
-      std::vector<LadderDesc> d(nm);
+    } else if (g.kind != RecordedOp::kPermute && g.kind != RecordedOp::kFill) {
+      std::vector<PairDesc> d(nm);
       std::vector<int64_t> pf(nm);
       for (int b = 0; b < nm; b++) {
         const RecordedOp& o = traces[b][k];
-        const int no = (int)o.d[0], nv = (int)o.d[1];
-        const int64_t nt = (nv + 31) / 32, n = (int64_t)no * no * nv * nv;
-        d[b] = LadderDesc{no, nv, b, o.alpha, o.in, o.in2, o.out, o.out2};
+        const int64_t no = o.d[0], nv = o.d[1], nt = (nv + 31) / 32;
+        const bool pairs = g.kind != RecordedOp::kRing;  // tile pairs of row pairs, or all tiles of all slices
+        d[b].no = (int)no, d[b].nv = (int)nv, d[b].prob = b;
+        d[b].tiles = g.kind == RecordedOp::kUnpackZ ? 1 : pairs ? nt * (nt + 1) / 2 : nt * nt;
+        std::copy(o.src, o.src + 5, d[b].src);
+        std::copy(o.dst, o.dst + 3, d[b].dst);
         pf[b] = g.total;
-        g.total += g.kind == RecordedOp::kPackTau ? nt * (nt + 1) / 2 * no * (no + 1) / 2 : (n + kChunk - 1) / kChunk;
+        g.total += g.kind == RecordedOp::kUnpackZ ? (no * no * no * nv + kChunk - 1) / kChunk
+                                                  : d[b].tiles * (pairs ? no * (no + 1) / 2 : no * no);
       }
-      g.ldesc.upload(d, B.stream);
+      g.pairs.upload(d, B.stream);
       g.prefix.upload(pf, B.stream);
     } else {
       std::vector<PermDesc> d(nm);
@@ -874,7 +876,7 @@ void build(ucc_batch& B) {
     }
   }
   // the split operations run one after the other and share one array of partial products
-  B.splitk.zeros((size_t)split_size, B.stream);
+  B.splitk.zeros((size_t)std::max<int64_t>(1, split_size), B.stream);
   for (size_t k = 0; k < nops; k++) {
     if (gemms[k].empty()) continue;
     double* part = B.splitk.p;

@@ -250,11 +250,38 @@ double flops_ccsd_iter(double no, double nv) {
                 8.0 * no * no * nv * nv * nv);
 }
 
-namespace {
+void pair_operator(Ctx& c) {
+  const int64_t no = c.no, nv = c.nv, vp = nv * (nv + 1) / 2, vm = nv * (nv - 1) / 2;
+  if (c.has("Vpp")) return;
+  Tensor Vp = c.alloc("Vpp", {vp + no * nv, vp}, false), Vm = c.alloc("Vmm", {vm + no * nv, vm}, false);
+  pack_vvvv(c, c.nv, 0, c.get("Vvvvv").p, Vp.p, Vm.p);
+  pack_ovvv(c, c.no, c.nv, c.get("Vovvv").p, Vp.p + vp * vp, Vm.p + vm * vm);
+}
 
-struct Amps {  // views of the packed [t1 | t2] buffers
-  Tensor t1, t2;
-};
+// R2 += alpha sum_ef W_abef amp_ijef on packed pairs (pairs.cu), W from an HBAR block: S = Tp Vp^T
+// over (i<=j, a<=b, e<=f) and A = Tm Vm^T over strict pairs, a quarter of the multiply-adds of
+// the plain contraction; amp must be invariant under (i,j,e,f) -> (j,i,f,e).  The packed
+// operator (names vp_name / vm_name, constant blocks) is built from block `src` once; mode 1
+// stores it as [e<=f][a<=b].
+void packed_ladder(Ctx& c, double alpha, const Tensor& amp, const char* src, int mode, const char* vp_name,
+                   const char* vm_name, double* R2) {
+  const int no = c.no, nv = c.nv;
+  const int64_t op = (int64_t)no * (no + 1) / 2, om = (int64_t)no * (no - 1) / 2;
+  const int64_t vp = (int64_t)nv * (nv + 1) / 2, vm = (int64_t)nv * (nv - 1) / 2;
+  if (!c.has(vp_name)) {
+    Tensor Vp = c.alloc(vp_name, {vp, vp}, false), Vm = c.alloc(vm_name, {vm, vm}, false);
+    pack_vvvv(c, nv, mode, c.get(src).p, Vp.p, Vm.p);
+  }
+  UCC_REQUIRE(amp.dense(), UCC_BAD_ARGS, "packed ladder: dense amplitudes");
+  Temp Tp(c, {op, vp}), Tm(c, {om, vm}), S(c, {op, vp}), A(c, {om, vm});
+  pack_tau(c, no, nv, amp.p, Tp->p, Tm->p);
+  const char* spec = mode == 1 ? "pe,eq->pq" : "pe,qe->pq";
+  contract(c, spec, 1.0, Tp, c.get(vp_name), 0.0, S);
+  contract(c, spec, 1.0, Tm, c.get(vm_name), 0.0, A);
+  unpack_ladder(c, no, nv, alpha, S->p, A->p, R2);
+}
+
+namespace {
 
 void copy_into(Ctx& c, const Tensor& src, Tensor dst) { permute_add(c, src, 1.0, 0.0, dst); }
 
@@ -273,147 +300,144 @@ void build_F(Ctx& c, const Tensor& t1, const Tensor& ttau) {
   contract(c, "nf,mnef->me", 1.0, t1, L(c, "oovv"), 1.0, Fov);
 }
 
-// build_W, ccwfn.cc:358-430
-void build_W(Ctx& c, const Tensor& t1, const Tensor& t2, const Tensor& tau) {
-  const int no = c.no, nv = c.nv;
-  Tensor Woooo = c.get("Woooo"), Wovov = c.get("Wovov"), Wovvo = c.get("Wovvo"), Zmbij = c.get("Zmbij");
+// Products of tau with the packed operator, one GEMM per symmetry: the particle ladder's rows
+// (a <= b) and, below them, the (m, b) rows of Zmbij = sum_ef <mb|ef> tau_ijef.  A batch whose
+// members' packed operators would not fit in memory goes without (S and A stay null).
+struct PairProducts {
+  std::unique_ptr<Temp> S, A;
+  PairProducts(Ctx& c, const Tensor& tau) {
+    if (recorder() && !recorder()->packed) return;
+    const int64_t no = c.no, nv = c.nv, op = no * (no + 1) / 2, om = no * (no - 1) / 2;
+    const int64_t vp = nv * (nv + 1) / 2, vm = nv * (nv - 1) / 2;
+    if (!recorder()) pair_operator(c);
+    S = std::make_unique<Temp>(c, std::vector<int64_t>{op, PairLd(no, nv).s});
+    A = std::make_unique<Temp>(c, std::vector<int64_t>{om, PairLd(no, nv).a});
+    Temp Tp(c, {op, vp}), Tm(c, {om, vm});
+    pack_tau(c, c.no, c.nv, tau.p, Tp->p, Tm->p);
+    product(c, Tp, c.get("Vpp"), S->t);
+    product(c, Tm, c.get("Vmm"), A->t);
+  }
+  const double* s() const { return S ? S->t.p : nullptr; }
+  const double* a() const { return A ? A->t.p : nullptr; }
+
+ private:
+  // out = T Op^T; a batch records it whatever the member's size, so that all members record
+  // the same operations (no = 1: no strict pairs of occupied indices, nv = 1: K = 0)
+  static void product(Ctx& c, const Tensor& T, const Tensor& Op, const Tensor& out) {
+    if (recorder()) {
+      GemmEpilogue epi;
+      epi.s_mhi = out.d[1];
+      dgemm_strided(c, T.d[0], Op.d[0], T.d[1], 1.0, T.p, T.d[1], 1, Op.p, 1, T.d[1], 0.0, out.p, epi, 1, 0, 0, 0,
+                    nullptr);
+    } else if (out.size() && !T.d[1]) {
+      fill(c, out.size(), 0.0, out.p);
+    } else {
+      contract(c, "pe,qe->pq", 1.0, T, Op, 0.0, out);
+    }
+  }
+};
+
+// build_W, ccwfn.cc:358-430, with the two ring intermediates
+//   Wovov[m,b,j,e]  (:390-404)  and  B = 2 Wovvo + Wovov(..je->..ej):
+// in B the amplitude products of Wovvo (:406-424) and Wovov collapse to one,
+//   B[m,b,e,j] = L_mbej + t1_jf L_mbef - t1_nb L_mnej + L_mnef P_jnfb,  P = t2(jnbf) - X,
+// so two products over (n, f) do the work of three (tests/test_ring_algebra.py).
+void build_W(Ctx& c, const Tensor& t1, const Tensor& tau, const Tensor& X, const Tensor& P) {
+  Tensor Woooo = c.get("Woooo"), Wovov = c.get("Wovov"), Bovvo = c.get("Bovvo");
   copy_into(c, V(c, "oooo"), Woooo);
   contract(c, "je,mnie->mnij", 1.0, t1, V(c, "ooov"), 1.0, Woooo);
   contract(c, "ie,mnej->mnij", 1.0, t1, V(c, "oovo"), 1.0, Woooo);
   contract(c, "ijef,mnef->mnij", 1.0, tau, V(c, "oovv"), 1.0, Woooo);
-  Temp X(c, {no, no, nv, nv});
-  if (!recorder()) {  // X = t2/2 + t1_jf t1_nb in one elementwise pass (as a K = 1 GEMM: DFMA tiles)
-    build_tau(c, no, nv, t1.p, t2.p, 1.0, X->p, 0.0, nullptr, 0.5);
-  } else {
-    axpby(c, X->size(), 0.5, t2.p, 0.0, X->p);
-    contract(c, "jf,nb->jnfb", 1.0, t1, t1, 1.0, X);
-  }
   permute_add(c, V(c, "ovov"), -1.0, 0.0, Wovov);
   contract(c, "jf,mbfe->mbje", -1.0, t1, V(c, "ovvv"), 1.0, Wovov);
   contract(c, "nb,mnje->mbje", 1.0, t1, V(c, "ooov"), 1.0, Wovov);
   contract(c, "mnfe,jnfb->mbje", 1.0, V(c, "oovv"), X, 1.0, Wovov);
-  copy_into(c, V(c, "ovvo"), Wovvo);
-  contract(c, "jf,mbef->mbej", 1.0, t1, V(c, "ovvv"), 1.0, Wovvo);
-  contract(c, "nb,mnej->mbej", -1.0, t1, V(c, "oovo"), 1.0, Wovvo);
-  contract(c, "mnef,jnfb->mbej", -1.0, V(c, "oovv"), X, 1.0, Wovvo);
-  contract(c, "mnef,njfb->mbej", 0.5, L(c, "oovv"), t2, 1.0, Wovvo);
-  contract(c, "mbef,ijef->mbij", 1.0, V(c, "ovvv"), tau, 0.0, Zmbij);
+  copy_into(c, L(c, "ovvo"), Bovvo);
+  contract(c, "jf,mbef->mbej", 1.0, t1, L(c, "ovvv"), 1.0, Bovvo);
+  contract(c, "nb,mnej->mbej", -1.0, t1, L(c, "oovo"), 1.0, Bovvo);
+  contract(c, "mnef,jnfb->mbej", 1.0, L(c, "oovv"), P, 1.0, Bovvo);
 }
 
-// build_t1, ccwfn.cc:432-469 (unscaled residual)
-void build_t1(Ctx& c, const Tensor& t1, const Tensor& t2, Tensor R1) {
-  const int no = c.no, nv = c.nv;
+// build_t1, ccwfn.cc:432-469 (unscaled residual); S = t2 - t2(ba)/2
+void build_t1(Ctx& c, const Tensor& t1, const Tensor& t2, const Tensor& S, Tensor R1) {
   transpose_add(c, "ai->ia", 1.0, Fk(c, "vo"), 0.0, R1);
   contract(c, "ie,ae->ia", 1.0, t1, c.get("Fvv"), 1.0, R1);
   contract(c, "ma,mi->ia", -1.0, t1, c.get("Foo"), 1.0, R1);
-  Temp t2x(c, {no, no, nv, nv});
-  transpose_add(c, "ijab->ijba", -1.0, t2, 0.0, t2x);
-  axpby(c, t2x->size(), 2.0, t2.p, 1.0, t2x->p);
-  contract(c, "imae,me->ia", 1.0, t2x, c.get("Fov"), 1.0, R1);
+  contract(c, "imae,me->ia", 2.0, S, c.get("Fov"), 1.0, R1);
   contract(c, "nf,nafi->ia", 1.0, t1, L(c, "ovvo"), 1.0, R1);
-  contract(c, "mief,maef->ia", 1.0, t2x, V(c, "ovvv"), 1.0, R1);
+  contract(c, "mief,maef->ia", 2.0, S, V(c, "ovvv"), 1.0, R1);
   contract(c, "mnae,nmei->ia", -1.0, t2, L(c, "oovo"), 1.0, R1);
 }
 
 // build_t2, ccwfn.cc:471-539 (unscaled residual).
 //
 // The residual is symmetric under the simultaneous swap (i<->j, a<->b): the reference
-// computes each term and its swapped partner explicitly.  Here one member of each pair
-// goes into a half residual Rh and R2 = <ij|ab> + Woooo.tau + ladder + Rh + Rh(ji,ba);
-// <ij|ab>, the hole ladder and the particle ladder are symmetric on their own.
-//
-}  // namespace
-
-void ladder_operator(Ctx& c, const char* src, int mode, const char* vp_name, const char* vm_name) {
-  const int64_t nv = c.nv, vp = nv * (nv + 1) / 2, vm = nv * (nv - 1) / 2;
-  if (c.has(vp_name)) return;
-  Tensor Vp = c.alloc(vp_name, {vp, vp}, false), Vm = c.alloc(vm_name, {vm, vm}, false);
-  pack_vvvv(c, c.nv, mode, c.get(src).p, Vp.p, Vm.p);
-}
-
-// R2 += alpha sum_ef W_abef amp_ijef on packed pairs (kernels_fp64.cu): S = Tp Vp^T over
-// (i<=j, a<=b, e<=f), A = Tm Vm^T over strict pairs, a quarter of the multiply-adds of the
-// plain contraction; amp must be invariant under (i,j,e,f) -> (j,i,f,e).  The packed
-// operator (names vp_name / vm_name, constant blocks) is built from block `src` once.
-void packed_ladder(Ctx& c, double alpha, const Tensor& amp, const char* src, int mode, const char* vp_name,
-                   const char* vm_name, double* R2) {
-  const int no = c.no, nv = c.nv;
-  const int64_t op = (int64_t)no * (no + 1) / 2, om = (int64_t)no * (no - 1) / 2;
-  const int64_t vp = (int64_t)nv * (nv + 1) / 2, vm = (int64_t)nv * (nv - 1) / 2;
-  if (!recorder()) ladder_operator(c, src, mode, vp_name, vm_name);
-  UCC_REQUIRE(amp.dense(), UCC_BAD_ARGS, "packed ladder: dense amplitudes");
-  Temp Tp(c, {op, vp}), Tm(c, {om, vm}), S(c, {op, vp}), A(c, {om, vm});
-  pack_tau(c, no, nv, amp.p, Tp->p, Tm->p);
-  contract(c, "pe,qe->pq", 1.0, Tp, c.get(vp_name), 0.0, S);
-  contract(c, "pe,qe->pq", 1.0, Tm, c.get(vm_name), 0.0, A);
-  unpack_ladder(c, no, nv, alpha, S->p, A->p, R2);
-}
-
-namespace {
-
-// particle ladder sum_ef <ab|ef> tau_ijef, ccwfn.cc:508-510, on packed pairs where there are
-// pairs: S = Tp Vp^T over (i<=j, a<=b, e<=f) and A = Tm Vm^T over strict pairs, a quarter of
-// the multiply-adds (the result is symmetric under the simultaneous swap
-// (i,j,a,b) -> (j,i,b,a) and the integrals under (a,b,e,f) -> (b,a,f,e))
-void ladder(Ctx& c, const Tensor& tau, const Tensor& R2) {
-  if (recorder() ? !recorder()->packed_ladder : c.no < 2 || c.nv < 2) {
-    contract(c, "ijef,abef->ijab", 1.0, tau, V(c, "vvvv"), 1.0, R2);
-    return;
-  }
-  packed_ladder(c, 1.0, tau, "Vvvvv", 0, "Vpp", "Vmm", R2.p);
-}
-
-void build_t2(Ctx& c, const Tensor& t1, const Tensor& t2, const Tensor& tau, Tensor R2, std::vector<cudaEvent_t>* ev) {
+// computes each term and its swapped partner explicitly.  Here one member of each pair (half
+// of the self-symmetric hole ladder) goes into a half residual Rh, the exchange ring
+// t2_imea Wovov_mbje into H, whose half and whose (i,j,b,a) transpose are the last two of the
+// reference's ring terms, and assemble_r2 adds <ij|ab>, the particle ladder, Q and Q(ji,ba)
+// with Q = Rh + H/2 + H(ijba) in one pass.
+void build_t2(Ctx& c, const Tensor& t1, const Tensor& t2, const Tensor& tau, const Tensor& S,
+              const PairProducts& pairs, Tensor R2) {
   const int no = c.no, nv = c.nv;
   Tensor Fvv = c.get("Fvv"), Foo = c.get("Foo"), Fov = c.get("Fov");
-  Tensor Woooo = c.get("Woooo"), Wovov = c.get("Wovov"), Wovvo = c.get("Wovvo"), Zmbij = c.get("Zmbij");
-  copy_into(c, V(c, "oovv"), R2);
-  contract(c, "mnab,mnij->ijab", 1.0, tau, Woooo, 1.0, R2);
-  if (ev) {
-    cudaEvent_t a, b;
-    cudaEventCreate(&a);
-    cudaEventCreate(&b);
-    cudaEventRecord(a, c.stream);
-    ladder(c, tau, R2);
-    cudaEventRecord(b, c.stream);
-    ev->push_back(a);
-    ev->push_back(b);
-  } else {
-    ladder(c, tau, R2);
-  }
-  Temp Rh(c, {no, no, nv, nv});
-  contract(c, "ijae,be->ijab", 1.0, t2, Fvv, 0.0, Rh);
+  Tensor Woooo = c.get("Woooo"), Wovov = c.get("Wovov"), Bovvo = c.get("Bovvo");
+  Temp Rh(c, {no, no, nv, nv}), H(c, {no, no, nv, nv});
   {
-    Temp tF(c, {nv, nv});
-    contract(c, "mb,me->be", 1.0, t1, Fov, 0.0, tF);
-    contract(c, "ijae,be->ijab", -0.5, t2, tF, 1.0, Rh);
-    Temp tF2(c, {no, no});
-    contract(c, "je,me->mj", 1.0, t1, Fov, 0.0, tF2);
-    axpby(c, tF2->size(), 0.5, tF2->p, 0.0, tF2->p);
-    axpby(c, Foo.size(), 1.0, Foo.p, 1.0, tF2->p);  // Foo + tF2 / 2
-    contract(c, "imab,mj->ijab", -1.0, t2, tF2, 1.0, Rh);
+    Temp F1(c, {nv, nv}), F2(c, {no, no});  // Fvv - t1 Fov / 2, Foo + t1 Fov / 2
+    copy_into(c, Fvv, F1);
+    contract(c, "mb,me->be", -0.5, t1, Fov, 1.0, F1);
+    copy_into(c, Foo, F2);
+    contract(c, "je,me->mj", 0.5, t1, Fov, 1.0, F2);
+    contract(c, "ijae,be->ijab", 1.0, t2, F1, 0.0, Rh);
+    contract(c, "imab,mj->ijab", -1.0, t2, F2, 1.0, Rh);
   }
+  contract(c, "mnab,mnij->ijab", 0.5, tau, Woooo, 1.0, Rh);
   contract(c, "ie,abej->ijab", 1.0, t1, V(c, "vvvo"), 1.0, Rh);
-  contract(c, "ma,mbij->ijab", -1.0, t1, V(c, "ovoo"), 1.0, Rh);
+  contract(c, "imae,mbej->ijab", 1.0, S, Bovvo, 1.0, Rh);
+  contract(c, "imea,mbje->ijab", 1.0, t2, Wovov, 0.0, H);
   {
-    // (t2 - t2(ba)) Wovvo + t2 (Wovvo + Wovov(..je->..ej)) = (2 t2 - t2(ba)) Wovvo + t2 Wovov^T
-    Temp t2x(c, {no, no, nv, nv});
-    transpose_add(c, "ijab->ijba", -1.0, t2, 0.0, t2x);
-    axpby(c, t2x->size(), 2.0, t2.p, 1.0, t2x->p);
-    contract(c, "imae,mbej->ijab", 1.0, t2x, Wovvo, 1.0, Rh);
-    contract(c, "imae,mbje->ijab", 1.0, t2, Wovov, 1.0, Rh);
-  }
-  contract(c, "mjae,mbie->ijab", 1.0, t2, Wovov, 1.0, Rh);
-  {
-    // Za[m,b,i,j] = Zmbij + t1[i,e] <mb|ej> + t1[j,e] <mb|ie>  ->  - t1[m,a] Za[m,b,i,j]
+    // Za[m,b,i,j] = <mb|ij> + Zmbij + t1[i,e] <mb|ej> + t1[j,e] <mb|ie>  ->  - t1[m,a] Za[m,b,i,j]
     Temp Za(c, {no, nv, no, no});
-    copy_into(c, Zmbij, Za);
+    if (pairs.s())
+      unpack_z(c, no, nv, pairs.s(), pairs.a(), Za->p);
+    else
+      contract(c, "mbef,ijef->mbij", 1.0, V(c, "ovvv"), tau, 0.0, Za);
+    permute_add(c, V(c, "ovoo"), 1.0, 1.0, Za);
     contract(c, "ie,mbej->mbij", 1.0, t1, V(c, "ovvo"), 1.0, Za);
     contract(c, "je,mbie->mbij", 1.0, t1, V(c, "ovov"), 1.0, Za);
     contract(c, "ma,mbij->ijab", -1.0, t1, Za, 1.0, Rh);
   }
-  axpby(c, Rh->size(), 1.0, Rh->p, 1.0, R2.p);
-  transpose_add(c, "jiba->ijab", 1.0, Rh, 1.0, R2);
+  if (!pairs.s()) contract(c, "ijef,abef->ijab", 0.5, tau, V(c, "vvvv"), 1.0, Rh);
+  assemble_r2(c, no, nv, V(c, "oovv").p, pairs.s(), pairs.a(), Rh->p, H->p, R2.p);
+}
+
+// the unscaled residual R(t_old) into r, given tau/ttau of t_old (ccwfn.cc:311-539); ev
+// collects event pairs around the packed products
+void residual(Ctx& c, const double* t_old, double* r, std::vector<cudaEvent_t>* ev) {
+  const int no = c.no, nv = c.nv;
+  Tensor t1 = amp1(c, const_cast<double*>(t_old)), t2 = amp2(c, const_cast<double*>(t_old)), tau = c.get("tau");
+  build_F(c, t1, c.get("ttau"));
+  cudaEvent_t a = nullptr, b = nullptr;
+  if (ev) {
+    cudaEventCreate(&a);
+    cudaEventCreate(&b);
+    cudaEventRecord(a, c.stream);
+  }
+  PairProducts pairs(c, tau);
+  if (ev) {
+    cudaEventRecord(b, c.stream);
+    ev->push_back(a);
+    ev->push_back(b);
+  }
+  Temp S(c, {no, no, nv, nv});
+  {
+    Temp X(c, {no, no, nv, nv}), P(c, {no, no, nv, nv});
+    ring_amplitudes(c, no, nv, t1.p, t2.p, X->p, P->p, S->p);
+    build_W(c, t1, tau, X, P);
+  }
+  build_t1(c, t1, t2, S, amp1(c, r));
+  build_t2(c, t1, t2, tau, S, pairs, amp2(c, r));
 }
 
 double energy(Ctx& c, const Tensor& t1, const Tensor& tau) {
@@ -442,18 +466,10 @@ void ccsd_alloc(Ctx& c) {
   c.alloc("Fov", {no, nv}, false);
   c.alloc("Woooo", {no, no, no, no}, false);
   c.alloc("Wovov", {no, nv, no, nv}, false);
-  c.alloc("Wovvo", {no, nv, nv, no}, false);
-  c.alloc("Zmbij", {no, nv, no, no}, false);
+  c.alloc("Bovvo", {no, nv, nv, no}, false);
 }
 
-// the unscaled residual R(t_old) into r, given tau/ttau of t_old (ccwfn.cc:311-539)
-void ccsd_residual(Ctx& c, const double* t_old, double* r) {
-  Tensor t1 = amp1(c, const_cast<double*>(t_old)), t2 = amp2(c, const_cast<double*>(t_old));
-  build_F(c, t1, c.get("ttau"));
-  build_W(c, t1, t2, c.get("tau"));
-  build_t1(c, t1, t2, amp1(c, r));
-  build_t2(c, t1, t2, c.get("tau"), amp2(c, r), nullptr);
-}
+void ccsd_residual(Ctx& c, const double* t_old, double* r) { residual(c, t_old, r, nullptr); }
 
 double ccsd_energy(Ctx& c, const double* t) { return energy(c, amp1(c, const_cast<double*>(t)), c.get("tau")); }
 
@@ -611,25 +627,12 @@ CCSDResult run_ccsd(Ctx& c) {
     double* to = c.get("Told").p;
     double* tn = c.get("T").p;
     double* r = c.get("R").p;
-    Tensor t1 = amp1(c, to), t2 = amp2(c, to);
     const MixedSweeps::Kind kind = sw.begin();
     {
       Fp64Scope scope(c, kind != MixedSweeps::kSplit);
-      build_F(c, t1, c.get("ttau"));
-      build_W(c, t1, t2, c.get("tau"));
-      build_t1(c, t1, t2, amp1(c, r));
-      build_t2(c, t1, t2, c.get("tau"), amp2(c, r), &ev);
+      residual(c, to, r, &ev);
     }
     sw.end();
-    if (kind == MixedSweeps::kSplit || kind == MixedSweeps::kDelta) {
-      // The exact residual is symmetric under (i,j,a,b) -> (j,i,b,a); rounding of the
-      // tensor-core products is not.  In the antisymmetric sector the Fock terms cancel
-      // and the Jacobi step does not damp, so project the noise out of R2.
-      Tensor R2 = amp2(c, r);
-      Temp S(c, {no, no, nv, nv});
-      transpose_add(c, "ijab->jiba", 1.0, R2, 0.0, S);
-      axpby(c, S->size(), 0.5, S->p, 0.5, R2.p);
-    }
     double noise = -1.0, drift = -1.0;
     if (c.opt.print >= 2 && mixed) {
       // diagnostics: distance of this residual from the FP64 one at the same amplitudes,

@@ -250,7 +250,7 @@ struct Ctx {
 // so that every problem yields the same operation sequence.
 // ----------------------------------------------------------------------------------
 struct RecordedOp {
-  enum Kind { kGemm = 0, kPermute = 1, kFill = 2, kPackTau = 3, kUnpack = 4 } kind = kGemm;
+  enum Kind { kGemm, kPermute, kFill, kPackTau, kRing, kAssemble, kUnpackZ } kind = kGemm;
   // GEMM: C[m*sCm + n*sCn] = alpha * sum_k A[m*sAm + k*sAk] B[k*sBk + n*sBn] + beta * C
   int64_t M = 0, N = 0, K = 0, sAm = 0, sAk = 0, sBk = 0, sBn = 0, sCm = 0, sCn = 0;
   const double* A = nullptr;
@@ -260,11 +260,11 @@ struct RecordedOp {
   // permute: out = alpha * in + beta * out over out's dims; fill: out = alpha
   int rank = 0;
   int64_t d[kMaxRank] = {}, si[kMaxRank] = {}, so[kMaxRank] = {};
-  // pack tau (in) into Tp, Tm (out, out2); unpack S, A (in, in2) into R2 (out): d = {no, nv}
   const double* in = nullptr;
   double* out = nullptr;
-  const double* in2 = nullptr;
-  double* out2 = nullptr;
+  // the amplitude passes of pairs.h: d = {no, nv}, arrays in the order of the launcher's arguments
+  const double* src[5] = {};
+  double* dst[3] = {};
 };
 
 struct Recorder {
@@ -279,7 +279,7 @@ struct Recorder {
   std::vector<std::string> tape;
   size_t tape_pos = 0;
   bool replay_tape = false;
-  bool packed_ladder = false;  // particle ladder on packed pairs (the operator built beforehand)
+  bool packed = true;  // products with the packed operator ("Vpp", "Vmm" built beforehand)
   void* alloc(size_t bytes);
   void release(void* p);
 };
@@ -336,9 +336,9 @@ double dot(Ctx& c, int64_t n, const double* x, const double* y);
 // Several dot products x_k . y at once (DIIS B-matrix row), results on the device.
 void multidot_async(Ctx& c, int nvec, const double* const* d_xs, const double* y, int64_t n, double* d_out);
 
-// tau = g t2 + f1 * t1(i,a) t1(j,b); ttau = g t2 + f2 * t1 t1  (ttau may be null; g = 1 or 1/2)
+// tau = t2 + f1 * t1(i,a) t1(j,b); ttau = t2 + f2 * t1 t1
 void build_tau(Ctx& c, int no, int nv, const double* t1, const double* t2, double f1, double* tau, double f2,
-               double* ttau, double g = 1.0);
+               double* ttau);
 
 // Jacobi update t_new = t_old + R / (D + shift), D built on the fly from the diagonals
 // do[no], dv[nv] in the reference's order ((d_i + d_j) - d_a) - d_b; the sum of R^2
@@ -374,13 +374,30 @@ void triples_energy_f32(Ctx& c, int no, int nv, int ntuple, const int* d_tuples,
 // Pair-symmetric particle ladder (sum_ef W_abef tau_ijef = S + sign A over packed pairs,
 // W and tau invariant under the simultaneous pair swap):
 // Vp[a<=b][e<=f] = W_abef + W_abfe (W_abee on e == f), Vm[a<b][e<f] = W_abef - W_abfe, with
-// W from a stored block by `mode` (0: H_abef; 1: H_efab + H_feba; 2: H_abef + H_bafe);
+// W from a stored block by `mode` (0: H_abef; 1: H_efab + H_feba, stored transposed as
+// Vp[e<=f][a<=b]; 2: H_abef + H_bafe);
 // Tp[i<=j][e<=f] = (tau_ijef + tau_ijfe)/2 (tau_ijee on e == f), Tm[i<j][e<f] = (tau_ijef - tau_ijfe)/2;
 // R2[ijab] += alpha (S[ij][ab] + sign A[ij][ab]) over the sorted pairs.  Pairs p <= q are
 // numbered q(q+1)/2 + p, strict pairs q(q-1)/2 + p.
 void pack_vvvv(Ctx& c, int nv, int mode, const double* H, double* Vp, double* Vm);
+// the (m, a) rows of <ma|ef> over the same pairs: Vp[ma][e<=f], Vm[ma][e<f]
+void pack_ovvv(Ctx& c, int no, int nv, const double* H, double* Vp, double* Vm);
 void pack_tau(Ctx& c, int no, int nv, const double* tau, double* Tp, double* Tm);
 void unpack_ladder(Ctx& c, int no, int nv, double alpha, const double* S, const double* A, double* R2);
+// Row lengths of S [pairs i<=j][a<=b pairs, then (m, b)] and A [pairs i<j][a<b pairs, then (m, b)],
+// the products of a ladder operator with the <mb|ef> rows below it
+struct PairLd {
+  int64_t s, a;
+  __host__ __device__ PairLd(int64_t no, int64_t nv) : s(nv * (nv + 1) / 2 + no * nv), a(nv * (nv - 1) / 2 + no * nv) {}
+};
+// X = t2/2 + t1 t1, P = t2(ijba) - X, S = t2 - t2(ijba)/2 in one pass
+void ring_amplitudes(Ctx& c, int no, int nv, const double* t1, const double* t2, double* X, double* P, double* S);
+// R2 = V + ladder(S, A) + Q + Q(ji,ba), Q = Rh + H/2 + H(ijba): exactly symmetric under (i,j,a,b) -> (j,i,b,a);
+// S and A may be null (no ladder)
+void assemble_r2(Ctx& c, int no, int nv, const double* V, const double* S, const double* A, const double* Rh,
+                 const double* H, double* R2);
+// Z[m][b][i][j] = sum_ef <mb|ef> tau_ijef from the (m, b) columns of S and A
+void unpack_z(Ctx& c, int no, int nv, const double* S, const double* A, double* Z);
 
 int64_t launches();  // kernels launched by this library so far (all contexts)
 

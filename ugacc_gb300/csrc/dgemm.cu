@@ -138,8 +138,7 @@ void launch(Ctx& c, const GemmArgs& g, int batch) {
 void dgemm_strided(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t sAm, int64_t sAk,
                    const double* B, int64_t sBk, int64_t sBn, double beta, double* C, const GemmEpilogue& epi,
                    int batch, int64_t bA, int64_t bB, int64_t bC, const GemmPtrs* ptrs) {
-  if (M <= 0 || N <= 0 || batch <= 0) return;
-  if (Recorder* r = recorder()) {
+  if (Recorder* r = recorder()) {  // an empty product too: all members record the same operations
     UCC_REQUIRE(batch == 1 && !ptrs && epi.msplit == 0, UCC_UNSUPPORTED, "dgemm: form not recordable");
     RecordedOp o;
     o.kind = RecordedOp::kGemm;
@@ -148,6 +147,7 @@ void dgemm_strided(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const 
     r->ops.push_back(o);
     return;
   }
+  if (M <= 0 || N <= 0 || batch <= 0) return;
   UCC_REQUIRE(batch <= 65535, UCC_BAD_ARGS, "dgemm: batch too large");
   UCC_REQUIRE((M + 63) / 64 <= 65535, UCC_BAD_ARGS, "dgemm: M too large");
   const DgemmPlan p = dgemm_plan({{M, N, K, batch}}, batch == 1 && !ptrs);

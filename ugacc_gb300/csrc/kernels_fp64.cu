@@ -13,7 +13,6 @@
 #include <memory>
 
 #include "core.h"
-#include "pairs.h"
 
 namespace ucc {
 
@@ -469,7 +468,7 @@ void multidot_async(Ctx& c, int nvec, const double* const* d_xs, const double* y
 namespace {
 template <class I>
 __global__ void tau_kernel(int no, int nv, const double* t1, const double* t2, double f1, double* tau, double f2,
-                           double* ttau, double g) {
+                           double* ttau) {
   const I n = (I)no * no * nv * nv, v_ = (I)nv, o_ = (I)no;
   for (I x = (I)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (I)gridDim.x * blockDim.x) {
     const I b = x % v_;
@@ -479,9 +478,9 @@ __global__ void tau_kernel(int no, int nv, const double* t1, const double* t2, d
     const I j = r % o_;
     const I i = r / o_;
     const double tt = t1[i * v_ + a] * t1[j * v_ + b];
-    const double v = g * t2[x];  // g = 1 or 1/2: exact
+    const double v = t2[x];
     tau[x] = fma(f1, tt, v);
-    if (ttau) ttau[x] = fma(f2, tt, v);
+    ttau[x] = fma(f2, tt, v);
   }
 }
 
@@ -528,14 +527,13 @@ __global__ void lincomb_kernel(int nvec, const double* const* vecs, const double
 }  // namespace
 
 void build_tau(Ctx& c, int no, int nv, const double* t1, const double* t2, double f1, double* tau, double f2,
-               double* ttau, double g) {
+               double* ttau) {
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
-  UCC_REQUIRE(g == 1.0 || g == 0.5, UCC_BAD_ARGS, "build_tau: t2 scale 1 or 1/2");
   const int64_t n = (int64_t)no * no * nv * nv;
   if (n + 152 * 32 * 256 < ((int64_t)1 << 31))
-    tau_kernel<uint32_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, t1, t2, f1, tau, f2, ttau, g);
+    tau_kernel<uint32_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, t1, t2, f1, tau, f2, ttau);
   else
-    tau_kernel<int64_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, t1, t2, f1, tau, f2, ttau, g);
+    tau_kernel<int64_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, t1, t2, f1, tau, f2, ttau);
   count_launch();
   check_launch("tau");
 }
@@ -916,151 +914,6 @@ __global__ void __launch_bounds__(EP_THREADS, 2)
 int64_t triples_f32_partials(int nv) {
   const int64_t T = (nv + ET - 1) / ET;
   return T * (T + 1) * (T + 2) / 6;
-}
-
-// ------------------------------------------------------------------------------------
-// Pair-symmetric particle ladder.  Pairs p <= q are numbered q(q+1)/2 + p, strict pairs
-// p < q are numbered q(q-1)/2 + p.
-// ------------------------------------------------------------------------------------
-namespace {
-__device__ __forceinline__ void pair_le(int64_t P, int& p, int& q) {
-  int j = (int)((sqrt(8.0 * (double)P + 1.0) - 1.0) * 0.5);
-  while ((int64_t)(j + 1) * (j + 2) / 2 <= P) j++;
-  while ((int64_t)j * (j + 1) / 2 > P) j--;
-  q = j;
-  p = (int)(P - (int64_t)j * (j + 1) / 2);
-}
-__device__ __forceinline__ void pair_lt(int64_t Q, int& p, int& q) {
-  int j = (int)((sqrt(8.0 * (double)Q + 1.0) + 1.0) * 0.5);
-  while ((int64_t)j * (j + 1) / 2 <= Q) j++;
-  while (j > 1 && (int64_t)(j - 1) * j / 2 > Q) j--;
-  q = j;
-  p = (int)(Q - (int64_t)j * (j - 1) / 2);
-}
-
-// the operator W_abef of a packed ladder, from a stored [nv]^4 block H:
-//   mode 0: H[a][b][e][f]                          (<ab|ef>, pair-symmetric itself)
-//   mode 1: H[e][f][a][b] + H[f][e][b][a]          (sum_ef Z_ijef H_efab of a Z + Z(ji,ba) residual)
-//   mode 2: H[a][b][e][f] + H[b][a][f][e]          (sum_ef Z_ijef H_abef of a Z + Z(ji,ba) residual)
-__device__ __forceinline__ double ladder_op(const double* H, int nv, int mode, int a, int b, int e, int f) {
-  auto at = [&](int p, int q, int r, int s) { return H[(((int64_t)p * nv + q) * nv + r) * nv + s]; };
-  if (mode == 1) return at(e, f, a, b) + at(f, e, b, a);
-  if (mode == 2) return at(a, b, e, f) + at(b, a, f, e);
-  return at(a, b, e, f);
-}
-
-// Vp[ab][ef] = W_abef + W_abfe (e < f), W_abee (e == f), a <= b;  Vm[ab][ef] = W_abef - W_abfe, a < b, e < f
-__global__ void pack_vvvv_kernel(int nv, int mode, const double* __restrict__ H, double* Vp, double* Vm) {
-  const int64_t np = (int64_t)nv * (nv + 1) / 2, nm = (int64_t)nv * (nv - 1) / 2;
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < np * np + nm * nm;
-       x += (int64_t)gridDim.x * blockDim.x) {
-    int a, b, e, f;
-    if (x < np * np) {
-      pair_le(x / np, a, b);
-      pair_le(x % np, e, f);
-      Vp[x] = e == f ? ladder_op(H, nv, mode, a, b, e, e)
-                     : ladder_op(H, nv, mode, a, b, e, f) + ladder_op(H, nv, mode, a, b, f, e);
-    } else {
-      const int64_t y = x - np * np;
-      pair_lt(y / nm, a, b);
-      pair_lt(y % nm, e, f);
-      Vm[y] = ladder_op(H, nv, mode, a, b, e, f) - ladder_op(H, nv, mode, a, b, f, e);
-    }
-  }
-}
-
-// Tp[ij][ef] = (tau_ijef + tau_ijfe)/2 (e < f), tau_ijee (e == f), i <= j;  Tm = (tau_ijef - tau_ijfe)/2, i < j, e < f
-__global__ void pack_tau_kernel(int no, int nv, const double* __restrict__ tau, double* Tp, double* Tm) {
-  const int64_t op = (int64_t)no * (no + 1) / 2, om = (int64_t)no * (no - 1) / 2;
-  const int64_t vp = (int64_t)nv * (nv + 1) / 2, vm = (int64_t)nv * (nv - 1) / 2;
-  const int64_t nv2 = (int64_t)nv * nv;
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < op * vp + om * vm;
-       x += (int64_t)gridDim.x * blockDim.x) {
-    int i, j, e, f;
-    if (x < op * vp) {
-      pair_le(x / vp, i, j);
-      pair_le(x % vp, e, f);
-      const double* t = tau + ((int64_t)i * no + j) * nv2;
-      Tp[x] = e == f ? t[(int64_t)e * nv + e] : 0.5 * (t[(int64_t)e * nv + f] + t[(int64_t)f * nv + e]);
-    } else {
-      const int64_t y = x - op * vp;
-      pair_lt(y / vm, i, j);
-      pair_lt(y % vm, e, f);
-      const double* t = tau + ((int64_t)i * no + j) * nv2;
-      Tm[y] = 0.5 * (t[(int64_t)e * nv + f] - t[(int64_t)f * nv + e]);
-    }
-  }
-}
-
-__global__ void pack_pairs_tiled_kernel(int nx, int nv, double h, const double* __restrict__ src, double* P,
-                                        double* M) {
-  pack_pairs_tile(nx, nv, h, src, P, M, (int)blockIdx.x, blockIdx.y);
-}
-
-// R2[ijab] += alpha * unpack_pair
-template <class I>
-__global__ void unpack_ladder_kernel(int no, int nv, double alpha, const double* __restrict__ S,
-                                     const double* __restrict__ A, double* R2) {
-  const I n = (I)no * no * nv * nv;
-  for (I x = (I)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (I)gridDim.x * blockDim.x)
-    R2[x] = combine(alpha, unpack_pair<I>(no, nv, S, A, x), 1.0, R2 + x);
-}
-}  // namespace
-
-void pack_vvvv(Ctx& c, int nv, int mode, const double* H, double* Vp, double* Vm) {
-  UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
-  const int64_t np = (int64_t)nv * (nv + 1) / 2, nm = (int64_t)nv * (nv - 1) / 2;
-  const int nt = (nv + 31) / 32;
-  if (mode == 0 && np <= 65535) {  // <ab|ef>: the (a, b) slice is one contiguous block
-    pack_pairs_tiled_kernel<<<dim3((unsigned)(nt * (nt + 1) / 2), (unsigned)np), dim3(32, 8), 0, c.stream>>>(
-        nv, nv, 1.0, H, Vp, Vm);
-    count_launch();
-    check_launch("pack_vvvv");
-    return;
-  }
-  pack_vvvv_kernel<<<grid_for(np * np + nm * nm), 256, 0, c.stream>>>(nv, mode, H, Vp, Vm);
-  count_launch();
-  check_launch("pack_vvvv");
-}
-
-void pack_tau(Ctx& c, int no, int nv, const double* tau, double* Tp, double* Tm) {
-  if (Recorder* r = recorder()) {
-    RecordedOp o;
-    o.kind = RecordedOp::kPackTau;
-    o.d[0] = no, o.d[1] = nv, o.in = tau, o.out = Tp, o.out2 = Tm;
-    r->ops.push_back(o);
-    return;
-  }
-  const int64_t op = (int64_t)no * (no + 1) / 2;
-  const int nt = (nv + 31) / 32;
-  if (op <= 65535) {
-    pack_pairs_tiled_kernel<<<dim3((unsigned)(nt * (nt + 1) / 2), (unsigned)op), dim3(32, 8), 0, c.stream>>>(
-        no, nv, 0.5, tau, Tp, Tm);
-    count_launch();
-    check_launch("pack_tau");
-    return;
-  }
-  const int64_t n = (int64_t)no * (no + 1) / 2 * nv * (nv + 1) / 2 + (int64_t)no * (no - 1) / 2 * nv * (nv - 1) / 2;
-  pack_tau_kernel<<<grid_for(n), 256, 0, c.stream>>>(no, nv, tau, Tp, Tm);
-  count_launch();
-  check_launch("pack_tau");
-}
-
-void unpack_ladder(Ctx& c, int no, int nv, double alpha, const double* S, const double* A, double* R2) {
-  if (Recorder* r = recorder()) {
-    RecordedOp o;
-    o.kind = RecordedOp::kUnpack;
-    o.d[0] = no, o.d[1] = nv, o.alpha = alpha, o.in = S, o.in2 = A, o.out = R2;
-    r->ops.push_back(o);
-    return;
-  }
-  const int64_t n = (int64_t)no * no * nv * nv;
-  if (n + 152 * 32 * 256 < ((int64_t)1 << 31))
-    unpack_ladder_kernel<uint32_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, alpha, S, A, R2);
-  else
-    unpack_ladder_kernel<int64_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, alpha, S, A, R2);
-  count_launch();
-  check_launch("unpack_ladder");
 }
 
 TriplesF32Layout triples_f32_layout(int no, int nv) {
