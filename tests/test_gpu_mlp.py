@@ -134,3 +134,19 @@ def test_family_workflow_batched_learned_guess():
     assert out["test_learned_guess"]["converged"] == out["test_mp2_guess"]["converged"] == 8
     assert out["max_abs_dE"] < 1e-7
     assert out["iterations_saved"] > 0
+
+
+@pytest.mark.parametrize("rows", [1, 7, 31, 33, 127, 129, 255, 257, 8193])
+def test_gradients_at_row_edges(rows):
+    """Rows at the edges of the 128-row tiles, the 32-row input blocks and the W2 row chunks."""
+    net = U.MLP(seed=9)
+    X, t = _data(rows, rows)
+    loss, g = net.loss_grad(X, t)
+    lref, gref = M.loss_grad(net.params.astype(np.float64), X.astype(np.float64), t.astype(np.float64))
+    assert abs(loss - lref) <= 1e-5 * lref
+    o = 0
+    for name, shape in M.SIZES:
+        n = int(np.prod(shape))
+        np.testing.assert_allclose(g[o:o + n], gref[o:o + n], rtol=0, atol=1e-4 * np.abs(gref[o:o + n]).max() + 1e-9,
+                                   err_msg=name)
+        o += n
