@@ -276,7 +276,7 @@ typedef struct ucc_stats {
   double tc_gemm_ms;         /* device time of the tensor-core GEMMs (CUDA events) */
   double tc_gemm_flops;      /* their algorithmic FLOPs, 2*M*N*K per GEMM */
   int anchored_iterations;   /* refinement iterations built as FP64 anchor + tensor-core corrections */
-  double fp64_gemm_ms;       /* device time of the FP64 GEMM launches (CUDA events) */
+  double fp64_gemm_ms;       /* device time of the FP64 GEMM launches (CUDA events; the short ones' own clock) */
   double fp64_gemm_flops;    /* their algorithmic FLOPs, 2*M*N*K per GEMM */
   int64_t fp64_gemm_launches;
   double sliced_gemm_ms;     /* device time of the sliced FP64 tensor-core GEMMs (slicing included) */

@@ -35,3 +35,18 @@ def test_fp64_gemm_nonfinite_stay_in_their_rows():
     assert np.array_equal(np.isnan(out), np.isnan(ref)) and np.array_equal(np.isinf(out), np.isinf(ref))
     fine = np.isfinite(ref)
     assert np.allclose(out[fine], ref[fine], rtol=0, atol=1e-13)
+
+
+@pytest.mark.parametrize("M,N,K", [(16, 16, 40000), (40, 9, 30000), (95, 95, 95)])
+def test_split_products_repeat_and_are_timed(M, N, K):
+    """The split's tickets come back to zero: a second product is the first one bit for bit; short
+    products are timed by their own CTAs."""
+    rng = np.random.default_rng(K)
+    A, B = rng.standard_normal((M, K)), rng.standard_normal((K, N))
+    ctx = U.Context()
+    first = ctx.gemm(A, B)
+    ctx.reset_stats()
+    assert np.array_equal(ctx.gemm(A, B), first)
+    st = ctx.stats()
+    assert st["fp64_gemm_launches"] == 1 and st["fp64_gemm_flops"] == 2.0 * M * N * K
+    assert 1e-4 < st["fp64_gemm_ms"] < 50.0

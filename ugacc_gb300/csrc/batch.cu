@@ -47,11 +47,10 @@ constexpr int kDiis = 8;
 constexpr int64_t kChunk = 2048;  // elements per work item of the elementwise kernels
 
 struct GemmDesc {
-  int64_t M, N, K, sAm, sAk, sBk, sBn, sCm, sCn;
-  const double* A;
-  const double* B;
+  int64_t M, N, K;
+  DView A, B;
   double* C;
-  double* part;  // partial products [zg][M][N] of a split operation
+  GemmEpilogue epi;
   double alpha, beta;
   int prob;
 };
@@ -137,44 +136,22 @@ __device__ __forceinline__ int find_item(const int64_t* __restrict__ prefix, int
 // ---------------------------------------------------------------------------------------
 template <class T, bool CLUSTER>
 __global__ void __launch_bounds__(T::THREADS) grouped_gemm(const GemmDesc* __restrict__ desc,
-                                                           const int64_t* __restrict__ prefix, int nd, int64_t total,
-                                                           int zc, int zg, const int* __restrict__ active) {
+                                                           const int64_t* __restrict__ prefix, int nd, int zc, int zg,
+                                                           double* part, unsigned int* tickets,
+                                                           const int* __restrict__ active) {
   __shared__ double smem[T::SMEM];
   const int rank = CLUSTER ? (int)dgemm_cluster_rank() : 0;
   const int64_t u = CLUSTER ? blockIdx.x / zc : blockIdx.x;
   // K share zi of tile t: the shares of one member's tiles are neighbours, its longest first
   const int64_t t = u / zg;
-  const int zi = (int)(u - t * zg);
   const int di = find_item(prefix, nd, t);
   const GemmDesc g = desc[di];
-  if (!active[g.prob]) return;  // the whole cluster
-  const int64_t local = t - prefix[di], ntn = (g.N + T::BN - 1) / T::BN;
-  const int64_t z = (int64_t)zc * zg, kchunk = (g.K + z - 1) / z;
-  const int64_t m0 = local / ntn * T::BM, n0 = local % ntn * T::BN, k0 = ((int64_t)zi * zc + rank) * kchunk;
-  const GemmEpilogue direct{0, g.sCm, 0, g.sCn}, partial{0, g.N, 0, 1};
-  dgemm_cta<T, CLUSTER>(smem, rank, zc, g.M, g.N, g.K, m0, n0, k0, kchunk, g.A, g.sAm, g.sAk, g.B, g.sBk, g.sBn,
-                        zg > 1 ? 1.0 : g.alpha, zg > 1 ? 0.0 : g.beta, zg > 1 ? g.part + (int64_t)zi * g.M * g.N : g.C,
-                        zg > 1 ? partial : direct);
-}
-
-// C = alpha * (the zg partial products, in order) + beta * C, kChunk outputs per work item
-__global__ void grouped_splitk_reduce(const GemmDesc* __restrict__ desc, const int64_t* __restrict__ prefix, int nd,
-                                      int64_t total, int zg, const int* __restrict__ active) {
-  for (int64_t t = blockIdx.x; t < total; t += gridDim.x) {
-    const int di = find_item(prefix, nd, t);
-    const GemmDesc& g = desc[di];
-    if (!active[g.prob]) continue;
-    const int64_t mn = g.M * g.N, e0 = (t - prefix[di]) * kChunk, e1 = min(e0 + kChunk, mn);
-    for (int64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-      double s = 0.0;
-#pragma unroll 8
-      for (int q = 0; q < zg; q++) s += g.part[(int64_t)q * mn + e];
-      const int64_t m = e / g.N, n = e - m * g.N;
-      double* c = g.C + m * g.sCm + n * g.sCn;
-      const double v = g.alpha * s;
-      *c = (g.beta == 0.0) ? v : fma(g.beta, *c, v);
-    }
-  }
+  if (!active[g.prob]) return;  // the whole cluster, and every share of the tile
+  const int64_t local = t - prefix[di], ntn = (g.N + T::BN - 1) / T::BN, z = (int64_t)zc * zg;
+  const DSplit split{zc, zg, rank, (int)(u - t * zg), (g.K + z - 1) / z, part + t * zg * (T::BM * T::BN),
+                     tickets + t * zc};
+  dgemm_cta<T, CLUSTER>(smem, split, g.A, g.B, g.M, g.N, g.K, local / ntn * T::BM, local % ntn * T::BN, g.alpha,
+                        g.beta, g.C, g.epi);
 }
 
 // The amplitude passes of pairs.h for all members: a work item is one (tile or tile pair, slice
@@ -572,8 +549,8 @@ struct GroupOp {
   DevArray<GemmDesc> gdesc;
   DevArray<PermDesc> pdesc;
   DevArray<PairDesc> pairs;
-  DevArray<int64_t> prefix, rprefix;  // work items; of a split GEMM's reduction
-  int64_t total = 0, rtotal = 0;
+  DevArray<int64_t> prefix;  // work items
+  int64_t total = 0;
   int nd = 0;
   double flops = 0.0;
 };
@@ -599,7 +576,8 @@ struct ucc_batch {
   int64_t total_np = 0, total_t2 = 0;
   DevArray<int> active, iterations, converged, status;
   DevArray<double> partial, dpartial, sumsq, rms, energy, Bmat, coef, epartial;
-  DevArray<double> splitk;  // partial products of the split GEMMs (one operation at a time)
+  DevArray<double> splitk;        // partial tiles of the split GEMMs and their tickets (one operation at a time)
+  DevArray<unsigned int> tickets;
   DevArray<SweepState> state;
   std::vector<std::unique_ptr<DeviceBuffer>> diis_store;
   cudaGraph_t graph = nullptr;
@@ -645,8 +623,8 @@ void launch_tiles(ucc_batch& B, GroupOp& op) {
   const DgemmPlan& p = op.plan;
   const unsigned grid = (unsigned)(op.total * p.zc * p.zg);
   if (p.zc == 1) {
-    grouped_gemm<T, false><<<grid, T::THREADS, 0, B.stream>>>(op.gdesc.p, op.prefix.p, op.nd, op.total, 1, p.zg,
-                                                              B.active.p);
+    grouped_gemm<T, false><<<grid, T::THREADS, 0, B.stream>>>(op.gdesc.p, op.prefix.p, op.nd, 1, 1, B.splitk.p,
+                                                              B.tickets.p, B.active.p);
     return;
   }
   cudaLaunchConfig_t cfg = {};
@@ -663,7 +641,7 @@ void launch_tiles(ucc_batch& B, GroupOp& op) {
   const GemmDesc* d = op.gdesc.p;
   const int64_t* pf = op.prefix.p;
   const int* act = B.active.p;
-  UCC_CUDA(cudaLaunchKernelEx(&cfg, grouped_gemm<T, true>, d, pf, op.nd, op.total, p.zc, p.zg, act));
+  UCC_CUDA(cudaLaunchKernelEx(&cfg, grouped_gemm<T, true>, d, pf, op.nd, p.zc, p.zg, B.splitk.p, B.tickets.p, act));
 }
 
 template <int KIND>
@@ -672,7 +650,7 @@ void launch_pairs(ucc_batch& B, GroupOp& op) {
                                                                         B.active.p);
 }
 
-// launches one operation of all members; the number of kernels
+// launches one operation of all members, one kernel (none if it is empty)
 int launch_op(ucc_batch& B, GroupOp& op) {
   int k = 0;
   if (op.total > 0) {
@@ -684,11 +662,6 @@ int launch_op(ucc_batch& B, GroupOp& op) {
           launch_tiles<DTile16>(B, op);
         else
           launch_tiles<DTile32>(B, op);
-        if (op.plan.zg > 1) {
-          grouped_splitk_reduce<<<grid_for(op.rtotal), 256, 0, B.stream>>>(op.gdesc.p, op.rprefix.p, op.nd, op.rtotal,
-                                                                           op.plan.zg, B.active.p);
-          k++;
-        }
         break;
       case RecordedOp::kPackTau: launch_pairs<RecordedOp::kPackTau>(B, op); break;
       case RecordedOp::kRing: launch_pairs<RecordedOp::kRing>(B, op); break;
@@ -726,30 +699,28 @@ void merge_axes(PermDesc& p) {
 }
 
 // a GEMM operation of all members: its plan, and the members longest K share first
-void group_gemm(ucc_batch& B, GroupOp& g, const std::vector<std::vector<RecordedOp>>& traces, size_t k,
-                std::vector<GemmDesc>& d) {
+void group_gemm(ucc_batch& B, GroupOp& g, const std::vector<std::vector<RecordedOp>>& traces, size_t k) {
   const int nm = (int)traces.size();
+  std::vector<GemmDesc> d;
   std::vector<GemmShape> shapes;
   for (int b = 0; b < nm; b++) {
     const RecordedOp& o = traces[b][k];
-    d.push_back(GemmDesc{o.M, o.N, o.K, o.sAm, o.sAk, o.sBk, o.sBn, o.sCm, o.sCn, o.A, o.B, o.C, nullptr, o.alpha,
-                         o.beta, b});
-    shapes.push_back({o.M, o.N, o.K, 1});
-    g.flops += 2.0 * (double)o.M * (double)o.N * (double)o.K;
+    const int64_t M = o.A.rows, N = o.B.rows, K = o.A.cols;
+    d.push_back(GemmDesc{M, N, K, dgemm_operand(o.A), dgemm_operand(o.B), o.C, o.epi, o.alpha, o.beta, b});
+    shapes.push_back({M, N, K, 1});
+    g.flops += 2.0 * (double)M * (double)N * (double)K;
   }
   g.plan = dgemm_plan(shapes, true);
   std::stable_sort(d.begin(), d.end(), [](const GemmDesc& x, const GemmDesc& y) { return x.K > y.K; });
   const int bm = g.plan.shape == 0 ? DTile16::BM : DTile32::BM, bn = g.plan.shape == 0 ? DTile16::BN : DTile32::BN;
-  std::vector<int64_t> pf(nm), rpf(nm);
+  std::vector<int64_t> pf(nm);
   for (int b = 0; b < nm; b++) {
     pf[b] = g.total;
     g.total += ((d[b].M + bm - 1) / bm) * ((d[b].N + bn - 1) / bn);
-    rpf[b] = g.rtotal;
-    g.rtotal += (d[b].M * d[b].N + kChunk - 1) / kChunk;
   }
   UCC_REQUIRE(g.total * g.plan.zc * g.plan.zg < ((int64_t)1 << 31), UCC_UNSUPPORTED, "batch: too many output tiles");
   g.prefix.upload(pf, B.stream);
-  if (g.plan.zg > 1) g.rprefix.upload(rpf, B.stream);
+  g.gdesc.upload(d, B.stream);
   B.info.shape_choice[g.plan.shape]++;
 }
 
@@ -816,17 +787,18 @@ void build(ucc_batch& B) {
   B.ops.clear();
   B.ops.resize(nops);
   for (int& n : B.info.shape_choice) n = 0;
-  std::vector<std::vector<GemmDesc>> gemms(nops);
-  int64_t split_size = 0;
+  int64_t split_size = 1, ticket_count = 1;
   for (size_t k = 0; k < nops; k++) {
     GroupOp& g = B.ops[k];
     g.kind = traces[0][k].kind;
     g.nd = nm;
     if (g.kind == RecordedOp::kGemm) {
-      group_gemm(B, g, traces, k, gemms[k]);
-      int64_t part = 0;
-      for (const GemmDesc& d : gemms[k]) part += d.M * d.N * g.plan.zg;
-      if (g.plan.zg > 1) split_size = std::max(split_size, part);
+      group_gemm(B, g, traces, k);
+      if (g.plan.zg > 1) {
+        const int64_t tile = g.plan.shape == 0 ? DTile16::BM * DTile16::BN : DTile32::BM * DTile32::BN;
+        split_size = std::max(split_size, g.total * g.plan.zg * tile);
+        ticket_count = std::max(ticket_count, g.total * g.plan.zc);
+      }
     } else if (g.kind != RecordedOp::kPermute && g.kind != RecordedOp::kFill) {
       std::vector<PairDesc> d(nm);
       std::vector<int64_t> pf(nm);
@@ -875,17 +847,9 @@ void build(ucc_batch& B) {
       g.prefix.upload(pf, B.stream);
     }
   }
-  // the split operations run one after the other and share one array of partial products
-  B.splitk.zeros((size_t)std::max<int64_t>(1, split_size), B.stream);
-  for (size_t k = 0; k < nops; k++) {
-    if (gemms[k].empty()) continue;
-    double* part = B.splitk.p;
-    for (GemmDesc& d : gemms[k]) {
-      d.part = part;
-      if (B.ops[k].plan.zg > 1) part += d.M * d.N * B.ops[k].plan.zg;
-    }
-    B.ops[k].gdesc.upload(gemms[k], B.stream);
-  }
+  // the split operations run one after the other and share one array of partial tiles
+  B.splitk.zeros((size_t)split_size, B.stream);
+  B.tickets.zeros((size_t)ticket_count, B.stream);
   // sweep tables
   std::vector<Member> mh(nm);
   std::vector<int64_t> pnp(nm), pt2(nm);

@@ -32,6 +32,7 @@ Ctx::~Ctx() {
     cudaEventDestroy(t.b);
   }
   for (auto e : event_pool) cudaEventDestroy(e);
+  if (words_) cudaFree(words_);
   anchors.clear();  // pool buffers are freed on the stream
   tc_cache.reset();
   perts.clear();

@@ -443,11 +443,11 @@ void residual(Ctx& c, const double* t_old, double* r, std::vector<cudaEvent_t>* 
 double energy(Ctx& c, const Tensor& t1, const Tensor& tau) {
   const int no = c.no, nv = c.nv, n = no + nv;
   // ccwfn.cc:270-273 assigns instead of accumulating: only the last (i,a) pair counts
-  double t1last = 0.0;
-  UCC_CUDA(cudaMemcpyAsync(&t1last, t1.p + (int64_t)no * nv - 1, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-  const double two = dot_all(c, tau, L(c, "oovv"));
-  const double one = 2.0 * c.fock[(size_t)(no - 1) * n + (n - 1)] * t1last;
-  return one + two;
+  DotList d(c);
+  const int two = dot_all(c, tau, L(c, "oovv"), d);
+  const int last = d.add(1, t1.p + (int64_t)no * nv - 1, nullptr);
+  d.fetch();
+  return 2.0 * c.fock[(size_t)(no - 1) * n + (n - 1)] * d[last] + d[two];
 }
 
 }  // namespace

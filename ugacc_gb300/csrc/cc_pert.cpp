@@ -362,12 +362,14 @@ void build_Y(Ctx& c, Perturbation& p, const Tensor& Y1o, const Tensor& Y2o, Tens
 double pseudoresponse(Ctx& c, Perturbation& p, double* amps) {  // ccpert.cc:233-253
   const int no = c.no, nv = c.nv;
   Tensor X1 = amp1(c, amps), X2 = amp2(c, amps);
-  double p1 = 2.0 * dot_all(c, X1, view(P(c, p, "Avo"), "ai->ia"));
+  DotList d(c);
+  dot_all(c, X1, view(P(c, p, "Avo"), "ai->ia"), d);
   Temp X(c, {no, no, nv, nv});
   transpose_add(c, "ijab->ijba", -1.0, X2, 0.0, X);
   axpby(c, X->size(), 2.0, X2.p, 1.0, X->p);
-  double p2 = 2.0 * dot_all(c, X, view(P(c, p, "Avvoo"), "abij->ijab"));
-  return -2.0 * (p1 + p2);
+  dot_all(c, X, view(P(c, p, "Avvoo"), "abij->ijab"), d);
+  d.fetch();
+  return -2.0 * (2.0 * d[0] + 2.0 * d[1]);
 }
 }  // namespace
 
@@ -491,44 +493,54 @@ double linresp(Ctx& c, int hx, int hy) {  // ccresp.cc:28-124
   Tensor X1y = amp1(c, yx), X2y = amp2(c, yx), Y1y = amp1(c, yy), Y2y = amp2(c, yy);
   Tensor Avo = P(c, X, "Avo"), Avv = P(c, X, "Avv"), Aoo = P(c, X, "Aoo"), Avvoo = P(c, X, "Avvoo");
   Tensor Avvvo = P(c, X, "Avvvo"), Aovoo = P(c, X, "Aovoo"), pov = P(c, X, "pov");
-  double polar1 = dot_all(c, view(Avo, "ai->ia"), Y1y);
+  // the dot products are added on the device's stream and read together at the end
+  DotList d(c);
+  std::vector<double> coef;  // of each dot product in the response function's two sums
+  auto add = [&](double f, const Tensor& A, const Tensor& B) {
+    dot_all(c, A, B, d);
+    coef.push_back(f);
+  };
+  add(1.0, view(Avo, "ai->ia"), Y1y);
   {
     Temp Ax(c, {no, no, nv, nv});
     transpose_add(c, "abij->ijab", 1.0, Avvoo, 0.0, Ax);
     transpose_add(c, "baji->ijab", 1.0, Avvoo, 1.0, Ax);
-    polar1 += 0.5 * dot_all(c, Ax, Y2y);
+    add(0.5, Ax, Y2y);
   }
-  double polar2 = 0.0;
+  const size_t first2 = coef.size();
   {
     Temp X(c, {no, no, nv, nv}), M(c, {no, nv});
     transpose_add(c, "ijab->ijba", -1.0, X2y, 0.0, X);
     axpby(c, X->size(), 2.0, X2y.p, 1.0, X->p);
     contract(c, "jb,ijab->ia", 1.0, pov, X, 0.0, M);
-    polar2 += dot_all(c, l1, M);
+    add(1.0, l1, M);
     contract(c, "ac,ic->ia", 1.0, Avv, X1y, 0.0, M);
-    polar2 += dot_all(c, l1, M);
+    add(1.0, l1, M);
     contract(c, "ki,ka->ia", 1.0, Aoo, X1y, 0.0, M);
-    polar2 -= dot_all(c, l1, M);
+    add(-1.0, l1, M);
     Temp A(c, {no, nv});  // A[i,a] = l2[i,j,b,c] Avvvo[b,c,a,j]
     contract(c, "ijbc,bcaj->ia", 1.0, l2, Avvvo, 0.0, A);
-    polar2 += dot_all(c, A, X1y);
+    add(1.0, A, X1y);
     Temp B(c, {no, nv});  // B[k,a] = l2[i,j,a,b] Aovoo[k,b,i,j]
     contract(c, "ijab,kbij->ka", 1.0, l2, Aovoo, 0.0, B);
-    polar2 -= 0.5 * dot_all(c, B, X1y);
+    add(-0.5, B, X1y);
     contract(c, "ijab,kaji->kb", 1.0, l2, Aovoo, 0.0, B);
-    polar2 -= 0.5 * dot_all(c, B, X1y);
+    add(-0.5, B, X1y);
     Temp G(c, {no, no});  // G[k,i] = l2[i,j,a,b] X2y[k,j,a,b]
     contract(c, "ijab,kjab->ki", 1.0, l2, X2y, 0.0, G);
-    polar2 -= 0.5 * dot_all(c, G, Aoo);
+    add(-0.5, G, Aoo);
     contract(c, "ijab,kiba->kj", 1.0, l2, X2y, 0.0, G);
-    polar2 -= 0.5 * dot_all(c, G, Aoo);
+    add(-0.5, G, Aoo);
     Temp H(c, {nv, nv});  // H[b,c] = l2[i,j,a,b] X2y[i,j,a,c]
     contract(c, "ijab,ijac->bc", 1.0, l2, X2y, 0.0, H);
-    polar2 += 0.5 * dot_all(c, H, Avv);
+    add(0.5, H, Avv);
     contract(c, "ijab,jibc->ac", 1.0, l2, X2y, 0.0, H);
-    polar2 += 0.5 * dot_all(c, H, Avv);
-    polar2 += 2.0 * dot_all(c, pov, X1y);
+    add(0.5, H, Avv);
+    add(2.0, pov, X1y);
   }
+  d.fetch();
+  double polar1 = 0.0, polar2 = 0.0;
+  for (size_t k = 0; k < coef.size(); k++) (k < first2 ? polar1 : polar2) += coef[k] * d[(int)k];
   return -(polar1 + polar2);
 }
 

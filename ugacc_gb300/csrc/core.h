@@ -101,6 +101,13 @@ struct MatView {
   bool k_contiguous() const { return (ksplit ? ks_lo : ks_hi) == 1; }  // unit stride along the columns
 };
 
+struct GemmEpilogue {  // C offset of element (m, n): (m / msplit) * s_mhi + (m % msplit) * s_mlo + n * s_n
+  int64_t msplit = 0;  // 0: plain, offset = m * s_mhi + n * s_n
+  int64_t s_mhi = 0, s_mlo = 0, s_n = 1;
+  // FP64 GEMM only: n as two runs as well, (n / nsplit) * s_n + (n % nsplit) * s_nlo; 0: plain
+  int64_t nsplit = 0, s_nlo = 0;
+};
+
 // FP64 buffer from the stream-ordered pool, freed in stream order (no device
 // synchronisation): per-sweep state such as the refinement anchors.
 struct PoolBuffer {
@@ -238,6 +245,20 @@ struct Ctx {
   cudaEvent_t take_event();
   void resolve_timers();  // synchronises the stream
 
+  // Zeroed device words that the kernels of this context's stream hand back as they found
+  // them (or add to): the clock of the short FP64 GEMMs and the tickets with which the last
+  // block of a reduction knows itself.  Allocated on first use.
+  struct DeviceWords {
+    unsigned long long start, total;  // dgemm_cta: start of the running GEMM (0: none), ns of all of them
+    unsigned int done, reduce;        // CTAs of the running GEMM that have ended; blocks of the running reduction
+    static constexpr int kTickets = 16384;
+    unsigned int tickets[kTickets];   // split-K: shares of a tile that have arrived
+  };
+  DeviceWords* words();
+  DeviceWords* words_ = nullptr;
+  double short_gemm_flops = 0.0;  // of the GEMMs that `total` times, until resolve_timers
+  int64_t short_gemm_launches = 0;
+
   ~Ctx();
 };
 
@@ -251,10 +272,9 @@ struct Ctx {
 // ----------------------------------------------------------------------------------
 struct RecordedOp {
   enum Kind { kGemm, kPermute, kFill, kPackTau, kRing, kAssemble, kUnpackZ } kind = kGemm;
-  // GEMM: C[m*sCm + n*sCn] = alpha * sum_k A[m*sAm + k*sAk] B[k*sBk + n*sBn] + beta * C
-  int64_t M = 0, N = 0, K = 0, sAm = 0, sAk = 0, sBk = 0, sBn = 0, sCm = 0, sCn = 0;
-  const double* A = nullptr;
-  const double* B = nullptr;
+  // GEMM: C(epi) = alpha * A B + beta * C, A: M x K, B: N x K
+  MatView A, B;
+  GemmEpilogue epi;
   double* C = nullptr;
   double alpha = 0.0, beta = 0.0;
   // permute: out = alpha * in + beta * out over out's dims; fill: out = alpha
@@ -288,11 +308,6 @@ Recorder*& recorder();  // the calling thread's recorder (null: launch normally)
 // ----------------------------------------------------------------------------------
 // Kernel launchers (kernels_fp64.cu).  All are asynchronous on ctx.stream.
 // ----------------------------------------------------------------------------------
-struct GemmEpilogue {  // C offset of element (m, n): (m / msplit) * s_mhi + (m % msplit) * s_mlo + n * s_n
-  int64_t msplit = 0;  // 0: plain, offset = m * s_mhi + n * s_n
-  int64_t s_mhi = 0, s_mlo = 0, s_n = 1;
-};
-
 // Blocked W3 layout of the mixed (T) path: W[a][b][c] of one tuple in 8 x 8 x 8 blocks,
 // block (a/8, b/8, c/8) at ((a/8 * T + b/8) * T + c/8) * 512 (T = ceil(nv/8) blocks per
 // index), element (x, y, z) = (a%8, b%8, c%8) of a block at 64 x + 8 (y ^ x) + (z ^ (5y % 8)).
@@ -312,9 +327,12 @@ struct GemmPtrs {
 // Status of the tensor-core launches since the last check (pipeline-wait timeout, sliced
 // operand out of range), read after synchronising the stream; throws on either.
 void tc_check(Ctx& c);
-// C = alpha * A B + beta * C with arbitrary operand strides: element (m, k) of A at A[m*sAm + k*sAk],
-// (k, n) of B at B[k*sBk + n*sBn].  Batched over `batch` with either strides or a device
-// array of pointer triples.
+// C = alpha * A B + beta * C, A: M x K and B: N x K views (rows = the output's columns)
+void dgemm_view(Ctx& c, double alpha, const MatView& A, const MatView& B, double beta, double* C,
+                const GemmEpilogue& epi);
+// The same with plain strides: element (m, k) of A at A[m*sAm + k*sAk], (k, n) of B at
+// B[k*sBk + n*sBn].  Batched over `batch` with either strides or a device array of pointer
+// triples.
 void dgemm_strided(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const double* A, int64_t sAm, int64_t sAk,
                    const double* B, int64_t sBk, int64_t sBn, double beta, double* C, const GemmEpilogue& epi,
                    int batch, int64_t bA, int64_t bB, int64_t bC, const GemmPtrs* ptrs);
@@ -332,6 +350,28 @@ void fill(Ctx& c, int64_t n, double v, double* y);
 // Sum of x[k] * y[k] (y == nullptr: sum of x) with compensated FP64 accumulation; the
 // result stays on the device.
 void dot_async(Ctx& c, int64_t n, const double* x, const double* y, double* d_out);
+// Dot products whose values are read together: one wait for all of them.
+class DotList {
+ public:
+  explicit DotList(Ctx& c) : c_(c), out_(c, sizeof(double) * kMax) {}
+  int add(int64_t n, const double* x, const double* y) {
+    UCC_REQUIRE(count_ < kMax, UCC_BAD_ARGS, "too many dot products in one list");
+    dot_async(c_, n, x, y, out_.d() + count_);
+    return count_++;
+  }
+  void fetch() {
+    UCC_CUDA(cudaMemcpyAsync(h_, out_.d(), sizeof(double) * count_, cudaMemcpyDeviceToHost, c_.stream));
+    UCC_CUDA(cudaStreamSynchronize(c_.stream));
+  }
+  double operator[](int k) const { return h_[k]; }
+
+ private:
+  static constexpr int kMax = 32;
+  Ctx& c_;
+  Scratch out_;
+  int count_ = 0;
+  double h_[kMax] = {};
+};
 double dot(Ctx& c, int64_t n, const double* x, const double* y);
 // Several dot products x_k . y at once (DIIS B-matrix row), results on the device.
 void multidot_async(Ctx& c, int nvec, const double* const* d_xs, const double* y, int64_t n, double* d_out);

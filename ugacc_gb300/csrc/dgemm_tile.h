@@ -32,6 +32,25 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// An index as one strided run or two (MatView); x < 2^31 as far as a split is used
+struct DRun {
+  int64_t hi, lo;
+  uint32_t split;
+  __host__ __device__ __forceinline__ int64_t off(int64_t x) const {
+    if (!split) return x * hi;
+    const uint32_t q = (uint32_t)x / split;
+    return (int64_t)q * hi + (int64_t)((uint32_t)x - q * split) * lo;
+  }
+  __host__ __device__ __forceinline__ int64_t step() const { return split ? lo : hi; }
+};
+// Operand: rows (m, or n) x K.  The index arithmetic of two runs costs nothing beside the
+// FMAs, and reading an operand in place saves the launch that would gather it.
+struct DView {
+  const double* p;
+  DRun r, k;
+  bool kfast;  // neighbouring threads load neighbouring k
+};
+
 // WM x WN warps, PM x PN patches of 8 x 4 outputs per warp, K in steps of BK through two
 // shared-memory stages filled by cp.async
 template <int WM_, int WN_, int PM_, int PN_, int BK_>
@@ -42,23 +61,22 @@ struct DTile {
   static constexpr int LDA = BM + 1, LDB = BN + 1, STAGE = BK * (LDA + LDB);
   static constexpr int SMEM = 2 * STAGE;  // doubles
 
-  // one stage: A(0..mrem, 0..krem) and B(0..krem, 0..nrem) relative to the given pointers
-  static __device__ __forceinline__ void load(double* st, const double* A, int64_t sAm, int64_t sAk, int mrem,
-                                              const double* B, int64_t sBk, int64_t sBn, int nrem, int krem,
-                                              bool a_kfast, bool b_nfast) {
+  // one stage: A rows m0.. (mrem of them), B rows n0.. (nrem), K from k0 (krem steps)
+  static __device__ __forceinline__ void load(double* st, const DView& A, int64_t m0, int mrem, const DView& B,
+                                              int64_t n0, int nrem, int64_t k0, int krem) {
     double* As = st;
     double* Bs = st + BK * LDA;
 #pragma unroll
     for (int e = threadIdx.x; e < BM * BK; e += THREADS) {
-      const int mm = a_kfast ? e / BK : e % BM, kk = a_kfast ? e % BK : e / BM;
+      const int mm = A.kfast ? e / BK : e % BM, kk = A.kfast ? e % BK : e / BM;
       const bool ok = mm < mrem && kk < krem;
-      cp_async8(As + kk * LDA + mm, ok ? A + mm * sAm + kk * sAk : A, ok);
+      cp_async8(As + kk * LDA + mm, ok ? A.p + A.r.off(m0 + mm) + A.k.off(k0 + kk) : A.p, ok);
     }
 #pragma unroll
     for (int e = threadIdx.x; e < BN * BK; e += THREADS) {
-      const int nn = b_nfast ? e % BN : e / BK, kk = b_nfast ? e / BN : e % BK;
+      const int nn = B.kfast ? e / BK : e % BN, kk = B.kfast ? e % BK : e / BN;
       const bool ok = nn < nrem && kk < krem;
-      cp_async8(Bs + kk * LDB + nn, ok ? B + kk * sBk + nn * sBn : B, ok);
+      cp_async8(Bs + kk * LDB + nn, ok ? B.p + B.r.off(n0 + nn) + B.k.off(k0 + kk) : B.p, ok);
     }
     cp_async_commit();
   }
@@ -85,14 +103,12 @@ struct DTile {
     }
   }
 
-  // acc = A(0..M, 0..K) B(0..K, 0..N) of this tile (M, N: rows and columns left from its
-  // corner, A and B the corner's pointers, K steps in ascending order)
-  static __device__ __forceinline__ void product(double* smem, const double* A, int64_t sAm, int64_t sAk,
-                                                 const double* B, int64_t sBk, int64_t sBn, int64_t M, int64_t N,
-                                                 int64_t K, double (&acc)[PM][PN]) {
+  // acc = the tile at (m0, n0) of an M x N product, K from k0 over kn steps in ascending order
+  static __device__ __forceinline__ void product(double* smem, const DView& A, const DView& B, int64_t M, int64_t N,
+                                                 int64_t m0, int64_t n0, int64_t k0, int64_t K,
+                                                 double (&acc)[PM][PN]) {
     const int warp = threadIdx.x / 32;
-    const int mrem = (int)(M < BM ? M : BM), nrem = (int)(N < BN ? N : BN);
-    const bool a_kfast = sAk == 1 || (sAm != 1 && sAk < sAm), b_nfast = sBn == 1 || (sBk != 1 && sBn < sBk);
+    const int mrem = (int)(M - m0 < BM ? M - m0 : BM), nrem = (int)(N - n0 < BN ? N - n0 : BN);
     // patch row i of the warp covers rows 8 (warp / WN + WM i) ..: the count inside the matrix
     const int pr = (mrem + 7) / 8 - warp / WN, pc = (nrem + 3) / 4 - warp % WN;
     const int pm = pr > 0 ? (pr + WM - 1) / WM : 0, pn = pc > 0 ? (pc + WN - 1) / WN : 0;
@@ -101,19 +117,18 @@ struct DTile {
 #pragma unroll
       for (int j = 0; j < PN; j++) acc[i][j] = 0.0;
     if (K <= 0) return;
-    load(smem, A, sAm, sAk, mrem, B, sBk, sBn, nrem, (int)(K < BK ? K : BK), a_kfast, b_nfast);
+    load(smem, A, m0, mrem, B, n0, nrem, k0, (int)(K < BK ? K : BK));
     int buf = 0;
-    for (int64_t k0 = 0; k0 < K; k0 += BK) {
-      const int64_t k1 = k0 + BK;
-      if (k1 < K) {
-        load(smem + (buf ^ 1) * STAGE, A + k1 * sAk, sAm, sAk, mrem, B + k1 * sBk, sBk, sBn, nrem,
-             (int)(K - k1 < BK ? K - k1 : BK), a_kfast, b_nfast);
+    for (int64_t kd = 0; kd < K; kd += BK) {
+      const int64_t kx = kd + BK;
+      if (kx < K) {
+        load(smem + (buf ^ 1) * STAGE, A, m0, mrem, B, n0, nrem, k0 + kx, (int)(K - kx < BK ? K - kx : BK));
         cp_async_wait<1>();
       } else {
         cp_async_wait<0>();
       }
       __syncthreads();
-      const int kn = (int)(K - k0 < BK ? K - k0 : BK);
+      const int kn = (int)(K - kd < BK ? K - kd : BK);
       if (pm == PM && pn == PN)
         fma_stage<true>(smem + buf * STAGE, kn, pm, pn, acc);
       else if (pm > 0 && pn > 0)
@@ -161,19 +176,49 @@ __device__ __forceinline__ double ld_cluster(const double* p, uint32_t rank) {
 }
 
 __device__ __forceinline__ int64_t dgemm_c_offset(const GemmEpilogue& ep, int64_t m, int64_t n) {
-  return (ep.msplit ? (m / ep.msplit) * ep.s_mhi + (m % ep.msplit) * ep.s_mlo : m * ep.s_mhi) + n * ep.s_n;
+  const int64_t mo = ep.msplit ? (m / ep.msplit) * ep.s_mhi + (m % ep.msplit) * ep.s_mlo : m * ep.s_mhi;
+  return mo + (ep.nsplit ? (n / ep.nsplit) * ep.s_n + (n % ep.nsplit) * ep.s_nlo : n * ep.s_n);
 }
 
-// One CTA's share of C = alpha A B + beta C: the tile at (m0, n0), K from k0 over at most kchunk
-// steps.  CLUSTER: the zc CTAs of a cluster hold the same tile's K shares, and their partial
-// tiles are added through distributed shared memory in rank order, so a split costs no second
-// launch and no trip through device memory.
+__device__ __forceinline__ unsigned long long dgemm_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+// Device time of a short GEMM, measured by its own CTAs: the first one to start sets `start`,
+// the last one to end adds the difference to `total` and clears the others.  A pair of CUDA
+// events costs the stream 4.5 us, more than the median FP64 GEMM of a small solve takes.
+__device__ __forceinline__ void dgemm_clock_start(Ctx::DeviceWords* w) {
+  if (w && threadIdx.x == 0) atomicCAS(&w->start, 0ull, dgemm_ns());
+}
+__device__ __forceinline__ void dgemm_clock_stop(Ctx::DeviceWords* w, unsigned int ctas) {
+  if (w && threadIdx.x == 0 && atomicAdd(&w->done, 1u) == ctas - 1) {
+    const unsigned long long t0 = *(volatile unsigned long long*)&w->start, t1 = dgemm_ns();
+    w->total += t1 > t0 ? t1 - t0 : 0ull;
+    w->start = 0ull;
+    w->done = 0u;
+  }
+}
+
+// K over zc CTAs of a cluster times zg clusters; the clusters' partial tiles go to part
+// [zg][BM * BN] and ticket[rank] counts those that have arrived
+struct DSplit {
+  int zc, zg, rank, zi;
+  int64_t kchunk;
+  double* part;
+  unsigned int* ticket;
+};
+
+// One CTA's share of C = alpha A B + beta C, the tile at (m0, n0).  CLUSTER: the zc CTAs of a
+// cluster hold shares of the same tile's K, and their partial tiles are added through
+// distributed shared memory in rank order; with zg > 1 the last cluster to finish adds the
+// clusters' sums in their order.  So a split needs no second launch.
 template <class T, bool CLUSTER>
-__device__ __forceinline__ void dgemm_cta(double* smem, int rank, int zc, int64_t M, int64_t N, int64_t K, int64_t m0,
-                                          int64_t n0, int64_t k0, int64_t kchunk, const double* A, int64_t sAm,
-                                          int64_t sAk, const double* B, int64_t sBk, int64_t sBn, double alpha,
-                                          double beta, double* C, const GemmEpilogue& epi) {
-  const int64_t kn = k0 < K ? (K - k0 < kchunk ? K - k0 : kchunk) : 0;
+__device__ __forceinline__ void dgemm_cta(double* smem, const DSplit& z, const DView& A, const DView& B, int64_t M,
+                                          int64_t N, int64_t K, int64_t m0, int64_t n0, double alpha, double beta,
+                                          double* C, const GemmEpilogue& epi) {
+  const int64_t k0 = ((int64_t)z.zi * z.zc + z.rank) * z.kchunk;
+  const int64_t kn = k0 < K ? (K - k0 < z.kchunk ? K - k0 : z.kchunk) : 0;
   double acc[T::PM][T::PN], old[T::PM][T::PN];
   if (!CLUSTER && beta != 0.0) {  // the old values travel while the product runs
 #pragma unroll
@@ -184,7 +229,7 @@ __device__ __forceinline__ void dgemm_cta(double* smem, int rank, int zc, int64_
         old[i][j] = m < M && n < N ? C[dgemm_c_offset(epi, m, n)] : 0.0;
       }
   }
-  T::product(smem, A + m0 * sAm + k0 * sAk, sAm, sAk, B + k0 * sBk + n0 * sBn, sBk, sBn, M - m0, N - n0, kn, acc);
+  T::product(smem, A, B, M, N, m0, n0, k0, kn, acc);
   if (!CLUSTER) {
 #pragma unroll
     for (int i = 0; i < T::PM; i++)
@@ -200,24 +245,47 @@ __device__ __forceinline__ void dgemm_cta(double* smem, int rank, int zc, int64_
   }
   // product() ended with a barrier: its stages are free for the partial tile, [m][n] or
   // [n][m] so that consecutive elements are consecutive in C where one of its indices allows
-  const bool mfast = epi.s_n != 1 && !epi.msplit && epi.s_mhi == 1;
+  const bool mfast = epi.s_n != 1 && !epi.msplit && !epi.nsplit && epi.s_mhi == 1;
 #pragma unroll
   for (int i = 0; i < T::PM; i++)
 #pragma unroll
     for (int j = 0; j < T::PN; j++)
       smem[mfast ? T::col(j) * T::BM + T::row(i) : T::row(i) * T::BN + T::col(j)] = acc[i][j];
   dgemm_cluster_barrier();
-  for (int e = rank * T::THREADS + (int)threadIdx.x; e < T::BM * T::BN; e += zc * T::THREADS) {
+  constexpr int kTile = T::BM * T::BN;
+  const int e0 = z.rank * T::THREADS + (int)threadIdx.x, step = z.zc * T::THREADS;  // this CTA's elements
+  auto store = [&](int e, double s) {
     const int64_t m = m0 + (mfast ? e % T::BM : e / T::BN), n = n0 + (mfast ? e / T::BM : e % T::BN);
-    if (m >= M || n >= N) continue;
+    if (m >= M || n >= N) return;
     double* cp = C + dgemm_c_offset(epi, m, n);
-    const double o = beta != 0.0 ? *cp : 0.0;
-    double s = 0.0;
-    for (int q = 0; q < zc; q++) s += ld_cluster(smem + e, (uint32_t)q);
     const double v = alpha * s;
-    *cp = beta == 0.0 ? v : fma(beta, o, v);
+    *cp = beta == 0.0 ? v : fma(beta, *cp, v);
+  };
+  for (int e = e0; e < kTile; e += step) {
+    double s = 0.0;
+    for (int q = 0; q < z.zc; q++) s += ld_cluster(smem + e, (uint32_t)q);
+    if (z.zg > 1)
+      z.part[(int64_t)z.zi * kTile + e] = s;
+    else
+      store(e, s);
   }
   dgemm_cluster_barrier();  // no CTA leaves while another still reads its partial tile
+  if (z.zg > 1) {
+    __shared__ unsigned int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&z.ticket[z.rank], 1u) == (unsigned)z.zg - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int e = e0; e < kTile; e += step) {
+      double s = 0.0;
+#pragma unroll 8
+      for (int q = 0; q < z.zg; q++) s += __ldcg(z.part + (int64_t)q * kTile + e);
+      store(e, s);
+    }
+    if (threadIdx.x == 0) z.ticket[z.rank] = 0u;
+  }
 }
 
 // `count` products of one shape in a launch
@@ -230,5 +298,6 @@ struct DgemmPlan {
   int zc, zg;  // K over the zc CTAs of a cluster, times zg partial products in device memory
 };
 DgemmPlan dgemm_plan(const std::vector<GemmShape>& probs, bool may_split);
+DView dgemm_operand(const MatView& v);
 
 }  // namespace ucc

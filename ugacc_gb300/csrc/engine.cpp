@@ -159,9 +159,28 @@ cudaEvent_t Ctx::take_event() {
   return e;
 }
 
+Ctx::DeviceWords* Ctx::words() {
+  if (!words_) {
+    UCC_CUDA(cudaMalloc(&words_, sizeof(DeviceWords)));
+    UCC_CUDA(cudaMemsetAsync(words_, 0, sizeof(DeviceWords), stream));
+  }
+  return words_;
+}
+
 void Ctx::resolve_timers() {
-  if (gemm_timers.empty()) return;
+  if (gemm_timers.empty() && !short_gemm_launches) return;
   UCC_CUDA(cudaStreamSynchronize(stream));
+  if (short_gemm_launches) {
+    unsigned long long ns = 0;
+    UCC_CUDA(cudaMemcpyAsync(&ns, &words_->total, sizeof ns, cudaMemcpyDeviceToHost, stream));
+    UCC_CUDA(cudaMemsetAsync(&words_->total, 0, sizeof ns, stream));
+    UCC_CUDA(cudaStreamSynchronize(stream));
+    stats.fp64_gemm_ms += 1e-6 * (double)ns;
+    stats.fp64_gemm_flops += short_gemm_flops;
+    stats.fp64_gemm_launches += short_gemm_launches;
+    short_gemm_flops = 0.0;
+    short_gemm_launches = 0;
+  }
   for (auto& t : gemm_timers) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, t.a, t.b);
@@ -423,7 +442,7 @@ void transpose_add(Ctx& c, const std::string& spec, double alpha, const Tensor& 
   permute_add(c, v, alpha, beta, C);
 }
 
-double dot_all(Ctx& c, const Tensor& A, const Tensor& B) {
+int dot_all(Ctx& c, const Tensor& A, const Tensor& B, DotList& list) {
   UCC_REQUIRE(A.rank == B.rank, UCC_BAD_ARGS, "dot_all: rank mismatch");
   for (int k = 0; k < A.rank; k++) UCC_REQUIRE(A.d[k] == B.d[k], UCC_BAD_ARGS, "dot_all: dim mismatch");
   std::unique_ptr<Scratch> ha, hb;
@@ -432,7 +451,14 @@ double dot_all(Ctx& c, const Tensor& A, const Tensor& B) {
   std::string lab = std::string("abcdef").substr(0, A.rank);
   if (!A.dense()) pa = gather(c, A, lab, lab, ha).p;
   if (!B.dense()) pb = gather(c, B, lab, lab, hb).p;
-  return dot(c, A.size(), pa, pb);
+  return list.add(A.size(), pa, pb);
+}
+
+double dot_all(Ctx& c, const Tensor& A, const Tensor& B) {
+  DotList d(c);
+  dot_all(c, A, B, d);
+  d.fetch();
+  return d[0];
 }
 
 void contract(Ctx& c, const std::string& spec, double alpha, const Tensor& A, const Tensor& B, double beta,
@@ -469,16 +495,22 @@ void contract(Ctx& c, const std::string& spec, double alpha, const Tensor& A, co
   const std::string Mcand[2] = {ordered(p.c, Ms), ordered(p.a, Ms)};
   const std::string Ncand[2] = {ordered(p.c, Ns), ordered(p.b, Ns)};
   const std::string Kcand[2] = {ordered(p.a, Ks), ordered(p.b, Ks)};
+  const bool mixed = c.opt.precision == UCC_MIXED;
   double best = 1e300;
+  // bytes that tensor T costs with row group r and column group k: none when each is one
+  // strided run, next to none for the FP64 GEMM when each is at most two, else a gather
+  auto cost_of = [&](const Tensor& T, const std::string& str, const std::string& r, const std::string& k, double copy) {
+    int64_t s1, s2, s3;
+    if (fusable(T, str, r, s1) && fusable(T, str, k, s1)) return 0.0;
+    if (!mixed && fusable2(T, str, r, s1, s2, s3) && fusable2(T, str, k, s1, s2, s3)) return 0.02 * (double)T.size();
+    return copy * (double)T.size();
+  };
   std::string bm, bn, bk;
   for (const auto& mo : Mcand)
     for (const auto& no_ : Ncand)
       for (const auto& ko : Kcand) {
-        int64_t s1, s2;
-        double cost = 0;
-        if (!(fusable(A, p.a, mo, s1) && fusable(A, p.a, ko, s2))) cost += (double)A.size();
-        if (!(fusable(B, p.b, ko, s1) && fusable(B, p.b, no_, s2))) cost += (double)B.size();
-        if (!(fusable(C, p.c, mo, s1) && fusable(C, p.c, no_, s2))) cost += 3.0 * (double)C.size();
+        const double cost =
+            cost_of(A, p.a, mo, ko, 1.0) + cost_of(B, p.b, no_, ko, 1.0) + cost_of(C, p.c, mo, no_, 3.0);
         if (cost < best) {
           best = cost;
           bm = mo;
@@ -503,7 +535,23 @@ void contract(Ctx& c, const std::string& spec, double alpha, const Tensor& A, co
   }
   std::unique_ptr<Scratch> hA, hB, hC;
   int64_t sCm, sCn;
+  bool done = false;
+  const bool anchored = c.anchors.mode != 0 && mixed && (double)M * N * K >= kAnchorMinWork && tc_eligible(M, N, K);
+  // a reduction rather than a GEMM: mostly padding on the sliced tensor tiles, DFMA where FP64 is asked for
+  const bool small_out = M <= 256 && N <= 256 && M * N <= 4096 && K >= 8192;
+  const bool tensor = mixed && !recorder() && !anchored && M > 1 && N > 1;  // may run on the tensor cores
+  // operands whose index groups are two strided runs are read in place: no gather
+  MatView av, bv;
+  const bool views = !anchored && ((M > 1 && N > 1) || recorder()) && view2(A, p.a, bm, bk, av) &&
+                     view2(B, p.b, bn, bk, bv);
   const bool cdirect = fusable(C, p.c, bm, sCm) && fusable(C, p.c, bn, sCn);
+  GemmEpilogue epi;  // of the FP64 GEMM: C's groups as one or two runs each
+  const bool c2 = views && !cdirect && fusable2(C, p.c, bm, epi.msplit, epi.s_mhi, epi.s_mlo) &&
+                  fusable2(C, p.c, bn, epi.nsplit, epi.s_n, epi.s_nlo);
+  if (!tensor && c2) {
+    dgemm_view(c, alpha, av, bv, beta, C.p, epi);
+    return;
+  }
   Tensor ct = C;
   if (!cdirect) {
     std::vector<int64_t> dims;
@@ -518,25 +566,29 @@ void contract(Ctx& c, const std::string& spec, double alpha, const Tensor& A, co
   if (sCm == 0) sCm = 1;  // empty groups: any stride works
   if (sCn == 0) sCn = 1;
   const double ga = cdirect ? alpha : 1.0, gb = cdirect ? beta : 0.0;
-  bool done = false;
-  const bool mixed = c.opt.precision == UCC_MIXED;
-  const bool anchored = c.anchors.mode != 0 && mixed && (double)M * N * K >= kAnchorMinWork && tc_eligible(M, N, K);
-  // a reduction rather than a GEMM: mostly padding on the tensor tiles, FP64 in every precision
-  const bool small_out = M <= 256 && N <= 256 && M * N <= 4096 && K >= 8192;
-  // the tensor-core paths read operands whose index groups are two strided runs directly:
-  // no gather
-  if (M > 1 && N > 1 && mixed && !recorder() && !anchored && !small_out) {
-    MatView av, bv;
-    if (view2(A, p.a, bm, bk, av) && view2(B, p.b, bn, bk, bv)) {
-      if (!c.force_fp64) done = mixed_gemm(c, M, N, K, ga, av, bv, gb, ct.p, sCm, sCn);
-      if (!done) {
-        const double t0 = c.stats.sliced_gemm_ms;
-        done = sliced_gemm(c, M, N, K, ga, av, bv, gb, ct.p, sCm, sCn);
-        if (done && c.opt.print >= 3)  // PRINT >= 3: every sliced FP64 GEMM with its shape and time
-          std::printf("\tsliced GEMM %s  M=%lld N=%lld K=%lld  %.3f ms\n", spec.c_str(), (long long)M, (long long)N,
-                      (long long)K, c.stats.sliced_gemm_ms - t0);
-      }
+  if (tensor && views) {
+    if (!c.force_fp64) done = mixed_gemm(c, M, N, K, ga, av, bv, gb, ct.p, sCm, sCn);
+    if (!done && !small_out) {
+      const double t0 = c.stats.sliced_gemm_ms;
+      done = sliced_gemm(c, M, N, K, ga, av, bv, gb, ct.p, sCm, sCn);
+      if (done && c.opt.print >= 3)  // PRINT >= 3: every sliced FP64 GEMM with its shape and time
+        std::printf("\tsliced GEMM %s  M=%lld N=%lld K=%lld  %.3f ms\n", spec.c_str(), (long long)M, (long long)N,
+                    (long long)K, c.stats.sliced_gemm_ms - t0);
     }
+  }
+  if (!done && views) {  // declined there, or FP64: the same operands in place
+    // PRINT >= 3 in the MIXED form: the FP64 (DFMA) GEMMs that remain, with their shapes
+    if (c.opt.print >= 3 && mixed && 2.0 * M * N * K >= 1e9)
+      std::printf("\tFP64 GEMM %s  M=%lld N=%lld K=%lld\n", spec.c_str(), (long long)M, (long long)N, (long long)K);
+    if (c2) {
+      dgemm_view(c, alpha, av, bv, beta, C.p, epi);
+      return;
+    }
+    GemmEpilogue e;
+    e.s_mhi = sCm;
+    e.s_n = sCn;
+    dgemm_view(c, ga, av, bv, gb, ct.p, e);
+    done = true;
   }
   Tensor a = A, b = B;
   int64_t sAm = 1, sAk = 1, sBk = 1, sBn = 1;
@@ -576,7 +628,7 @@ void contract(Ctx& c, const std::string& spec, double alpha, const Tensor& A, co
     done = mixed_gemm(c, M, N, K, ga, a.p, sAm, sAk, b.p, sBk, sBn, gb, ct.p, sCm, sCn);
   // the FP64 work of the MIXED form (refinement sweeps, one-shot builds): sliced operands
   // on the tensor cores, FP64-accurate
-  if (!done && c.opt.precision == UCC_MIXED && !recorder() && !small_out) {
+  if (!done && tensor && !small_out) {
     const double t0 = c.stats.sliced_gemm_ms;
     done = sliced_gemm(c, M, N, K, ga, a.p, sAm, sAk, b.p, sBk, sBn, gb, ct.p, sCm, sCn);
     if (done && c.opt.print >= 3)  // PRINT >= 3: every sliced FP64 GEMM with its shape and time
@@ -584,14 +636,13 @@ void contract(Ctx& c, const std::string& spec, double alpha, const Tensor& A, co
                   (long long)K, c.stats.sliced_gemm_ms - t0);
   }
   if (!done) {
-    GemmEpilogue epi;
-    epi.msplit = 0;
-    epi.s_mhi = sCm;
-    epi.s_n = sCn;
+    GemmEpilogue e;
+    e.s_mhi = sCm;
+    e.s_n = sCn;
     // PRINT >= 3 in the MIXED form: the FP64 (DFMA) GEMMs that remain, with their shapes
     if (c.opt.print >= 3 && c.opt.precision == UCC_MIXED && 2.0 * M * N * K >= 1e9)
       std::printf("\tFP64 GEMM %s  M=%lld N=%lld K=%lld\n", spec.c_str(), (long long)M, (long long)N, (long long)K);
-    dgemm_strided(c, M, N, K, ga, a.p, sAm, sAk, b.p, sBk, sBn, gb, ct.p, epi, 1, 0, 0, 0, nullptr);
+    dgemm_strided(c, M, N, K, ga, a.p, sAm, sAk, b.p, sBk, sBn, gb, ct.p, e, 1, 0, 0, 0, nullptr);
   }
   if (!cdirect) {
     // ct is laid out (bm, bn); view it with C's label order and accumulate

@@ -22,6 +22,8 @@ Tensor view(const Tensor& T, const std::string& spec);
 
 // Full contraction sum A[a] B[a] (same labels, any layouts), result on the host.
 double dot_all(Ctx& c, const Tensor& A, const Tensor& B);
+// The same into a list whose values are read together; its index there.
+int dot_all(Ctx& c, const Tensor& A, const Tensor& B, DotList& list);
 
 // Dense scratch tensor (stream-ordered allocation freed when the holder dies).
 struct Temp {

@@ -365,11 +365,17 @@ void fill(Ctx& c, int64_t n, double v, double* y) {
 }
 
 // ------------------------------------------------------------------------------------
-// Compensated reductions.  Pass 1: each block writes (sum, compensation) of its
-// grid-stride share; pass 2: one block folds the partials.  Fixed grid => deterministic.
+// Compensated reductions in one launch: each block writes the sum of its grid-stride share,
+// and the last block to arrive (a ticket) folds the blocks' sums in their order.  The grid
+// depends on n alone, so a result does not depend on the order in which blocks ran.  A second
+// launch for the fold cost 2-3 us, as much as the first one on the small solves' vectors.
 // ------------------------------------------------------------------------------------
 namespace {
 constexpr int RED_BLOCKS = 512, RED_THREADS = 256;
+// blocks of a reduction over n elements: about eight elements per thread, RED_BLOCKS at most
+unsigned red_blocks(int64_t n) {
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + 8 * RED_THREADS - 1) / (8 * RED_THREADS), RED_BLOCKS));
+}
 
 __device__ inline void neumaier(double& s, double& c, double x) {
   const double t = s + x;
@@ -394,21 +400,41 @@ __device__ double block_sum(double v) {
   return v;
 }
 
-// partial[(vec * gridDim.x + block)] ; x may be indexed per vector via xs
-__global__ void dot_pass1(int64_t n, const double* const* xs, const double* x0, const double* y, double* partial) {
-  const double* x = xs ? xs[blockIdx.y] : x0;
+// out = the sum over the gridDim.x blocks of tot (thread 0's value); the ticket goes back to 0
+__device__ void fold_blocks(double tot, double* partial, unsigned int* ticket, double* out) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = tot;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double s = 0.0, cc = 0.0;
+  for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) neumaier(s, cc, __ldcg(partial + i));
+  const double all = block_sum(s + cc);
+  if (threadIdx.x == 0) {
+    *out = all;
+    *ticket = 0u;
+  }
+}
+
+// sum x y, or sum x (y null)
+__global__ void dot_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ y, double* partial,
+                           unsigned int* ticket, double* out) {
   double s = 0.0, cc = 0.0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     neumaier(s, cc, y ? x[i] * y[i] : x[i]);
-  const double tot = block_sum(s + cc);
-  if (threadIdx.x == 0) partial[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = tot;
+  fold_blocks(block_sum(s + cc), partial, ticket, out);
 }
 
 // The DIIS overlaps: one FMA per element per thread (a thread's share is ~n / 131072
 // terms), the block and cross-block folds as above.  The compensated per-element form
 // costs about six FP64 operations per element and bounded this kernel on GB300's FP64
 // pipe; the overlaps only feed the extrapolation coefficients.
-__global__ void multidot_pass1(int64_t n, const double* const* xs, const double* y, double* partial) {
+__global__ void multidot_kernel(int64_t n, const double* const* xs, const double* __restrict__ y, double* partial,
+                                unsigned int* tickets, double* out) {
   const double* __restrict__ x = xs[blockIdx.y];
   double s0 = 0.0, s1 = 0.0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -418,26 +444,15 @@ __global__ void multidot_pass1(int64_t n, const double* const* xs, const double*
     s1 = fma(x[i + stride], y[i + stride], s1);
   }
   if (i < n) s0 = fma(x[i], y[i], s0);
-  const double tot = block_sum(s0 + s1);
-  if (threadIdx.x == 0) partial[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = tot;
-}
-
-__global__ void sum_pass2(int nparts, const double* partial, double* out) {
-  // one block per output
-  const double* p = partial + (int64_t)blockIdx.x * nparts;
-  double s = 0.0, cc = 0.0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) neumaier(s, cc, p[i]);
-  const double tot = block_sum(s + cc);
-  if (threadIdx.x == 0) out[blockIdx.x] = tot;
+  fold_blocks(block_sum(s0 + s1), partial + (int64_t)blockIdx.y * gridDim.x, tickets + blockIdx.y, out + blockIdx.y);
 }
 }  // namespace
 
 void dot_async(Ctx& c, int64_t n, const double* x, const double* y, double* d_out) {
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
-  Scratch part(c, sizeof(double) * RED_BLOCKS);
-  dot_pass1<<<dim3(RED_BLOCKS, 1), RED_THREADS, 0, c.stream>>>(n, nullptr, x, y, part.d());
-  sum_pass2<<<1, RED_THREADS, 0, c.stream>>>(RED_BLOCKS, part.d(), d_out);
-  count_launch();
+  const unsigned nb = red_blocks(n);
+  Scratch part(c, sizeof(double) * nb);
+  dot_kernel<<<nb, RED_THREADS, 0, c.stream>>>(n, x, y, part.d(), &c.words()->reduce, d_out);
   count_launch();
   check_launch("dot");
 }
@@ -454,10 +469,9 @@ double dot(Ctx& c, int64_t n, const double* x, const double* y) {
 void multidot_async(Ctx& c, int nvec, const double* const* d_xs, const double* y, int64_t n, double* d_out) {
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
   if (nvec <= 0) return;
-  Scratch part(c, sizeof(double) * RED_BLOCKS * nvec);
-  multidot_pass1<<<dim3(RED_BLOCKS, nvec), RED_THREADS, 0, c.stream>>>(n, d_xs, y, part.d());
-  sum_pass2<<<nvec, RED_THREADS, 0, c.stream>>>(RED_BLOCKS, part.d(), d_out);
-  count_launch();
+  const unsigned nb = red_blocks(n);
+  Scratch part(c, sizeof(double) * nb * nvec);
+  multidot_kernel<<<dim3(nb, nvec), RED_THREADS, 0, c.stream>>>(n, d_xs, y, part.d(), c.words()->tickets, d_out);
   count_launch();
   check_launch("multidot");
 }
@@ -490,7 +504,7 @@ __global__ void tau_kernel(int no, int nv, const double* t1, const double* t2, d
 template <class I>
 __global__ void jacobi_kernel(int no, int nv, const double* d_do, const double* d_dv, double shift, const double* R1,
                               const double* R2, const double* t1o, const double* t2o, double* t1n, double* t2n,
-                              double* partial) {
+                              double* partial, unsigned int* ticket, double* sumsq) {
   const I n1 = (I)no * nv, n2 = (I)no * no * nv * nv, v = (I)nv, o = (I)no;
   double s = 0.0;
   for (I x = (I)blockIdx.x * blockDim.x + threadIdx.x; x < n1 + n2; x += (I)gridDim.x * blockDim.x) {
@@ -513,8 +527,7 @@ __global__ void jacobi_kernel(int no, int nv, const double* d_do, const double* 
       t2n[y] = t2o[y] + r / (D + shift);
     }
   }
-  const double tot = block_sum(s);
-  if (threadIdx.x == 0) partial[blockIdx.x] = tot;
+  fold_blocks(block_sum(s), partial, ticket, sumsq);
 }
 
 __global__ void lincomb_kernel(int nvec, const double* const* vecs, const double* coef, int64_t n, double* out) {
@@ -542,16 +555,16 @@ void jacobi_update(Ctx& c, int no, int nv, const double* d_do, const double* d_d
                    const double* R2, const double* t1old, const double* t2old, double* t1new, double* t2new,
                    double* d_sumsq) {
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
-  Scratch part(c, sizeof(double) * RED_BLOCKS);
   const int64_t n = (int64_t)no * nv + (int64_t)no * no * nv * nv;
+  const unsigned nb = red_blocks(n);
+  Scratch part(c, sizeof(double) * nb);
+  unsigned int* ticket = &c.words()->reduce;
   if (n + (int64_t)RED_BLOCKS * RED_THREADS < ((int64_t)1 << 31))
-    jacobi_kernel<uint32_t><<<RED_BLOCKS, RED_THREADS, 0, c.stream>>>(no, nv, d_do, d_dv, shift, R1, R2, t1old, t2old,
-                                                                      t1new, t2new, part.d());
+    jacobi_kernel<uint32_t><<<nb, RED_THREADS, 0, c.stream>>>(no, nv, d_do, d_dv, shift, R1, R2, t1old, t2old, t1new,
+                                                              t2new, part.d(), ticket, d_sumsq);
   else
-    jacobi_kernel<int64_t><<<RED_BLOCKS, RED_THREADS, 0, c.stream>>>(no, nv, d_do, d_dv, shift, R1, R2, t1old, t2old,
-                                                                     t1new, t2new, part.d());
-  sum_pass2<<<1, RED_THREADS, 0, c.stream>>>(RED_BLOCKS, part.d(), d_sumsq);
-  count_launch();
+    jacobi_kernel<int64_t><<<nb, RED_THREADS, 0, c.stream>>>(no, nv, d_do, d_dv, shift, R1, R2, t1old, t2old, t1new,
+                                                             t2new, part.d(), ticket, d_sumsq);
   count_launch();
   check_launch("jacobi");
 }
@@ -1069,8 +1082,9 @@ void dgemv_strided(Ctx& c, int64_t N, int64_t K, double alpha, const double* x, 
   if (Recorder* r = recorder()) {  // a GEMM with one row
     RecordedOp o;
     o.kind = RecordedOp::kGemm;
-    o.M = 1, o.N = N, o.K = K, o.sAm = 0, o.sAk = sx, o.sBk = sk, o.sBn = sn, o.sCm = 0, o.sCn = sy;
-    o.A = x, o.B = A, o.C = y, o.alpha = alpha, o.beta = beta;
+    o.A = MatView::strided(x, 1, K, 0, sx), o.B = MatView::strided(A, N, K, sn, sk);
+    o.epi.s_n = sy;
+    o.C = y, o.alpha = alpha, o.beta = beta;
     r->ops.push_back(o);
     return;
   }
