@@ -55,8 +55,11 @@ inline int cluster_m(int mtiles) { return mtiles >= 2 ? 2 : 1; }
 constexpr size_t GEMM_RING = 216 * 1024;
 constexpr size_t GEMM_SMEM_BYTES = 1024 + GEMM_RING + 256;
 // instruction descriptor, kind::f16: D f32 (bit 4), A bf16 (bits 7-9 = 1), B bf16
-// (bits 10-12 = 1), both K-major, N>>3 at bits 17-22, M>>4 at bits 24-28
-constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+// (bits 10-12 = 1), both K-major, N>>3 at bits 17-22, M>>4 at bits 24-28; the CTAs of a pair
+// work on M = 256 rows together
+__device__ __forceinline__ uint32_t idesc_of(int cm, int bn) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(cm * BM >> 4) << 24);
+}
 
 struct Params {
   int M, N, kblocks, mtiles, ntiles;
@@ -126,11 +129,6 @@ __device__ __forceinline__ void seg_parts(int nparts, int seg, int& pa, int& pb)
   }
 }
 
-__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-      "l"(a), "l"(b), "r"(IDESC), "r"(acc));
-}
 // N tiles per raster band: the tiles of one problem run band by band, and inside a band M
 // group by M group with the band's N tiles fastest, so that the ~150 tiles in flight at a
 // time cover about a dozen M groups x RASTER_N N tiles: each A tile is then read by
@@ -165,11 +163,18 @@ __device__ __forceinline__ void tile_coords(const Params& p, int mgroups, int ti
   }
 }
 
-// CM CTAs per cluster along M (1 or 2).  With CM = 2 the two CTAs of a cluster take M tiles
-// 2j and 2j+1 of the same N tile: each loads half of the B tile's rows and multicasts it
-// into both CTAs' rings (the B tensor maps have boxes of bn / 2 rows), so every B byte
-// crosses from L2 once per pair; a ring stage is refilled only after the MMAs of both CTAs
-// released it (each MMA commit arrives on the stage's empty barrier in both CTAs).
+// CM CTAs per cluster along M (1 or 2).  With CM = 2 the two CTAs of a cluster work as a pair
+// (cta_group::2) on M tiles 2j and 2j+1 of one N tile: each CTA's ring holds its own 128 rows
+// of A and half of the B tile's rows (the B tensor maps have boxes of bn / 2 rows), rank 0
+// issues MMAs of 256 rows that read both rings, and each CTA's tensor memory gets its own
+// 128 rows of the result.  Rank 0's full barriers count the bytes of both CTAs' loads, its
+// MMA commits arrive on the empty and accumulator barriers of both, and both epilogues
+// release an accumulator on rank 0's barrier.
+//
+// What bounds it is the shared-memory port (128 bytes per SM clock), which TMA writes and
+// operand reads share: a 128 x 256 x 16 MMA (128 clocks) reads 12 KB, and filling the ring
+// with a whole B tile per CTA adds 96 KB per three products of a K block (1536 clocks), 160
+// bytes per clock together; as a pair it is 8 KB and 64 KB, 106 bytes.
 template <int CM>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap mAhi, const __grid_constant__ CUtensorMap mAlo,
@@ -189,39 +194,34 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int nst = p.fused ? p.nst : STAGES;  // ring stages (at most STAGES)
   const int rank = CM > 1 ? (int)cluster_rank() : 0;
-  constexpr uint16_t kMask = (uint16_t)((1u << CM) - 1u);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], CM);  // released by the MMAs of every CTA that reads the multicast B
+      mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; a++) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 128);
+      mbar_init(&tempty[a], 128 * CM);  // the epilogues of both CTAs, on rank 0's barrier
     }
     mbar_init(mdone, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                 "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  if (warp == 1) tmem_alloc<CM>(tslot, TMEM_COLS);
   fence_before();
   __syncthreads();
   fence_after();
-  if (CM > 1) cluster_sync();  // the peer's barriers exist before its multicasts or arrivals reach them
+  if (CM > 1) cluster_sync();  // the peer's barriers exist before loads, commits or arrivals reach them
   const uint32_t tmem = *tslot;
   // M tiles in groups of CM (one per CTA of the cluster); the clusters walk the groups
   const int mgroups = (p.mtiles + CM - 1) / CM;
   const int tiles_per = mgroups * p.ntiles;
   const int ntile = tiles_per * (p.nprob ? p.nprob : (p.ksplit > 1 ? p.ksplit : 1));
   const int cid = blockIdx.x / CM, ncl = gridDim.x / CM;
-  const int bh = p.bn / CM;  // B rows this CTA loads (for every CTA of the cluster)
+  const int bh = p.bn / CM;  // B rows this CTA loads
   // ring items per K block and term: one fused stage, or one stage per split product
   const int nseg = p.fused ? 1 : (p.nparts == 3 ? 6 : 3);
-  const uint32_t b_tile = (uint32_t)(p.bn * BK * 2);
+  const uint32_t b_tile = (uint32_t)(bh * BK * 2);
   // K chunks of one tile (in-kernel chunking) and the K blocks of chunk ch
   const int nch = p.kc > 0 ? (p.kblocks + p.kc - 1) / p.kc : 1;
 
@@ -255,29 +255,30 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             const int term = kb / (nseg * kn), w = kb - term * nseg * kn;
             const int seg = w / kn, kk = (k0 + w - seg * kn) * BK;
-            // this CTA's share of the B tile (all of it when CM = 1) goes to every CTA of the cluster
-            auto load_b = [&](uint8_t* dst, const CUtensorMap* map, int row) {
+            // rank 0 counts the bytes of the pair's loads
+            const uint32_t fbar = CM > 1 ? map_rank(&full[stage], 0) : 0u;
+            auto load = [&](uint8_t* dst, const CUtensorMap* map, int row) {
               if (CM == 1)
                 tma_load(dst, map, &full[stage], kk, row);
               else
-                tma_load_mc(dst + (size_t)rank * bh * BK * 2, map, &full[stage], kk, row, kMask);
+                tma_load_pair(dst, map, fbar, kk, row);
             };
             if (p.fused) {  // A_hi | A_lo | B_hi | B_lo of K block kk
               uint8_t* st = smem + (size_t)stage * p.stage_bytes;
-              mbar_expect_tx(&full[stage], (uint32_t)(2 * A_BYTES) + 2 * b_tile);
-              tma_load(st, term == 0 ? &mAhi : &mA2hi, &full[stage], kk, term == 0 ? ar0 : ar1);
-              tma_load(st + A_BYTES, term == 0 ? &mAlo : &mA2lo, &full[stage], kk, term == 0 ? ar0 : ar1);
-              load_b(st + 2 * A_BYTES, &mBhi, term == 0 ? br0 : br1);
-              load_b(st + 2 * A_BYTES + b_tile, &mBlo, term == 0 ? br0 : br1);
+              if (rank == 0) mbar_expect_tx(&full[stage], CM * ((uint32_t)(2 * A_BYTES) + 2 * b_tile));
+              load(st, term == 0 ? &mAhi : &mA2hi, term == 0 ? ar0 : ar1);
+              load(st + A_BYTES, term == 0 ? &mAlo : &mA2lo, term == 0 ? ar0 : ar1);
+              load(st + 2 * A_BYTES, &mBhi, term == 0 ? br0 : br1);
+              load(st + 2 * A_BYTES + b_tile, &mBlo, term == 0 ? br0 : br1);
             } else {
               int pa, pbp;
               seg_parts(p.nparts, seg, pa, pbp);
               const CUtensorMap* ma = term == 0 ? (pa == 0 ? &mAhi : (pa == 1 && p.nparts == 3) ? &mAmid : &mAlo)
                                                 : (pa == 0 ? &mA2hi : &mA2lo);
               const CUtensorMap* mb = pbp == 0 ? &mBhi : (pbp == 1 && p.nparts == 3) ? &mBmid : &mBlo;
-              mbar_expect_tx(&full[stage], (uint32_t)A_BYTES + b_tile);
-              tma_load(sA + stage * A_BYTES, ma, &full[stage], kk, term == 0 ? ar0 : ar1);
-              load_b(sB + stage * B_BYTES, mb, term == 0 ? br0 : br1);
+              if (rank == 0) mbar_expect_tx(&full[stage], CM * ((uint32_t)A_BYTES + b_tile));
+              load(sA + stage * A_BYTES, ma, term == 0 ? ar0 : ar1);
+              load(sB + stage * B_BYTES, mb, term == 0 ? br0 : br1);
             }
             ++issued;
             if (++stage == nst) {
@@ -288,17 +289,20 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
       }
       // the last ring loads must have landed before the CTA may exit (matters only on an
-      // error path; normally the epilogue's final wait already implies it)
-      for (int64_t n = issued > nst ? issued - nst : 0; n < issued; n++)
-        mbar_wait_deadline(&full[n % nst], (uint32_t)((n / nst) & 1));
+      // error path; normally the epilogue's final wait already implies it); rank 0's barriers
+      // see the loads of both, and the cluster leaves together
+      if (rank == 0)
+        for (int64_t n = issued > nst ? issued - nst : 0; n < issued; n++)
+          mbar_wait_deadline(&full[n % nst], (uint32_t)((n / nst) & 1));
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && rank != 0) {
+      mbar_wait_deadline(mdone, 0);  // rank 0 issues the pair's MMAs
+    } else if (lane == 0) {
       int stage = 0, acc = 0;
       uint32_t phase = 0, aphase = 0;
       bool ok = true;
-      const uint32_t idesc =
-          (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint32_t idesc = idesc_of(CM, p.bn);
       for (int tile = cid; tile < ntile && ok; tile += ncl) {
         for (int ch = 0; ch < nch && ok; ch++) {
           int kn = p.kblocks;
@@ -327,24 +331,21 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint64_t ad = pr == 2 ? alo : ahi, bd = pr == 1 ? blo : bhi;
 #pragma unroll
                 for (int k = 0; k < BK / 16; k++)
-                  mma_i(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb | pr | k) != 0);
+                  mma_i<CM>(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb | pr | k) != 0);
               }
             } else {
               const uint64_t ad = sdesc(sA + stage * A_BYTES), bd = sdesc(sB + stage * B_BYTES);
 #pragma unroll
               for (int k = 0; k < BK / 16; k++)  // +32 bytes along K per 16-element step
-                mma_i(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+                mma_i<CM>(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb | k) != 0);
             }
-            if (CM == 1)
-              mma_commit(&empty[stage]);
-            else
-              mma_commit_mc(&empty[stage], kMask);  // the stage is free here and in the peer
+            mma_commit<CM>(&empty[stage]);
             if (++stage == nst) {
               stage = 0;
               phase ^= 1u;
             }
           }
-          mma_commit(&tfull[acc]);
+          mma_commit<CM>(&tfull[acc]);
           if (++acc == 2) {
             acc = 0;
             aphase ^= 1u;
@@ -353,7 +354,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       // on an error path the loop may end with MMAs still running: wait for all of them
       // before the CTA releases tensor memory
-      mma_commit(mdone);
+      mma_commit<CM>(mdone);
       mbar_wait_deadline(mdone, 0);
     }
   } else {
@@ -469,7 +470,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         }
       }
       fence_before();
-      mbar_arrive(&tempty[acc]);
+      if (CM == 1)
+        mbar_arrive(&tempty[acc]);
+      else
+        mbar_arrive_cluster(map_rank(&tempty[acc], 0));
       if (++acc == 2) {
         acc = 0;
         aphase ^= 1u;
@@ -478,11 +482,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
   fence_before();
   __syncthreads();
-  // no CTA leaves while its peer may still multicast into its ring or arrive on its barriers
+  // no CTA leaves while MMAs may still read its ring or its peer arrive on its barriers
   if (CM > 1) cluster_sync();
   if (warp == 1) {
     fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    tmem_dealloc<CM>(tmem, TMEM_COLS);
   }
 }
 
@@ -560,46 +564,46 @@ __device__ __forceinline__ double pow2i(int e) {  // 2^e for -1022 <= e <= 1023
   return __longlong_as_double((long long)(e + 1023) << 52);
 }
 
+// ring stages of the sliced kernel, of A_BYTES + B_BYTES / cm each
+constexpr int sliced_stages(int cm) { return cm == 2 ? 6 : STAGES; }
+static_assert(6 * (A_BYTES + B_BYTES / 2) <= STAGES * (A_BYTES + B_BYTES), "the pair's ring fits the same space");
 // shared memory of the sliced kernel: the operand ring, barriers, and a 32 x 33 FP32
 // transpose buffer per epilogue warp
 constexpr size_t SLICED_SMEM_BYTES = SMEM_BYTES + 4 * 32 * 33 * sizeof(float);
 
-// CM = 2: as gemm_kernel<2>, the two CTAs of a cluster take neighbouring M tiles and each
-// multicasts half of every B slice tile into both rings.
+// CM = 2: as gemm_kernel<2>, the two CTAs of a cluster work as a pair on neighbouring M tiles,
+// each with its own A rows and half of every B slice tile in its ring.  Every slice product of
+// a K block is its own ring item, so the shared-memory port sees 96 bytes of fill and 96 of
+// operand reads per clock without the pair (two thirds of the MMA rate at best) and 64 and 64
+// as a pair; half tiles of B also leave room for six stages instead of four.
 template <int CM>
 __global__ void __launch_bounds__(THREADS, 1)
     sliced_gemm_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, SParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA = smem;
-  uint8_t* sB = smem + STAGES * A_BYTES;
-  uint64_t* full = (uint64_t*)(sB + STAGES * B_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* tfull = empty + STAGES;
+  uint64_t* full = (uint64_t*)(smem + STAGES * (A_BYTES + B_BYTES));
+  uint64_t* empty = full + sliced_stages(2);
+  uint64_t* tfull = empty + sliced_stages(2);
   uint64_t* tempty = tfull + 2;
   uint64_t* mdone = tempty + 2;  // every MMA of this CTA has completed (before TMEM is released)
   uint32_t* tslot = (uint32_t*)(mdone + 1);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int rank = CM > 1 ? (int)cluster_rank() : 0;
-  constexpr uint16_t kMask = (uint16_t)((1u << CM) - 1u);
+  constexpr int NST = sliced_stages(CM), STAGE = A_BYTES + B_BYTES / CM;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; s++) {
+    for (int s = 0; s < NST; s++) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], CM);
+      mbar_init(&empty[s], 1);
     }
     for (int a = 0; a < 2; a++) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 128);
+      mbar_init(&tempty[a], 128 * CM);
     }
     mbar_init(mdone, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                 "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
+  if (warp == 1) tmem_alloc<CM>(tslot, TMEM_COLS);
   fence_before();
   __syncthreads();
   fence_after();
@@ -642,31 +646,37 @@ __global__ void __launch_bounds__(THREADS, 1)
                   ok = false;
                   break;
                 }
-                mbar_expect_tx(&full[stage], (uint32_t)(A_BYTES + p.bn * BK * 2));
-                tma_load(sA + stage * A_BYTES, &mA, &full[stage], kb * BK, s * p.a_rows + m0);
-                if (CM == 1)
-                  tma_load(sB + stage * B_BYTES, &mB, &full[stage], kb * BK, (g - s) * p.b_rows + n0);
-                else
-                  tma_load_mc(sB + stage * B_BYTES + (size_t)rank * bh * BK * 2, &mB, &full[stage], kb * BK,
-                              (g - s) * p.b_rows + n0, kMask);
+                uint8_t* st = smem + (size_t)stage * STAGE;
+                const int arow = s * p.a_rows + m0, brow = (g - s) * p.b_rows + n0;
+                if (rank == 0) mbar_expect_tx(&full[stage], (uint32_t)(CM * A_BYTES + p.bn * BK * 2));
+                if (CM == 1) {
+                  tma_load(st, &mA, &full[stage], kb * BK, arow);
+                  tma_load(st + A_BYTES, &mB, &full[stage], kb * BK, brow);
+                } else {
+                  const uint32_t fbar = map_rank(&full[stage], 0);
+                  tma_load_pair(st, &mA, fbar, kb * BK, arow);
+                  tma_load_pair(st + A_BYTES, &mB, fbar, kb * BK, brow);
+                }
                 ++issued;
-                if (++stage == STAGES) {
+                if (++stage == NST) {
                   stage = 0;
                   phase ^= 1u;
                 }
               }
         }
       }
-      for (int64_t n = issued > STAGES ? issued - STAGES : 0; n < issued; n++)
-        mbar_wait_deadline(&full[n % STAGES], (uint32_t)((n / STAGES) & 1));
+      if (rank == 0)
+        for (int64_t n = issued > NST ? issued - NST : 0; n < issued; n++)
+          mbar_wait_deadline(&full[n % NST], (uint32_t)((n / NST) & 1));
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && rank != 0) {
+      mbar_wait_deadline(mdone, 0);
+    } else if (lane == 0) {
       int stage = 0, acc = 0;
       uint32_t phase = 0, aphase = 0;
       bool ok = true;
-      const uint32_t idesc =
-          (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      const uint32_t idesc = idesc_of(CM, p.bn);
       for (int tile = cid; tile < ntile && ok; tile += ncl) {
         int k0, kn;
         krange(tile, k0, kn);
@@ -685,27 +695,25 @@ __global__ void __launch_bounds__(THREADS, 1)
               break;
             }
             fence_after();
-            const uint64_t ad = sdesc(sA + stage * A_BYTES), bd = sdesc(sB + stage * B_BYTES);
+            const uint8_t* st = smem + (size_t)stage * STAGE;
+            const uint64_t ad = sdesc(st), bd = sdesc(st + A_BYTES);
 #pragma unroll
             for (int k = 0; k < BK / 16; k++)
-              mma_i(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb | k) != 0);
-            if (CM == 1)
-              mma_commit(&empty[stage]);
-            else
-              mma_commit_mc(&empty[stage], kMask);
-            if (++stage == STAGES) {
+              mma_i<CM>(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc, (kb | k) != 0);
+            mma_commit<CM>(&empty[stage]);
+            if (++stage == NST) {
               stage = 0;
               phase ^= 1u;
             }
           }
-          mma_commit(&tfull[acc]);
+          mma_commit<CM>(&tfull[acc]);
           if (++acc == 2) {
             acc = 0;
             aphase ^= 1u;
           }
         }
       }
-      mma_commit(mdone);  // as in gemm_kernel: no MMA in flight when TMEM is released
+      mma_commit<CM>(mdone);  // as in gemm_kernel: no MMA in flight when TMEM is released
       mbar_wait_deadline(mdone, 0);
     }
   } else {
@@ -801,7 +809,10 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
         }
         fence_before();
-        mbar_arrive(&tempty[acc]);
+        if (CM == 1)
+          mbar_arrive(&tempty[acc]);
+        else
+          mbar_arrive_cluster(map_rank(&tempty[acc], 0));
         if (++acc == 2) {
           acc = 0;
           aphase ^= 1u;
@@ -814,7 +825,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (CM > 1) cluster_sync();  // the peer no longer multicasts into this ring
   if (warp == 1) {
     fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    tmem_dealloc<CM>(tmem, TMEM_COLS);
   }
 }
 
@@ -1471,9 +1482,9 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
 
 namespace tc {
 // ring layout of a two-part launch: fused stages (A_hi | A_lo | B_hi | B_lo), as many as fit
-static void set_fused(Params& p, bool fused) {
+static void set_fused(Params& p, bool fused, int cm) {
   p.fused = fused ? 1 : 0;
-  p.stage_bytes = 2 * A_BYTES + 2 * p.bn * BK * 2;
+  p.stage_bytes = 2 * A_BYTES + 2 * p.bn * BK * 2 / cm;
   p.nst = fused ? (int)std::min<size_t>(STAGES, GEMM_RING / (size_t)p.stage_bytes) : STAGES;
 }
 
@@ -1596,7 +1607,7 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
   p.a_row1 = p.b_row1 = nullptr;
   p.C32 = nullptr;
   p.nparts = parts;
-  set_fused(p, parts == 2 && p.kc == 0);
+  set_fused(p, parts == 2 && p.kc == 0, cm);
   launch_gemm(c, k, cm, tiles * p.ksplit, a_hi, a_lo, b_hi, b_lo, a_hi, a_lo, parts == 3 ? a_mid : a_hi,
               parts == 3 ? b_mid : b_hi, p);
   if (part) splitk_reduce(c, M, N, p.ksplit, part->d(), alpha, beta, C, epi);
@@ -1910,7 +1921,7 @@ bool mixed_triples_batch(Ctx& c, int nb, const int* tuples, float* W3, int tblk)
     const int tiles = p.mtiles * p.ntiles * nb;
     p.nparts = 2;
     p.kc = 0;
-    set_fused(p, true);
+    set_fused(p, true, 2);
     launch_gemm(c, k, 2, tiles, T.A.mhi, T.A.mlo, T.B.mhi, T.B.mlo, T.A2.mhi, T.A2.mlo, T.A.mhi, T.B.mhi, p);
   }
   UCC_CUDA(cudaEventRecord(ev1, c.stream));
