@@ -523,6 +523,7 @@ struct SParams {
   const int* eb;
   int* err;
   int ksplit, kchunk;  // split-K into FP64 partials at C + z*M*N (alpha 1, beta 0)
+  int klast;           // sliced_short_kernel: 16-element K steps of the last K block that hold data
 };
 
 struct SUnit {
@@ -826,6 +827,292 @@ __global__ void __launch_bounds__(THREADS, 1)
   if (warp == 1) {
     fence_after();
     tmem_dealloc<CM>(tmem, TMEM_COLS);
+  }
+}
+
+// ------------------------------------------------------------------------------------
+// The same product for a short K (at most kShortK elements): the accumulators of all S orders of
+// a 128 x SN tile stay in tensor memory (at most nine of SN columns), so a K block's slices of
+// both operands are loaded once for all its S (S + 1) / 2 products, and the output is written
+// once, not once per order.  The ring kernel above reads an A and a B tile from L2 for each
+// product and passes over C eight times; at K = 256 the passes (FP64 multiply-adds on a pipe of
+// two per clock, a trip to memory each) took ten times the products' time.
+//
+// An MMA of 128 rows takes 130 to 150 clocks however few columns it has (measured with SN = 32
+// and 64), so one MMA does several slices of B: they lie one after the other in shared memory,
+// 128 SN bytes each, and A slice s times slices t0 .. t1 of B as one operand of (t1 - t0 + 1) SN
+// rows lands in the columns of orders s + t0 .. s + t1, which are neighbours too.  SN = 48 (two
+// groups of 4 and 5 slices, 14 MMAs for 45 products), 32 (8 and 1) or 16 (all nine at once).
+//
+// The epilogue needs no FP64 operation but the add onto an old value: the accumulators are
+// integers below 2^22 in units of 2^-SB(g+2) (K (g+1) 2^10).  A 64-bit integer sum of them, in
+// quarters of the last order but one's unit (2^-56 of the row and column maxima's product at
+// nine digits; below 448 2^54 of those), is turned into a double by its bit fields.  All
+// accumulators of a tile are read and released before C is touched, so the writes overlap the
+// next tile's products.
+//
+// Every slice has its own slot and barriers.  A K block's products run by rows, A slice s with B
+// slices 0 .. S-1-s, from s = S-1 down: A slices free up one by one and are loaded again under
+// the rest.  All B slices are in use until row 0 ends, so the ones that the next K block begins
+// with (all of them where they fit, the first four at SN = 48) have two slots.
+//
+// Measured (kernel alone, nine digits): 8192 x 8192 x 256 1.56 ms (2.81 with one MMA per
+// product), 200000 x 16 x 160 0.14 ms (0.42; 0.56 on the ring kernel); a K block takes 8.7
+// thousand clocks where its 56 MMAs need 7.2.
+// ------------------------------------------------------------------------------------
+constexpr int kShortK = 448, kShortThreads = 64 + 512;
+constexpr int short_double(int sn) { return sn == 48 ? 4 : kSlices; }  // B slices with two slots
+constexpr int short_group(int sn) { return sn == 48 ? 4 : 256 / sn; }  // B slices of the first MMA of a row
+constexpr size_t short_smem(int sn) {
+  return 1024 + (size_t)kSlices * A_BYTES + (size_t)(kSlices + short_double(sn)) * sn * BK * 2 + 768;
+}
+static_assert(short_smem(48) <= 227 * 1024 && short_smem(32) <= 227 * 1024, "nine slices of both operands");
+static_assert((kSlices - short_group(48)) * 48 <= 256, "the second group is one MMA");
+
+// V 2^e as a double (round to nearest, ties away), integer operations only while the result
+// is a normal number
+__device__ __forceinline__ double fixed_to_f64(long long v, int e) {
+  if (v == 0) return 0.0;
+  const unsigned long long u = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  const int lz = __clzll((long long)u);
+  const unsigned long long m = u << lz, sgn = (unsigned long long)v & 0x8000000000000000ull;
+  const unsigned long long mant = (m >> 11) + ((m >> 10) & 1ull);  // 2^52 .. 2^53: adds 1 (or 2) to the exponent
+  const int ex = 1022 + 63 - lz + e;
+  if (ex > 0 && ex < 2045) return __longlong_as_double((long long)(sgn | (((unsigned long long)ex << 52) + mant)));
+  const double d = __longlong_as_double((long long)(sgn | ((1022ull << 52) + mant)));  // times 2^(63 - lz + e)
+  const int h = (63 - lz + e) / 2;
+  return d * pow2i(h) * pow2i(63 - lz + e - h);
+}
+
+template <int SN>
+__global__ void __launch_bounds__(kShortThreads, 1)
+    sliced_short_kernel(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB, SParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  constexpr int kB = SN * BK * 2, DB = short_double(SN), G0 = short_group(SN);
+  constexpr int NBUF = 2 * kSlices * SN <= 512 ? 2 : 1;  // two sets of accumulators where they fit
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + kSlices * A_BYTES;
+  uint64_t* fullA = (uint64_t*)(sB + (kSlices + DB) * kB);
+  uint64_t* fullB = fullA + kSlices;  // by slot: slice t < DB of K block n at t + (n & 1) DB, else DB + t
+  uint64_t* emptyA = fullB + 2 * kSlices;
+  uint64_t* emptyB = emptyA + kSlices;
+  uint64_t* tfull = emptyB + 2 * kSlices;
+  uint64_t* tempty = tfull + 2;
+  uint64_t* mdone = tempty + 2;
+  uint32_t* tslot = (uint32_t*)(mdone + 1);
+  // slot of slice t in the CTA's K block n, and the parity of the slot's use there
+  auto bslot = [](int t, uint32_t n) { return t < DB ? t + (int)(n & 1u) * DB : DB + t; };
+  auto bpar = [](int t, uint32_t n) { return (t < DB ? n >> 1 : n) & 1u; };
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, S = p.S;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kSlices; s++) {
+      mbar_init(&fullA[s], 1);
+      mbar_init(&emptyA[s], 1);
+    }
+    for (int s = 0; s < kSlices + DB; s++) {
+      mbar_init(&fullB[s], 1);
+      mbar_init(&emptyB[s], 1);
+    }
+    for (int a = 0; a < 2; a++) {
+      mbar_init(&tfull[a], 1);
+      mbar_init(&tempty[a], 512);
+    }
+    mbar_init(mdone, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc<1>(tslot, 512);
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const uint32_t tmem = *tslot;
+  const int ntile = p.mtiles * p.ntiles;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t n = 0;  // K blocks of this CTA so far, over all its tiles
+      bool ok = true;
+      int part = 0;    // loads of K block n that were issued (fewer than 2 S only after an error)
+      for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x) {
+        int mt, nt;
+        raster(p.mtiles, p.ntiles, tile, mt, nt);
+        for (int kb = 0; kb < p.kblocks && ok; kb++) {
+          part = 0;
+          for (int i = 0; i < S; i++) {  // A slice S-1-i and B slice i in the order of their first use
+            const int s = S - 1 - i, bs = bslot(i, n);
+            if (!(ok = mbar_wait(&emptyA[s], (n & 1u) ^ 1u, p.err))) break;
+            mbar_expect_tx(&fullA[s], A_BYTES);
+            tma_load(sA + s * A_BYTES, &mA, &fullA[s], kb * BK, s * p.a_rows + mt * BM);
+            part++;
+            if (!(ok = mbar_wait(&emptyB[bs], bpar(i, n) ^ 1u, p.err))) break;
+            mbar_expect_tx(&fullB[bs], (uint32_t)kB);
+            tma_load(sB + bs * kB, &mB, &fullB[bs], kb * BK, i * p.b_rows + nt * SN);
+            part++;
+          }
+          if (ok) n++;
+        }
+      }
+      if (!ok) {
+        // the loads in flight must land before the CTA exits: a slot's last load is that of the
+        // broken K block n (the first `part` of its loads), or the one before it in that slot
+        for (int i = 0; i < S; i++) {
+          const int s = S - 1 - i;
+          const bool a = 2 * i < part, b = 2 * i + 1 < part;
+          if (a || n >= 1) mbar_wait_deadline(&fullA[s], (a ? n : n - 1) & 1u);
+          const uint32_t gap = i < DB ? 2 : 1;  // K blocks between two uses of a B slot
+          if (b || n >= gap) mbar_wait_deadline(&fullB[bslot(i, n)], bpar(i, b ? n : n - gap));
+          if (i < DB && n >= 1) mbar_wait_deadline(&fullB[bslot(i, n - 1)], bpar(i, n - 1));
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      uint32_t n = 0, aphase = 0;
+      int buf = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x) {
+        if (!mbar_wait(&tempty[buf], aphase ^ 1u, p.err)) break;
+        fence_after();
+        const uint32_t d0 = tmem + (uint32_t)(buf * kSlices * SN);
+        for (int kb = 0; kb < p.kblocks && ok; kb++, n++) {
+          const int ksteps = kb == p.kblocks - 1 ? p.klast : BK / 16;
+          for (int s = S - 1; s >= 0; s--) {
+            const int cnt = S - s;  // B slices of this row; order s + t of the tile in columns (s + t) SN
+            if (!(ok = mbar_wait(&fullA[s], n & 1u, p.err) &&
+                       mbar_wait(&fullB[bslot(cnt - 1, n)], bpar(cnt - 1, n), p.err)))
+              break;
+            fence_after();
+            const uint64_t ad = sdesc(sA + s * A_BYTES);
+            for (int t0 = 0; t0 < cnt; t0 += t0 == 0 ? G0 : kSlices) {
+              const int nt = min(cnt - t0, t0 == 0 ? G0 : kSlices);
+              const uint64_t bd = sdesc(sB + bslot(t0, n) * kB);
+              const uint32_t d = d0 + (uint32_t)((s + t0) * SN);
+              for (int k = 0; k < ksteps; k++) {
+                if (kb == 0 && k == 0 && t0 == 0) {  // order s begins here, the later ones have begun
+                  mma_i(d, ad, bd, idesc_of(1, SN), 0u);
+                  if (nt > 1)
+                    mma_i(d + (uint32_t)SN, ad, bd + (uint64_t)(kB >> 4), idesc_of(1, (nt - 1) * SN), 1u);
+                } else {
+                  mma_i(d, ad + (uint64_t)(k * 2), bd + (uint64_t)(k * 2), idesc_of(1, nt * SN), 1u);
+                }
+              }
+              if (s == 0)
+                for (int t = t0; t < t0 + nt; t++) mma_commit(&emptyB[bslot(t, n)]);
+            }
+            mma_commit(&emptyA[s]);
+          }
+        }
+        if (!ok) break;
+        mma_commit(&tfull[buf]);
+        if (++buf == NBUF) {
+          buf = 0;
+          aphase ^= 1u;
+        }
+      }
+      mma_commit(mdone);  // no MMA in flight when TMEM is released
+      mbar_wait_deadline(mdone, 0);
+    }
+  } else {
+    // warps 2 .. 17: the tile's rows of lane quarter q, SN / 4 columns each
+    const int q = warp & 3, part = (warp - 2) / 4, lsb = -SB * S - 2;
+    constexpr int NC = SN / 4;
+    uint32_t aphase = 0;
+    int buf = 0;
+    const GemmEpilogue ep = p.epi;
+    // a power-of-two alpha goes into the exponent
+    const long long ab = __double_as_longlong(p.alpha);
+    const bool apow2 = (ab & 0xFFFFFFFFFFFFFll) == 0;
+    const int aexp = apow2 ? (int)((ab >> 52) & 0x7FF) - 1023 : 0;
+    const bool rows_contiguous = ep.msplit == 0 && ep.s_mhi == 1;
+    for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+      int mt, nt;
+      raster(p.mtiles, p.ntiles, tile, mt, nt);
+      if (!__all_sync(0xffffffffu, mbar_wait(&tfull[buf], aphase, p.err))) break;
+      fence_after();
+      long long v[NC];
+      // n = acc 2^(SB (g + 2)), exact, by adding 1.5 2^23
+      auto whole = [&](uint32_t x, int g) {
+        const float sc = __int_as_float((127 + SB * (g + 2)) << 23);
+        return __float_as_int(fmaf(__uint_as_float(x), sc, 12582912.f)) - 0x4B400000;
+      };
+#pragma unroll
+      for (int c0 = 0; c0 < NC; c0 += 4) {
+        const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * kSlices * SN + part * NC + c0);
+        uint32_t r[kSlices][4];  // by order from the last one, r[0]; orders that fewer digits lack stay unread
+#pragma unroll
+        for (int u = 0; u < kSlices; u++)
+          if (u < S) tmem_ld4(base + (uint32_t)((S - 1 - u) * SN), r[u]);
+        tmem_wait();
+        // orders in pairs from the most significant: w = 2^SB n_hi + n_lo in 32 bits, then 64-bit
+        // sums; the pairs end at the last order but one, then the last in quarters of its unit
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          long long x = 0;
+#pragma unroll
+          for (int u = 8; u >= 2; u -= 2) {
+            int w = 0;
+            if (u < S) w = whole(r[u][j], S - 1 - u) * (1 << SB);
+            if (u - 1 < S) w += whole(r[u - 1][j], S - u);
+            x = u == 8 ? (long long)w : x * (1ll << (2 * SB)) + w;
+          }
+          v[c0 + j] = x * 4 + ((whole(r[0][j], S - 1) + 8) >> 4);
+        }
+      }
+      fence_before();
+      mbar_arrive(&tempty[buf]);
+      if (++buf == NBUF) {
+        buf = 0;
+        aphase ^= 1u;
+      }
+      const int64_t m = (int64_t)mt * BM + q * 32 + lane, n0 = (int64_t)nt * SN + part * NC;
+      if (m < p.M && n0 < p.N) {
+        const int em = p.ea[m] + lsb + aexp;
+        const int ncol = (int)(p.N - n0 < NC ? p.N - n0 : NC);
+        double* Cm = p.C + (ep.msplit ? (m / ep.msplit) * ep.s_mhi + (m % ep.msplit) * ep.s_mlo : m * ep.s_mhi) +
+                     n0 * ep.s_n;
+        auto value = [&](int j) {
+          const double d = fixed_to_f64(v[j], em + p.eb[n0 + j]);
+          return apow2 ? (ab < 0 ? -d : d) : p.alpha * d;
+        };
+        if (!rows_contiguous && ep.s_n == 1 && ncol == NC && ((uintptr_t)Cm & 15) == 0) {
+          double2* C2 = reinterpret_cast<double2*>(Cm);  // a lane's columns are contiguous: 16-byte accesses
+          double2 old[NC / 2];
+          if (p.beta != 0.0) {
+#pragma unroll
+            for (int j = 0; j < NC / 2; j++) old[j] = C2[j];
+          }
+#pragma unroll
+          for (int j = 0; j < NC / 2; j++) {
+            double2 x = make_double2(value(2 * j), value(2 * j + 1));
+            if (p.beta == 1.0) {
+              x.x += old[j].x;
+              x.y += old[j].y;
+            } else if (p.beta != 0.0) {
+              x.x = fma(p.beta, old[j].x, x.x);
+              x.y = fma(p.beta, old[j].y, x.y);
+            }
+            C2[j] = x;
+          }
+        } else {
+          double old[NC];
+#pragma unroll
+          for (int j = 0; j < NC; j++) old[j] = p.beta != 0.0 && j < ncol ? Cm[j * ep.s_n] : 0.0;
+#pragma unroll
+          for (int j = 0; j < NC; j++)
+            if (j < ncol) {
+              const double x = value(j);
+              Cm[j * ep.s_n] = p.beta == 0.0 ? x : p.beta == 1.0 ? old[j] + x : fma(p.beta, old[j], x);
+            }
+        }
+      }
+      __syncwarp();
+    }
+  }
+  fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    fence_after();
+    tmem_dealloc<1>(tmem, 512);
   }
 }
 
@@ -1268,7 +1555,7 @@ static Sliced* slice_prepare(Ctx& c, const MatView& x, int pad_rows, int box_row
   slice_absmax_kernel<<<dim3((unsigned)((cols + kchunk - 1) / kchunk), (unsigned)rblocks), blk, 0, c.stream>>>(
       x, kchunk, static_cast<unsigned long long*>(amax.p));
   count_kernel_launch();
-  slice_digits_kernel<<<dim3((unsigned)(s->kp / 64), (unsigned)(s->rows_p / 32)), blk, 0, c.stream>>>(
+  slice_digits_kernel<<<dim3((unsigned)(s->kp / 64), (unsigned)((s->rows_p + 31) / 32)), blk, 0, c.stream>>>(
       x, s->rows_p, s->kp, static_cast<const unsigned long long*>(amax.p), S, s->d, s->e, k.range);
   count_kernel_launch();
   UCC_CUDA(cudaGetLastError());
@@ -1318,8 +1605,10 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   UCC_REQUIRE(S >= 2 && SB * S <= 56, UCC_BAD_ARGS, "sliced GEMM: 2 to 9 slices");
   const double aa = std::fabs(alpha);
   if (!(aa >= 0x1p-20 && aa <= 0x1p20) || M > INT32_MAX || N > INT32_MAX) return false;
-  // N tile (pick_bn): no more tiles than 256-column ones would need, padded to multiples of 32
-  const int bn = pick_bn(N);
+  // a short K: the kernel that keeps every order in tensor memory (tiles of 48 columns, 32 or 16 for
+  // a thin product); otherwise the ring kernel with N tiles of pick_bn
+  const bool short_k = K <= kShortK;
+  const int bn = short_k ? (N > 32 ? 48 : N > 16 ? 32 : 16) : pick_bn(N);
   Cache& k = cache(c);
   {
     const int64_t Mp = (M + BM - 1) / BM * BM, Np = (N + bn - 1) / bn * bn, kp = (K + BK - 1) / BK * BK;
@@ -1365,7 +1654,7 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   UCC_CUDA(cudaEventRecord(ev0, c.stream));  // the time includes the slicing of non-cached operands
   std::unique_ptr<Sliced> ta, tb;
   // neighbouring M tiles pair up in clusters that share each B slice tile (boxes of bn / 2)
-  const int cm = cluster_m((int)((M + BM - 1) / BM));
+  const int cm = short_k ? 1 : cluster_m((int)((M + BM - 1) / BM));
   Sliced* a = slice_prepare(c, A, BM, BM, S, ta, allow_cache);
   const CUtensorMap amap = a ? a->map : CUtensorMap{};  // copied: A and B may be one cached operand
   Sliced* b = a ? slice_prepare(c, B, bn, bn / cm, S, tb, allow_cache) : nullptr;
@@ -1381,6 +1670,12 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
                                   (int)SLICED_SMEM_BYTES));
     UCC_CUDA(cudaFuncSetAttribute(sliced_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)SLICED_SMEM_BYTES));
+    UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)short_smem(32)));
+    UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)short_smem(16)));
+    UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<48>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)short_smem(48)));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * k.sms);
     cfg.blockDim = dim3(THREADS);
@@ -1417,13 +1712,14 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   p.err = k.err;
   p.ksplit = 1;
   p.kchunk = p.kblocks;
+  p.klast = (int)((K - (int64_t)(p.kblocks - 1) * BK + 15) / 16);
   const int tiles = p.mtiles * p.ntiles;
   std::unique_ptr<Scratch> part;
   // split K when the tiles fill the SMs poorly: the split z (chunks of >= 8 K blocks, FP64
   // partials of at most 2 GB) with the shortest time in waves, ceil(tiles z / SMs) / z,
   // a larger z only for a 5 % gain; fixed-order FP64 reduce
   int ks = 1;
-  {
+  if (!short_k) {
     const int zmax = (int)std::min<int64_t>(std::min<int64_t>(p.kblocks / 8, 256),
                                             std::max<int64_t>(1, 8LL * k.sms / tiles));
     double best = (double)((tiles + k.sms - 1) / k.sms);
@@ -1448,7 +1744,15 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
       p.epi.s_n = 1;
     }
   }
-  if (cm == 1) {
+  if (short_k) {
+    const int grid = std::min(tiles, k.sms);
+    if (bn == 16)
+      sliced_short_kernel<16><<<grid, kShortThreads, short_smem(16), c.stream>>>(amap, bmap, p);
+    else if (bn == 32)
+      sliced_short_kernel<32><<<grid, kShortThreads, short_smem(32), c.stream>>>(amap, bmap, p);
+    else
+      sliced_short_kernel<48><<<grid, kShortThreads, short_smem(48), c.stream>>>(amap, bmap, p);
+  } else if (cm == 1) {
     sliced_gemm_kernel<1><<<std::min(tiles * p.ksplit, k.sms), THREADS, SLICED_SMEM_BYTES, c.stream>>>(amap, bmap,
                                                                                                         p);
   } else {
