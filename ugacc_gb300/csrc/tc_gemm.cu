@@ -1508,18 +1508,18 @@ static Sliced* slice_map(Sliced* s, int box_rows) {
 }
 
 // slice (and cache when the source is a constant block and memory allows) a rows x cols
-// FP64 operand; the slice arrays are padded to whole tiles of pad_rows rows so that no tile
-// reaches into the next slice, and read with boxes of box_rows rows (pad_rows or a half).
+// FP64 operand, the slice arrays padded to 32 rows and read with boxes of box_rows rows (the
+// last tile's box may reach into the next slice: rows or columns that no output uses).
 // A cached operand always holds all kSlices digits: a product with S < kSlices digits reads
 // the leading S of them (they differ from x by less than one unit of digit S-1, like an
 // S-digit split).  nullptr when the slices do not fit in free memory.
-static Sliced* slice_prepare(Ctx& c, const MatView& x, int pad_rows, int box_rows, int S,
-                             std::unique_ptr<Sliced>& temp, bool allow_cache) {
+static Sliced* slice_prepare(Ctx& c, const MatView& x, int box_rows, int S, std::unique_ptr<Sliced>& temp,
+                             bool allow_cache) {
   Cache& k = cache(c);
   bool constant = allow_cache && c.is_constant(x.p);
   const int64_t rows = x.rows, cols = x.cols;
   UCC_REQUIRE(rows < INT32_MAX && cols < INT32_MAX, UCC_BAD_ARGS, "sliced GEMM: operand too large");
-  const Key key = make_key(x, pad_rows, kSlices);
+  const Key key = make_key(x, 0, kSlices);
   if (constant) {
     auto it = k.sliced.find(key);
     if (it != k.sliced.end()) return slice_map(it->second.get(), box_rows);
@@ -1527,7 +1527,7 @@ static Sliced* slice_prepare(Ctx& c, const MatView& x, int pad_rows, int box_row
   }
   auto s = std::make_unique<Sliced>();
   s->rows = rows;
-  s->rows_p = (rows + pad_rows - 1) / pad_rows * pad_rows;
+  s->rows_p = (rows + 31) / 32 * 32;
   s->kp = (cols + BK - 1) / BK * BK;
   s->S = S;
   const size_t nel = (size_t)S * s->rows_p * s->kp;
@@ -1555,7 +1555,7 @@ static Sliced* slice_prepare(Ctx& c, const MatView& x, int pad_rows, int box_row
   slice_absmax_kernel<<<dim3((unsigned)((cols + kchunk - 1) / kchunk), (unsigned)rblocks), blk, 0, c.stream>>>(
       x, kchunk, static_cast<unsigned long long*>(amax.p));
   count_kernel_launch();
-  slice_digits_kernel<<<dim3((unsigned)(s->kp / 64), (unsigned)((s->rows_p + 31) / 32)), blk, 0, c.stream>>>(
+  slice_digits_kernel<<<dim3((unsigned)(s->kp / 64), (unsigned)(s->rows_p / 32)), blk, 0, c.stream>>>(
       x, s->rows_p, s->kp, static_cast<const unsigned long long*>(amax.p), S, s->d, s->e, k.range);
   count_kernel_launch();
   UCC_CUDA(cudaGetLastError());
@@ -1568,6 +1568,84 @@ static Sliced* slice_prepare(Ctx& c, const MatView& x, int pad_rows, int box_row
   return raw;
 }
 
+}  // namespace tc
+
+namespace tc {
+static void set_sliced_attrs(Cache& k) {
+  if (k.sattr_set) return;
+  UCC_CUDA(cudaFuncSetAttribute(sliced_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)SLICED_SMEM_BYTES));
+  UCC_CUDA(cudaFuncSetAttribute(sliced_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)SLICED_SMEM_BYTES));
+  UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)short_smem(32)));
+  UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)short_smem(16)));
+  UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<48>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)short_smem(48)));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * k.sms);
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = SLICED_SMEM_BYTES;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  UCC_CUDA(cudaOccupancyMaxActiveClusters(&n, sliced_gemm_kernel<2>, &cfg));
+  k.max_pairs_sliced = std::max(1, n);
+  k.sattr_set = true;
+}
+
+// The N tile and the K split of a single product: the least of a time model over N tiles of 32 to
+// 256 columns and splits z,
+//   waves * sum over units of max(items t(bn), e(bn)),  waves = ceil(tiles z / slots),
+// with t the time of a ring item (a K block: three products of the split form, one of the
+// sliced) measured at 4864 x 6144 x 2048 on full waves, and e that of an epilogue pass: 33 ns a
+// column for the split form's one (a 64-bit operation per element on two per clock), 120 ns for
+// each of the sliced form's (it reads and writes C again per unit).  z > 1 adds the partial
+// products' way through memory at about 4 TB/s.  An MMA's time hardly falls below 128 columns,
+// so narrow tiles pay only where they fill a wave.  The rule before (the widest tile that wastes
+// no column, the split with the fewest waves) counted neither: 2560^3 ran as z = 3 of
+// 256-column tiles, 228 us split and 2154 us sliced at nine digits; in two waves of 192-column
+// tiles it is 91 and 1272, and 160 x 40960 x 2048 at nine digits 2586 -> 1510.
+struct TilePlan {
+  int bn, z;
+};
+static TilePlan plan_tiles(int64_t M, int64_t N, int kblocks, int cm, int slots, const double (&t)[8], double products,
+                           int units, int min_blocks) {
+  // ring items per K block of unit u: order u of the sliced form, the tail the rest
+  auto unit_items = [&](int u) { return u + 1 < units ? u + 1.0 : products - 0.5 * u * (u + 1); };
+  TilePlan best{256, 1};
+  double best_us = 1e300;
+  const double groups = cm == 2 ? (double)(((M + BM - 1) / BM + 1) / 2) : (double)((M + BM - 1) / BM);
+  for (int bn = 256; bn >= 32; bn -= 32) {
+    const double nt = (double)((N + bn - 1) / bn);
+    if (bn > 32 && N <= bn - 32) continue;  // a whole step of padding
+    static const int zs[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64, 96, 128, 192, 256};
+    for (int z : zs) {
+      if (z > 1 && (kblocks / z < min_blocks || 8.0 * (double)M * N * z > 2e9)) break;
+      const double kb = (double)((kblocks + z - 1) / z), epi = (units > 1 ? 0.12 : 0.033) * bn;
+      const double mb = 8e-6 * (double)M * N;
+      double tile = 0.0;
+      for (int u = 0; u < units; u++) tile += std::max(unit_items(u) * kb * t[bn / 32 - 1], epi);
+      double us = std::ceil(groups * nt * z / slots) * tile + epi;
+      if (units > 1 && mb * z > 100.0) us = std::max(us, mb * z * 2.0 * units / 4.0);
+      if (z > 1) us += 5.0 + mb * ((units > 1 ? 2.0 : 1.0) * z + z + 2.0) / 4.0;
+      if (us < best_us) {
+        best_us = us;
+        best = TilePlan{bn, z};
+      }
+    }
+  }
+  return best;
+}
+// microseconds of a ring item by columns / 32: a fused K block of the split form, a slice product
+constexpr double kSplitItem[8] = {0.56, 0.61, 0.66, 0.79, 0.94, 1.10, 1.28, 1.46};
+constexpr double kSliceItem[8] = {0.269, 0.276, 0.290, 0.306, 0.329, 0.364, 0.406, 0.450};
 }  // namespace tc
 
 // the smallest GEMM the sliced FP64 GEMM takes
@@ -1606,17 +1684,22 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   const double aa = std::fabs(alpha);
   if (!(aa >= 0x1p-20 && aa <= 0x1p20) || M > INT32_MAX || N > INT32_MAX) return false;
   // a short K: the kernel that keeps every order in tensor memory (tiles of 48 columns, 32 or 16 for
-  // a thin product); otherwise the ring kernel with N tiles of pick_bn
+  // a thin product); otherwise the ring kernel with the N tile and K split of plan_tiles
   const bool short_k = K <= kShortK;
-  const int bn = short_k ? (N > 32 ? 48 : N > 16 ? 32 : 16) : pick_bn(N);
   Cache& k = cache(c);
+  set_sliced_attrs(k);
+  // neighbouring M tiles pair up in clusters (boxes of bn / 2 rows of B)
+  const int cm = short_k ? 1 : cluster_m((int)((M + BM - 1) / BM));
+  TilePlan plan{N > 32 ? 48 : N > 16 ? 32 : 16, 1};
+  if (!short_k)
+    plan = plan_tiles(M, N, (int)((K + BK - 1) / BK), cm, cm == 2 ? k.max_pairs_sliced : k.sms, kSliceItem,
+                      0.5 * S * (S + 1), std::max(1, S - 2) + 1, 8);
+  const int bn = plan.bn;
   {
-    const int64_t Mp = (M + BM - 1) / BM * BM, Np = (N + bn - 1) / bn * bn, kp = (K + BK - 1) / BK * BK;
-    auto cached = [&](const MatView& x, int box) {
-      return allow_cache && k.sliced.count(make_key(x, box, kSlices)) != 0;
-    };
-    const double needA = cached(A, BM) ? 0.0 : 2.0 * S * (double)Mp * kp;
-    const double needB = cached(B, bn) ? 0.0 : 2.0 * S * (double)Np * kp;
+    const int64_t Mp = (M + 31) / 32 * 32, Np = (N + 31) / 32 * 32, kp = (K + BK - 1) / BK * BK;
+    auto cached = [&](const MatView& x) { return allow_cache && k.sliced.count(make_key(x, 0, kSlices)) != 0; };
+    const double needA = cached(A) ? 0.0 : 2.0 * S * (double)Mp * kp;
+    const double needB = cached(B) ? 0.0 : 2.0 * S * (double)Np * kp;
     size_t free_b = 0, total_b = 0;
     UCC_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const bool too_big = (double)S * Mp >= 2e9 || (double)S * Np >= 2e9 || Np / 32 > 65535 || Mp / 32 > 65535 ||
@@ -1653,11 +1736,9 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   cudaEvent_t ev0 = c.take_event(), ev1 = c.take_event();
   UCC_CUDA(cudaEventRecord(ev0, c.stream));  // the time includes the slicing of non-cached operands
   std::unique_ptr<Sliced> ta, tb;
-  // neighbouring M tiles pair up in clusters that share each B slice tile (boxes of bn / 2)
-  const int cm = short_k ? 1 : cluster_m((int)((M + BM - 1) / BM));
-  Sliced* a = slice_prepare(c, A, BM, BM, S, ta, allow_cache);
+  Sliced* a = slice_prepare(c, A, BM, S, ta, allow_cache);
   const CUtensorMap amap = a ? a->map : CUtensorMap{};  // copied: A and B may be one cached operand
-  Sliced* b = a ? slice_prepare(c, B, bn, bn / cm, S, tb, allow_cache) : nullptr;
+  Sliced* b = a ? slice_prepare(c, B, bn / cm, S, tb, allow_cache) : nullptr;
   if (!a || !b) {
     c.event_pool.push_back(ev0);
     c.event_pool.push_back(ev1);
@@ -1665,33 +1746,6 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   }
   const CUtensorMap bmap = b->map;
   wrote = true;
-  if (!k.sattr_set) {
-    UCC_CUDA(cudaFuncSetAttribute(sliced_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)SLICED_SMEM_BYTES));
-    UCC_CUDA(cudaFuncSetAttribute(sliced_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)SLICED_SMEM_BYTES));
-    UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)short_smem(32)));
-    UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)short_smem(16)));
-    UCC_CUDA(cudaFuncSetAttribute(sliced_short_kernel<48>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)short_smem(48)));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * k.sms);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = SLICED_SMEM_BYTES;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = 2;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    UCC_CUDA(cudaOccupancyMaxActiveClusters(&n, sliced_gemm_kernel<2>, &cfg));
-    k.max_pairs_sliced = std::max(1, n);
-    k.sattr_set = true;
-  }
   SParams p;
   p.M = (int)M;
   p.N = (int)N;
@@ -1715,22 +1769,8 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   p.klast = (int)((K - (int64_t)(p.kblocks - 1) * BK + 15) / 16);
   const int tiles = p.mtiles * p.ntiles;
   std::unique_ptr<Scratch> part;
-  // split K when the tiles fill the SMs poorly: the split z (chunks of >= 8 K blocks, FP64
-  // partials of at most 2 GB) with the shortest time in waves, ceil(tiles z / SMs) / z,
-  // a larger z only for a 5 % gain; fixed-order FP64 reduce
-  int ks = 1;
-  if (!short_k) {
-    const int zmax = (int)std::min<int64_t>(std::min<int64_t>(p.kblocks / 8, 256),
-                                            std::max<int64_t>(1, 8LL * k.sms / tiles));
-    double best = (double)((tiles + k.sms - 1) / k.sms);
-    for (int z = 2; z <= zmax && 8.0 * M * N * z <= 2e9; z++) {
-      const double t = (double)((tiles * z + k.sms - 1) / k.sms) / z;
-      if (t < 0.95 * best) {
-        best = t;
-        ks = z;
-      }
-    }
-  }
+  // FP64 partial products of the K chunks, added in a fixed order
+  const int ks = plan.z;
   {
     if (ks > 1) {
       p.kchunk = (p.kblocks + ks - 1) / ks;
@@ -1850,9 +1890,15 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
   using namespace tc;
   UCC_REQUIRE(parts == 2 || parts == 3, UCC_BAD_ARGS, "tensor-core GEMM: 2 or 3 split parts");
   Cache& k = cache(c);
+  set_gemm_attrs(k);
   std::unique_ptr<Split> ta, tb;
-  const int bn = pick_bn(N);
   const int cm = cluster_m((int)((M + BM - 1) / BM));
+  // K chunks of one tile summed in FP64 (kc) are not split further
+  const int kblocks = (int)((K + BK - 1) / BK);
+  const bool chunks = kc > 0 && kc < kblocks;
+  const TilePlan plan = plan_tiles(M, N, kblocks, cm, cm == 2 ? k.max_pairs : k.sms, kSplitItem, parts == 2 ? 1.0 : 2.0,
+                                   1, chunks ? kblocks + 1 : 4);
+  const int bn = plan.bn;
   // the maps are copied at once: A and B may be one cached operand read with two boxes
   Split* a = prepare(c, A, BM, ta, parts);
   const CUtensorMap a_hi = a->mhi, a_lo = a->mlo, a_mid = a->mmid;
@@ -1876,23 +1922,11 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
   p.ksplit = 1;
   p.kchunk = p.kblocks;
   const int tiles = p.mtiles * p.ntiles;
-  // tiles that fill the SMs poorly and a long K: split K (chunks of >= 4 K blocks, FP64
-  // partials of at most 2 GB) for the shortest time in waves, ceil(tiles z / SMs) / z, a
-  // larger z only for a 5 % gain; fixed-order reduce
   std::unique_ptr<Scratch> part;
-  p.kc = kc > 0 && kc < p.kblocks ? kc : 0;
-  if (p.kc == 0 && p.kblocks >= 8) {
-    int ks = 1;
-    const int zmax = (int)std::min<int64_t>(std::min<int64_t>(p.kblocks / 4, 256),
-                                            std::max<int64_t>(1, 8LL * k.sms / tiles));
-    double best = (double)((tiles + k.sms - 1) / k.sms);
-    for (int z = 2; z <= zmax && 8.0 * M * N * z <= 2e9; z++) {
-      const double t = (double)((tiles * z + k.sms - 1) / k.sms) / z;
-      if (t < 0.95 * best) {
-        best = t;
-        ks = z;
-      }
-    }
+  p.kc = chunks ? kc : 0;
+  {
+    // FP64 partial products of the K chunks, added in a fixed order
+    const int ks = plan.z;
     if (ks > 1) {
       p.kchunk = (p.kblocks + ks - 1) / ks;
       p.ksplit = (p.kblocks + p.kchunk - 1) / p.kchunk;
