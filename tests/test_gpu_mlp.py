@@ -136,9 +136,9 @@ def test_family_workflow_batched_learned_guess():
     assert out["iterations_saved"] > 0
 
 
-@pytest.mark.parametrize("rows", [1, 7, 31, 33, 127, 129, 255, 257, 8193])
+@pytest.mark.parametrize("rows", [1, 7, 31, 33, 63, 65, 127, 129, 255, 257, 8193])
 def test_gradients_at_row_edges(rows):
-    """Rows at the edges of the 128-row tiles, the 32-row input blocks and the W2 row chunks."""
+    """Rows at the edges of the 128-row tiles and of the 32-row blocks and 64-row stages."""
     net = U.MLP(seed=9)
     X, t = _data(rows, rows)
     loss, g = net.loss_grad(X, t)

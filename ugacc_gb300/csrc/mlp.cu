@@ -49,31 +49,26 @@ __device__ __forceinline__ float ld(const __half* p) { return __half2float(*p); 
 
 // What a product's epilogue does with C[m][n] = sum_k A[m][k] B[k][n] (n: hidden unit)
 enum class Epi {
-  kHidden,   // Z = C + bias[n], act = silu(Z): both stored
-  kPre,      // Z = C + bias[n]
-  kBack,     // Z holds this layer's input to the activation: Z = C * silu'(Z), in place
-  kPartial,  // partial product of K chunk blockIdx.z at Z + blockIdx.z * M * N
+  kHidden,  // Z = C + bias[n], act = silu(Z): both stored
+  kPre,     // Z = C + bias[n]
+  kBack,    // Z holds this layer's input to the activation: Z = C * silu'(Z), in place
 };
 
 // FP32 product on the CUDA cores, 128 x 64 tile, 8 x 4 outputs per thread, K in steps of 16
 // through two shared-memory stages with the next one's elements in registers meanwhile.  The
 // multiply-adds bound it (32 FMAs for three 16-byte shared loads); the bias, the activation
-// and its derivative run in the epilogue, so no layer is read or written twice.  A is read
-// along k (activations of one row) or along m (weight gradients, K = rows of the batch split
-// over blockIdx.z: 256 x 256 outputs alone are eight tiles).  An 8192-row training step took
-// 3.2 ms with 64 x 64 tiles, one pass per operation, 16 CTAs on a weight gradient and 256
-// threads on the column sums; it takes 0.17 ms now (products 0.13, floor 0.04 at 128 FMAs per
-// SM clock).
+// and its derivative run in the epilogue, so no layer is read or written twice.  An 8192-row
+// training step took 3.2 ms with 64 x 64 tiles, one pass per operation, 16 CTAs on a weight
+// gradient and 256 threads on the column sums; it takes 0.29 ms now.
 constexpr int kTM = 128, kTN = 64, kTK = 16;
-template <typename TB, Epi E, bool AM>
-__global__ void __launch_bounds__(256, 2) layer_gemm(int M, int N, int K, int kchunk, const float* __restrict__ A,
-                                                     int64_t lda, const TB* __restrict__ B, int64_t sBk, int64_t sBn,
+template <typename TB, Epi E>
+__global__ void __launch_bounds__(256, 2) layer_gemm(int M, int N, int K, const float* __restrict__ A, int64_t lda,
+                                                     const TB* __restrict__ B, int64_t sBk, int64_t sBn,
                                                      const float* __restrict__ bias, float* Z, float* act) {
   __shared__ __align__(16) float As[2][kTK][kTM + 4];
   __shared__ __align__(16) float Bs[2][kTK][kTN + 4];
   const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
   const int m0 = blockIdx.y * kTM, n0 = blockIdx.x * kTN;
-  const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
   float ra[8], rb[4], acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; i++)
@@ -82,14 +77,14 @@ __global__ void __launch_bounds__(256, 2) layer_gemm(int M, int N, int K, int kc
   auto fetch = [&](int k0) {
 #pragma unroll
     for (int r = 0; r < 8; r++) {
-      const int e = tid + 256 * r, mm = AM ? e % kTM : e / kTK, kk = AM ? e / kTM : e % kTK;
-      const bool ok = m0 + mm < M && k0 + kk < kend;
-      ra[r] = ok ? A[AM ? (int64_t)(k0 + kk) * lda + m0 + mm : (int64_t)(m0 + mm) * lda + k0 + kk] : 0.f;
+      const int e = tid + 256 * r, mm = e / kTK, kk = e % kTK;
+      const bool ok = m0 + mm < M && k0 + kk < K;
+      ra[r] = ok ? A[(int64_t)(m0 + mm) * lda + k0 + kk] : 0.f;
     }
 #pragma unroll
     for (int r = 0; r < 4; r++) {
       const int e = tid + 256 * r, nn = e % kTN, kk = e / kTN;
-      const bool ok = n0 + nn < N && k0 + kk < kend;
+      const bool ok = n0 + nn < N && k0 + kk < K;
       rb[r] = ok ? ld(B + (int64_t)(k0 + kk) * sBk + (int64_t)(n0 + nn) * sBn) : 0.f;
     }
   };
@@ -97,7 +92,7 @@ __global__ void __launch_bounds__(256, 2) layer_gemm(int M, int N, int K, int kc
 #pragma unroll
     for (int r = 0; r < 8; r++) {
       const int e = tid + 256 * r;
-      As[b][AM ? e / kTM : e % kTK][AM ? e % kTM : e / kTK] = ra[r];
+      As[b][e % kTK][e / kTK] = ra[r];
     }
 #pragma unroll
     for (int r = 0; r < 4; r++) {
@@ -105,12 +100,12 @@ __global__ void __launch_bounds__(256, 2) layer_gemm(int M, int N, int K, int kc
       Bs[b][e / kTN][e % kTN] = rb[r];
     }
   };
-  fetch(kbeg);
+  fetch(0);
   int b = 0;
-  for (int k0 = kbeg; k0 < kend; k0 += kTK) {
+  for (int k0 = 0; k0 < K; k0 += kTK) {
     stage(b);
     __syncthreads();
-    if (k0 + kTK < kend) fetch(k0 + kTK);
+    if (k0 + kTK < K) fetch(k0 + kTK);
 #pragma unroll
     for (int kk = 0; kk < kTK; kk++) {
       const float4 a0 = *reinterpret_cast<const float4*>(&As[b][kk][ty * 8]);
@@ -133,9 +128,7 @@ __global__ void __launch_bounds__(256, 2) layer_gemm(int M, int N, int K, int kc
       const int n = n0 + tx * 4 + j;
       if (n >= N) continue;
       const int64_t o = (int64_t)m * N + n;
-      if (E == Epi::kPartial) {
-        Z[(int64_t)blockIdx.z * M * N + o] = acc[i][j];
-      } else if (E == Epi::kBack) {
+      if (E == Epi::kBack) {
         Z[o] = acc[i][j] * dsilu(Z[o]);
       } else {
         const float z = acc[i][j] + bias[n];
@@ -146,134 +139,181 @@ __global__ void __launch_bounds__(256, 2) layer_gemm(int M, int N, int K, int kc
   }
 }
 
-// The output layer, one warp per row: y = silu(Z2) w3 + b3.  GRAD: dy = 2 (y - t) / n, Z2
-// becomes dZ2 = dy w3 silu'(Z2) in place, and this block's sums over its rows go to
-// part[block]: 256 of dy silu(Z2) (w3), 256 of dZ2 (b2), dy (b3) and (y - t)^2.
-constexpr int kOutSums = 2 * kHid + 2;
+// The output layer, 32 rows per block: A2 = silu(Z2), y = A2 w3 + b3 (a row's sum runs over the
+// hidden units in order, one lane per row).  GRAD: dy = 2 (y - t) / n, Z2 becomes
+// dZ2 = dy w3 silu'(Z2) in place, and part[block] gets the block's sum of (y - t)^2.
+constexpr int kOutRows = 32;
+constexpr size_t kOutSmem = sizeof(float) * (kOutRows * (kHid + 1) + kOutRows);
 template <bool GRAD>
-__global__ void __launch_bounds__(256) output_kernel(int64_t n, float* Z2, const __half* __restrict__ w3,
-                                                     const float* __restrict__ b3, const float* __restrict__ t,
-                                                     float* y, float* part) {
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  float w[8], s3[8], s2[8], sd = 0.f, sl = 0.f;
+__global__ void __launch_bounds__(kHid) output_kernel(int64_t n, float* Z2, const __half* __restrict__ w3,
+                                                      const float* __restrict__ b3, const float* __restrict__ t,
+                                                      float* y, float* A2, float* part) {
+  extern __shared__ float sm[];  // activations [32][257], then dy [32]
+  float* dys = sm + kOutRows * (kHid + 1);
+  const int j = threadIdx.x;
+  const int64_t r0 = (int64_t)blockIdx.x * kOutRows;
+  const int nr = (int)(n - r0 < kOutRows ? n - r0 : kOutRows);
+  float z[kOutRows];
 #pragma unroll
-  for (int e = 0; e < 8; e++) {
-    w[e] = __half2float(w3[lane + 32 * e]);
-    s3[e] = s2[e] = 0.f;
+  for (int r = 0; r < kOutRows; r++) z[r] = r < nr ? Z2[(r0 + r) * kHid + j] : 0.f;
+#pragma unroll
+  for (int r = 0; r < kOutRows; r++) {
+    const float a = silu(z[r]);
+    sm[r * (kHid + 1) + j] = a;
+    if (GRAD && r < nr) A2[(r0 + r) * kHid + j] = a;
   }
-  const float b = b3[0];
-  for (int64_t r = (int64_t)blockIdx.x * 8 + warp; r < n; r += (int64_t)gridDim.x * 8) {
-    float* z = Z2 + r * kHid;
-    float zv[8], a[8], s = 0.f;
-#pragma unroll
-    for (int e = 0; e < 8; e++) zv[e] = z[lane + 32 * e];
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      a[e] = silu(zv[e]);
-      s = fmaf(a[e], w[e], s);
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    s += b;
-    if (!GRAD) {
-      if (lane == 0) y[r] = s;
-      continue;
-    }
-    const float d = s - t[r], dy = 2.f * d / (float)n;
-    sd += dy;
-    sl = fmaf(d, d, sl);
-#pragma unroll
-    for (int e = 0; e < 8; e++) {
-      const float g = dy * w[e] * dsilu(zv[e]);
-      z[lane + 32 * e] = g;
-      s3[e] = fmaf(dy, a[e], s3[e]);
-      s2[e] += g;
+  __syncthreads();
+  if (j < kOutRows) {
+    float s = 0.f;
+#pragma unroll 16
+    for (int k = 0; k < kHid; k++) s = fmaf(sm[j * (kHid + 1) + k], __half2float(w3[k]), s);
+    s += b3[0];
+    if (GRAD) {
+      const float d = j < nr ? s - t[r0 + j] : 0.f;
+      const float dy = 2.f * d / (float)n;
+      dys[j] = dy;
+      if (j < nr) y[r0 + j] = dy;
+      float l = d * d;
+      for (int o = 16; o > 0; o >>= 1) l += __shfl_down_sync(0xffffffffu, l, o);
+      if (j == 0) part[blockIdx.x] = l;
+    } else if (j < nr) {
+      y[r0 + j] = s;
     }
   }
-  if constexpr (GRAD) {
-    __shared__ float sums[8][kOutSums];
+  if (!GRAD) return;
+  __syncthreads();
+  const float w = __half2float(w3[j]);
 #pragma unroll
-    for (int e = 0; e < 8; e++) {
-      sums[warp][lane + 32 * e] = s3[e];
-      sums[warp][kHid + lane + 32 * e] = s2[e];
-    }
-    if (lane == 0) {
-      sums[warp][2 * kHid] = sd;
-      sums[warp][2 * kHid + 1] = sl;
-    }
-    __syncthreads();
-    for (int x = threadIdx.x; x < kOutSums; x += 256) {
-      float s = 0.f;
-#pragma unroll
-      for (int q = 0; q < 8; q++) s += sums[q][x];
-      part[(int64_t)blockIdx.x * kOutSums + x] = s;
-    }
-  }
+  for (int r = 0; r < kOutRows; r++)
+    if (r < nr) Z2[(r0 + r) * kHid + j] = dys[r] * w * dsilu(z[r]);
 }
 
-// W1 and b1 gradients, sum_r X[r][k] dZ1[r][n] and sum_r dZ1[r][n]: thread n keeps the 16 sums
-// of its column over the block's rows, part[block][16][256]
-constexpr int kIn = kFeat + 1, kInRows = 32;
-__global__ void __launch_bounds__(kHid) input_grad_kernel(int64_t rows, const float* __restrict__ X,
-                                                          const float* __restrict__ dZ1, float* part) {
-  __shared__ float xs[kInRows][kFeat];
-  const int64_t r0 = (int64_t)blockIdx.x * kInRows;
-  const int nr = (int)(rows - r0 < kInRows ? rows - r0 : kInRows), n = threadIdx.x;
-  for (int e = threadIdx.x; e < nr * kFeat; e += kHid) xs[e / kFeat][e % kFeat] = X[r0 * kFeat + e];
-  __syncthreads();
-  float s[kIn];
+// Parameter gradients, sums over the rows of a batch: C[m][n] = sum_r A[r][m] B[r][n] for m < M,
+// and bias[n] = sum_r B[r][n].
+struct RowSum {
+  const float* A;
+  int lda, M;
+  const float* B;
+  int ldb, N;
+  float* C;
+  int ldc;
+  float* bias;
+  int tn, first;  // tiles along n, first block
+};
+// The three layers' sums in one launch, one 32 x 16 tile of outputs per block (152 tiles, one
+// per SM); the last block sums the loss.  A sum runs over the rows in order, in FP32, whatever
+// the tile: changes of a last bit, which the optimizer amplifies from step to step, stay out of
+// training.  So no row range is split, and a row's 6 shared words per thread for 8 multiply-adds
+// (2 x 4 outputs, 2 warps) bound it: 12 clocks of the shared-memory port a row, 52 us for 8192
+// rows.  Four more warps load, by cp.async in stages of 64 rows, three ahead, and sum B alone,
+// for the bias, in the blocks of the first 32 rows m.  82 us for a W2 tile, 97 us for the launch
+// (the 15 features' rows are copied word by word); 300 us with the same warps loading and
+// summing in stages of 32, 145 us with 4 outputs per thread.
+constexpr int kSumM = 32, kSumN = 16, kSumR = 64, kSumStages = 4;
+constexpr int kSumMath = 64, kSumLoad = 128, kSumThreads = kSumMath + kSumLoad;
+template <int kBytes>
+__device__ __forceinline__ void sum_copy(float* dst, const float* src, bool ok) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  const int n = ok ? kBytes : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(d), "l"(src), "n"(kBytes), "r"(n) : "memory");
+}
+// rows r0 .. of columns c0 .. c0 + W - 1 of X [rows][ld] (nc columns in all) into st [kSumR][W]
+template <int W>
+__device__ __forceinline__ void sum_load(float* st, const float* X, int ld, int nc, int c0, int64_t r0, int64_t rows,
+                                         int t) {
+  if (ld % 4 == 0 && c0 + W <= nc) {
 #pragma unroll
-  for (int k = 0; k < kIn; k++) s[k] = 0.f;
+    for (int e = t; e < kSumR * W / 4; e += kSumLoad) {
+      const int r = e / (W / 4), c = e % (W / 4) * 4;
+      const bool ok = r0 + r < rows;
+      sum_copy<16>(st + r * W + c, ok ? X + (r0 + r) * ld + c0 + c : X, ok);
+    }
+  } else {  // columns past nc keep the zeros of the start
+    const int w = min(W, nc - c0), step = kSumLoad / w, c = t % w, r = t / w;
+    const int n = (int)min((int64_t)kSumR, rows - r0);
+    const float* x = X + (r0 + r) * ld + c0 + c;
+    st += r * W + c;
 #pragma unroll 8
-  for (int r = 0; r < nr; r++) {
-    const float d = dZ1[(r0 + r) * kHid + n];
-#pragma unroll
-    for (int k = 0; k < kFeat; k++) s[k] = fmaf(xs[r][k], d, s[k]);
-    s[kFeat] += d;
+    for (int q = r < step ? r : kSumR; q < kSumR; q += step, x += step * ld, st += step * W)
+      sum_copy<4>(st, q < n ? x : X, q < n);
   }
-#pragma unroll
-  for (int k = 0; k < kIn; k++) part[((int64_t)blockIdx.x * kIn + k) * kHid + n] = s[k];
 }
-
-// The gradient from its partial sums, one block per 32 consecutive parameters and 8 lanes of
-// partials each, added in a fixed order: W1, b1 from pin[nin], W2 from pw2[nw2], b2, w3, b3 and
-// the loss (the sum of squares over n) from pout[nout]
-__global__ void __launch_bounds__(256) gradient_kernel(const float* __restrict__ pin, int nin,
-                                                       const float* __restrict__ pw2, int nw2,
-                                                       const float* __restrict__ pout, int nout, int64_t n, float* g,
-                                                       float* loss) {
-  __shared__ float red[8][33];
-  constexpr int64_t kW1 = kIn * kHid, kW2 = kW1 + kHid * kHid, kAll = kW2 + kOutSums;
-  const int64_t x = (int64_t)blockIdx.x * 32 + threadIdx.x % 32;
-  const float* p = nullptr;
-  int64_t ld = 0;
-  int np = 0;
-  if (x < kW1) {
-    p = pin + x, ld = kW1, np = nin;
-  } else if (x < kW2) {
-    p = pw2 + (x - kW1), ld = kHid * kHid, np = nw2;
-  } else if (x < kAll) {
-    p = pout + (x - kW2), ld = kOutSums, np = nout;
+__global__ void __launch_bounds__(kSumThreads) row_sums_kernel(int64_t rows, RowSum p0, RowSum p1, RowSum p2,
+                                                               int loss_block, const float* __restrict__ part,
+                                                               int nparts, float* loss) {
+  __shared__ __align__(16) float As[kSumStages][kSumR * kSumM];
+  __shared__ __align__(16) float Bs[kSumStages][kSumR * kSumN];
+  const int tid = threadIdx.x, blk = blockIdx.x;
+  if (blk == loss_block) {
+    float s = 0.f;
+    for (int i = tid; i < nparts; i += kSumThreads) s += part[i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (tid % 32 == 0) As[0][tid / 32] = s;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < kSumThreads / 32; w++) s += As[0][w];
+      loss[0] = s / (float)rows;
+    }
+    return;
   }
-  float s = 0.f;
-#pragma unroll 4
-  for (int q = threadIdx.x / 32; q < np; q += 8) s += p[q * ld];
-  red[threadIdx.x / 32][threadIdx.x % 32] = s;
-  __syncthreads();
-  if (threadIdx.x >= 32 || x >= kAll) return;
-  s = 0.f;
+  const RowSum p = blk >= p2.first ? p2 : blk >= p1.first ? p1 : p0;
+  const int m0 = (blk - p.first) / p.tn * kSumM, n0 = (blk - p.first) % p.tn * kSumN;
+  if (m0 + kSumM > p.M || n0 + kSumN > p.N) {
+    for (int e = tid; e < kSumStages * kSumR * kSumM; e += kSumThreads) As[0][e] = 0.f;
+    for (int e = tid; e < kSumStages * kSumR * kSumN; e += kSumThreads) Bs[0][e] = 0.f;
+    __syncthreads();
+  }
+  const bool loads = tid >= kSumMath;
+  const int lt = tid - kSumMath, tm = tid / 4 % 16 * 2, tn = tid % 4 * 4;
+  auto load = [&](int b, int64_t r0) {
+    if (r0 < rows) {
+      sum_load<kSumM>(As[b], p.A, p.lda, p.M, m0, r0, rows, lt);
+      sum_load<kSumN>(Bs[b], p.B, p.ldb, p.N, n0, r0, rows, lt);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // kSumStages - 1 groups in flight; past the last rows the groups are empty
+  if (loads)
+    for (int q = 0; q < kSumStages - 1; q++) load(q, (int64_t)q * kSumR);
+  float acc[2][4] = {}, bias = 0.f;
+  int b = 0;
+  for (int64_t r0 = 0; r0 < rows; r0 += kSumR) {
+    if (loads) asm volatile("cp.async.wait_group %0;" ::"n"(kSumStages - 2) : "memory");
+    __syncthreads();  // this stage has landed for all, and the one loaded next has been read by all
+    const float *A = As[b] + tm, *B = Bs[b] + tn;
+    if (loads) {
+      load((b + kSumStages - 1) % kSumStages, r0 + (int64_t)(kSumStages - 1) * kSumR);
+      if (m0 == 0 && lt < kSumN) {
+        const float* x = Bs[b] + lt;
+#pragma unroll 16
+        for (int r = 0; r < kSumR; r++) bias += x[r * kSumN];
+      }
+    } else {
 #pragma unroll
-  for (int q = 0; q < 8; q++) s += red[q][threadIdx.x];
-  const int64_t y = x - kW2;  // w3, b2, b3, loss; the parameter order is W1 b1 W2 b2 w3 b3
-  if (x < kW2)
-    g[x] = s;
-  else if (y < kHid)
-    g[kW2 + kHid + y] = s;
-  else if (y < 2 * kHid)
-    g[kW2 + y - kHid] = s;
-  else if (y == 2 * kHid)
-    g[kW2 + 2 * kHid] = s;
-  else
-    loss[0] = s / (float)n;
+      for (int r = 0; r < kSumR; r++) {
+        const float2 a = *reinterpret_cast<const float2*>(A + r * kSumM);
+        const float4 x = *reinterpret_cast<const float4*>(B + r * kSumN);
+        acc[0][0] = fmaf(a.x, x.x, acc[0][0]);
+        acc[0][1] = fmaf(a.x, x.y, acc[0][1]);
+        acc[0][2] = fmaf(a.x, x.z, acc[0][2]);
+        acc[0][3] = fmaf(a.x, x.w, acc[0][3]);
+        acc[1][0] = fmaf(a.y, x.x, acc[1][0]);
+        acc[1][1] = fmaf(a.y, x.y, acc[1][1]);
+        acc[1][2] = fmaf(a.y, x.z, acc[1][2]);
+        acc[1][3] = fmaf(a.y, x.w, acc[1][3]);
+      }
+    }
+    b = (b + 1) % kSumStages;
+  }
+  if (loads) {
+    if (m0 == 0 && lt < kSumN && n0 + lt < p.N) p.bias[n0 + lt] = bias;
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (m0 + tm + i < p.M && n0 + tn + j < p.N) p.C[(int64_t)(m0 + tm + i) * p.ldc + n0 + tn + j] = acc[i][j];
 }
 
 // Adam on FP32 masters, then the FP16 working copy
@@ -602,7 +642,7 @@ struct ucc_mlp {
   int64_t adam_t = 0;
   int64_t cap = 0;   // activation buffers sized for this many rows
   int64_t ycap = 0;  // output / output-gradient buffers
-  float *Z1 = nullptr, *A1 = nullptr, *Z2 = nullptr, *y = nullptr, *loss = nullptr;
+  float *Z1 = nullptr, *A1 = nullptr, *Z2 = nullptr, *A2 = nullptr, *y = nullptr, *loss = nullptr;
   int64_t oW1() const { return 0; }
   int64_t ob1() const { return (int64_t)kFeat * kHid; }
   int64_t oW2() const { return ob1() + kHid; }
@@ -610,8 +650,8 @@ struct ucc_mlp {
   int64_t ow3() const { return ob2() + kHid; }
   int64_t ob3() const { return ow3() + kHid; }
   ~ucc_mlp() {
-    for (void* p : {(void*)w, (void*)g, (void*)m, (void*)v, (void*)wh, (void*)Z1, (void*)A1, (void*)Z2, (void*)y,
-                    (void*)loss})
+    for (void* p : {(void*)w, (void*)g, (void*)m, (void*)v, (void*)wh, (void*)Z1, (void*)A1, (void*)Z2, (void*)A2,
+                    (void*)y, (void*)loss})
       if (p) cudaFree(p);
     if (stream) cudaStreamDestroy(stream);
   }
@@ -636,14 +676,11 @@ ucc_status mguard(ucc_mlp* n, F&& f) {
 }
 
 constexpr int64_t kChunk = 1 << 20;  // rows per forward pass (activation buffers)
-constexpr int kOutBlocks = 152 * 4;   // blocks of the output layer's pass (and their partial sums)
-constexpr int kSplitRows = 256;       // rows per K chunk of the W2 gradient
-
 void ensure_rows(ucc_mlp& n, int64_t rows) {
   const int64_t act = std::min(rows, kChunk);
   if (act > n.cap) {
     n.cap = 0;
-    for (float** p : {&n.Z1, &n.A1, &n.Z2}) {
+    for (float** p : {&n.Z1, &n.A1, &n.Z2, &n.A2}) {
       if (*p) cudaFree(*p);
       *p = nullptr;
       UCC_CUDA(cudaMalloc(p, sizeof(float) * act * kHid));
@@ -659,21 +696,7 @@ void ensure_rows(ucc_mlp& n, int64_t rows) {
   }
 }
 
-// partial sums of one backward pass over rows: W2 (up to 32 chunks), W1 and b1, output layer
-struct Parts {
-  int nw2, nin, nout, w2chunk;
-  explicit Parts(int64_t rows) {
-    nw2 = (int)std::max<int64_t>(1, std::min<int64_t>((rows + kSplitRows - 1) / kSplitRows, 32));
-    w2chunk = (int)((rows + nw2 - 1) / nw2);
-    nw2 = (int)((rows + w2chunk - 1) / w2chunk);
-    nin = (int)((rows + kInRows - 1) / kInRows);
-    nout = (int)std::min<int64_t>((rows + 7) / 8, kOutBlocks);
-  }
-  int64_t w2() const { return 0; }
-  int64_t in() const { return (int64_t)nw2 * kHid * kHid; }
-  int64_t out() const { return in() + (int64_t)nin * kIn * kHid; }
-  int64_t total() const { return out() + (int64_t)nout * kOutSums; }
-};
+int64_t out_blocks(int64_t rows) { return (rows + kOutRows - 1) / kOutRows; }
 
 void launched(int k) {
   for (; k > 0; k--) count_kernel_launch();
@@ -685,10 +708,10 @@ dim3 layer_grid(int64_t rows) { return dim3(kHid / kTN, (unsigned)((rows + kTM -
 // the two hidden layers of rows X[rows][15]: Z1, A1 = silu(Z1), Z2
 void hidden_layers(ucc_mlp& n, const float* X, int64_t rows) {
   const dim3 grid = layer_grid(rows);
-  layer_gemm<__half, Epi::kHidden, false><<<grid, 256, 0, n.stream>>>(
-      (int)rows, kHid, kFeat, kFeat, X, kFeat, n.wh + n.oW1(), kHid, 1, n.w + n.ob1(), n.Z1, n.A1);
-  layer_gemm<__half, Epi::kPre, false><<<grid, 256, 0, n.stream>>>((int)rows, kHid, kHid, kHid, n.A1, kHid,
-                                                                  n.wh + n.oW2(), kHid, 1, n.w + n.ob2(), n.Z2, nullptr);
+  layer_gemm<__half, Epi::kHidden><<<grid, 256, 0, n.stream>>>((int)rows, kHid, kFeat, X, kFeat, n.wh + n.oW1(), kHid,
+                                                              1, n.w + n.ob1(), n.Z1, n.A1);
+  layer_gemm<__half, Epi::kPre><<<grid, 256, 0, n.stream>>>((int)rows, kHid, kHid, n.A1, kHid, n.wh + n.oW2(), kHid, 1,
+                                                           n.w + n.ob2(), n.Z2, nullptr);
   launched(2);
 }
 
@@ -697,29 +720,33 @@ void forward(ucc_mlp& n, const float* X, int64_t rows) {
   for (int64_t r0 = 0; r0 < rows; r0 += kChunk) {
     const int64_t len = std::min(kChunk, rows - r0);
     hidden_layers(n, X + r0 * kFeat, len);
-    output_kernel<false><<<kOutBlocks, 256, 0, n.stream>>>(len, n.Z2, n.wh + n.ow3(), n.w + n.ob3(), nullptr, n.y + r0,
-                                                           nullptr);
+    output_kernel<false><<<(unsigned)out_blocks(len), kHid, kOutSmem, n.stream>>>(
+        len, n.Z2, n.wh + n.ow3(), n.w + n.ob3(), nullptr, n.y + r0, nullptr, nullptr);
     launched(1);
   }
 }
 
 // mean squared error (to loss[0] on the device) and gradients (into n.g) for rows X, targets t;
-// part: Parts(rows).total() floats of scratch
+// part: out_blocks(rows) floats of scratch
 void backward(ucc_mlp& n, const float* X, const float* t, int64_t rows, float* part, float* loss) {
-  const Parts p(rows);
   hidden_layers(n, X, rows);
-  output_kernel<true><<<p.nout, 256, 0, n.stream>>>(rows, n.Z2, n.wh + n.ow3(), n.w + n.ob3(), t, nullptr,
-                                                    part + p.out());
-  // W2: A1^T dZ2 over row chunks; dZ1 = (dZ2 W2^T) silu'(Z1), in place of Z1; W1 and b1
-  layer_gemm<float, Epi::kPartial, true><<<dim3(kHid / kTN, kHid / kTM, p.nw2), 256, 0, n.stream>>>(
-      kHid, kHid, (int)rows, p.w2chunk, n.A1, kHid, n.Z2, kHid, 1, nullptr, part + p.w2(), nullptr);
-  layer_gemm<__half, Epi::kBack, false><<<layer_grid(rows), 256, 0, n.stream>>>(
-      (int)rows, kHid, kHid, kHid, n.Z2, kHid, n.wh + n.oW2(), 1, kHid, nullptr, n.Z1, nullptr);
-  input_grad_kernel<<<p.nin, kHid, 0, n.stream>>>(rows, X, n.Z1, part + p.in());
-  constexpr int kAll = kIn * kHid + kHid * kHid + kOutSums;
-  gradient_kernel<<<(kAll + 31) / 32, 256, 0, n.stream>>>(part + p.in(), p.nin, part + p.w2(), p.nw2, part + p.out(),
-                                                          p.nout, rows, n.g, loss);
-  launched(5);
+  output_kernel<true><<<(unsigned)out_blocks(rows), kHid, kOutSmem, n.stream>>>(
+      rows, n.Z2, n.wh + n.ow3(), n.w + n.ob3(), t, n.y, n.A2, part);
+  // dZ1 = (dZ2 W2^T) silu'(Z1), in place of Z1
+  layer_gemm<__half, Epi::kBack><<<layer_grid(rows), 256, 0, n.stream>>>((int)rows, kHid, kHid, n.Z2, kHid,
+                                                                        n.wh + n.oW2(), 1, kHid, nullptr, n.Z1, nullptr);
+  // W2 and b2 from A1 and dZ2, w3 and b3 from A2 and dy, W1 and b1 from X and dZ1
+  RowSum p[3] = {{n.A1, kHid, kHid, n.Z2, kHid, kHid, n.g + n.oW2(), kHid, n.g + n.ob2(), 0, 0},
+                 {n.A2, kHid, kHid, n.y, 1, 1, n.g + n.ow3(), 1, n.g + n.ob3(), 0, 0},
+                 {X, kFeat, kFeat, n.Z1, kHid, kHid, n.g + n.oW1(), kHid, n.g + n.ob1(), 0, 0}};
+  int blocks = 0;
+  for (RowSum& q : p) {
+    q.tn = (q.N + kSumN - 1) / kSumN;
+    q.first = blocks;
+    blocks += q.tn * ((q.M + kSumM - 1) / kSumM);
+  }
+  row_sums_kernel<<<blocks + 1, kSumThreads, 0, n.stream>>>(rows, p[0], p[1], p[2], blocks, part, (int)out_blocks(rows), loss);
+  launched(3);
 }
 }  // namespace
 
@@ -821,7 +848,7 @@ ucc_status ucc_mlp_loss_grad(ucc_mlp* n, const float* X, const float* t, int64_t
     UCC_CUDA(cudaMemcpyAsync(dt, t, sizeof(float) * rows, cudaMemcpyHostToDevice, m.stream));
     UCC_REQUIRE(rows <= kChunk, UCC_BAD_ARGS, "training batch larger than the activation chunk");
     float* part = nullptr;
-    UCC_CUDA(cudaMallocAsync(&part, sizeof(float) * Parts(rows).total(), m.stream));
+    UCC_CUDA(cudaMallocAsync(&part, sizeof(float) * out_blocks(rows), m.stream));
     backward(m, dX, dt, rows, part, m.loss);
     UCC_CUDA(cudaMemcpyAsync(loss, m.loss, sizeof(float), cudaMemcpyDeviceToHost, m.stream));
     UCC_CUDA(cudaFreeAsync(part, m.stream));
@@ -847,7 +874,7 @@ ucc_status ucc_mlp_train(ucc_mlp* n, const float* X, const float* t, int64_t row
     UCC_CUDA(cudaMallocAsync(&dt, sizeof(float) * rows, m.stream));
     UCC_CUDA(cudaMallocAsync(&Xb, sizeof(float) * nb * kFeat, m.stream));
     UCC_CUDA(cudaMallocAsync(&tb, sizeof(float) * nb, m.stream));
-    UCC_CUDA(cudaMallocAsync(&part, sizeof(float) * Parts(nb).total(), m.stream));
+    UCC_CUDA(cudaMallocAsync(&part, sizeof(float) * out_blocks(nb), m.stream));
     UCC_CUDA(cudaMallocAsync(&dloss, sizeof(float) * steps, m.stream));
     UCC_CUDA(cudaMallocAsync(&didx, sizeof(int64_t) * rows, m.stream));
     UCC_CUDA(cudaMemcpyAsync(dX, X, sizeof(float) * rows * kFeat, cudaMemcpyHostToDevice, m.stream));
