@@ -391,6 +391,8 @@ void jacobi_update(Ctx& c, int no, int nv, const double* d_do, const double* d_d
 void lincomb(Ctx& c, int nvec, const double* const* d_vecs, const double* coef, int64_t n, double* out);
 
 // (T) energy over a batch of (i>=j>=k) tuples, given W3 for each tuple.
+// W3 of the n tuples in d_list (2 t + 0: exchange a and b, + 1: exchange b and c), in place: W3 + W3(exchanged)
+void triples_fold(Ctx& c, int nv, int n, const int* d_list, double* W3);
 void triples_energy(Ctx& c, int no, int nv, int ntuple, const int* d_tuples, const double* W3,
                     const double* t1, const double* Voovv, const double* eps, double* d_partial);
 // The same from an FP32 W3 (mixed form) held as nparts partial arrays part_stride floats

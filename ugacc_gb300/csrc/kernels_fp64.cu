@@ -627,6 +627,40 @@ __global__ void triples_energy_kernel(int no, int nv, const int* tuples, const d
   if (threadIdx.x == 0) partial[(int64_t)t * nv + a] = tot;
 }
 
+// W += W(exchanged) of the tuples whose W3 was made from half its products, each pair of
+// elements by one thread, in place.  Two passes over the tuple's memory bound it.  Block (x, a,
+// list entry): exchanging a and b, rows c of the pairs (a, b >= a), b from a + x in steps of the
+// grid; exchanging b and c, the tile pair x of plane a, through shared memory so that both sides
+// are read along c.
+constexpr int kFold = 32;
+__global__ void __launch_bounds__(256) triples_fold_kernel(int nv, const int* __restrict__ list, double* W3) {
+  __shared__ double ta[kFold][kFold + 1], tb[kFold][kFold + 1];
+  const int e = list[blockIdx.z], a = blockIdx.y;
+  const int64_t nv2 = (int64_t)nv * nv;
+  double* W = W3 + (int64_t)(e / 2) * nv2 * nv;
+  if (e % 2 == 0) {
+    for (int b = a + blockIdx.x; b < nv; b += gridDim.x) {
+      double *x = W + a * nv2 + (int64_t)b * nv, *y = W + b * nv2 + (int64_t)a * nv;
+      for (int c = threadIdx.x; c < nv; c += 256) x[c] = y[c] = x[c] + y[c];
+    }
+    return;
+  }
+  int hi = 0;
+  while ((hi + 1) * (hi + 2) / 2 <= (int)blockIdx.x) hi++;
+  const int b0 = hi * kFold, c0 = ((int)blockIdx.x - hi * (hi + 1) / 2) * kFold;  // b0 >= c0
+  double* P = W + a * nv2;
+  const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+  for (int r = ty; r < kFold; r += 8) {
+    if (b0 + r < nv && c0 + tx < nv) ta[r][tx] = P[(int64_t)(b0 + r) * nv + c0 + tx];
+    if (c0 + r < nv && b0 + tx < nv) tb[r][tx] = P[(int64_t)(c0 + r) * nv + b0 + tx];
+  }
+  __syncthreads();
+  for (int r = ty; r < kFold; r += 8) {
+    if (b0 + r < nv && c0 + tx < nv) P[(int64_t)(b0 + r) * nv + c0 + tx] = ta[r][tx] + tb[tx][r];
+    if (b0 != c0 && c0 + r < nv && b0 + tx < nv) P[(int64_t)(c0 + r) * nv + b0 + tx] = tb[r][tx] + ta[tx][r];
+  }
+}
+
 // FP32 W3 (mixed form): the per-element V3/X3/Y3/Z3 algebra in FP32, the sums in FP64.
 // W3 arrives as up to three partial arrays (one per pair of W3 terms, each written without
 // a read-modify-write by its tensor-core GEMM), nparts * part_stride floats apart; their
@@ -1013,6 +1047,15 @@ void triples_energy_f32(Ctx& c, int no, int nv, int ntuple, const int* d_tuples,
   count_launch();
   check_launch("triples_energy_f32");
   UCC_CUDA(cudaStreamSynchronize(c.stream));  // the tile list is freed on return
+}
+
+void triples_fold(Ctx& c, int nv, int n, const int* d_list, double* W3) {
+  UCC_REQUIRE(n <= 65535 && nv <= 65535, UCC_BAD_ARGS, "triples_fold: too many tuples per batch");
+  const int64_t t = (nv + kFold - 1) / kFold;
+  triples_fold_kernel<<<dim3((unsigned)(t * (t + 1) / 2), (unsigned)nv, (unsigned)n), 256, 0, c.stream>>>(nv, d_list,
+                                                                                                      W3);
+  count_launch();
+  check_launch("triples_fold");
 }
 
 void triples_energy(Ctx& c, int no, int nv, int ntuple, const int* d_tuples, const double* W3, const double* t1,

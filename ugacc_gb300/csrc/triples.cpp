@@ -42,30 +42,51 @@ void triples_operands_fp64(Ctx& c, Tensor& Acat, Tensor& Bcat) {
 }
 
 // W3 of nb tuples (host triples (i,j,k)) into W3 + b*nv^3, FP64; d_ptrs holds 6*nb
-// pointer triples and is reused: the call synchronises before returning
+// pointer triples and is reused: the call synchronises before returning.
+//
+// With i == j the terms 5, 4 and 3 have the operands of 0, 1 and 2 and their output with a and
+// b exchanged; with j == k the terms 1, 5 and 4 those of 0, 2 and 3 with b and c exchanged.  So
+// half the products make S, and one pass over it W3 = S + S(exchanged): with FP64
+// multiply-adds the bound of (T), 43 % of the products go at no = 5 and 9 % at no = 32 (with
+// (i,i,i), below).  no=8/nv=96: the products took 112 ms with six for every tuple, 110 ms being
+// the floor of their multiply-adds, and take 79 ms; the pass takes 0.16 ms.
 void triples_w3_fp64(Ctx& c, const Tensor& Acat, const Tensor& Bcat, const int* h_tuples, int nb, double* W3,
                      GemmPtrs* d_ptrs) {
   const int no = c.no, nv = c.nv;
   const int64_t nv2 = (int64_t)nv * nv, nv3 = nv2 * nv, Kp = nv + no;
   TriplesTerm terms[6];
   triples_terms(nv, terms);
-  std::vector<GemmPtrs> all((size_t)nb * 6);
-  for (int q = 0; q < 6; q++)
+  std::vector<GemmPtrs> all;
+  all.reserve((size_t)nb * 6);
+  std::vector<int> fold;  // 2 b + (0: exchange a and b, 1: exchange b and c)
+  int first[7] = {0};
+  for (int q = 0; q < 6; q++) {
     for (int b = 0; b < nb; b++) {
       const int* ijk = h_tuples + 3 * b;
       const TriplesTerm& tm = terms[q];
-      all[(size_t)q * nb + b] = {Acat.p + (int64_t)ijk[tm.x] * Kp * nv2,
-                                 Bcat.p + ((int64_t)ijk[tm.y] * no + ijk[tm.z]) * Kp * nv, W3 + (int64_t)b * nv3};
+      const bool ij = ijk[0] == ijk[1], jk = !ij && ijk[1] == ijk[2];
+      if ((ij && q > 2) || (jk && (q == 1 || q > 3))) continue;
+      if (q == 0 && (ij || jk)) fold.push_back(2 * b + (jk ? 1 : 0));
+      all.push_back({Acat.p + (int64_t)ijk[tm.x] * Kp * nv2,
+                     Bcat.p + ((int64_t)ijk[tm.y] * no + ijk[tm.z]) * Kp * nv, W3 + (int64_t)b * nv3});
     }
+    first[q + 1] = (int)all.size();
+  }
   UCC_CUDA(cudaMemcpyAsync(d_ptrs, all.data(), sizeof(GemmPtrs) * all.size(), cudaMemcpyHostToDevice, c.stream));
   for (int q = 0; q < 6; q++) {
+    if (first[q + 1] == first[q]) continue;
     GemmEpilogue epi;
     epi.msplit = nv;
     epi.s_mhi = terms[q].su;
     epi.s_mlo = terms[q].sv;
     epi.s_n = terms[q].sw;
-    dgemm_strided(c, nv2, nv, Kp, 1.0, nullptr, 1, nv2, nullptr, nv, 1, q == 0 ? 0.0 : 1.0, nullptr, epi, nb, 0, 0, 0,
-                  d_ptrs + (size_t)q * nb);
+    dgemm_strided(c, nv2, nv, Kp, 1.0, nullptr, 1, nv2, nullptr, nv, 1, q == 0 ? 0.0 : 1.0, nullptr, epi,
+                  first[q + 1] - first[q], 0, 0, 0, d_ptrs + first[q]);
+  }
+  if (!fold.empty()) {
+    // the pointers have been read: their space (24 bytes a product) takes the list
+    UCC_CUDA(cudaMemcpyAsync(d_ptrs, fold.data(), sizeof(int) * fold.size(), cudaMemcpyHostToDevice, c.stream));
+    triples_fold(c, nv, (int)fold.size(), reinterpret_cast<const int*>(d_ptrs), W3);
   }
   // the pointer array is reused by the next batch: keep the copy ordered after use
   UCC_CUDA(cudaStreamSynchronize(c.stream));
@@ -78,15 +99,19 @@ double run_triples(Ctx& c) {
   double* T = c.get("T").p;
   Tensor t1 = amp1(c, T);
 
+  // (i,i,i) is left out: W3 and V3 are then symmetric in a, b, c, X3 = 6 W V, Y3 = Z3 = 3 V, and
+  // (Y3 - 2 Z3) 3 W + (Z3 - 2 Y3) 3 W + 3 X3 = 0
   std::vector<int> tuples;
   for (int i = 0; i < no; i++)
     for (int j = 0; j <= i; j++)
       for (int k = 0; k <= j; k++) {
+        if (k == i) continue;
         tuples.push_back(i);
         tuples.push_back(j);
         tuples.push_back(k);
       }
   const int ntup = (int)tuples.size() / 3;
+  if (!ntup) return 0.0;
   size_t free_b = 0, total_b = 0;
   UCC_CUDA(cudaMemGetInfo(&free_b, &total_b));
   // larger batches let more tuples that share an A operand read it from L2 (the batched
