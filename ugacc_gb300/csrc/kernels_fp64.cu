@@ -605,11 +605,12 @@ __global__ void triples_energy_kernel(int no, int nv, const int* tuples, const d
   for (int q = threadIdx.x; q < npair; q += blockDim.x) {
     const int b = q / (a + 1), c = q % (a + 1);
     if (c > b) continue;
+    // the divisor 1, 2 or 4 is the same for all six orders of (a, b, c), and exact as a factor
+    const double same = a == b && b == c ? 0.25 : a == b || b == c ? 0.5 : 1.0;
     auto Wv = [&](int x, int y, int z) { return W[(int64_t)x * nv2 + (int64_t)y * nv + z]; };
     auto Vv = [&](int x, int y, int z) {
-      const double num = Wv(x, y, z) + Vij[(int64_t)x * nv + y] * t1k[z] + Vik[(int64_t)x * nv + z] * t1j[y] +
-                         Vjk[(int64_t)y * nv + z] * t1i[x];
-      return num / (1.0 + (double)((x == y) + (x == z) + (y == z)));
+      return same * (Wv(x, y, z) + Vij[(int64_t)x * nv + y] * t1k[z] + Vik[(int64_t)x * nv + z] * t1j[y] +
+                     Vjk[(int64_t)y * nv + z] * t1i[x]);
     };
     const double wabc = Wv(a, b, c), wacb = Wv(a, c, b), wbac = Wv(b, a, c);
     const double wbca = Wv(b, c, a), wcab = Wv(c, a, b), wcba = Wv(c, b, a);
