@@ -5,6 +5,7 @@
 #include <memory>
 #include <vector>
 
+#include "chain.h"
 #include "core.h"
 #include "dgemm_tile.h"
 
@@ -34,6 +35,7 @@ struct GemmArgs {
 template <class T, bool CLUSTER>
 __global__ void __launch_bounds__(T::THREADS) dgemm_kernel(GemmArgs g) {
   __shared__ double smem[T::SMEM];
+  chain_enter();
   if (g.timed) dgemm_clock_start(g.words);
   const int rank = CLUSTER ? (int)dgemm_cluster_rank() : 0;
   const int t = CLUSTER ? (int)blockIdx.x / g.zc : (int)blockIdx.x;
@@ -126,22 +128,10 @@ namespace {
 template <class T>
 void launch(Ctx& c, const GemmArgs& g, int batch) {
   const dim3 grid((unsigned)((int64_t)g.tiles * g.zc * g.zg), (unsigned)batch);
-  if (g.zc == 1) {
-    dgemm_kernel<T, false><<<grid, T::THREADS, 0, c.stream>>>(g);
-    return;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(T::THREADS);
-  cfg.stream = c.stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)g.zc;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  UCC_CUDA(cudaLaunchKernelEx(&cfg, dgemm_kernel<T, true>, g));
+  if (g.zc == 1)
+    launch_chained(dgemm_kernel<T, false>, grid, dim3(T::THREADS), c.stream, 1, g);
+  else
+    launch_chained(dgemm_kernel<T, true>, grid, dim3(T::THREADS), c.stream, (unsigned)g.zc, g);
 }
 
 }  // namespace

@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <memory>
 
+#include "chain.h"
 #include "core.h"
 
 namespace ucc {
@@ -96,6 +97,7 @@ struct PermArgs {
 // axes shorten that, and the row kernel below pays it once per row.
 template <class I>
 __global__ void permute_kernel_elem(PermArgs a) {
+  chain_enter();
   I od[kMaxRank], is[kMaxRank], os[kMaxRank];
   for (int k = 0; k < a.rank; k++) od[k] = (I)a.od[k], is[k] = (I)a.is[k], os[k] = (I)a.os[k];
   const I total = (I)a.total;
@@ -116,6 +118,7 @@ __global__ void permute_kernel_elem(PermArgs a) {
 // four loads per lane in flight before the stores.
 template <class I>
 __global__ void permute_kernel_rows(PermArgs a) {
+  chain_enter();
   const int r = a.rank;
   I od[kMaxRank], is[kMaxRank], os[kMaxRank];
   for (int k = 0; k < r; k++) od[k] = (I)a.od[k], is[k] = (I)a.is[k], os[k] = (I)a.os[k];
@@ -174,6 +177,7 @@ struct TileArgs {
 
 template <class I>
 __global__ void permute_kernel_tile(TileArgs t) {
+  chain_enter();
   __shared__ double tile[32][33];
   const int r = t.p.rank;
   const I dl = (I)t.p.od[r - 1], dq = (I)t.p.od[t.q];
@@ -295,24 +299,24 @@ void permute_add(Ctx& c, const Tensor& in, double alpha, double beta, const Tens
     const int64_t tiles_q = (a.od[q] + 31) / 32;
     dim3 grid((unsigned)(t.tiles_last * tiles_q), (unsigned)std::min<int64_t>(t.rest_total, 65535));
     if (narrow)
-      permute_kernel_tile<uint32_t><<<grid, dim3(32, 8), 0, c.stream>>>(t);
+      launch_chained(permute_kernel_tile<uint32_t>, grid, dim3(32, 8), c.stream, 1, t);
     else
-      permute_kernel_tile<int64_t><<<grid, dim3(32, 8), 0, c.stream>>>(t);
+      launch_chained(permute_kernel_tile<int64_t>, grid, dim3(32, 8), c.stream, 1, t);
   } else if (a.od[r - 1] >= 32) {
     const int threads = 256;
     const int64_t items = (a.total / a.od[r - 1]) * ((a.od[r - 1] + 127) / 128);
     const int64_t blocks = std::min<int64_t>((items + 7) / 8, 152 * 16);
     if (narrow)
-      permute_kernel_rows<uint32_t><<<(unsigned)blocks, threads, 0, c.stream>>>(a);
+      launch_chained(permute_kernel_rows<uint32_t>, (unsigned)blocks, threads, c.stream, 1, a);
     else
-      permute_kernel_rows<int64_t><<<(unsigned)blocks, threads, 0, c.stream>>>(a);
+      launch_chained(permute_kernel_rows<int64_t>, (unsigned)blocks, threads, c.stream, 1, a);
   } else {
     const int threads = 256;
     const int64_t blocks = std::min<int64_t>((a.total + threads - 1) / threads, 152 * 64);
     if (narrow)
-      permute_kernel_elem<uint32_t><<<(unsigned)blocks, threads, 0, c.stream>>>(a);
+      launch_chained(permute_kernel_elem<uint32_t>, (unsigned)blocks, threads, c.stream, 1, a);
     else
-      permute_kernel_elem<int64_t><<<(unsigned)blocks, threads, 0, c.stream>>>(a);
+      launch_chained(permute_kernel_elem<int64_t>, (unsigned)blocks, threads, c.stream, 1, a);
   }
   count_launch();
   check_launch("permute");
@@ -323,11 +327,13 @@ void permute_add(Ctx& c, const Tensor& in, double alpha, double beta, const Tens
 // ------------------------------------------------------------------------------------
 namespace {
 __global__ void axpby_kernel(int64_t n, double alpha, const double* x, double beta, double* y) {
+  chain_enter();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     y[i] = combine(alpha, x[i], beta, y + i);
   }
 }
 __global__ void fill_kernel(int64_t n, double v, double* y) {
+  chain_enter();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     y[i] = v;
 }
@@ -351,7 +357,7 @@ static void record_flat(Recorder* r, RecordedOp::Kind kind, int64_t n, double al
 void axpby(Ctx& c, int64_t n, double alpha, const double* x, double beta, double* y) {
   if (n <= 0) return;
   if (Recorder* r = recorder()) return record_flat(r, RecordedOp::kPermute, n, alpha, x, beta, y);
-  axpby_kernel<<<grid_for(n), 256, 0, c.stream>>>(n, alpha, x, beta, y);
+  launch_chained(axpby_kernel, grid_for(n), 256, c.stream, 1, n, alpha, x, beta, y);
   count_launch();
   check_launch("axpby");
 }
@@ -359,7 +365,7 @@ void axpby(Ctx& c, int64_t n, double alpha, const double* x, double beta, double
 void fill(Ctx& c, int64_t n, double v, double* y) {
   if (n <= 0) return;
   if (Recorder* r = recorder()) return record_flat(r, RecordedOp::kFill, n, v, nullptr, 0.0, y);
-  fill_kernel<<<grid_for(n), 256, 0, c.stream>>>(n, v, y);
+  launch_chained(fill_kernel, grid_for(n), 256, c.stream, 1, n, v, y);
   count_launch();
   check_launch("fill");
 }
@@ -421,8 +427,9 @@ __device__ void fold_blocks(double tot, double* partial, unsigned int* ticket, d
 }
 
 // sum x y, or sum x (y null)
-__global__ void dot_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ y, double* partial,
-                           unsigned int* ticket, double* out) {
+__global__ void dot_kernel(int64_t n, const double* x, const double* y, double* partial, unsigned int* ticket,
+                           double* out) {
+  chain_enter();
   double s = 0.0, cc = 0.0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     neumaier(s, cc, y ? x[i] * y[i] : x[i]);
@@ -433,9 +440,10 @@ __global__ void dot_kernel(int64_t n, const double* __restrict__ x, const double
 // terms), the block and cross-block folds as above.  The compensated per-element form
 // costs about six FP64 operations per element and bounded this kernel on GB300's FP64
 // pipe; the overlaps only feed the extrapolation coefficients.
-__global__ void multidot_kernel(int64_t n, const double* const* xs, const double* __restrict__ y, double* partial,
+__global__ void multidot_kernel(int64_t n, const double* const* xs, const double* y, double* partial,
                                 unsigned int* tickets, double* out) {
-  const double* __restrict__ x = xs[blockIdx.y];
+  chain_enter();
+  const double* x = xs[blockIdx.y];
   double s0 = 0.0, s1 = 0.0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -452,7 +460,7 @@ void dot_async(Ctx& c, int64_t n, const double* x, const double* y, double* d_ou
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
   const unsigned nb = red_blocks(n);
   Scratch part(c, sizeof(double) * nb);
-  dot_kernel<<<nb, RED_THREADS, 0, c.stream>>>(n, x, y, part.d(), &c.words()->reduce, d_out);
+  launch_chained(dot_kernel, nb, RED_THREADS, c.stream, 1, n, x, y, part.d(), &c.words()->reduce, d_out);
   count_launch();
   check_launch("dot");
 }
@@ -471,7 +479,8 @@ void multidot_async(Ctx& c, int nvec, const double* const* d_xs, const double* y
   if (nvec <= 0) return;
   const unsigned nb = red_blocks(n);
   Scratch part(c, sizeof(double) * nb * nvec);
-  multidot_kernel<<<dim3(nb, nvec), RED_THREADS, 0, c.stream>>>(n, d_xs, y, part.d(), c.words()->tickets, d_out);
+  launch_chained(multidot_kernel, dim3(nb, nvec), RED_THREADS, c.stream, 1, n, d_xs, y, part.d(), c.words()->tickets,
+                 d_out);
   count_launch();
   check_launch("multidot");
 }
@@ -483,6 +492,7 @@ namespace {
 template <class I>
 __global__ void tau_kernel(int no, int nv, const double* t1, const double* t2, double f1, double* tau, double f2,
                            double* ttau) {
+  chain_enter();
   const I n = (I)no * no * nv * nv, v_ = (I)nv, o_ = (I)no;
   for (I x = (I)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (I)gridDim.x * blockDim.x) {
     const I b = x % v_;
@@ -505,6 +515,7 @@ template <class I>
 __global__ void jacobi_kernel(int no, int nv, const double* d_do, const double* d_dv, double shift, const double* R1,
                               const double* R2, const double* t1o, const double* t2o, double* t1n, double* t2n,
                               double* partial, unsigned int* ticket, double* sumsq) {
+  chain_enter();
   const I n1 = (I)no * nv, n2 = (I)no * no * nv * nv, v = (I)nv, o = (I)no;
   double s = 0.0;
   for (I x = (I)blockIdx.x * blockDim.x + threadIdx.x; x < n1 + n2; x += (I)gridDim.x * blockDim.x) {
@@ -531,6 +542,7 @@ __global__ void jacobi_kernel(int no, int nv, const double* d_do, const double* 
 }
 
 __global__ void lincomb_kernel(int nvec, const double* const* vecs, const double* coef, int64_t n, double* out) {
+  chain_enter();
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
     for (int p = 0; p < nvec; p++) s += coef[p] * vecs[p][x];
@@ -544,9 +556,9 @@ void build_tau(Ctx& c, int no, int nv, const double* t1, const double* t2, doubl
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
   const int64_t n = (int64_t)no * no * nv * nv;
   if (n + 152 * 32 * 256 < ((int64_t)1 << 31))
-    tau_kernel<uint32_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, t1, t2, f1, tau, f2, ttau);
+    launch_chained(tau_kernel<uint32_t>, grid_for(n), 256, c.stream, 1, no, nv, t1, t2, f1, tau, f2, ttau);
   else
-    tau_kernel<int64_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, t1, t2, f1, tau, f2, ttau);
+    launch_chained(tau_kernel<int64_t>, grid_for(n), 256, c.stream, 1, no, nv, t1, t2, f1, tau, f2, ttau);
   count_launch();
   check_launch("tau");
 }
@@ -560,11 +572,11 @@ void jacobi_update(Ctx& c, int no, int nv, const double* d_do, const double* d_d
   Scratch part(c, sizeof(double) * nb);
   unsigned int* ticket = &c.words()->reduce;
   if (n + (int64_t)RED_BLOCKS * RED_THREADS < ((int64_t)1 << 31))
-    jacobi_kernel<uint32_t><<<nb, RED_THREADS, 0, c.stream>>>(no, nv, d_do, d_dv, shift, R1, R2, t1old, t2old, t1new,
-                                                              t2new, part.d(), ticket, d_sumsq);
+    launch_chained(jacobi_kernel<uint32_t>, nb, RED_THREADS, c.stream, 1, no, nv, d_do, d_dv, shift, R1, R2, t1old,
+                   t2old, t1new, t2new, part.d(), ticket, d_sumsq);
   else
-    jacobi_kernel<int64_t><<<nb, RED_THREADS, 0, c.stream>>>(no, nv, d_do, d_dv, shift, R1, R2, t1old, t2old, t1new,
-                                                             t2new, part.d(), ticket, d_sumsq);
+    launch_chained(jacobi_kernel<int64_t>, nb, RED_THREADS, c.stream, 1, no, nv, d_do, d_dv, shift, R1, R2, t1old,
+                   t2old, t1new, t2new, part.d(), ticket, d_sumsq);
   count_launch();
   check_launch("jacobi");
 }
@@ -573,7 +585,7 @@ void lincomb(Ctx& c, int nvec, const double* const* d_vecs, const double* coef, 
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
   Scratch dc(c, sizeof(double) * nvec);
   UCC_CUDA(cudaMemcpyAsync(dc.p, coef, sizeof(double) * nvec, cudaMemcpyHostToDevice, c.stream));
-  lincomb_kernel<<<grid_for(n), 256, 0, c.stream>>>(nvec, d_vecs, dc.d(), n, out);
+  launch_chained(lincomb_kernel, grid_for(n), 256, c.stream, 1, nvec, d_vecs, dc.d(), n, out);
   count_launch();
   check_launch("lincomb");
   // the host coefficient array may go out of scope once the copy has been consumed
@@ -1078,6 +1090,7 @@ namespace {
 // K chunk it writes y, otherwise the chunk sums go to P[z][n] for gemv_reduce (fixed order).
 __global__ void gemv_ncontig(int64_t N, int64_t K, int64_t kc, double alpha, const double* x, int64_t sx,
                              const double* A, int64_t sk, int64_t sn, double beta, double* y, int64_t sy, double* P) {
+  chain_enter();
   // blockDim = (32, 8): threadIdx.x over n (coalesced when sn == 1), threadIdx.y over k
   __shared__ double red[8][33];
   const int64_t n = (int64_t)blockIdx.x * 32 + threadIdx.x;
@@ -1096,8 +1109,9 @@ __global__ void gemv_ncontig(int64_t N, int64_t K, int64_t kc, double alpha, con
       y[n * sy] = combine(alpha, t, beta, y + n * sy);
   }
 }
-__global__ void gemv_reduce(int64_t N, int nz, const double* __restrict__ P, double alpha, double beta, double* y,
+__global__ void gemv_reduce(int64_t N, int nz, const double* P, double alpha, double beta, double* y,
                             int64_t sy) {
+  chain_enter();
   for (int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; n < N; n += (int64_t)gridDim.x * blockDim.x) {
     double t = P[n];
     for (int z = 1; z < nz; z++) t += P[(int64_t)z * N + n];
@@ -1106,6 +1120,7 @@ __global__ void gemv_reduce(int64_t N, int nz, const double* __restrict__ P, dou
 }
 __global__ void gemv_kcontig(int64_t N, int64_t K, double alpha, const double* x, int64_t sx, const double* A,
                              int64_t sk, int64_t sn, double beta, double* y, int64_t sy) {
+  chain_enter();
   // one warp per n, lanes over k (coalesced when sk == 1)
   const int64_t n = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
@@ -1134,8 +1149,8 @@ void dgemv_strided(Ctx& c, int64_t N, int64_t K, double alpha, const double* x, 
   }
   if (sk == 1 && sn != 1) {
     const int wpb = 8;
-    gemv_kcontig<<<(unsigned)((N + wpb - 1) / wpb), 32 * wpb, 0, c.stream>>>(N, K, alpha, x, sx, A, sk, sn, beta, y,
-                                                                            sy);
+    launch_chained(gemv_kcontig, (unsigned)((N + wpb - 1) / wpb), 32 * wpb, c.stream, 1, N, K, alpha, x, sx, A, sk,
+                   sn, beta, y, sy);
   } else {
     // enough blocks for ~4 per SM: split K into chunks of at least 256 when the n tiles are few
     const int64_t nb = (N + 31) / 32;
@@ -1144,13 +1159,13 @@ void dgemv_strided(Ctx& c, int64_t N, int64_t K, double alpha, const double* x, 
     const int64_t kc = nz > 1 ? (K + nz - 1) / nz : K;
     if (nz > 1) nz = (K + kc - 1) / kc;
     if (nz <= 1) {
-      gemv_ncontig<<<dim3((unsigned)nb, 1), dim3(32, 8), 0, c.stream>>>(N, K, K, alpha, x, sx, A, sk, sn, beta, y, sy,
-                                                                         nullptr);
+      launch_chained(gemv_ncontig, dim3((unsigned)nb, 1), dim3(32, 8), c.stream, 1, N, K, K, alpha, x, sx, A, sk, sn,
+                     beta, y, sy, nullptr);
     } else {
       Scratch part(c, sizeof(double) * nz * N);
-      gemv_ncontig<<<dim3((unsigned)nb, (unsigned)nz), dim3(32, 8), 0, c.stream>>>(N, K, kc, alpha, x, sx, A, sk, sn,
-                                                                                   beta, y, sy, part.d());
-      gemv_reduce<<<grid_for(N), 256, 0, c.stream>>>(N, (int)nz, part.d(), alpha, beta, y, sy);
+      launch_chained(gemv_ncontig, dim3((unsigned)nb, (unsigned)nz), dim3(32, 8), c.stream, 1, N, K, kc, alpha, x, sx,
+                     A, sk, sn, beta, y, sy, part.d());
+      launch_chained(gemv_reduce, grid_for(N), 256, c.stream, 1, N, (int)nz, part.d(), alpha, beta, y, sy);
       count_launch();
     }
   }

@@ -2,6 +2,7 @@
 // operators and amplitudes, the ring terms' combinations, the doubles residual's assembly.
 #include <algorithm>
 
+#include "chain.h"
 #include "core.h"
 #include "pairs.h"
 
@@ -50,30 +51,31 @@ __global__ void pack_rows_kernel(int64_t rows, int nv, const double* __restrict_
     pack_slice_tile(s, nv, 1.0, H + R * nv2, nullptr, true, false, Vp + R * np, Vm + R * nm, (int)blockIdx.x);
 }
 
-__global__ void pack_tau_kernel(int no, int nv, const double* __restrict__ tau, double* Tp, double* Tm) {
+__global__ void pack_tau_kernel(int no, int nv, const double* tau, double* Tp, double* Tm) {
+  chain_enter();
   __shared__ TileBuf s;
   const int64_t op = (int64_t)no * (no + 1) / 2;
   for (int64_t R = blockIdx.y; R < op; R += gridDim.y) pack_tau_tile(s, no, nv, tau, Tp, Tm, (int)blockIdx.x, R);
 }
 
-__global__ void ring_kernel(int no, int nv, const double* __restrict__ t1, const double* __restrict__ t2, double* X,
-                            double* P, double* S) {
+__global__ void ring_kernel(int no, int nv, const double* t1, const double* t2, double* X, double* P, double* S) {
+  chain_enter();
   __shared__ TileBuf s;
   const int64_t slices = (int64_t)no * no;
   for (int64_t R = blockIdx.y; R < slices; R += gridDim.y) ring_tile(s, no, nv, t1, t2, X, P, S, (int)blockIdx.x, R);
 }
 
-__global__ void assemble_kernel(int no, int nv, const double* __restrict__ V, const double* __restrict__ S,
-                                int64_t ldS, const double* __restrict__ A, int64_t ldA, const double* __restrict__ Rh,
-                                const double* __restrict__ H, double* R2) {
+__global__ void assemble_kernel(int no, int nv, const double* V, const double* S, int64_t ldS, const double* A,
+                                int64_t ldA, const double* Rh, const double* H, double* R2) {
+  chain_enter();
   __shared__ TileBuf s;
   const int64_t op = (int64_t)no * (no + 1) / 2;
   for (int64_t R = blockIdx.y; R < op; R += gridDim.y)
     assemble_tile(s, no, nv, V, S, ldS, A, ldA, Rh, H, R2, (int)blockIdx.x, R);
 }
 
-__global__ void unpack_z_kernel(int no, int nv, const double* __restrict__ S, int64_t ldS,
-                                const double* __restrict__ A, int64_t ldA, double* Z) {
+__global__ void unpack_z_kernel(int no, int nv, const double* S, int64_t ldS, const double* A, int64_t ldA, double* Z) {
+  chain_enter();
   const int64_t n = (int64_t)no * no * no * nv;
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x)
     Z[x] = z_element(no, nv, S, ldS, A, ldA, x);
@@ -81,8 +83,8 @@ __global__ void unpack_z_kernel(int no, int nv, const double* __restrict__ S, in
 
 // R2[ijab] += alpha * unpack_pair
 template <class I>
-__global__ void unpack_ladder_kernel(int no, int nv, double alpha, const double* __restrict__ S,
-                                     const double* __restrict__ A, double* R2) {
+__global__ void unpack_ladder_kernel(int no, int nv, double alpha, const double* S, const double* A, double* R2) {
+  chain_enter();
   const I n = (I)no * no * nv * nv;
   for (I x = (I)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (I)gridDim.x * blockDim.x)
     R2[x] = fma(alpha, unpack_pair<I>(no, nv, S, A, x), R2[x]);
@@ -123,14 +125,15 @@ static void record(RecordedOp::Kind kind, int no, int nv, const std::vector<cons
 
 void pack_tau(Ctx& c, int no, int nv, const double* tau, double* Tp, double* Tm) {
   if (recorder()) return record(RecordedOp::kPackTau, no, nv, {tau}, {Tp, Tm});
-  pack_tau_kernel<<<tile_grid(tile_pairs(nv), (int64_t)no * (no + 1) / 2), kBlock, 0, c.stream>>>(no, nv, tau, Tp, Tm);
+  launch_chained(pack_tau_kernel, tile_grid(tile_pairs(nv), (int64_t)no * (no + 1) / 2), kBlock, c.stream, 1, no, nv,
+                 tau, Tp, Tm);
   launched("pack_tau");
 }
 
 void ring_amplitudes(Ctx& c, int no, int nv, const double* t1, const double* t2, double* X, double* P, double* S) {
   if (recorder()) return record(RecordedOp::kRing, no, nv, {t1, t2}, {X, P, S});
   const int64_t nt = (nv + 31) / 32;
-  ring_kernel<<<tile_grid(nt * nt, (int64_t)no * no), kBlock, 0, c.stream>>>(no, nv, t1, t2, X, P, S);
+  launch_chained(ring_kernel, tile_grid(nt * nt, (int64_t)no * no), kBlock, c.stream, 1, no, nv, t1, t2, X, P, S);
   launched("ring_amplitudes");
 }
 
@@ -138,15 +141,15 @@ void assemble_r2(Ctx& c, int no, int nv, const double* V, const double* S, const
                  const double* H, double* R2) {
   if (recorder()) return record(RecordedOp::kAssemble, no, nv, {V, S, A, Rh, H}, {R2});
   const PairLd ld(no, nv);
-  assemble_kernel<<<tile_grid(tile_pairs(nv), (int64_t)no * (no + 1) / 2), kBlock, 0, c.stream>>>(
-      no, nv, V, S, ld.s, A, ld.a, Rh, H, R2);
+  launch_chained(assemble_kernel, tile_grid(tile_pairs(nv), (int64_t)no * (no + 1) / 2), kBlock, c.stream, 1, no, nv, V,
+                 S, ld.s, A, ld.a, Rh, H, R2);
   launched("assemble_r2");
 }
 
 void unpack_z(Ctx& c, int no, int nv, const double* S, const double* A, double* Z) {
   if (recorder()) return record(RecordedOp::kUnpackZ, no, nv, {S, A}, {Z});
   const PairLd ld(no, nv);
-  unpack_z_kernel<<<grid_for((int64_t)no * no * no * nv), 256, 0, c.stream>>>(no, nv, S, ld.s, A, ld.a, Z);
+  launch_chained(unpack_z_kernel, grid_for((int64_t)no * no * no * nv), 256, c.stream, 1, no, nv, S, ld.s, A, ld.a, Z);
   launched("unpack_z");
 }
 
@@ -154,9 +157,9 @@ void unpack_ladder(Ctx& c, int no, int nv, double alpha, const double* S, const 
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
   const int64_t n = (int64_t)no * no * nv * nv;
   if (n + 152 * 32 * 256 < ((int64_t)1 << 31))
-    unpack_ladder_kernel<uint32_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, alpha, S, A, R2);
+    launch_chained(unpack_ladder_kernel<uint32_t>, grid_for(n), 256, c.stream, 1, no, nv, alpha, S, A, R2);
   else
-    unpack_ladder_kernel<int64_t><<<grid_for(n), 256, 0, c.stream>>>(no, nv, alpha, S, A, R2);
+    launch_chained(unpack_ladder_kernel<int64_t>, grid_for(n), 256, c.stream, 1, no, nv, alpha, S, A, R2);
   launched("unpack_ladder");
 }
 
