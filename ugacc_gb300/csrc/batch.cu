@@ -1031,8 +1031,15 @@ ucc_status ucc_batch_create(ucc_batch** out, int device) {
 
 ucc_status ucc_batch_destroy(ucc_batch* b) {
   if (!b) return UCC_BAD_ARGS;
-  cudaSetDevice(b->device);
+  const int device = b->device;
+  cudaSetDevice(device);
   delete b;
+  // the members' blocks went back to the stream-ordered pool, which keeps them: hand them back
+  cudaMemPool_t pool;
+  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
+    cudaDeviceSynchronize();
+    cudaMemPoolTrimTo(pool, 0);
+  }
   return UCC_OK;
 }
 

@@ -33,6 +33,7 @@ Ctx::~Ctx() {
   }
   for (auto e : event_pool) cudaEventDestroy(e);
   if (words_) cudaFree(words_);
+  for (double* h : host_all) cudaFreeHost(h);
   anchors.clear();  // pool buffers are freed on the stream
   tc_cache.reset();
   perts.clear();

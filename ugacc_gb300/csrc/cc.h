@@ -26,21 +26,25 @@ Tensor narrow(const Tensor& t, int axis, int64_t start, int64_t len);
 // used through psi4's DIISManager at ccwfn.cc:206-221.
 class Diis {
  public:
-  Diis(Ctx& c, int64_t n, int nmax = 8);
-  ~Diis();
-  void add(const double* vnew, const double* vold);
+  Diis(Ctx& c, int64_t n, int nmax = VecList::kMax);
+  // The entry that a sweep fills before it is known whether the entry counts: err() = new - old
+  // and vec() = new by the Jacobi update, its overlaps (nmax words, host) by overlaps(), all
+  // read with the residual norm behind one wait; accept() then adds it.
+  double* err() { return err_.p + (size_t)slot() * n_; }
+  double* vec() { return vec_.p + (size_t)slot() * n_; }
+  void overlaps(double* out);
+  void accept(const HostBlock& h, int first);
   int size() const { return count_; }
   void extrapolate(double* out);
   void reset();
 
  private:
+  int slot() const { return count_ < nmax_ ? count_ : (int)(nadded_ % nmax_); }
   Ctx& c_;
   int64_t n_;
   int nmax_, count_ = 0;
   long nadded_ = 0;
   DeviceBuffer err_, vec_;
-  const double** d_errp_ = nullptr;
-  const double** d_vecp_ = nullptr;
   std::vector<double> B_;
 };
 

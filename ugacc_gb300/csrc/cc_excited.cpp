@@ -232,7 +232,7 @@ CCSDResult run_lambda(Ctx& c) {  // :93-129
     c.drop("Lam_guess");
   }
   Tensor eps = c.get("eps");
-  Scratch sumsq(c, sizeof(double));
+  HostBlock sums(c);  // of a sweep: sum of squares, then the DIIS overlaps
   Diis diis(c, np, 8);
   auto pseudo = [&](double* buf) { return 0.5 * dot_all(c, V(c, "oovv"), amp2(c, buf)); };
   if (c.opt.print) {
@@ -258,11 +258,11 @@ CCSDResult run_lambda(Ctx& c) {  // :93-129
       lambda_l2(c, l1, l2, Goo, Gvv, amp2(c, r));
     }
     sw.end();
-    jacobi_update(c, no, nv, eps.p, eps.p + no, 0.0, r, r + n1, lo, lo + n1, ln, ln + n1, sumsq.d());
-    double ss = 0.0;
-    UCC_CUDA(cudaMemcpyAsync(&ss, sumsq.p, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    jacobi_update(c, no, nv, eps.p, eps.p + no, 0.0, r, r + n1, lo, lo + n1, ln, ln + n1, sums.p,
+                  c.opt.diis ? diis.err() : nullptr, c.opt.diis ? diis.vec() : nullptr);
+    if (c.opt.diis) diis.overlaps(sums.p + 1);
     UCC_CUDA(cudaStreamSynchronize(c.stream));
-    rms = std::sqrt(ss);
+    rms = std::sqrt(sums[0]);
     tc_check(c);
     UCC_REQUIRE(std::isfinite(rms), UCC_NAN_DETECTED, "Lambda residual is not finite");
     bool restart = false;
@@ -272,7 +272,7 @@ CCSDResult run_lambda(Ctx& c) {  // :93-129
     }
     if (restart) diis.reset();
     if (c.opt.diis && !restart) {
-      diis.add(ln, lo);
+      diis.accept(sums, 1);
       if (diis.size() > 2) diis.extrapolate(ln);
     }
     if (c.opt.print) {

@@ -151,37 +151,19 @@ Tensor Fk(Ctx& c, const std::string& b) { return c.get("f" + b); }
 // DIIS
 // ---------------------------------------------------------------------------------------
 Diis::Diis(Ctx& c, int64_t n, int nmax)
-    : c_(c), n_(n), nmax_(nmax), err_((size_t)n * nmax), vec_((size_t)n * nmax), B_((size_t)nmax * nmax, 0.0) {
-  UCC_CUDA(cudaMalloc(&d_errp_, sizeof(double*) * nmax));
-  UCC_CUDA(cudaMalloc(&d_vecp_, sizeof(double*) * nmax));
-  std::vector<const double*> e(nmax), v(nmax);
-  for (int p = 0; p < nmax; p++) {
-    e[p] = err_.p + (size_t)p * n;
-    v[p] = vec_.p + (size_t)p * n;
-  }
-  UCC_CUDA(cudaMemcpy(d_errp_, e.data(), sizeof(double*) * nmax, cudaMemcpyHostToDevice));
-  UCC_CUDA(cudaMemcpy(d_vecp_, v.data(), sizeof(double*) * nmax, cudaMemcpyHostToDevice));
-}
+    : c_(c), n_(n), nmax_(nmax), err_((size_t)n * nmax, c.stream), vec_((size_t)n * nmax, c.stream),
+      B_((size_t)nmax * nmax, 0.0) {}
 
-Diis::~Diis() {
-  cudaFree(d_errp_);
-  cudaFree(d_vecp_);
-}
-
-void Diis::add(const double* vnew, const double* vold) {
-  const int slot = count_ < nmax_ ? count_ : (int)(nadded_ % nmax_);
-  double* e = err_.p + (size_t)slot * n_;
-  double* v = vec_.p + (size_t)slot * n_;
-  axpby(c_, n_, 1.0, vnew, 0.0, e);
-  axpby(c_, n_, -1.0, vold, 1.0, e);
-  UCC_CUDA(cudaMemcpyAsync(v, vnew, sizeof(double) * n_, cudaMemcpyDeviceToDevice, c_.stream));
+void Diis::overlaps(double* out) {
+  VecList e;
   const int cnt = std::min(count_ + 1, nmax_);
-  Scratch d(c_, sizeof(double) * nmax_);
-  multidot_async(c_, cnt, d_errp_, e, n_, d.d());
-  std::vector<double> row(cnt);
-  UCC_CUDA(cudaMemcpyAsync(row.data(), d.p, sizeof(double) * cnt, cudaMemcpyDeviceToHost, c_.stream));
-  UCC_CUDA(cudaStreamSynchronize(c_.stream));
-  for (int p = 0; p < cnt; p++) B_[(size_t)slot * nmax_ + p] = B_[(size_t)p * nmax_ + slot] = row[p];
+  for (int p = 0; p < cnt; p++) e.p[p] = err_.p + (size_t)p * n_;
+  multidot_async(c_, cnt, e, err(), n_, out);
+}
+
+void Diis::accept(const HostBlock& h, int first) {
+  const int s = slot(), cnt = std::min(count_ + 1, nmax_);
+  for (int p = 0; p < cnt; p++) B_[(size_t)s * nmax_ + p] = B_[(size_t)p * nmax_ + s] = h[first + p];
   count_ = cnt;
   nadded_++;
 }
@@ -238,8 +220,10 @@ void Diis::extrapolate(double* out) {
   std::vector<double> Bn((size_t)n * n);
   for (int p = 0; p < n; p++)
     for (int q = 0; q < n; q++) Bn[(size_t)p * n + q] = B_[(size_t)p * nmax_ + q];
-  std::vector<double> coef = diis_coefficients(Bn, n);
-  lincomb(c_, n, d_vecp_, coef.data(), n_, out);
+  const std::vector<double> coef = diis_coefficients(Bn, n);
+  VecList v;
+  for (int p = 0; p < n; p++) v.p[p] = vec_.p + (size_t)p * n_, v.coef[p] = coef[p];
+  lincomb(c_, n, v, n_, out);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -440,15 +424,18 @@ void residual(Ctx& c, const double* t_old, double* r, std::vector<cudaEvent_t>* 
   build_t2(c, t1, t2, tau, S, pairs, amp2(c, r));
 }
 
-double energy(Ctx& c, const Tensor& t1, const Tensor& tau) {
-  const int no = c.no, nv = c.nv, n = no + nv;
-  // ccwfn.cc:270-273 assigns instead of accumulating: only the last (i,a) pair counts
-  DotList d(c);
-  const int two = dot_all(c, tau, L(c, "oovv"), d);
-  const int last = d.add(1, t1.p + (int64_t)no * nv - 1, nullptr);
-  d.fetch();
-  return 2.0 * c.fock[(size_t)(no - 1) * n + (n - 1)] * d[last] + d[two];
-}
+// ccwfn.cc:270-273 assigns instead of accumulating: only the last (i,a) pair counts
+struct Energy {
+  DotList d;
+  double fov;
+  int two, last;
+  Energy(Ctx& c, const Tensor& t1, const Tensor& tau)
+      : d(c), fov(c.fock[(size_t)(c.no - 1) * (c.no + c.nv) + (c.no + c.nv - 1)]) {
+    two = dot_all(c, tau, L(c, "oovv"), d);
+    last = d.add(1, t1.p + (int64_t)c.no * c.nv - 1, nullptr);
+  }
+  double value() const { return 2.0 * fov * d[last] + d[two]; }  // after a wait for the stream
+};
 
 }  // namespace
 
@@ -471,7 +458,11 @@ void ccsd_alloc(Ctx& c) {
 
 void ccsd_residual(Ctx& c, const double* t_old, double* r) { residual(c, t_old, r, nullptr); }
 
-double ccsd_energy(Ctx& c, const double* t) { return energy(c, amp1(c, const_cast<double*>(t)), c.get("tau")); }
+double ccsd_energy(Ctx& c, const double* t) {
+  Energy e(c, amp1(c, const_cast<double*>(t)), c.get("tau"));
+  e.d.fetch();
+  return e.value();
+}
 
 // residual norm near which BF16 hi+lo split products with FP32 accumulation stop
 // resolving the update (measured ~1.5e-6 at no=16/nv=160)
@@ -587,7 +578,7 @@ CCSDResult run_ccsd(Ctx& c) {
   Tensor eps = c.get("eps");
   const double* d_do = eps.p;
   const double* d_dv = eps.p + no;
-  Scratch sumsq(c, sizeof(double));
+  HostBlock sums(c);  // of a sweep: sum of squares, then the DIIS overlaps
 
   // MP2 guess t1 = f_ia / D1, t2 = <ij|ab> / D2 (ccwfn.cc:75-87), unless amplitudes were given
   if (!c.has("T_guess")) {
@@ -595,7 +586,7 @@ CCSDResult run_ccsd(Ctx& c) {
     copy_into(c, Fk(c, "ov"), amp1(c, R0->p));
     copy_into(c, V(c, "oovv"), amp2(c, R0->p));
     jacobi_update(c, no, nv, d_do, d_dv, 0.0, R0->p, R0->p + (int64_t)no * nv, Told.p, Told.p + (int64_t)no * nv, T.p,
-                  T.p + (int64_t)no * nv, sumsq.d());
+                  T.p + (int64_t)no * nv, sums.p);
   } else {  // a supplied guess (restart file, learned guess) applies to this solve only
     UCC_CUDA(cudaMemcpyAsync(T.p, c.get("T_guess").p, sizeof(double) * np, cudaMemcpyDeviceToDevice, c.stream));
     UCC_CUDA(cudaStreamSynchronize(c.stream));
@@ -606,7 +597,10 @@ CCSDResult run_ccsd(Ctx& c) {
   };
   tau_of(c.get("T").p);
   CCSDResult res;
-  res.e_mp2 = energy(c, amp1(c, c.get("T").p), c.get("tau"));
+  auto en = std::make_unique<Energy>(c, amp1(c, c.get("T").p), c.get("tau"));
+  en->d.fetch();
+  res.e_mp2 = en->value();
+  en.reset();
   if (c.opt.print) {
     std::printf("\n\tThe Coupled-Cluster Iteration:\n");
     std::printf("\t---------------------------------------------------\n");
@@ -656,11 +650,11 @@ CCSDResult run_ccsd(Ctx& c) {
       }
     }
     jacobi_update(c, no, nv, d_do, d_dv, 0.0, r, r + (int64_t)no * nv, to, to + (int64_t)no * nv, tn,
-                  tn + (int64_t)no * nv, sumsq.d());
-    double ss = 0.0;
-    UCC_CUDA(cudaMemcpyAsync(&ss, sumsq.p, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    UCC_CUDA(cudaStreamSynchronize(c.stream));
-    rms = std::sqrt(ss);
+                  tn + (int64_t)no * nv, sums.p, c.opt.diis ? diis.err() : nullptr, c.opt.diis ? diis.vec() : nullptr);
+    if (c.opt.diis) diis.overlaps(sums.p + 1);
+    UCC_CUDA(cudaStreamSynchronize(c.stream));  // the only wait of a sweep
+    if (en) eccsd = en->value();
+    rms = std::sqrt(sums[0]);
     tc_check(c);
     UCC_REQUIRE(std::isfinite(rms), UCC_NAN_DETECTED, "CCSD residual is not finite");
     bool restart = false;
@@ -670,12 +664,14 @@ CCSDResult run_ccsd(Ctx& c) {
     }
     if (restart) diis.reset();
     if (c.opt.diis && !restart) {
-      diis.add(tn, to);
+      diis.accept(sums, 1);
       if (diis.size() > 2) diis.extrapolate(tn);
     }
     tau_of(tn);
-    eccsd = energy(c, amp1(c, tn), c.get("tau"));
+    en = std::make_unique<Energy>(c, amp1(c, tn), c.get("tau"));
     if (c.opt.print) {
+      en->d.fetch();
+      eccsd = en->value();
       double t1n = std::sqrt(dot(c, (int64_t)no * nv, tn, tn) / (2 * no));
       static const char* tag[] = {"", " split", " record", " delta"};
       const auto t_now = std::chrono::steady_clock::now();
@@ -694,6 +690,7 @@ CCSDResult run_ccsd(Ctx& c) {
   const int fp64_iters = mixed ? sw.record : std::min(iter, c.opt.maxiter);
   tau_of(c.get("T").p);
   UCC_CUDA(cudaStreamSynchronize(c.stream));
+  if (en) eccsd = en->value();
   for (size_t k = 0; k + 1 < ev.size(); k += 2) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ev[k], ev[k + 1]);

@@ -382,13 +382,15 @@ int pert_create(Ctx& c, const double* pert, double omega) {
   pp->omega = omega;
   pp->pfx = "P" + std::to_string(pp->id) + ":";
   Perturbation& p = *pp;
+  std::vector<double> blocks[4];  // read by the copies until the wait below
+  int nb = 0;
   auto put = [&](const char* nm, int r0, int nr, int c0, int nc) {
-    std::vector<double> h((size_t)nr * nc);
+    std::vector<double>& h = blocks[nb++];
+    h.resize((size_t)nr * nc);
     for (int i = 0; i < nr; i++)
       for (int j = 0; j < nc; j++) h[(size_t)i * nc + j] = pert[(size_t)(r0 + i) * n + c0 + j];
     Tensor t = c.alloc(p.pfx + nm, {nr, nc}, false);
     UCC_CUDA(cudaMemcpyAsync(t.p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice, c.stream));
-    UCC_CUDA(cudaStreamSynchronize(c.stream));
   };
   put("poo", 0, no, 0, no);
   put("pov", 0, no, no, nv);
@@ -426,7 +428,7 @@ CCSDResult pert_solve(Ctx& c, int h, bool right) {  // ccpert.cc:177-229
   const int64_t np = npacked(c), n1 = (int64_t)no * nv;
   const std::string cur = p.pfx + (right ? "X" : "Y"), old = p.pfx + (right ? "Xold" : "Yold");
   Tensor hd = c.get("Hdiag");
-  Scratch sumsq(c, sizeof(double));
+  HostBlock sums(c);  // of a sweep: sum of squares, then the DIIS overlaps
   Temp R(c, {np});
   Diis diis(c, np, 8);
   if (c.opt.print) {
@@ -451,11 +453,11 @@ CCSDResult pert_solve(Ctx& c, int h, bool right) {  // ccpert.cc:177-229
         build_Y(c, p, amp1(c, o), amp2(c, o), amp1(c, R->p), amp2(c, R->p));
     }
     sw.end();
-    jacobi_update(c, no, nv, hd.p, hd.p + no, p.omega, R->p, R->p + n1, o, o + n1, nw, nw + n1, sumsq.d());
-    double ss = 0.0;
-    UCC_CUDA(cudaMemcpyAsync(&ss, sumsq.p, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    jacobi_update(c, no, nv, hd.p, hd.p + no, p.omega, R->p, R->p + n1, o, o + n1, nw, nw + n1, sums.p,
+                  c.opt.diis ? diis.err() : nullptr, c.opt.diis ? diis.vec() : nullptr);
+    if (c.opt.diis) diis.overlaps(sums.p + 1);
     UCC_CUDA(cudaStreamSynchronize(c.stream));
-    rms = std::sqrt(ss);
+    rms = std::sqrt(sums[0]);
     tc_check(c);
     UCC_REQUIRE(std::isfinite(rms), UCC_NAN_DETECTED, "perturbed-wavefunction residual is not finite");
     bool restart = false;
@@ -465,7 +467,7 @@ CCSDResult pert_solve(Ctx& c, int h, bool right) {  // ccpert.cc:177-229
     }
     if (restart) diis.reset();
     if (c.opt.diis && !restart) {
-      diis.add(nw, o);
+      diis.accept(sums, 1);
       if (diis.size() > 2) diis.extrapolate(nw);
     }
     if (c.opt.print) {

@@ -123,12 +123,18 @@ struct PoolBuffer {
   PoolBuffer& operator=(const PoolBuffer&) = delete;
 };
 
-// Owned device buffer (cudaMalloc; freed on destruction).
+// Owned device buffer.  With a stream, up to kPooled bytes come from the stream-ordered pool
+// (0.7 us; cudaMalloc and cudaFree take 10 to 25 us each and wait for the device, 10 % of a
+// solve at no=5/nv=19), to be used on that stream or after a wait for it.  Larger ones, and those
+// without a stream, are cudaMalloc's: what the pool holds back is not there for the cached
+// tensor-core operands of a large problem.
 struct DeviceBuffer {
+  static constexpr size_t kPooled = (size_t)32 << 20;
   double* p = nullptr;
   size_t n = 0;
+  cudaStream_t pool = nullptr;  // of a pooled buffer
   DeviceBuffer() = default;
-  explicit DeviceBuffer(size_t count);
+  explicit DeviceBuffer(size_t count, cudaStream_t stream = nullptr);
   ~DeviceBuffer();
   DeviceBuffer(const DeviceBuffer&) = delete;
   DeviceBuffer& operator=(const DeviceBuffer&) = delete;
@@ -256,6 +262,8 @@ struct Ctx {
   };
   DeviceWords* words();
   DeviceWords* words_ = nullptr;
+  std::vector<double*> host_free;  // HostBlocks not in use
+  std::vector<double*> host_all;
   double short_gemm_flops = 0.0;  // of the GEMMs that `total` times, until resolve_timers
   int64_t short_gemm_launches = 0;
 
@@ -350,31 +358,48 @@ void fill(Ctx& c, int64_t n, double v, double* y);
 // Sum of x[k] * y[k] (y == nullptr: sum of x) with compensated FP64 accumulation; the
 // result stays on the device.
 void dot_async(Ctx& c, int64_t n, const double* x, const double* y, double* d_out);
+// Host memory that the kernels of a context's stream write their scalars to, read after a wait
+// for the stream: no copy behind the kernel.  The blocks belong to the context.  A wait, with
+// the idle time until the next kernel, takes 15 to 25 us; a sweep of a solve has one, for its
+// norm, DIIS overlaps and (CCSD) the energy of the sweep before.  With five of them, copies for
+// the DIIS coefficients and entries, and cudaMalloc for every block, the solve at no=5/nv=19
+// took 1.67 ms (1.43 now), six perturbed solves at no=6/nv=22 18.4 ms (14.9).
+struct HostBlock {
+  static constexpr int kWords = 32;
+  Ctx& c;
+  double* p;
+  explicit HostBlock(Ctx& ctx);
+  ~HostBlock() { c.host_free.push_back(p); }
+  HostBlock(const HostBlock&) = delete;
+  HostBlock& operator=(const HostBlock&) = delete;
+  double operator[](int k) const { return static_cast<volatile const double*>(p)[k]; }
+};
 // Dot products whose values are read together: one wait for all of them.
 class DotList {
  public:
-  explicit DotList(Ctx& c) : c_(c), out_(c, sizeof(double) * kMax) {}
+  explicit DotList(Ctx& c) : c_(c), out_(c) {}
   int add(int64_t n, const double* x, const double* y) {
-    UCC_REQUIRE(count_ < kMax, UCC_BAD_ARGS, "too many dot products in one list");
-    dot_async(c_, n, x, y, out_.d() + count_);
+    UCC_REQUIRE(count_ < HostBlock::kWords, UCC_BAD_ARGS, "too many dot products in one list");
+    dot_async(c_, n, x, y, out_.p + count_);
     return count_++;
   }
-  void fetch() {
-    UCC_CUDA(cudaMemcpyAsync(h_, out_.d(), sizeof(double) * count_, cudaMemcpyDeviceToHost, c_.stream));
-    UCC_CUDA(cudaStreamSynchronize(c_.stream));
-  }
-  double operator[](int k) const { return h_[k]; }
+  void fetch() { UCC_CUDA(cudaStreamSynchronize(c_.stream)); }
+  double operator[](int k) const { return out_[k]; }
 
  private:
-  static constexpr int kMax = 32;
   Ctx& c_;
-  Scratch out_;
+  HostBlock out_;
   int count_ = 0;
-  double h_[kMax] = {};
 };
 double dot(Ctx& c, int64_t n, const double* x, const double* y);
-// Several dot products x_k . y at once (DIIS B-matrix row), results on the device.
-void multidot_async(Ctx& c, int nvec, const double* const* d_xs, const double* y, int64_t n, double* d_out);
+// Up to kMax vectors and coefficients, passed to a kernel by value.
+struct VecList {
+  static constexpr int kMax = 8;
+  const double* p[kMax] = {};
+  double coef[kMax] = {};
+};
+// Several dot products x_k . y at once (DIIS B-matrix row).
+void multidot_async(Ctx& c, int nvec, const VecList& xs, const double* y, int64_t n, double* out);
 
 // tau = t2 + f1 * t1(i,a) t1(j,b); ttau = t2 + f2 * t1 t1
 void build_tau(Ctx& c, int no, int nv, const double* t1, const double* t2, double f1, double* tau, double f2,
@@ -382,13 +407,14 @@ void build_tau(Ctx& c, int no, int nv, const double* t1, const double* t2, doubl
 
 // Jacobi update t_new = t_old + R / (D + shift), D built on the fly from the diagonals
 // do[no], dv[nv] in the reference's order ((d_i + d_j) - d_a) - d_b; the sum of R^2
-// (compensated) goes to the device scalar d_sumsq.
+// (compensated) goes to *sumsq.  With e, the packed [1 | 2] vectors e = t_new - t_old and
+// v = t_new are written as well (a DIIS entry).
 void jacobi_update(Ctx& c, int no, int nv, const double* d_do, const double* d_dv, double shift, const double* R1,
                    const double* R2, const double* t1old, const double* t2old, double* t1new, double* t2new,
-                   double* d_sumsq);
+                   double* sumsq, double* e = nullptr, double* v = nullptr);
 
-// out = sum_p coef[p] * vecs[p] (device pointers, host coefficients), n elements
-void lincomb(Ctx& c, int nvec, const double* const* d_vecs, const double* coef, int64_t n, double* out);
+// out = sum_p coef[p] * p[p] over the first nvec vectors, n elements
+void lincomb(Ctx& c, int nvec, const VecList& vecs, int64_t n, double* out);
 
 // (T) energy over a batch of (i>=j>=k) tuples, given W3 for each tuple.
 // W3 of the n tuples in d_list (2 t + 0: exchange a and b, + 1: exchange b and c), in place: W3 + W3(exchanged)

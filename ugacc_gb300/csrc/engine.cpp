@@ -56,11 +56,33 @@ Tensor Tensor::slice0(int64_t i) const {
   return r;
 }
 
-DeviceBuffer::DeviceBuffer(size_t count) : n(count) {
-  if (count) UCC_CUDA(cudaMalloc(&p, count * sizeof(double)));
+DeviceBuffer::DeviceBuffer(size_t count, cudaStream_t stream) : n(count) {
+  if (!count) return;
+  if (stream && count * sizeof(double) <= kPooled) {
+    UCC_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&p), count * sizeof(double), stream));
+    pool = stream;
+  } else {
+    UCC_CUDA(cudaMalloc(&p, count * sizeof(double)));
+  }
 }
 DeviceBuffer::~DeviceBuffer() {
-  if (p) cudaFree(p);
+  if (!p) return;
+  if (pool)
+    cudaFreeAsync(p, pool);
+  else
+    cudaFree(p);
+}
+
+HostBlock::HostBlock(Ctx& ctx) : c(ctx) {
+  if (c.host_free.empty()) {
+    void* h = nullptr;
+    UCC_CUDA(cudaHostAlloc(&h, sizeof(double) * kWords, cudaHostAllocPortable));
+    c.host_all.push_back(static_cast<double*>(h));
+    c.host_free.reserve(c.host_all.size());  // returning a block does not allocate
+    c.host_free.push_back(c.host_all.back());
+  }
+  p = c.host_free.back();
+  c.host_free.pop_back();
 }
 
 Scratch::Scratch(Ctx& c, size_t bytes) : ctx(&c) {
@@ -134,7 +156,7 @@ Tensor Ctx::alloc(const std::string& name, const std::vector<int64_t>& dims, boo
   auto it = store.find(name);
   if (it == store.end() || it->second->n != n) {
     store[name].reset();
-    store[name] = std::make_unique<DeviceBuffer>(n);
+    store[name] = std::make_unique<DeviceBuffer>(n, stream);
   }
   shapes[name] = dims;
   if (zero && n) UCC_CUDA(cudaMemsetAsync(store[name]->p, 0, n * sizeof(double), stream));

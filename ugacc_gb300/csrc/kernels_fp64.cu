@@ -440,10 +440,10 @@ __global__ void dot_kernel(int64_t n, const double* x, const double* y, double* 
 // terms), the block and cross-block folds as above.  The compensated per-element form
 // costs about six FP64 operations per element and bounded this kernel on GB300's FP64
 // pipe; the overlaps only feed the extrapolation coefficients.
-__global__ void multidot_kernel(int64_t n, const double* const* xs, const double* y, double* partial,
+__global__ void multidot_kernel(int64_t n, const __grid_constant__ VecList xs, const double* y, double* partial,
                                 unsigned int* tickets, double* out) {
   chain_enter();
-  const double* x = xs[blockIdx.y];
+  const double* x = xs.p[blockIdx.y];
   double s0 = 0.0, s1 = 0.0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -466,21 +466,18 @@ void dot_async(Ctx& c, int64_t n, const double* x, const double* y, double* d_ou
 }
 
 double dot(Ctx& c, int64_t n, const double* x, const double* y) {
-  Scratch out(c, sizeof(double));
-  dot_async(c, n, x, y, out.d());
-  double h = 0.0;
-  UCC_CUDA(cudaMemcpyAsync(&h, out.d(), sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-  UCC_CUDA(cudaStreamSynchronize(c.stream));
-  return h;
+  DotList d(c);
+  d.add(n, x, y);
+  d.fetch();
+  return d[0];
 }
 
-void multidot_async(Ctx& c, int nvec, const double* const* d_xs, const double* y, int64_t n, double* d_out) {
+void multidot_async(Ctx& c, int nvec, const VecList& xs, const double* y, int64_t n, double* out) {
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
   if (nvec <= 0) return;
   const unsigned nb = red_blocks(n);
   Scratch part(c, sizeof(double) * nb * nvec);
-  launch_chained(multidot_kernel, dim3(nb, nvec), RED_THREADS, c.stream, 1, n, d_xs, y, part.d(), c.words()->tickets,
-                 d_out);
+  launch_chained(multidot_kernel, dim3(nb, nvec), RED_THREADS, c.stream, 1, n, xs, y, part.d(), c.words()->tickets, out);
   count_launch();
   check_launch("multidot");
 }
@@ -514,7 +511,7 @@ __global__ void tau_kernel(int no, int nv, const double* t1, const double* t2, d
 template <class I>
 __global__ void jacobi_kernel(int no, int nv, const double* d_do, const double* d_dv, double shift, const double* R1,
                               const double* R2, const double* t1o, const double* t2o, double* t1n, double* t2n,
-                              double* partial, unsigned int* ticket, double* sumsq) {
+                              double* partial, unsigned int* ticket, double* sumsq, double* err, double* vec) {
   chain_enter();
   const I n1 = (I)no * nv, n2 = (I)no * no * nv * nv, v = (I)nv, o = (I)no;
   double s = 0.0;
@@ -523,7 +520,9 @@ __global__ void jacobi_kernel(int no, int nv, const double* d_do, const double* 
       const I a = x % v, i = x / v;
       const double r = R1[x];
       s = fma(r, r, s);
-      t1n[x] = t1o[x] + r / ((d_do[i] - d_dv[a]) + shift);
+      const double told = t1o[x], tnew = told + r / ((d_do[i] - d_dv[a]) + shift);
+      t1n[x] = tnew;
+      if (err) err[x] = tnew - told, vec[x] = tnew;
     } else {
       const I y = x - n1;
       const I b = y % v;
@@ -535,17 +534,21 @@ __global__ void jacobi_kernel(int no, int nv, const double* d_do, const double* 
       const double r = R2[y];
       s = fma(r, r, s);
       const double D = ((d_do[i] + d_do[j]) - d_dv[a]) - d_dv[b];
-      t2n[y] = t2o[y] + r / (D + shift);
+      const double told = t2o[y], tnew = told + r / (D + shift);
+      t2n[y] = tnew;
+      if (err) err[x] = tnew - told, vec[x] = tnew;
     }
   }
   fold_blocks(block_sum(s), partial, ticket, sumsq);
 }
 
-__global__ void lincomb_kernel(int nvec, const double* const* vecs, const double* coef, int64_t n, double* out) {
+__global__ void lincomb_kernel(int nvec, const __grid_constant__ VecList vecs, int64_t n, double* out) {
   chain_enter();
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
-    for (int p = 0; p < nvec; p++) s += coef[p] * vecs[p][x];
+#pragma unroll
+    for (int p = 0; p < VecList::kMax; p++)
+      if (p < nvec) s += vecs.coef[p] * vecs.p[p][x];
     out[x] = s;
   }
 }
@@ -565,7 +568,7 @@ void build_tau(Ctx& c, int no, int nv, const double* t1, const double* t2, doubl
 
 void jacobi_update(Ctx& c, int no, int nv, const double* d_do, const double* d_dv, double shift, const double* R1,
                    const double* R2, const double* t1old, const double* t2old, double* t1new, double* t2new,
-                   double* d_sumsq) {
+                   double* sumsq, double* e, double* v) {
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
   const int64_t n = (int64_t)no * nv + (int64_t)no * no * nv * nv;
   const unsigned nb = red_blocks(n);
@@ -573,23 +576,19 @@ void jacobi_update(Ctx& c, int no, int nv, const double* d_do, const double* d_d
   unsigned int* ticket = &c.words()->reduce;
   if (n + (int64_t)RED_BLOCKS * RED_THREADS < ((int64_t)1 << 31))
     launch_chained(jacobi_kernel<uint32_t>, nb, RED_THREADS, c.stream, 1, no, nv, d_do, d_dv, shift, R1, R2, t1old,
-                   t2old, t1new, t2new, part.d(), ticket, d_sumsq);
+                   t2old, t1new, t2new, part.d(), ticket, sumsq, e, v);
   else
     launch_chained(jacobi_kernel<int64_t>, nb, RED_THREADS, c.stream, 1, no, nv, d_do, d_dv, shift, R1, R2, t1old,
-                   t2old, t1new, t2new, part.d(), ticket, d_sumsq);
+                   t2old, t1new, t2new, part.d(), ticket, sumsq, e, v);
   count_launch();
   check_launch("jacobi");
 }
 
-void lincomb(Ctx& c, int nvec, const double* const* d_vecs, const double* coef, int64_t n, double* out) {
+void lincomb(Ctx& c, int nvec, const VecList& vecs, int64_t n, double* out) {
   UCC_REQUIRE(!recorder(), UCC_UNSUPPORTED, "not recordable");
-  Scratch dc(c, sizeof(double) * nvec);
-  UCC_CUDA(cudaMemcpyAsync(dc.p, coef, sizeof(double) * nvec, cudaMemcpyHostToDevice, c.stream));
-  launch_chained(lincomb_kernel, grid_for(n), 256, c.stream, 1, nvec, d_vecs, dc.d(), n, out);
+  launch_chained(lincomb_kernel, grid_for(n), 256, c.stream, 1, nvec, vecs, n, out);
   count_launch();
   check_launch("lincomb");
-  // the host coefficient array may go out of scope once the copy has been consumed
-  UCC_CUDA(cudaStreamSynchronize(c.stream));
 }
 
 // ------------------------------------------------------------------------------------
