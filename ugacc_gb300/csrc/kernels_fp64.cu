@@ -47,6 +47,7 @@ __device__ __forceinline__ double combine(double alpha, double x, double beta, c
 // C(epi) = alpha * sum_z P[z][m][n] + beta * C(epi), the fixed-order split-K reduction
 __global__ void splitk_reduce_kernel(int64_t M, int64_t N, int nsplit, const double* P, double alpha, double beta,
                                      double* C, GemmEpilogue ep) {
+  chain_enter();
   const int64_t MN = M * N;
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < MN; x += (int64_t)gridDim.x * blockDim.x) {
     double s = 0.0;
@@ -72,7 +73,7 @@ void splitk_reduce(Ctx& c, int64_t M, int64_t N, int nsplit, const double* P, do
                    const GemmEpilogue& epi) {
   const int64_t MN = M * N;
   const unsigned blocks = (unsigned)std::min<int64_t>((MN + 255) / 256, 152 * 16);
-  splitk_reduce_kernel<<<blocks, 256, 0, c.stream>>>(M, N, nsplit, P, alpha, beta, C, epi);
+  launch_chained(splitk_reduce_kernel, blocks, 256, c.stream, 1, M, N, nsplit, P, alpha, beta, C, epi);
   count_launch();
   check_launch("split-K reduce");
 }

@@ -24,6 +24,7 @@
 #include <tuple>
 
 #include "cc.h"
+#include "chain.h"
 #include "core.h"
 #include "tc_ptx.h"
 
@@ -1134,8 +1135,11 @@ __device__ __forceinline__ bool mv_kcontig(const MatView& v) { return (v.ksplit 
 // row maxima |x| of a rows x cols FP64 view as bit patterns (non-negative doubles order
 // like their bits, so the maximum is an integer one); block (x, y) covers 32 rows and the
 // K range [x kchunk, (x+1) kchunk), lanes along k (sk == 1) or along the rows (transposed
-// views), and merges into amax (zeroed by the caller) with one atomicMax per row
+// views), and merges into amax (zeroed by the caller) with one atomicMax per row; a single
+// chunk writes its rows' maxima
 __global__ void slice_absmax_kernel(MatView x, int64_t kchunk, unsigned long long* amax) {
+  chain_enter();
+  const bool single = gridDim.x == 1;
   __shared__ unsigned long long t[8][32];
   const int64_t rows = x.rows, cols = x.cols;
   const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * kchunk;
@@ -1150,7 +1154,12 @@ __global__ void slice_absmax_kernel(MatView x, int64_t kchunk, unsigned long lon
         for (int64_t k = k0 + tx; k < k1; k += 32)
           mm = max(mm, (unsigned long long)__double_as_longlong(mv_at(x, r, k)) & absmask);
       for (int o = 16; o > 0; o >>= 1) mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-      if (tx == 0 && r < rows && mm) atomicMax(amax + r, mm);
+      if (tx == 0 && r < rows) {
+        if (single)
+          amax[r] = mm;
+        else if (mm)
+          atomicMax(amax + r, mm);
+      }
     }
   } else {
     const int64_t r = r0 + tx;
@@ -1162,7 +1171,10 @@ __global__ void slice_absmax_kernel(MatView x, int64_t kchunk, unsigned long lon
     __syncthreads();
     if (ty == 0 && r < rows) {
       for (int i = 1; i < 8; i++) mm = max(mm, t[i][tx]);
-      if (mm) atomicMax(amax + r, mm);
+      if (single)
+        amax[r] = mm;
+      else if (mm)
+        atomicMax(amax + r, mm);
     }
   }
 }
@@ -1203,8 +1215,9 @@ __device__ __forceinline__ long long slice_fixed(double x, int e, int bits) {
 // reads coalesced along whichever stride is 1; each thread then slices two neighbouring
 // elements of a row and stores each digit pair as one bf16x2 (a warp writes 128
 // contiguous bytes of a slice plane per store; kp is a multiple of 64).
-__global__ void slice_digits_kernel(MatView x, int64_t rows_p, int64_t kp, const unsigned long long* __restrict__ amax,
-                                    int S, __nv_bfloat16* slices, int* e_out, int* range) {
+__global__ void slice_digits_kernel(MatView x, int64_t rows_p, int64_t kp, const unsigned long long* amax, int S,
+                                    __nv_bfloat16* slices, int* e_out, int* range) {
+  chain_enter();
   __shared__ double t[32][65];
   const int64_t rows = x.rows, cols = x.cols;
   const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 64;
@@ -1286,6 +1299,7 @@ __global__ void slice_digits_kernel(MatView x, int64_t rows_p, int64_t kp, const
 // multiple of 64).  Two parts are formed in FP32 (x truncated to FP32 first, from its bit
 // fields: 2^-23, far below the lo part's 2^-17), three parts in FP64.
 __global__ void split_kernel(MatView x, int64_t kp, __nv_bfloat16* hi, __nv_bfloat16* lo, __nv_bfloat16* mid) {
+  chain_enter();
   __shared__ double t[32][65];
   const int64_t rows = x.rows, cols = x.cols;
   const int64_t k0 = (int64_t)blockIdx.x * 64;
@@ -1392,7 +1406,8 @@ struct Cache {
   std::map<Key, std::unique_ptr<Split>> ops;
   std::map<Key, std::unique_ptr<Sliced>> sliced;
   int* range = nullptr;    // device flag: a sliced operand row maximum beyond the range (sticky)
-  int* pinned = nullptr;   // host copies of err and range, refreshed in stream order after launches
+  int* pinned = nullptr;   // host copies of err and range (tc_check)
+  bool unchecked = false;  // launches since the last check
   bool sattr_set = false;
   int max_pairs_sliced = 0;  // clusters of two sliced_gemm_kernel CTAs resident at once
   std::shared_ptr<Triples> triples;
@@ -1485,8 +1500,8 @@ static Split* prepare(Ctx& c, const MatView& x, int box_rows, std::unique_ptr<Sp
     s->lo = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(s->tmp->p) + plane);
     if (parts == 3) s->mid = reinterpret_cast<__nv_bfloat16*>(static_cast<char*>(s->tmp->p) + 2 * plane);
   }
-  split_kernel<<<dim3((unsigned)(s->kp / 64), (unsigned)std::min<int64_t>((rows + 31) / 32, 65535)), dim3(32, 8), 0,
-                 c.stream>>>(x, s->kp, s->hi, s->lo, s->mid);
+  launch_chained(split_kernel, dim3((unsigned)(s->kp / 64), (unsigned)std::min<int64_t>((rows + 31) / 32, 65535)),
+                 dim3(32, 8), c.stream, 1, x, s->kp, s->hi, s->lo, s->mid);
   count_kernel_launch();
   UCC_CUDA(cudaGetLastError());
   maps_for(s.get(), box_rows, parts);
@@ -1546,17 +1561,18 @@ static Sliced* slice_prepare(Ctx& c, const MatView& x, int box_rows, int S, std:
     s->e = reinterpret_cast<int*>(static_cast<char*>(s->tmp->p) + ((sizeof(__nv_bfloat16) * nel + 15) / 16) * 16);
   }
   Scratch amax(c, sizeof(unsigned long long) * rows);
-  UCC_CUDA(cudaMemsetAsync(amax.p, 0, sizeof(unsigned long long) * rows, c.stream));
   // K chunks of >= 1024 elements, enough blocks to cover the SMs a few times
   const int64_t rblocks = (rows + 31) / 32;
   const int64_t want = std::max<int64_t>(1, (int64_t)k.sms * 8 / rblocks);
   const int64_t kchunk = std::max<int64_t>(1024, (cols + want - 1) / want);
   const dim3 blk(32, 8);
-  slice_absmax_kernel<<<dim3((unsigned)((cols + kchunk - 1) / kchunk), (unsigned)rblocks), blk, 0, c.stream>>>(
-      x, kchunk, static_cast<unsigned long long*>(amax.p));
+  const unsigned nchunks = (unsigned)((cols + kchunk - 1) / kchunk);
+  unsigned long long* am = static_cast<unsigned long long*>(amax.p);
+  if (nchunks > 1) UCC_CUDA(cudaMemsetAsync(am, 0, sizeof(unsigned long long) * rows, c.stream));
+  launch_chained(slice_absmax_kernel, dim3(nchunks, (unsigned)rblocks), blk, c.stream, 1, x, kchunk, am);
   count_kernel_launch();
-  slice_digits_kernel<<<dim3((unsigned)(s->kp / 64), (unsigned)(s->rows_p / 32)), blk, 0, c.stream>>>(
-      x, s->rows_p, s->kp, static_cast<const unsigned long long*>(amax.p), S, s->d, s->e, k.range);
+  launch_chained(slice_digits_kernel, dim3((unsigned)(s->kp / 64), (unsigned)(s->rows_p / 32)), blk, c.stream, 1, x,
+                 s->rows_p, s->kp, am, S, s->d, s->e, k.range);
   count_kernel_launch();
   UCC_CUDA(cudaGetLastError());
   slice_map(s.get(), box_rows);
@@ -1820,7 +1836,7 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   // other GEMM timers and the status flags are read at the next synchronisation (tc_check)
   c.gemm_timers.push_back({ev0, ev1, 2.0 * (double)M * (double)N * (double)K, 2, 0.5 * S * (S + 1)});
   if (c.gemm_timers.size() >= 4096) c.resolve_timers();
-  UCC_CUDA(cudaMemcpyAsync(k.pinned, k.err, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  k.unchecked = true;
   return true;
 }
 
@@ -1953,7 +1969,7 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
   // no synchronisation (see sliced_gemm_part)
   c.gemm_timers.push_back({ev0, ev1, 2.0 * (double)M * (double)N * (double)K, 1});
   if (c.gemm_timers.size() >= 4096) c.resolve_timers();
-  UCC_CUDA(cudaMemcpyAsync(k.pinned, k.err, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  k.unchecked = true;
 }
 
 // the status of the tensor-core launches since the last check, after a synchronisation of
@@ -1962,10 +1978,15 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
 void tc_check(Ctx& c) {
   if (!c.tc_cache) return;
   tc::Cache& k = *static_cast<tc::Cache*>(c.tc_cache.get());
+  if (!k.unchecked) return;
+  // the flags are sticky: one copy per check (a copy behind every launch, with the idle time on
+  // both its sides, and plain launches of the split and slicing passes took 3.9 of the 162.7 ms
+  // of a mixed CCSD(T) solve at no=16/nv=160)
+  UCC_CUDA(cudaMemcpyAsync(k.pinned, k.err, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
   UCC_CUDA(cudaStreamSynchronize(c.stream));
+  k.unchecked = false;
   const int herr = k.pinned[0], hrange = k.pinned[1];
   if (!herr && !hrange) return;
-  k.pinned[0] = k.pinned[1] = 0;
   UCC_CUDA(cudaMemsetAsync(k.err, 0, 2 * sizeof(int), c.stream));
   UCC_CUDA(cudaStreamSynchronize(c.stream));
   if (herr) throw Error(UCC_DEVICE_TIMEOUT, "tensor-core GEMM: a pipeline wait timed out");
@@ -1980,7 +2001,7 @@ void wait_selftest(Ctx& c, unsigned long long limit_ns) {
   tc::wait_selftest_kernel<<<1, 32, 0, c.stream>>>(k.err, limit_ns);
   count_kernel_launch();
   UCC_CUDA(cudaGetLastError());
-  UCC_CUDA(cudaMemcpyAsync(k.pinned, k.err, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  k.unchecked = true;
   tc_check(c);
 }
 
@@ -2089,6 +2110,7 @@ namespace tc {
 __global__ void split_into_kernel(int64_t rows, int64_t cols, const double* src, int64_t rsplit, int64_t sr_hi,
                                   int64_t sr, int64_t sk, double scale, __nv_bfloat16* hi, __nv_bfloat16* lo,
                                   int64_t ld, int64_t row0, int64_t col0) {
+  chain_enter();
   __shared__ double t[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
   for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
@@ -2128,8 +2150,8 @@ static void split_into(Ctx& c, int64_t rows, int64_t cols, const double* src, in
   dim3 grid((unsigned)((cols + 31) / 32), (unsigned)((rows + 31) / 32));
   UCC_REQUIRE(grid.y <= 65535, UCC_BAD_ARGS, "split_into: too many rows");
   if (rsplit <= 0) rsplit = rows;  // one level: r * sr
-  split_into_kernel<<<grid, dim3(32, 8), 0, c.stream>>>(rows, cols, src, rsplit, sr_hi, sr, sk, scale, dst.hi, dst.lo,
-                                                        dst.kp, row0, col0);
+  launch_chained(split_into_kernel, grid, dim3(32, 8), c.stream, 1, rows, cols, src, rsplit, sr_hi, sr, sk, scale,
+                 dst.hi, dst.lo, dst.kp, row0, col0);
   count_kernel_launch();
   UCC_CUDA(cudaGetLastError());
 }
@@ -2266,7 +2288,7 @@ bool mixed_triples_batch(Ctx& c, int nb, const int* tuples, float* W3, int tblk)
   // timed with the other GEMMs (resolved lazily); the status flags are read at the next check
   c.gemm_timers.push_back({ev0, ev1, 2.0 * 6.0 * (double)nv2 * (double)nv * (double)(nv + no) * nb, 1});
   if (c.gemm_timers.size() >= 4096) c.resolve_timers();
-  UCC_CUDA(cudaMemcpyAsync(k.pinned, k.err, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+  k.unchecked = true;
   return true;
 }
 
