@@ -1132,50 +1132,122 @@ __device__ __forceinline__ const double& mv_at(const MatView& v, int64_t r, int6
 }
 __device__ __forceinline__ bool mv_kcontig(const MatView& v) { return (v.ksplit ? v.ks_lo : v.ks_hi) == 1; }
 
+// Offsets of 32 rows and 64 columns of an operand: one division per element of the two index
+// lists instead of up to two per matrix element, which bounded the passes below.
+struct TileOffsets {
+  int64_t r[32], k[64];
+};
+__device__ __forceinline__ int64_t mv_off(int64_t i, int64_t split, int64_t hi, int64_t lo) {
+  if (!split) return i * hi;
+  const uint32_t s = (uint32_t)min(split, (int64_t)INT32_MAX), q = (uint32_t)i / s;  // extents are below 2^31
+  return (int64_t)q * hi + (int64_t)((uint32_t)i - q * s) * lo;
+}
+__device__ __forceinline__ void row_offsets(const MatView& x, int64_t r0, TileOffsets& o, int tid) {
+  if (tid < 32) o.r[tid] = mv_off(r0 + tid, x.rsplit, x.rs_hi, x.rs_lo);
+}
+__device__ __forceinline__ void col_offsets(const MatView& x, int64_t k0, int64_t* k, int tid) {
+  if (tid >= 64 && tid < 128) k[tid - 64] = mv_off(k0 + tid - 64, x.ksplit, x.ks_hi, x.ks_lo);
+}
+
 // row maxima |x| of a rows x cols FP64 view as bit patterns (non-negative doubles order
 // like their bits, so the maximum is an integer one); block (x, y) covers 32 rows and the
-// K range [x kchunk, (x+1) kchunk), lanes along k (sk == 1) or along the rows (transposed
-// views), and merges into amax (zeroed by the caller) with one atomicMax per row; a single
-// chunk writes its rows' maxima
+// K range [x kchunk, (x+1) kchunk) (kchunk a multiple of 64), lanes along k (sk == 1) or along
+// the rows (transposed views), and merges into amax (zeroed by the caller) with one atomicMax
+// per row; a single chunk writes its rows' maxima.  Reading bounds it, with eight loads per
+// thread in flight: 6.6e6 elements (rows and columns of two strided runs) take 20 us, and took
+// 48 us with divisions for each element and K chunks of 1024.
 __global__ void slice_absmax_kernel(MatView x, int64_t kchunk, unsigned long long* amax) {
   chain_enter();
-  const bool single = gridDim.x == 1;
+  constexpr int kCols = 512;  // columns of an offset list
   __shared__ unsigned long long t[8][32];
-  const int64_t rows = x.rows, cols = x.cols;
+  __shared__ int64_t ro[32], ko[kCols];
+  const bool single = gridDim.x == 1, kc = mv_kcontig(x);
   const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * kchunk;
-  const int64_t k1 = min(cols, k0 + kchunk);
-  const int tx = threadIdx.x, ty = threadIdx.y;
+  const int64_t k1 = min(x.cols, k0 + kchunk);
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+  const int nr = (int)min((int64_t)32, x.rows - r0);
   const unsigned long long absmask = 0x7FFFFFFFFFFFFFFFull;
-  if (mv_kcontig(x)) {
-    for (int i = ty; i < 32; i += 8) {
-      const int64_t r = r0 + i;
-      unsigned long long mm = 0;
-      if (r < rows)
-        for (int64_t k = k0 + tx; k < k1; k += 32)
-          mm = max(mm, (unsigned long long)__double_as_longlong(mv_at(x, r, k)) & absmask);
-      for (int o = 16; o > 0; o >>= 1) mm = max(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-      if (tx == 0 && r < rows) {
+  if (tid < 32) ro[tid] = mv_off(r0 + tid, x.rsplit, x.rs_hi, x.rs_lo);
+  unsigned long long mm[4] = {0, 0, 0, 0};
+  for (int64_t kt = k0; kt < k1; kt += kCols) {
+    const int nk = (int)min((int64_t)kCols, k1 - kt);
+    __syncthreads();
+    for (int j = tid; j < nk; j += 256) ko[j] = mv_off(kt + j, x.ksplit, x.ks_hi, x.ks_lo);
+    __syncthreads();
+#pragma unroll 2
+    for (int j0 = 0; j0 < nk; j0 += 64) {
+      unsigned long long v[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int i = kc ? ty + 8 * (q / 2) : tx, j = j0 + (kc ? tx + 32 * (q % 2) : ty + 8 * q);
+        v[q] = i < nr && j < nk ? (unsigned long long)__double_as_longlong(x.p[ro[i] + ko[j]]) & absmask : 0;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++) mm[q / 2] = max(mm[q / 2], v[q]);
+    }
+  }
+  if (kc) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int i = ty + 8 * q;
+      for (int o = 16; o > 0; o >>= 1) mm[q] = max(mm[q], __shfl_xor_sync(0xffffffffu, mm[q], o));
+      if (tx == 0 && i < nr) {
         if (single)
-          amax[r] = mm;
-        else if (mm)
-          atomicMax(amax + r, mm);
+          amax[r0 + i] = mm[q];
+        else if (mm[q])
+          atomicMax(amax + r0 + i, mm[q]);
       }
     }
   } else {
-    const int64_t r = r0 + tx;
-    unsigned long long mm = 0;
-    if (r < rows)
-      for (int64_t k = k0 + ty; k < k1; k += 8)
-        mm = max(mm, (unsigned long long)__double_as_longlong(mv_at(x, r, k)) & absmask);
-    t[ty][tx] = mm;
+    t[ty][tx] = max(max(mm[0], mm[1]), max(mm[2], mm[3]));
     __syncthreads();
-    if (ty == 0 && r < rows) {
-      for (int i = 1; i < 8; i++) mm = max(mm, t[i][tx]);
+    if (ty == 0 && tx < nr) {
+      unsigned long long m = t[0][tx];
+      for (int i = 1; i < 8; i++) m = max(m, t[i][tx]);
       if (single)
-        amax[r] = mm;
-      else if (mm)
-        atomicMax(amax + r, mm);
+        amax[r0 + tx] = m;
+      else if (m)
+        atomicMax(amax + r0 + tx, m);
     }
+  }
+}
+
+// The 32 x 64 tile at (r0, k0) of an operand in pairs of neighbouring columns: v0[q], v1[q] are
+// elements (ty + 8 q, 2 tx) and (ty + 8 q, 2 tx + 1), zero outside the matrix.  Rows with unit
+// stride are read directly, others along the rows, through shared memory; either way a
+// thread's eight loads are in flight together.  The split of 6.6e6 elements into two parts took
+// 39 us (2 TB/s) with a division or two per element, one load at a time ahead of its shared
+// store, and an FP64-pipe conversion per element; it takes 20 us.  The slicing into nine digits
+// took 40 us and takes 34 us (5 TB/s).
+struct TileStage {
+  TileOffsets off;
+  double t[32][65];
+};
+__device__ __forceinline__ void load_pairs(TileStage& s, const MatView& x, int64_t r0, int64_t k0, double (&v0)[4],
+                                           double (&v1)[4]) {
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+  row_offsets(x, r0, s.off, tid);
+  col_offsets(x, k0, s.off.k, tid);
+  __syncthreads();
+  const int nr = (int)min((int64_t)32, x.rows - r0), nk = (int)min((int64_t)64, x.cols - k0);
+  if (mv_kcontig(x)) {
+    const int64_t c0 = s.off.k[2 * tx], c1 = s.off.k[2 * tx + 1];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int i = ty + 8 * q;
+      v0[q] = i < nr && 2 * tx < nk ? x.p[s.off.r[i] + c0] : 0.0;
+      v1[q] = i < nr && 2 * tx + 1 < nk ? x.p[s.off.r[i] + c1] : 0.0;
+    }
+  } else {
+    const double* p = x.p + s.off.r[tx];
+    double v[8];  // all eight loads before the first store, which might alias them
+#pragma unroll
+    for (int q = 0; q < 8; q++) v[q] = tx < nr && ty + 8 * q < nk ? p[s.off.k[ty + 8 * q]] : 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) s.t[tx][ty + 8 * q] = v[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) v0[q] = s.t[ty + 8 * q][2 * tx], v1[q] = s.t[ty + 8 * q][2 * tx + 1];
   }
 }
 
@@ -1218,39 +1290,30 @@ __device__ __forceinline__ long long slice_fixed(double x, int e, int bits) {
 __global__ void slice_digits_kernel(MatView x, int64_t rows_p, int64_t kp, const unsigned long long* amax, int S,
                                     __nv_bfloat16* slices, int* e_out, int* range) {
   chain_enter();
-  __shared__ double t[32][65];
-  const int64_t rows = x.rows, cols = x.cols;
-  const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 64;
+  __shared__ TileStage st;
+  const int64_t rows = x.rows, r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 64;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  if (mv_kcontig(x)) {
-    for (int i = ty; i < 32; i += 8)
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int64_t r = r0 + i, k = k0 + tx + 32 * h;
-        t[i][tx + 32 * h] = (r < rows && k < cols) ? mv_at(x, r, k) : 0.0;
-      }
-  } else {
-    for (int j = ty; j < 64; j += 8) {
-      const int64_t r = r0 + tx, k = k0 + j;
-      t[tx][j] = (r < rows && k < cols) ? mv_at(x, r, k) : 0.0;
-    }
-  }
-  __syncthreads();
+  double v0[4], v1[4];
+  load_pairs(st, x, r0, k0, v0, v1);
   const size_t plane2 = (size_t)rows_p * kp / 2;  // a slice plane in bf16 pairs
   constexpr int H = 1 << (SB - 1);
-  for (int i = ty; i < 32; i += 8) {
-    const int64_t r = r0 + i, k = k0 + 2 * tx;
+#pragma unroll
+  for (int q4 = 0; q4 < 4; q4++) {
+    const int64_t r = r0 + ty + 8 * q4, k = k0 + 2 * tx;
     if (r >= rows_p) continue;
     const int e = r < rows ? slice_exponent(amax[r], range) : 0;
     if (k == 0 && r < rows) e_out[r] = e;
-    long long X0 = r < rows ? slice_fixed(t[i][2 * tx], e, SB * S) : 0;
-    long long X1 = r < rows ? slice_fixed(t[i][2 * tx + 1], e, SB * S) : 0;
+    long long X0 = r < rows ? slice_fixed(v0[q4], e, SB * S) : 0;
+    long long X1 = r < rows ? slice_fixed(v1[q4], e, SB * S) : 0;
     __nv_bfloat162* dst = reinterpret_cast<__nv_bfloat162*>(slices + (size_t)r * kp + k);
     // digit s (|d| <= 2^(SB-1)): a 32-bit conversion, exact, and exact in bf16 after the
     // power-of-2 scale
+    // (the sum 1.5 2^23 + d as bits, scaled and shifted by one exact FMA: an integer conversion
+    // runs at a quarter of the rate)
     auto put = [&](int s, int d0, int d1) {
-      const float sc = __int_as_float((127 - SB * (s + 1)) << 23);
-      dst[(size_t)s * plane2] = __floats2bfloat162_rn((float)d0 * sc, (float)d1 * sc);
+      const float sc = __int_as_float((127 - SB * (s + 1)) << 23), off = -12582912.0f * sc;
+      dst[(size_t)s * plane2] = __floats2bfloat162_rn(fmaf(__int_as_float(0x4B400000 + d0), sc, off),
+                                                      fmaf(__int_as_float(0x4B400000 + d1), sc, off));
     };
     if (S >= 6) {
       // balanced digits in 32-bit arithmetic: the low 30 bits hold the 5 least significant
@@ -1298,34 +1361,21 @@ __global__ void slice_digits_kernel(MatView x, int64_t rows_p, int64_t kp, const
 // and stores each part as one bf16x2 (128 contiguous bytes per warp store; kp is a
 // multiple of 64).  Two parts are formed in FP32 (x truncated to FP32 first, from its bit
 // fields: 2^-23, far below the lo part's 2^-17), three parts in FP64.
-__global__ void split_kernel(MatView x, int64_t kp, __nv_bfloat16* hi, __nv_bfloat16* lo, __nv_bfloat16* mid) {
+__global__ void __launch_bounds__(256, 6) split_kernel(MatView x, int64_t kp, __nv_bfloat16* hi, __nv_bfloat16* lo, __nv_bfloat16* mid) {
   chain_enter();
-  __shared__ double t[32][65];
-  const int64_t rows = x.rows, cols = x.cols;
-  const int64_t k0 = (int64_t)blockIdx.x * 64;
+  __shared__ TileStage st;
+  const int64_t rows = x.rows, k0 = (int64_t)blockIdx.x * 64;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  const bool kc = mv_kcontig(x);
   for (int64_t r0 = (int64_t)blockIdx.y * 32; r0 < rows; r0 += (int64_t)gridDim.y * 32) {  // row tiles
   __syncthreads();
-  if (kc) {
-    for (int i = ty; i < 32; i += 8)
+  double w0[4], w1[4];
+  load_pairs(st, x, r0, k0, w0, w1);
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int64_t r = r0 + i, k = k0 + tx + 32 * h;
-        t[i][tx + 32 * h] = (r < rows && k < cols) ? mv_at(x, r, k) : 0.0;
-      }
-  } else {
-    for (int j = ty; j < 64; j += 8) {
-      const int64_t r = r0 + tx, k = k0 + j;
-      t[tx][j] = (r < rows && k < cols) ? mv_at(x, r, k) : 0.0;
-    }
-  }
-  __syncthreads();
-  for (int i = ty; i < 32; i += 8) {
-    const int64_t r = r0 + i, k = k0 + 2 * tx;
+  for (int q4 = 0; q4 < 4; q4++) {
+    const int64_t r = r0 + ty + 8 * q4, k = k0 + 2 * tx;
     if (r >= rows) continue;
     const int64_t o2 = (r * kp + k) / 2;  // bf16 pair index
-    const double v0 = t[i][2 * tx], v1 = t[i][2 * tx + 1];
+    const double v0 = w0[q4], v1 = w1[q4];
     if (mid) {
       const __nv_bfloat16 h0 = __double2bfloat16(v0), h1 = __double2bfloat16(v1);
       double r0d = v0 - (double)__bfloat162float(h0), r1d = v1 - (double)__bfloat162float(h1);
@@ -1561,10 +1611,10 @@ static Sliced* slice_prepare(Ctx& c, const MatView& x, int box_rows, int S, std:
     s->e = reinterpret_cast<int*>(static_cast<char*>(s->tmp->p) + ((sizeof(__nv_bfloat16) * nel + 15) / 16) * 16);
   }
   Scratch amax(c, sizeof(unsigned long long) * rows);
-  // K chunks of >= 1024 elements, enough blocks to cover the SMs a few times
+  // K chunks of >= 256 elements, enough blocks to cover the SMs a few times
   const int64_t rblocks = (rows + 31) / 32;
   const int64_t want = std::max<int64_t>(1, (int64_t)k.sms * 8 / rblocks);
-  const int64_t kchunk = std::max<int64_t>(1024, (cols + want - 1) / want);
+  const int64_t kchunk = (std::max<int64_t>(256, (cols + want - 1) / want) + 63) / 64 * 64;
   const dim3 blk(32, 8);
   const unsigned nchunks = (unsigned)((cols + kchunk - 1) / kchunk);
   unsigned long long* am = static_cast<unsigned long long*>(amax.p);
@@ -2113,11 +2163,16 @@ __global__ void split_into_kernel(int64_t rows, int64_t cols, const double* src,
   chain_enter();
   __shared__ double t[32][33];
   const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
-  for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
-    const int64_t r = r0 + threadIdx.x, k = k0 + yy;
-    const double x = (r < rows && k < cols) ? src[(r / rsplit) * sr_hi + (r % rsplit) * sr + k * sk] : 0.0;
-    t[yy][threadIdx.x] = scale == 1.0 ? x : scale * x;
+  double v[4];  // all loads before the first store, which might alias them
+  const int64_t rl = r0 + threadIdx.x;
+  const double* p = src + (rl / rsplit) * sr_hi + (rl % rsplit) * sr;
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int64_t k = k0 + threadIdx.y + 8 * q;
+    v[q] = rl < rows && k < cols ? p[k * sk] : 0.0;
   }
+#pragma unroll
+  for (int q = 0; q < 4; q++) t[threadIdx.y + 8 * q][threadIdx.x] = scale == 1.0 ? v[q] : scale * v[q];
   __syncthreads();
   for (int yy = threadIdx.y; yy < 32; yy += blockDim.y) {
     const int64_t r = r0 + yy, k = k0 + threadIdx.x;

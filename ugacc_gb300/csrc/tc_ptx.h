@@ -158,15 +158,20 @@ __device__ __forceinline__ double f32_bits_to_f64(uint32_t fb) {
 }
 
 // FP64 -> FP32 truncated toward zero by moving the bit fields (relative error below 2^-23,
-// integer pipe); zeros keep their sign, values outside FP32's normal range take the
-// converting instruction
+// integer pipe); zeros keep their sign
 __device__ __forceinline__ float f64_to_f32_trunc(double v) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const uint32_t sgn = (uint32_t)(b >> 32) & 0x80000000u;
-  if ((b << 1) == 0ull) return __uint_as_float(sgn);
   const int e = (int)((b >> 52) & 0x7FF) - 1023;
-  if (e < -126 || e > 127) return (float)v;
-  return __uint_as_float(sgn | ((uint32_t)(e + 127) << 23) | (uint32_t)((b >> 29) & 0x7FFFFFu));
+  if (e >= -126 && e <= 127) return __uint_as_float(sgn | ((uint32_t)(e + 127) << 23) | (uint32_t)((b >> 29) & 0x7FFFFFu));
+  // beyond FP32's normal range as the conversion instruction rounds, without it: a compiler that
+  // evaluates both sides of this branch puts one FP64-pipe conversion on every element
+  if (e > 127) return __uint_as_float(sgn | (e == 1024 && (b << 12) ? 0x7FFFFFFFu : 0x7F800000u));
+  const int sh = -126 - e + 29;  // >= 30; the FP64 subnormals (e = -1023) come out as zero
+  if (sh > 54) return __uint_as_float(sgn);
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52), half = 1ull << (sh - 1);
+  const unsigned long long q = m >> sh, rem = m & (2 * half - 1);
+  return __uint_as_float(sgn | (uint32_t)(q + (rem > half || (rem == half && (q & 1)))));
 }
 
 __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {  // tmem_wait before use
