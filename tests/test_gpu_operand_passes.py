@@ -57,3 +57,14 @@ def test_row_maxima_of_one_and_several_column_chunks(ctx):
             A[1, pos] = 2.0 ** 20
             out = ctx.gemm(A, np.ones((K, 2)), digits=9)
             np.testing.assert_array_equal(out, A @ np.ones((K, 2)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(33, 32, 64), (130, 64, 40), (7, 66, 64), (129, 100, 128)])
+def test_accumulating_product_by_sectors_and_by_elements(ctx, M, N, K):
+    """C += A B: rows of C on 32-byte boundaries and not, whole and ragged blocks of 32 columns."""
+    A, B, a, b = _operands(N, M, N, K, False, False)
+    C = np.random.default_rng(N + 1).standard_normal((M, N))
+    bound = np.abs(A) @ np.abs(B)
+    out = ctx.gemm(a, b, C=C, beta=1.0, precision=U.MIXED)
+    assert np.all(np.abs(out - (C + A @ B)) <= (3 * EPS2 + 3 * K * 2.0 ** -24) * bound + 1e-15 * np.abs(C))

@@ -146,15 +146,30 @@ __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// FP32 -> FP64 by moving the bit fields (integer pipe, GB300 has few FP64 units); zero,
-// subnormal, infinite and NaN inputs take the converting instruction
+// FP32 -> FP64 by moving the bit fields (integer pipe, GB300 has few FP64 units)
 __device__ __forceinline__ double f32_bits_to_f64(uint32_t fb) {
-  const uint32_t e = (fb >> 23) & 0xFFu;
-  if (e == 0u || e == 0xFFu) return (double)__uint_as_float(fb);
-  const unsigned long long sgn = (unsigned long long)(fb >> 31) << 63;
-  const unsigned long long ex = (unsigned long long)(e + 896u) << 52;
-  const unsigned long long mt = (unsigned long long)(fb & 0x7FFFFFu) << 29;
-  return __longlong_as_double((long long)(sgn | ex | mt));
+  const uint32_t e = (fb >> 23) & 0xFFu, m = fb & 0x7FFFFFu, sgn = fb & 0x80000000u;
+  uint32_t ex = e + 896u, mt = m;
+  if (e - 1u >= 0xFEu) {  // zero, subnormal, infinite, NaN
+    if (e) {
+      ex = 0x7FFu;
+    } else if (m) {
+      const int s = __clz(m) - 8;
+      ex = 897u - s;
+      mt = (m << s) & 0x7FFFFFu;
+    } else {
+      ex = 0u;
+    }
+  }
+  return __hiloint2double((int)(sgn | (ex << 20) | (mt >> 3)), (int)(mt << 29));
+}
+
+// 32 bytes of a lane, a whole sector, in one access (p: a multiple of 32 bytes)
+__device__ __forceinline__ void st_global4(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ void ld_global4(const double* p, double* v) {
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p) : "memory");
 }
 
 // FP64 -> FP32 truncated toward zero by moving the bit fields (relative error below 2^-23,
