@@ -2,7 +2,7 @@
 //
 //  (the GEMM itself is dgemm.cu)
 //  * permute_kernel_*  -- tensor transposition with alpha/beta through a 32x33 shared tile
-//  * reductions        -- compensated (Neumaier) FP64 sums in two deterministic passes
+//  * reductions        -- compensated (Neumaier) FP64 sums, folded in a fixed order in one launch
 //  * amplitude kernels -- tau/ttau, Jacobi update with on-the-fly denominators, DIIS
 //                         linear combination
 //  * triples_energy    -- the (T) energy of ccwfn.cc:795-852 for a batch of i>=j>=k
