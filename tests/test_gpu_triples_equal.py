@@ -19,3 +19,17 @@ def test_triples_of_few_occupied(no, nv):
     # both sides' amplitudes are within some 1e-11 of the solution, and (T) is quadratic in
     # them: 2 |E(T)| 1e-11 / |t|, below 1e-10 for these energies
     assert abs(cc.triples() - ref.tcorr_tjl()) < 1e-10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("no,nv", [(2, 64), (2, 66), (3, 68), (3, 71)])
+def test_mixed_triples_of_few_occupied(no, nv):
+    """The mixed form's half sets of products and the exchange in both energy kernels (nv % 4 == 0 or not)."""
+    h = make_hamiltonian(no, nv, seed=100 * no + nv)
+    H = U.Hamiltonian(h.no, h.nv, h.fock, B=h.B)
+    cc = U.CCWfn(H, {"R_CONVERGENCE": 1e-11, "MAXITER": 100})
+    cc.compute_energy()
+    e64 = cc.triples()
+    mixed = U.CCWfn(H, {"R_CONVERGENCE": 1e-11, "MAXITER": 100, "PRECISION": "MIXED"}).triples()
+    # two bf16 parts leave 2^-16 of a product; the energy's sums of W V cancel to a tenth or so
+    assert abs(mixed - e64) < 1e-3 * abs(e64)

@@ -423,7 +423,8 @@ void triples_energy(Ctx& c, int no, int nv, int ntuple, const int* d_tuples, con
                     const double* t1, const double* Voovv, const double* eps, double* d_partial);
 // The same from an FP32 W3 (mixed form) held as nparts partial arrays part_stride floats
 // apart (W3 = their sum): per-element arithmetic in FP32, the energy sum in FP64
-// (compensated).
+// (compensated).  With three arrays a tuple with i == j (j == k) has no array 2 (1) and the sum
+// of the other two is S, W3 = S + S(a and b (b and c) exchanged).
 // With f32in (FP32 copies of Voovv, t1 and eps made once per (T) call by triples_f32_inputs,
 // laid out by triples_f32_layout; nv % 4 == 0) the pipelined kernel runs on W3 in the
 // blocked layout of w3_block_offset, part_stride floats per array; without it the

@@ -705,6 +705,24 @@ constexpr int ET = 8;
 // make exact: thread t, iteration k covers element t + TNT*k of each loop.
 constexpr int TNT = 128;
 static_assert(TNT == 2 * ET * ET && (ET * ET * ET) % TNT == 0 && (6 * ET * ET) % TNT == 0, "tile/thread layout");
+// A tuple with i == j or j == k has two partial arrays of three, with S, W3 = S + S(a and b, or
+// b and c, exchanged): the array that is not there (0: all are)
+template <int NP>
+__device__ __forceinline__ int skipped_part(int i, int j, int k) {
+  return NP != 3 ? 0 : i == j ? 2 : j == k ? 1 : 0;
+}
+__device__ __forceinline__ void add_exchanged(int skip, float& abc, float& acb, float& bac, float& bca, float& cab,
+                                              float& cba) {
+  if (skip == 2) {
+    abc = bac = abc + bac;
+    acb = cab = acb + cab;
+    bca = cba = bca + cba;
+  } else if (skip == 1) {
+    abc = acb = abc + acb;
+    bac = bca = bac + bca;
+    cab = cba = cab + cba;
+  }
+}
 template <int NP>  // W3 partial arrays (1 or 3), a compile-time count so that all loads are in flight together
 __global__ void __launch_bounds__(TNT) triples_energy_f32_tiled_kernel(int no, int nv, const int* __restrict__ tuples,
                                                                       const int* __restrict__ tri, int ntri,
@@ -722,6 +740,7 @@ __global__ void __launch_bounds__(TNT) triples_energy_f32_tiled_kernel(int no, i
   const int Ra = (code & 1023) * ET, Rb = ((code >> 10) & 1023) * ET, Rc = (code >> 20) * ET;
   auto R0 = [&](int role) { return role == 0 ? Ra : (role == 1 ? Rb : Rc); };  // range start of a role
   const int i = tuples[3 * t], j = tuples[3 * t + 1], k = tuples[3 * t + 2];
+  const int skip = skipped_part<NP>(i, j, k);
   const int64_t nv2 = (int64_t)nv * nv;
   const float* W = W3 + (int64_t)t * nv2 * nv;
   // role order of each permutation tile p, two bits per role: W[x in role 0][y in 1][z in 2]
@@ -740,7 +759,8 @@ __global__ void __launch_bounds__(TNT) triples_energy_f32_tiled_kernel(int no, i
       const int64_t o = (int64_t)gx * nv2 + (int64_t)gy * nv + gz;
       w = W[o];
 #pragma unroll
-      for (int q = 1; q < NP; q++) w += W[o + q * part_stride];
+      for (int q = 1; q < NP; q++)
+        if (q != skip) w += W[o + q * part_stride];
     }
     Ws[p][x][ty][tz] = w;
   }
@@ -781,8 +801,9 @@ __global__ void __launch_bounds__(TNT) triples_energy_f32_tiled_kernel(int no, i
     const int la = tx + 2 * it, lb = ty, lc = tz;
     const int a = Ra + la, b = Rb + lb, c = Rc + lc;
     if (a >= nv || b > a || c > b) continue;
-    const float wabc = Ws[0][la][lb][lc], wacb = Ws[1][la][lc][lb], wbac = Ws[2][lb][la][lc];
-    const float wbca = Ws[3][lb][lc][la], wcab = Ws[4][lc][la][lb], wcba = Ws[5][lc][lb][la];
+    float wabc = Ws[0][la][lb][lc], wacb = Ws[1][la][lc][lb], wbac = Ws[2][lb][la][lc];
+    float wbca = Ws[3][lb][lc][la], wcab = Ws[4][lc][la][lb], wcba = Ws[5][lc][lb][la];
+    add_exchanged(skip, wabc, wacb, wbac, wbca, wcab, wcba);
     const float vabc = Vp(wabc, 0, la, 1, lb, 2, lc, a, b, c), vacb = Vp(wacb, 0, la, 2, lc, 1, lb, a, c, b);
     const float vbac = Vp(wbac, 1, lb, 0, la, 2, lc, b, a, c), vbca = Vp(wbca, 1, lb, 2, lc, 0, la, b, c, a);
     const float vcab = Vp(wcab, 2, lc, 0, la, 1, lb, c, a, b), vcba = Vp(wcba, 2, lc, 1, lb, 0, la, c, b, a);
@@ -882,6 +903,8 @@ __global__ void __launch_bounds__(EP_THREADS, 2)
     ranges(item, Ra, Rb, Rc, t);
     auto R0 = [&](int role) { return role == 0 ? Ra : (role == 1 ? Rb : Rc); };
     const float* Wt = W3 + (int64_t)t * per;
+    const int i = tuples[3 * t], j = tuples[3 * t + 1], k = tuples[3 * t + 2];
+    const int skip = skipped_part<NP>(i, j, k);
 #pragma unroll
     for (int pp = 0; pp < 3; pp++) {
       const int p = 3 * h + pp;
@@ -890,9 +913,8 @@ __global__ void __launch_bounds__(EP_THREADS, 2)
       const float* src = Wt + ((X * T + Y) * T + Z) * EP_WTILE + 4 * c16;
       float* dst = &st[s].W[0][p][4 * c16];
 #pragma unroll
-      for (int q = 0; q < NP; q++) ep_cp16(dst + q * 6 * EP_WTILE, src + q * part_stride, true);
+      for (int q = 0; q < NP; q++) ep_cp16(dst + q * 6 * EP_WTILE, src + q * part_stride, !q || q != skip);
     }
-    const int i = tuples[3 * t], j = tuples[3 * t + 1], k = tuples[3 * t + 2];
     for (int c = tid; c < EP_SIDE_CHUNKS; c += EP_THREADS) {
       const float* src;
       float* dst;
@@ -958,8 +980,9 @@ __global__ void __launch_bounds__(EP_THREADS, 2)
       const int lc = ((tid >> 4) & 1) | (((tid >> 3) & 1) << 1) | ((it & 1) << 2);
       const int a = Ra + la, b = Rb + lb, c = Rc + lc;
       if (a >= nv || b > a || c > b) continue;
-      const float wabc = W(0, la, lb, lc), wacb = W(1, la, lc, lb), wbac = W(2, lb, la, lc);
-      const float wbca = W(3, lb, lc, la), wcab = W(4, lc, la, lb), wcba = W(5, lc, lb, la);
+      float wabc = W(0, la, lb, lc), wacb = W(1, la, lc, lb), wbac = W(2, lb, la, lc);
+      float wbca = W(3, lb, lc, la), wcab = W(4, lc, la, lb), wcba = W(5, lc, lb, la);
+      add_exchanged(skipped_part<NP>(i, j, k), wabc, wacb, wbac, wbca, wcab, wcba);
       const float vabc = Vp(wabc, 0, la, 1, lb, 2, lc), vacb = Vp(wacb, 0, la, 2, lc, 1, lb);
       const float vbac = Vp(wbac, 1, lb, 0, la, 2, lc), vbca = Vp(wbca, 1, lb, 2, lc, 0, la);
       const float vcab = Vp(wcab, 2, lc, 0, la, 1, lb), vcba = Vp(wcba, 2, lc, 1, lb, 0, la);

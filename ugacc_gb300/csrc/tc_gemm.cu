@@ -79,8 +79,9 @@ struct Params {
   // of the three split products and writes a plain [M][N] FP64 partial at C + z*M*N
   int ksplit, kchunk;
   // nterms = 2 (batched problems only): a second product accumulated into the same tile,
-  // A from the second pair of tensor maps at rows a_row1[p], B at rows b_row1[p]
-  int nterms;
+  // A from the second pair of tensor maps at rows a_row1[p], B at rows b_row1[p], for the
+  // problems p < npair
+  int nterms, npair;
   const int* a_row1;
   const int* b_row1;
   // C32 != null: FP32 output C32[off] = alpha * acc (+ C32[off] when beta != 0), no FP64
@@ -238,8 +239,9 @@ __global__ void __launch_bounds__(THREADS, 1)
         const int mt = mg * CM + rank;
         const int ar0 = (p.nprob ? p.a_row0[pb] : 0) + mt * BM;
         const int br0 = (p.nprob ? p.b_row0[pb] : 0) + nt * p.bn + rank * bh;
-        const int ar1 = p.nterms > 1 ? p.a_row1[pb] + mt * BM : 0;
-        const int br1 = p.nterms > 1 ? p.b_row1[pb] + nt * p.bn + rank * bh : 0;
+        const int terms = p.nterms > 1 && pb < p.npair ? 2 : 1;
+        const int ar1 = terms > 1 ? p.a_row1[pb] + mt * BM : 0;
+        const int br1 = terms > 1 ? p.b_row1[pb] + nt * p.bn + rank * bh : 0;
         for (int ch = 0; ch < nch && ok; ch++) {
           int k0 = 0, kn = p.kblocks;
           if (p.ksplit > 1) {
@@ -249,7 +251,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             k0 = ch * p.kc;
             kn = min(p.kblocks - k0, p.kc);
           }
-          for (int kb = 0; kb < p.nterms * nseg * kn; kb++) {
+          for (int kb = 0; kb < terms * nseg * kn; kb++) {
             if (!mbar_wait(&empty[stage], phase ^ 1u, p.err)) {
               ok = false;
               break;
@@ -305,6 +307,12 @@ __global__ void __launch_bounds__(THREADS, 1)
       bool ok = true;
       const uint32_t idesc = idesc_of(CM, p.bn);
       for (int tile = cid; tile < ntile && ok; tile += ncl) {
+        int terms = 1;
+        if (p.nterms > 1) {
+          int pb, mg, nt;
+          tile_coords(p, mgroups, tile, pb, mg, nt);
+          terms = pb < p.npair ? 2 : 1;
+        }
         for (int ch = 0; ch < nch && ok; ch++) {
           int kn = p.kblocks;
           if (p.ksplit > 1)
@@ -317,7 +325,7 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
           fence_after();
           const uint32_t d = tmem + (uint32_t)(acc * BN);
-          for (int kb = 0; kb < p.nterms * nseg * kn; kb++) {
+          for (int kb = 0; kb < terms * nseg * kn; kb++) {
             if (!mbar_wait(&full[stage], phase, p.err)) {
               ok = false;
               break;
@@ -2031,6 +2039,7 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
   cudaEvent_t ev0 = c.take_event(), ev1 = c.take_event();
   UCC_CUDA(cudaEventRecord(ev0, c.stream));
   p.nterms = 1;
+  p.npair = 0;
   p.a_row1 = p.b_row1 = nullptr;
   p.C32 = nullptr;
   p.nparts = parts;
@@ -2293,9 +2302,9 @@ void mixed_triples_release(Ctx& c) {
 // W3 + (pq * nb + b) * S for tuple b with beta 0 (no read-modify-write of W3 in the
 // epilogue), S = nv^3 in the plain [a][b][c] layout (tblk = 0) or tblk^3 * 512 in the
 // blocked layout of w3_block_offset; triples_energy_f32 adds the three while staging its
-// tiles.  The three launches go out back to back with their own row tables; the caller
+// tiles.  The launches go out back to back with their own row tables; the caller
 // synchronises.
-bool mixed_triples_batch(Ctx& c, int nb, const int* tuples, float* W3, int tblk) {
+bool mixed_triples_batch(Ctx& c, int nb, const int* tuples, float* W3, int tblk, bool halves) {
   using namespace tc;
   Cache& k = cache(c);
   Triples& T = *k.triples;
@@ -2305,31 +2314,53 @@ bool mixed_triples_batch(Ctx& c, int nb, const int* tuples, float* W3, int tblk)
               "mixed (T): blocked W3 needs whole 8-wide blocks and < 2^31 floats per tuple");
   TriplesTerm terms[6];
   triples_terms(nv, terms);
-  // The six terms in pairs that write the same W3 layout: the first term of a pair uses
-  // A's natural (a,b) rows, the second the (b,a) copy, so that one tile accumulates both
+  // The six terms in pairs that write the same W3 layout: one term of a pair uses
+  // A's natural (a,b) rows, the other the (b,a) copy, so that one tile accumulates both
   // in tensor memory; every pair's fastest-varying output row index has W3 stride 1 or
   // its column index does.
-  const int pairs[3][2] = {{0, 5}, {1, 2}, {4, 3}};
-  std::vector<int> arow(6 * nb), brow(6 * nb);
-  std::vector<int64_t> coff(3 * nb);
-  for (int pq = 0; pq < 3; pq++) {
-    for (int b = 0; b < nb; b++) coff[pq * nb + b] = ((int64_t)pq * nb + b) * per;
-    for (int t = 0; t < 2; t++) {
-      const TriplesTerm& tm = terms[pairs[pq][t]];
-      for (int b = 0; b < nb; b++) {
-        const int* ijk = tuples + 3 * b;
-        arow[(2 * pq + t) * nb + b] = (int)(ijk[tm.x] * nv2);
-        brow[(2 * pq + t) * nb + b] = (int)((ijk[tm.y] * no + ijk[tm.z]) * nv);
-      }
-    }
+  // halves: with i == j the terms 5, 4, 3 are 0, 1, 2 with a and b exchanged, with j == k the terms
+  // 1, 5, 4 are 0, 2, 3 with b and c exchanged.  Such a tuple's arrays then hold S with
+  // W3 = S + S(exchanged): term 0 and the second pair (array 2 is not written), or the first
+  // pair and term 3 (array 1 is not); the energy kernels add the exchange in registers.  15 % of
+  // the products go at no = 16, 12 % at no = 20, 8 % at no = 32 (CCSD(T) no=16/nv=160
+  // 148.3 -> 146.6 ms, no=20/nv=200 409.7 -> 402.5 ms).  Half tuples come last in a launch, so a
+  // problem's number tells how many terms it has.
+  // In the last pair the (b,a) copy comes first: a half tuple takes a pair's first term alone.
+  const int pairs[3][2] = {{0, 5}, {1, 2}, {3, 4}};
+  std::vector<int> both[3], one[3];  // tuples with both terms of a pair, with the first
+  for (int b = 0; b < nb; b++) {
+    const int* ijk = tuples + 3 * b;
+    const bool ij = halves && ijk[0] == ijk[1], jk = halves && !ij && ijk[1] == ijk[2];
+    (ij ? one : both)[0].push_back(b);
+    if (!jk) both[1].push_back(b);
+    if (!ij) (jk ? one : both)[2].push_back(b);
   }
-  UCC_CUDA(cudaMemcpyAsync(T.d_coff, coff.data(), sizeof(int64_t) * 3 * nb, cudaMemcpyHostToDevice, c.stream));
-  UCC_CUDA(cudaMemcpyAsync(T.d_arow, arow.data(), sizeof(int) * 6 * nb, cudaMemcpyHostToDevice, c.stream));
-  UCC_CUDA(cudaMemcpyAsync(T.d_brow, brow.data(), sizeof(int) * 6 * nb, cudaMemcpyHostToDevice, c.stream));
+  std::vector<int> arow, brow;
+  std::vector<int64_t> coff;
+  for (int pq = 0; pq < 3; pq++) {
+    for (const auto* l : {&both[pq], &one[pq]})
+      for (int b : *l) coff.push_back(((int64_t)pq * nb + b) * per);
+    auto rows = [&](const TriplesTerm& tm, const std::vector<int>& l) {
+      for (int b : l) {
+        const int* ijk = tuples + 3 * b;
+        arow.push_back((int)(ijk[tm.x] * nv2));
+        brow.push_back((int)((ijk[tm.y] * no + ijk[tm.z]) * nv));
+      }
+    };
+    rows(terms[pairs[pq][0]], both[pq]);
+    rows(terms[pairs[pq][0]], one[pq]);
+    rows(terms[pairs[pq][1]], both[pq]);
+  }
+  UCC_CUDA(cudaMemcpyAsync(T.d_coff, coff.data(), sizeof(int64_t) * coff.size(), cudaMemcpyHostToDevice, c.stream));
+  UCC_CUDA(cudaMemcpyAsync(T.d_arow, arow.data(), sizeof(int) * arow.size(), cudaMemcpyHostToDevice, c.stream));
+  UCC_CUDA(cudaMemcpyAsync(T.d_brow, brow.data(), sizeof(int) * brow.size(), cudaMemcpyHostToDevice, c.stream));
   cudaEvent_t ev0 = c.take_event(), ev1 = c.take_event();
   UCC_CUDA(cudaEventRecord(ev0, c.stream));
+  size_t row = 0, off = 0;
   for (int pq = 0; pq < 3; pq++) {
-    const TriplesTerm& t0 = terms[pairs[pq][0]];
+    const int n2 = (int)both[pq].size(), n = n2 + (int)one[pq].size();
+    if (!n) continue;
+    const TriplesTerm& t0 = terms[pq == 2 ? 4 : pairs[pq][0]];  // output strides for A's natural rows
     Params p;
     p.M = (int)nv2;
     p.N = (int)nv;
@@ -2347,20 +2378,24 @@ bool mixed_triples_batch(Ctx& c, int nb, const int* tuples, float* W3, int tblk)
     p.epi.s_mlo = t0.sv;
     p.epi.s_n = t0.sw;
     p.err = k.err;
-    p.nprob = nb;
+    p.nprob = n;
     p.ksplit = 1;
     p.kchunk = p.kblocks;
-    p.a_row0 = T.d_arow + 2 * pq * nb;
-    p.b_row0 = T.d_brow + 2 * pq * nb;
-    p.c_off = T.d_coff + pq * nb;
-    p.nterms = 2;
-    p.a_row1 = T.d_arow + (2 * pq + 1) * nb;
-    p.b_row1 = T.d_brow + (2 * pq + 1) * nb;
-    const int tiles = p.mtiles * p.ntiles * nb;
+    p.nterms = n2 ? 2 : 1;
+    p.npair = n2;
+    p.a_row0 = T.d_arow + row;
+    p.b_row0 = T.d_brow + row;
+    p.a_row1 = T.d_arow + row + n;
+    p.b_row1 = T.d_brow + row + n;
+    p.c_off = T.d_coff + off;
+    row += (size_t)n + n2;
+    off += n;
+    const int tiles = p.mtiles * p.ntiles * n;
     p.nparts = 2;
     p.kc = 0;
     set_fused(p, true, 2);
-    launch_gemm(c, k, 2, tiles, T.A.mhi, T.A.mlo, T.B.mhi, T.B.mlo, T.A2.mhi, T.A2.mlo, T.A.mhi, T.B.mhi, p);
+    const Split &A0 = pq == 2 ? T.A2 : T.A, &A1 = pq == 2 ? T.A : T.A2;
+    launch_gemm(c, k, 2, tiles, A0.mhi, A0.mlo, T.B.mhi, T.B.mlo, A1.mhi, A1.mlo, A0.mhi, T.B.mhi, p);
   }
   UCC_CUDA(cudaEventRecord(ev1, c.stream));
   // timed with the other GEMMs (resolved lazily); the status flags are read at the next check

@@ -40,7 +40,7 @@
 namespace ucc {
 
 void count_kernel_launch();
-bool mixed_triples_batch(Ctx& c, int nbatch, const int* h_tuples, float* W3, int tblk = 0);
+bool mixed_triples_batch(Ctx& c, int nbatch, const int* h_tuples, float* W3, int tblk, bool halves);
 bool mixed_triples_prepare(Ctx& c, int max_batch);
 void mixed_triples_release(Ctx& c);
 void triples_operands_fp64(Ctx& c, Tensor& Acat, Tensor& Bcat);
@@ -244,7 +244,7 @@ void run_triples_gradient(Ctx& c) {
       const int64_t total = (int64_t)nt * nv3;
       const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 152 * 32));
       if (tc) {
-        mixed_triples_batch(c, nt, tuples.data(), static_cast<float*>(W32->p));
+        mixed_triples_batch(c, nt, tuples.data(), static_cast<float*>(W32->p), 0, false);
         tg_prep_kernel<float><<<g, 256, 0, c.stream>>>(no, nv, nt, static_cast<int*>(dtup.p),
                                                        static_cast<const float*>(W32->p), 3, (int64_t)nt * nv3,
                                                        Mb.d(), Nb.d(), eps, t1.p, t2.p, Voovv, fov);

@@ -21,7 +21,7 @@ namespace ucc {
 double flops_triples(double no, double nv) { return 2.0 * no * (no + 1) * (no + 2) * nv * nv * nv * (nv + no); }
 
 // mixed-precision tuple GEMMs (tc_gemm.cu); false if not available for this shape
-bool mixed_triples_batch(Ctx& c, int nbatch, const int* h_tuples, float* W3, int tblk = 0);
+bool mixed_triples_batch(Ctx& c, int nbatch, const int* h_tuples, float* W3, int tblk, bool halves);
 bool mixed_triples_prepare(Ctx& c, int max_batch);
 void mixed_triples_release(Ctx& c);
 
@@ -151,7 +151,7 @@ double run_triples(Ctx& c) {
   for (int t0 = 0; t0 < ntup; t0 += batch) {
     const int nb = std::min(batch, ntup - t0);
     if (mixed)
-      mixed_triples_batch(c, nb, tuples.data() + 3 * t0, static_cast<float*>(W3.p), f32in ? tblk : 0);
+      mixed_triples_batch(c, nb, tuples.data() + 3 * t0, static_cast<float*>(W3.p), f32in ? tblk : 0, true);
     else
       triples_w3_fp64(c, Acat, Bcat, tuples.data() + 3 * t0, nb, W3.d(), dp);
     if (mixed)
