@@ -610,7 +610,9 @@ CCSDResult run_ccsd(Ctx& c) {
   }
   Diis diis(c, np, 8);
   std::vector<cudaEvent_t> ev;
-  double rms = INFINITY, eccsd = NAN;
+  // a solve that stops in its first sweep reports the energy of its starting amplitudes, as any
+  // other reports that of the amplitudes its last sweep started from
+  double rms = INFINITY, eccsd = res.e_mp2;
   MixedSweeps sw(c);  // mixed precision: split, record and delta sweeps (cc.h)
   const bool mixed = sw.mixed();
   bool converged = false;
