@@ -94,7 +94,7 @@ struct Params {
   // accumulator added into the FP64 output by the epilogue (the first with beta, the
   // rest with 1), which bounds the FP32 accumulation chain; FP64 output only
   int kc;
-  // fused (two parts, kc == 0): one ring stage holds A_hi, A_lo, B_hi and B_lo of a K block
+  // fused (two parts): one ring stage holds A_hi, A_lo, B_hi and B_lo of a K block
   // and the three products are issued from it (a third less operand traffic than one
   // stage per product); nst stages of stage_bytes each
   int fused, nst, stage_bytes;
@@ -1707,38 +1707,78 @@ static void set_sliced_attrs(Cache& k) {
 // products' way through memory at about 4 TB/s.  An MMA's time hardly falls below 128 columns,
 // so narrow tiles pay only where they fill a wave.  The rule before (the widest tile that wastes
 // no column, the split with the fewest waves) counted neither: 2560^3 ran as z = 3 of
-// 256-column tiles, 228 us split and 2154 us sliced at nine digits; in two waves of 192-column
-// tiles it is 91 and 1272, and 160 x 40960 x 2048 at nine digits 2586 -> 1510.
+// 256-column tiles, 237 us split and 2154 us sliced at nine digits; in two waves of 192-column
+// tiles it is 126 (three passes over K) and 1272, and 160 x 40960 x 2048 at nine digits 2586 -> 1510.
+//
+// chain: the most K blocks that one accumulation in tensor memory may cover (accumulation_blocks;
+// kblocks where it does not matter).  z splits obey it; so do, where C is cheap to pass over
+// again (in_place), kc K blocks per pass with the passes added in C in FP64: a pass is added
+// behind the next one's products, which a z split's partial products are not (2560^3 in one
+// pass, with an accumulation nearly three times too long, took 74 us; 4000^3 220, in two 240 us).
 struct TilePlan {
-  int bn, z;
+  int bn, z, kc;  // N tile, K split, K blocks per pass (0: one pass)
 };
 static TilePlan plan_tiles(int64_t M, int64_t N, int kblocks, int cm, int slots, const double (&t)[8], double products,
-                           int units, int min_blocks) {
+                           int units, int min_blocks, int chain, bool in_place) {
   // ring items per K block of unit u: order u of the sliced form, the tail the rest
   auto unit_items = [&](int u) { return u + 1 < units ? u + 1.0 : products - 0.5 * u * (u + 1); };
-  TilePlan best{256, 1};
+  TilePlan best{256, 1, 0};
   double best_us = 1e300;
+  auto take = [&](double us, const TilePlan& p) {
+    if (us < best_us) best_us = us, best = p;
+  };
   const double groups = cm == 2 ? (double)(((M + BM - 1) / BM + 1) / 2) : (double)((M + BM - 1) / BM);
+  const double mb = 8e-6 * (double)M * N;
+  std::vector<int> zs = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64, 96, 128, 192, 256};
+  const int passes = (kblocks + chain - 1) / chain;
+  zs.push_back(passes);
   for (int bn = 256; bn >= 32; bn -= 32) {
     const double nt = (double)((N + bn - 1) / bn);
     if (bn > 32 && N <= bn - 32) continue;  // a whole step of padding
-    static const int zs[] = {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16, 20, 24, 32, 40, 48, 64, 96, 128, 192, 256};
+    const double epi = (units > 1 ? 0.12 : 0.033) * bn;
     for (int z : zs) {
-      if (z > 1 && (kblocks / z < min_blocks || 8.0 * (double)M * N * z > 2e9)) break;
-      const double kb = (double)((kblocks + z - 1) / z), epi = (units > 1 ? 0.12 : 0.033) * bn;
-      const double mb = 8e-6 * (double)M * N;
+      const int kb = (kblocks + z - 1) / z;
+      if (kb > chain) continue;
+      if (z > 1 && z != passes && (kblocks / z < min_blocks || 8.0 * (double)M * N * z > 2e9)) continue;
       double tile = 0.0;
       for (int u = 0; u < units; u++) tile += std::max(unit_items(u) * kb * t[bn / 32 - 1], epi);
       double us = std::ceil(groups * nt * z / slots) * tile + epi;
       if (units > 1 && mb * z > 100.0) us = std::max(us, mb * z * 2.0 * units / 4.0);
       if (z > 1) us += 5.0 + mb * ((units > 1 ? 2.0 : 1.0) * z + z + 2.0) / 4.0;
-      if (us < best_us) {
-        best_us = us;
-        best = TilePlan{bn, z};
-      }
+      take(us, TilePlan{bn, z, 0});
+    }
+    if (passes > 1 && in_place) {
+      const int kc = (kblocks + passes - 1) / passes;
+      const double tile = passes * std::max(products * kc * t[bn / 32 - 1], 2.0 * epi);
+      take(std::max(std::ceil(groups * nt / slots) * tile + epi, mb * 2.0 * passes / 4.0), TilePlan{bn, 1, kc});
     }
   }
   return best;
+}
+
+// K blocks that one FP32 accumulation of a split product may cover.  The tensor core truncates
+// its sums: at operands of one sign an accumulation over K elements loses 4.4e-9 K of the
+// result, which passes the 4.6e-6 that two bf16 parts leave near K = 1000.  These are the lengths
+// that the mixed form's stated accuracy was measured with: K in the number of parts (of at
+// least four blocks) that gives tiles as wide as possible the fewest waves of CTAs, one more part
+// only for a 5 % gain.  Lengths from time alone were up to five times as long, and so were the
+// errors (relative, normal / uniform operands):
+//   2560 x 2560 x 2560     896 elements 5.4e-6 / 3.4e-6,  2560 elements 9.9e-6 / 1.3e-5
+//   15440 x 136 x 12880   2624 elements 1.0e-5 / 1.3e-5, 12880 elements 4.5e-5 / 8.7e-5
+//   160 x 160 x 40960      576 elements 4.9e-6 / 2.3e-6,  1280 elements 6.3e-6 / 5.6e-6
+static int accumulation_blocks(int64_t M, int64_t N, int kblocks, int sms) {
+  if (kblocks < 8) return kblocks;
+  const int bn = pick_bn(N);
+  const int64_t tiles = (M + BM - 1) / BM * ((N + bn - 1) / bn);
+  const int zmax =
+      (int)std::min<int64_t>(std::min<int64_t>(kblocks / 4, 256), std::max<int64_t>(1, 8LL * sms / tiles));
+  int z = 1;
+  double best = (double)((tiles + sms - 1) / sms);
+  for (int y = 2; y <= zmax && 8.0 * M * N * y <= 2e9; y++) {
+    const double waves = (double)((tiles * y + sms - 1) / sms) / y;
+    if (waves < 0.95 * best) best = waves, z = y;
+  }
+  return (kblocks + z - 1) / z;
 }
 // microseconds of a ring item by columns / 32: a fused K block of the split form, a slice product
 constexpr double kSplitItem[8] = {0.56, 0.61, 0.66, 0.79, 0.94, 1.10, 1.28, 1.46};
@@ -1787,10 +1827,10 @@ static bool sliced_gemm_part(Ctx& c, int64_t M, int64_t N, int64_t K, double alp
   set_sliced_attrs(k);
   // neighbouring M tiles pair up in clusters (boxes of bn / 2 rows of B)
   const int cm = short_k ? 1 : cluster_m((int)((M + BM - 1) / BM));
-  TilePlan plan{N > 32 ? 48 : N > 16 ? 32 : 16, 1};
+  TilePlan plan{N > 32 ? 48 : N > 16 ? 32 : 16, 1, 0};
   if (!short_k)
     plan = plan_tiles(M, N, (int)((K + BK - 1) / BK), cm, cm == 2 ? k.max_pairs_sliced : k.sms, kSliceItem,
-                      0.5 * S * (S + 1), std::max(1, S - 2) + 1, 8);
+                      0.5 * S * (S + 1), std::max(1, S - 2) + 1, 8, (int)((K + BK - 1) / BK), false);
   const int bn = plan.bn;
   {
     const int64_t Mp = (M + 31) / 32 * 32, Np = (N + 31) / 32 * 32, kp = (K + BK - 1) / BK * BK;
@@ -1993,8 +2033,13 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
   // K chunks of one tile summed in FP64 (kc) are not split further
   const int kblocks = (int)((K + BK - 1) / BK);
   const bool chunks = kc > 0 && kc < kblocks;
+  // rows of C in whole sectors, or lanes along its contiguous rows
+  const bool in_place = parts == 2 && ((epi.s_n == 1 && (reinterpret_cast<uintptr_t>(C) & 31u) == 0 && epi.s_mhi % 4 == 0 &&
+                                        (!epi.msplit || epi.s_mlo % 4 == 0)) ||
+                                       (epi.s_mhi == 1 && !epi.msplit));
   const TilePlan plan = plan_tiles(M, N, kblocks, cm, cm == 2 ? k.max_pairs : k.sms, kSplitItem, parts == 2 ? 1.0 : 2.0,
-                                   1, chunks ? kblocks + 1 : 4);
+                                   1, chunks ? kblocks + 1 : 4,
+                                   chunks ? kblocks : accumulation_blocks(M, N, kblocks, k.sms), in_place);
   const int bn = plan.bn;
   // the maps are copied at once: A and B may be one cached operand read with two boxes
   Split* a = prepare(c, A, BM, ta, parts);
@@ -2020,7 +2065,7 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
   p.kchunk = p.kblocks;
   const int tiles = p.mtiles * p.ntiles;
   std::unique_ptr<Scratch> part;
-  p.kc = chunks ? kc : 0;
+  p.kc = chunks ? kc : plan.kc;
   {
     // FP64 partial products of the K chunks, added in a fixed order
     const int ks = plan.z;
@@ -2043,7 +2088,7 @@ void tc_gemm_run(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const Ma
   p.a_row1 = p.b_row1 = nullptr;
   p.C32 = nullptr;
   p.nparts = parts;
-  set_fused(p, parts == 2 && p.kc == 0, cm);
+  set_fused(p, parts == 2, cm);
   launch_gemm(c, k, cm, tiles * p.ksplit, a_hi, a_lo, b_hi, b_lo, a_hi, a_lo, parts == 3 ? a_mid : a_hi,
               parts == 3 ? b_mid : b_hi, p);
   if (part) splitk_reduce(c, M, N, p.ksplit, part->d(), alpha, beta, C, epi);
