@@ -165,6 +165,28 @@ __device__ __forceinline__ void tile_coords(const Params& p, int mgroups, int ti
   }
 }
 
+// The loads of a pair's ring complete on rank 0's barriers, and rank 0 waits for those of the stages
+// that it issued itself.  After a wait that ran out its peer can be up to a ring ahead, with loads in
+// flight into its own shared memory that nobody waits for.  So both producers leave their count of
+// issued stages with both CTAs (issued[rank], before the cluster's last barrier), and when the
+// counts differ rank 0 expects and awaits the peer's surplus, `bytes` a stage, before either leaves.
+// Without an error the counts are equal and nothing more is done.
+__device__ __forceinline__ void pair_tell(int64_t* issued, int rank, int64_t n) {
+  issued[rank] = n;
+  asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(map_rank(issued + rank, (uint32_t)(rank ^ 1))), "l"(n)
+               : "memory");
+}
+__device__ __forceinline__ void pair_drain(uint64_t* full, int nst, const int64_t* issued, int rank, uint32_t bytes) {
+  const int64_t n0 = issued[0], n1 = issued[1];
+  if (n0 == n1) return;
+  if (rank == 0 && threadIdx.x == 0)
+    for (int64_t n = n0; n < n1; n++) {
+      mbar_expect_tx(&full[n % nst], bytes);
+      mbar_wait_deadline(&full[n % nst], (uint32_t)((n / nst) & 1));
+    }
+  cluster_sync();
+}
+
 // CM CTAs per cluster along M (1 or 2).  With CM = 2 the two CTAs of a cluster work as a pair
 // (cta_group::2) on M tiles 2j and 2j+1 of one N tile: each CTA's ring holds its own 128 rows
 // of A and half of the B tile's rows (the B tensor maps have boxes of bn / 2 rows), rank 0
@@ -192,7 +214,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint64_t* tfull = empty + STAGES;
   uint64_t* tempty = tfull + 2;
   uint64_t* mdone = tempty + 2;  // every MMA of this CTA has completed (before TMEM is released)
-  uint32_t* tslot = (uint32_t*)(mdone + 1);
+  int64_t* issued_of = (int64_t*)(mdone + 1);  // stages issued by the CTAs of a pair
+  uint32_t* tslot = (uint32_t*)(issued_of + 2);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int nst = p.fused ? p.nst : STAGES;  // ring stages (at most STAGES)
   const int rank = CM > 1 ? (int)cluster_rank() : 0;
@@ -293,10 +316,11 @@ __global__ void __launch_bounds__(THREADS, 1)
       }
       // the last ring loads must have landed before the CTA may exit (matters only on an
       // error path; normally the epilogue's final wait already implies it); rank 0's barriers
-      // see the loads of both, and the cluster leaves together
+      // see the loads of both (pair_drain)
       if (rank == 0)
         for (int64_t n = issued > nst ? issued - nst : 0; n < issued; n++)
           mbar_wait_deadline(&full[n % nst], (uint32_t)((n / nst) & 1));
+      if (CM > 1) pair_tell(issued_of, rank, issued);
     }
   } else if (warp == 1) {
     if (lane == 0 && rank != 0) {
@@ -514,8 +538,11 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
   fence_before();
   __syncthreads();
-  // no CTA leaves while MMAs may still read its ring or its peer arrive on its barriers
-  if (CM > 1) cluster_sync();
+  // no CTA leaves while MMAs may still read its ring, its peer arrive on its barriers or loads be in flight
+  if (CM > 1) {
+    cluster_sync();
+    pair_drain(full, nst, issued_of, rank, p.fused ? (uint32_t)(2 * A_BYTES) + 2 * b_tile : (uint32_t)A_BYTES + b_tile);
+  }
   if (warp == 1) {
     fence_after();
     tmem_dealloc<CM>(tmem, TMEM_COLS);
@@ -619,7 +646,8 @@ __global__ void __launch_bounds__(THREADS, 1)
   uint64_t* tfull = empty + sliced_stages(2);
   uint64_t* tempty = tfull + 2;
   uint64_t* mdone = tempty + 2;  // every MMA of this CTA has completed (before TMEM is released)
-  uint32_t* tslot = (uint32_t*)(mdone + 1);
+  int64_t* issued_of = (int64_t*)(mdone + 1);  // stages issued by the CTAs of a pair
+  uint32_t* tslot = (uint32_t*)(issued_of + 2);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int rank = CM > 1 ? (int)cluster_rank() : 0;
   constexpr int NST = sliced_stages(CM), STAGE = A_BYTES + B_BYTES / CM;
@@ -701,6 +729,7 @@ __global__ void __launch_bounds__(THREADS, 1)
       if (rank == 0)
         for (int64_t n = issued > NST ? issued - NST : 0; n < issued; n++)
           mbar_wait_deadline(&full[n % NST], (uint32_t)((n / NST) & 1));
+      if (CM > 1) pair_tell(issued_of, rank, issued);
     }
   } else if (warp == 1) {
     if (lane == 0 && rank != 0) {
@@ -855,7 +884,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   }
   fence_before();
   __syncthreads();
-  if (CM > 1) cluster_sync();  // the peer no longer multicasts into this ring
+  if (CM > 1) {  // as in gemm_kernel
+    cluster_sync();
+    pair_drain(full, NST, issued_of, rank, (uint32_t)(A_BYTES + bh * BK * 2));
+  }
   if (warp == 1) {
     fence_after();
     tmem_dealloc<CM>(tmem, TMEM_COLS);
