@@ -13,8 +13,8 @@
 //
 // Rules: chain_enter() is the first statement, before any access to global memory.  As every
 // kernel of a chain waits for its predecessor's end, the wait covers all that came before.  The
-// kernel's pointers are not __restrict__: what is read through such a pointer could be fetched
-// ahead of the wait.  A launch without the attribute, a copy or an event between two kernels
+// kernel's pointers are not __restrict__, nor are those of the functions inlined into it: what is
+// read through such a pointer could be fetched ahead of the wait.  A launch without the attribute, a copy or an event between two kernels
 // waits as always.
 #pragma once
 

@@ -134,8 +134,8 @@ __global__ void permute_kernel_rows(PermArgs a) {
   const I warp = ((I)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const I per = (items + nwarps - 1) / nwarps;
   const I w0 = warp * per, w1 = (w0 + per < items) ? w0 + per : items;
-  const double* __restrict__ in = a.in;
-  double* __restrict__ out = a.out;
+  const double* in = a.in;
+  double* out = a.out;
   I cur = (I)-1, bi = 0, bo = 0;
   for (I w = w0; w < w1; w++) {
     const I row = w / nseg, x0 = (w - row * nseg) * 128;

@@ -6,7 +6,9 @@
 // Pairs p <= q are numbered q(q+1)/2 + p, strict pairs p < q are numbered q(q-1)/2 + p.
 // The passes are HBM-bound; the pair numbers of a tile and a slice come from one decode per
 // block, since an FP64 square root per element would keep GB300's FP64 pipe (two operations
-// per SM clock) busier than the memory.
+// per SM clock) busier than the memory.  The functions are inlined into kernels whose first
+// statement waits for the kernel before (chain.h), so no pointer is __restrict__; each loads what a
+// thread needs of a tile before its first store, which might alias it.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -33,32 +35,37 @@ struct TileBuf {
 //             W[e][f] itself with `plain`
 //   M[e<f]  = h (W[e][f] - W[f][e])   (M may be null)
 // written along e, which is contiguous in both for a fixed f.
-__device__ __forceinline__ void pack_slice_tile(TileBuf& s, int nv, double h, const double* __restrict__ t,
-                                                const double* __restrict__ u, bool keep_diag, bool plain, double* P,
+__device__ __forceinline__ void pack_slice_tile(TileBuf& s, int nv, double h, const double* t,
+                                                const double* u, bool keep_diag, bool plain, double* P,
                                                 double* M, int tp) {
   int E, F;
   pair_of(tp, E, F);
   const int e0 = E * 32, f0 = F * 32, tx = threadIdx.x, ty = threadIdx.y;
+  double va[4], vb[4];
 #pragma unroll
-  for (int r = ty; r < 32; r += 8) {
-    const int ea = e0 + r, fa = f0 + tx, fb = f0 + r, eb = e0 + tx;
-    const bool oka = ea < nv && fa < nv, okb = fb < nv && eb < nv;
-    s.a[r][tx] = oka ? t[(int64_t)ea * nv + fa] : 0.0;  // a[e][f] = t[e][f]
-    s.b[tx][r] = okb ? t[(int64_t)fb * nv + eb] : 0.0;  // b[e][f] = t[f][e]
+  for (int q = 0; q < 4; q++) {
+    const int ea = e0 + ty + 8 * q, fa = f0 + tx, fb = f0 + ty + 8 * q, eb = e0 + tx;
+    va[q] = ea < nv && fa < nv ? t[(int64_t)ea * nv + fa] : 0.0;
+    vb[q] = fb < nv && eb < nv ? t[(int64_t)fb * nv + eb] : 0.0;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    s.a[ty + 8 * q][tx] = va[q];  // a[e][f] = t[e][f]
+    s.b[tx][ty + 8 * q] = vb[q];  // b[e][f] = t[f][e]
   }
   if (u) {
-    __syncthreads();
 #pragma unroll
-    for (int r = ty; r < 32; r += 8) {
-      const int ea = e0 + r, fa = f0 + tx;
-      if (ea < nv && fa < nv) s.b[r][tx] += u[(int64_t)ea * nv + fa];  // W[f][e] has u[e][f]
+    for (int q = 0; q < 4; q++) {
+      const int ea = e0 + ty + 8 * q, fa = f0 + tx, fb = f0 + ty + 8 * q, eb = e0 + tx;
+      va[q] = ea < nv && fa < nv ? u[(int64_t)ea * nv + fa] : 0.0;
+      vb[q] = fb < nv && eb < nv ? u[(int64_t)fb * nv + eb] : 0.0;
     }
     __syncthreads();
 #pragma unroll
-    for (int r = ty; r < 32; r += 8) {
-      const int fb = f0 + r, eb = e0 + tx;
-      if (fb < nv && eb < nv) s.a[tx][r] += u[(int64_t)fb * nv + eb];  // W[e][f] has u[f][e]
-    }
+    for (int q = 0; q < 4; q++) s.b[ty + 8 * q][tx] += va[q];  // W[f][e] has u[e][f]
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; q++) s.a[tx][ty + 8 * q] += vb[q];  // W[e][f] has u[f][e]
   }
   __syncthreads();
   for (int c = ty; c < 32; c += 8) {  // f = f0 + c, e = e0 + tx along the lanes
@@ -83,31 +90,36 @@ __device__ __forceinline__ void pack_tau_tile(TileBuf& s, int no, int nv, const 
 
 // The ring terms' combinations of one slice (i, j), tile (E, F) of all nt^2 tiles:
 //   X[ijef] = t2/2 + t1[ie] t1[jf];  P[ijef] = t2[ijfe] - X[ijef];  S[ijef] = t2 - t2[ijfe]/2
-__device__ __forceinline__ void ring_tile(TileBuf& s, int no, int nv, const double* __restrict__ t1,
-                                          const double* __restrict__ t2, double* X, double* P, double* S, int tile,
+__device__ __forceinline__ void ring_tile(TileBuf& s, int no, int nv, const double* t1,
+                                          const double* t2, double* X, double* P, double* S, int tile,
                                           int64_t slice) {
   const int nt = (nv + 31) / 32, e0 = tile / nt * 32, f0 = tile % nt * 32, tx = threadIdx.x, ty = threadIdx.y;
   const int64_t base = slice * (int64_t)nv * nv;
   const double* t = t2 + base;
   const double* ti = t1 + slice / no * nv;
   const double* tj = t1 + slice % no * nv;
-#pragma unroll
-  for (int r = ty; r < 32; r += 8) {
-    const int fb = f0 + r, eb = e0 + tx;
-    s.b[tx][r] = fb < nv && eb < nv ? t[(int64_t)fb * nv + eb] : 0.0;
-  }
-  __syncthreads();
   const int f = f0 + tx;
   const double tjf = f < nv ? tj[f] : 0.0;
+  double vb[4], v[4], ti4[4];
 #pragma unroll
-  for (int r = ty; r < 32; r += 8) {
-    const int e = e0 + r;
+  for (int q = 0; q < 4; q++) {
+    const int fb = f0 + ty + 8 * q, eb = e0 + tx, e = e0 + ty + 8 * q;
+    vb[q] = fb < nv && eb < nv ? t[(int64_t)fb * nv + eb] : 0.0;
+    v[q] = e < nv && f < nv ? t[(int64_t)e * nv + f] : 0.0;
+    ti4[q] = e < nv ? ti[e] : 0.0;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) s.b[tx][ty + 8 * q] = vb[q];
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int r = ty + 8 * q, e = e0 + r;
     if (e >= nv || f >= nv) continue;
     const int64_t o = (int64_t)e * nv + f;
-    const double v = t[o], w = s.b[r][tx], x = fma(0.5, v, ti[e] * tjf);
+    const double w = s.b[r][tx], x = fma(0.5, v[q], ti4[q] * tjf);
     X[base + o] = x;
     P[base + o] = w - x;
-    S[base + o] = fma(-0.5, w, v);
+    S[base + o] = fma(-0.5, w, v[q]);
   }
   __syncthreads();
 }
@@ -118,9 +130,9 @@ __device__ __forceinline__ void ring_tile(TileBuf& s, int no, int nv, const doub
 // exactly one of i > j, a > b holds; A = 0 on i == j or a == b; S null: no such term).  One value goes to ijab and
 // jiba and one to ijba and jiab, so R2 is exactly symmetric whatever the rounding of Rh and H:
 // in the antisymmetric sector the Jacobi step of the solver does not damp.
-__device__ __forceinline__ void assemble_tile(TileBuf& s, int no, int nv, const double* __restrict__ V,
-                                              const double* __restrict__ S, int64_t ldS, const double* __restrict__ A,
-                                              int64_t ldA, const double* __restrict__ Rh, const double* __restrict__ H,
+__device__ __forceinline__ void assemble_tile(TileBuf& s, int no, int nv, const double* V,
+                                              const double* S, int64_t ldS, const double* A,
+                                              int64_t ldA, const double* Rh, const double* H,
                                               double* R2, int tp, int64_t R) {
   int ta, tb, i, j;
   pair_of(tp, ta, tb);
@@ -129,34 +141,45 @@ __device__ __forceinline__ void assemble_tile(TileBuf& s, int no, int nv, const 
   const int64_t nv2 = (int64_t)nv * nv, ij = ((int64_t)i * no + j) * nv2, ji = ((int64_t)j * no + i) * nv2;
   const double* Srow = S + R * ldS;
   const double* Arow = A + ((int64_t)j * (j - 1) / 2 + i) * ldA;  // read for i < j only
+  double u1[4], u2[4];
 #pragma unroll
-  for (int r = ty; r < 32; r += 8) {  // along a: the transposed elements and the packed ones
-    const int b = b0 + r, a = a0 + tx;
-    double u1 = 0.0, u2 = 0.0;
+  for (int q = 0; q < 4; q++) {  // along a: the transposed elements and the packed ones
+    const int b = b0 + ty + 8 * q, a = a0 + tx;
+    u1[q] = u2[q] = 0.0;
     if (b < nv && a <= b) {
       const int64_t o = (int64_t)b * nv + a;
       const double h3 = H[ij + o], h2 = H[ji + o];
       const double sp = S ? Srow[(int64_t)b * (b + 1) / 2 + a] : 0.0;
       const double am = S && i < j && a < b ? Arow[(int64_t)b * (b - 1) / 2 + a] : 0.0;
-      u1 = (fma(0.5, h2, Rh[ji + o]) + h3) + (sp + am);
-      u2 = (fma(0.5, h3, Rh[ij + o]) + h2) + (sp - am);
+      u1[q] = (fma(0.5, h2, Rh[ji + o]) + h3) + (sp + am);
+      u2[q] = (fma(0.5, h3, Rh[ij + o]) + h2) + (sp - am);
     }
-    s.a[tx][r] = u1;
-    s.b[tx][r] = u2;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    s.a[tx][ty + 8 * q] = u1[q];
+    s.b[tx][ty + 8 * q] = u2[q];
   }
   __syncthreads();
 #pragma unroll
-  for (int r = ty; r < 32; r += 8) {
-    const int a = a0 + r, b = b0 + tx;
+  for (int q = 0; q < 4; q++) {
+    const int r = ty + 8 * q, a = a0 + r, b = b0 + tx;
     if (b < nv && a <= b) {
       const int64_t o = (int64_t)a * nv + b;
       const double h1 = H[ij + o], h4 = H[ji + o];
-      const double r1 = ((fma(0.5, h1, Rh[ij + o]) + h4) + s.a[r][tx]) + V[ij + o];
-      const double r2 = ((fma(0.5, h4, Rh[ji + o]) + h1) + s.b[r][tx]) + V[ji + o];
-      R2[ij + o] = r1;
-      if (i < j) R2[ji + o] = r2;
-      s.a[r][tx] = r1;
-      s.b[r][tx] = r2;
+      u1[q] = ((fma(0.5, h1, Rh[ij + o]) + h4) + s.a[r][tx]) + V[ij + o];
+      u2[q] = ((fma(0.5, h4, Rh[ji + o]) + h1) + s.b[r][tx]) + V[ji + o];
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int r = ty + 8 * q, a = a0 + r, b = b0 + tx;
+    if (b < nv && a <= b) {
+      const int64_t o = (int64_t)a * nv + b;
+      R2[ij + o] = u1[q];
+      if (i < j) R2[ji + o] = u2[q];
+      s.a[r][tx] = u1[q];
+      s.b[r][tx] = u2[q];
     }
   }
   __syncthreads();
@@ -174,8 +197,8 @@ __device__ __forceinline__ void assemble_tile(TileBuf& s, int no, int nv, const 
 
 // Element x of Z[m][b][i][j] = (S + sign A)[(i,j) sorted][off + mb], off the number of packed
 // ladder columns before the (m,b) ones
-__device__ __forceinline__ double z_element(int no, int nv, const double* __restrict__ S, int64_t ldS,
-                                            const double* __restrict__ A, int64_t ldA, int64_t x) {
+__device__ __forceinline__ double z_element(int no, int nv, const double* S, int64_t ldS,
+                                            const double* A, int64_t ldA, int64_t x) {
   const int64_t oo = (int64_t)no * no, mb = x / oo;
   const int y = (int)(x - mb * oo), i = y / no, j = y - i * no;
   const int p = i < j ? i : j, q = i < j ? j : i;
@@ -190,8 +213,8 @@ __device__ __forceinline__ double z_element(int no, int nv, const double* __rest
 
 // Element x of [no][no][nv][nv] from the packed S and A (see assemble_tile)
 template <class I>
-__device__ __forceinline__ double unpack_pair(int no, int nv, const double* __restrict__ S,
-                                              const double* __restrict__ A, I x) {
+__device__ __forceinline__ double unpack_pair(int no, int nv, const double* S,
+                                              const double* A, I x) {
   const I v_ = (I)nv, o_ = (I)no, vp = v_ * (v_ + 1) / 2, vm = v_ * (v_ - 1) / 2;
   const I b = x % v_;
   I r = x / v_;
