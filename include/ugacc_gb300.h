@@ -274,7 +274,7 @@ typedef struct ucc_stats {
   int64_t tc_gemm_launches;  /* tensor-core (BF16 split) GEMM launches */
   int mixed_iterations;      /* CCSD iterations with split-product residuals */
   double tc_gemm_ms;         /* device time of the tensor-core GEMMs (CUDA events) */
-  double tc_gemm_flops;      /* their algorithmic FLOPs, 2*M*N*K per GEMM */
+  double tc_gemm_flops;      /* their algorithmic FLOPs, 2*M*N*K per product that was launched */
   int anchored_iterations;   /* refinement iterations built as FP64 anchor + tensor-core corrections */
   double fp64_gemm_ms;       /* device time of the FP64 GEMM launches (CUDA events; the short ones' own clock) */
   double fp64_gemm_flops;    /* their algorithmic FLOPs, 2*M*N*K per GEMM */

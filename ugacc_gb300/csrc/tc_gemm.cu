@@ -2475,8 +2475,9 @@ bool mixed_triples_batch(Ctx& c, int nb, const int* tuples, float* W3, int tblk,
     launch_gemm(c, k, 2, tiles, A0.mhi, A0.mlo, T.B.mhi, T.B.mlo, A1.mhi, A1.mlo, A0.mhi, T.B.mhi, p);
   }
   UCC_CUDA(cudaEventRecord(ev1, c.stream));
-  // timed with the other GEMMs (resolved lazily); the status flags are read at the next check
-  c.gemm_timers.push_back({ev0, ev1, 2.0 * 6.0 * (double)nv2 * (double)nv * (double)(nv + no) * nb, 1});
+  // timed with the other GEMMs (resolved lazily), `row` products of one term each; the status flags are read
+  // at the next check
+  c.gemm_timers.push_back({ev0, ev1, 2.0 * (double)row * (double)nv2 * (double)nv * (double)(nv + no), 1});
   if (c.gemm_timers.size() >= 4096) c.resolve_timers();
   k.unchecked = true;
   return true;
