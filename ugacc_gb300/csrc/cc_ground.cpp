@@ -234,12 +234,27 @@ double flops_ccsd_iter(double no, double nv) {
                 8.0 * no * no * nv * nv * nv);
 }
 
+// Two blocks that are there together and filled, or not at all: their presence says that they are built.
+template <typename F>
+static void build_blocks(Ctx& c, const char* p, const std::vector<int64_t>& pdims, const char* m,
+                         const std::vector<int64_t>& mdims, F&& fill) {
+  if (c.has(p)) return;
+  try {
+    Tensor P = c.alloc(p, pdims, false), M = c.alloc(m, mdims, false);
+    fill(P.p, M.p);
+  } catch (...) {
+    c.drop(p);
+    c.drop(m);
+    throw;
+  }
+}
+
 void pair_operator(Ctx& c) {
   const int64_t no = c.no, nv = c.nv, vp = nv * (nv + 1) / 2, vm = nv * (nv - 1) / 2;
-  if (c.has("Vpp")) return;
-  Tensor Vp = c.alloc("Vpp", {vp + no * nv, vp}, false), Vm = c.alloc("Vmm", {vm + no * nv, vm}, false);
-  pack_vvvv(c, c.nv, 0, c.get("Vvvvv").p, Vp.p, Vm.p);
-  pack_ovvv(c, c.no, c.nv, c.get("Vovvv").p, Vp.p + vp * vp, Vm.p + vm * vm);
+  build_blocks(c, "Vpp", {vp + no * nv, vp}, "Vmm", {vm + no * nv, vm}, [&](double* P, double* M) {
+    pack_vvvv(c, c.nv, 0, c.get("Vvvvv").p, P, M);
+    pack_ovvv(c, c.no, c.nv, c.get("Vovvv").p, P + vp * vp, M + vm * vm);
+  });
 }
 
 // R2 += alpha sum_ef W_abef amp_ijef on packed pairs (pairs.cu), W from an HBAR block: S = Tp Vp^T
@@ -252,10 +267,8 @@ void packed_ladder(Ctx& c, double alpha, const Tensor& amp, const char* src, int
   const int no = c.no, nv = c.nv;
   const int64_t op = (int64_t)no * (no + 1) / 2, om = (int64_t)no * (no - 1) / 2;
   const int64_t vp = (int64_t)nv * (nv + 1) / 2, vm = (int64_t)nv * (nv - 1) / 2;
-  if (!c.has(vp_name)) {
-    Tensor Vp = c.alloc(vp_name, {vp, vp}, false), Vm = c.alloc(vm_name, {vm, vm}, false);
-    pack_vvvv(c, nv, mode, c.get(src).p, Vp.p, Vm.p);
-  }
+  build_blocks(c, vp_name, {vp, vp}, vm_name, {vm, vm},
+               [&](double* P, double* M) { pack_vvvv(c, nv, mode, c.get(src).p, P, M); });
   UCC_REQUIRE(amp.dense(), UCC_BAD_ARGS, "packed ladder: dense amplitudes");
   Temp Tp(c, {op, vp}), Tm(c, {om, vm}), S(c, {op, vp}), A(c, {om, vm});
   pack_tau(c, no, nv, amp.p, Tp->p, Tm->p);

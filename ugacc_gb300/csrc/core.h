@@ -50,9 +50,12 @@ struct Error : std::runtime_error {
   Error(ucc_status s, const std::string& m) : std::runtime_error(m), status(s) {}
 };
 
+// An allocation that fails leaves the context usable: the runtime's record of it is cleared, so that
+// the check after the next launch does not find it.
 #define UCC_CUDA(call)                                                                     \
   do {                                                                                     \
     cudaError_t e_ = (call);                                                               \
+    if (e_ == cudaErrorMemoryAllocation) cudaGetLastError();                               \
     if (e_ != cudaSuccess)                                                                 \
       throw ::ucc::Error(e_ == cudaErrorMemoryAllocation ? UCC_OUT_OF_MEMORY : UCC_CUDA_ERROR, \
                          std::string(#call) + ": " + cudaGetErrorString(e_));             \

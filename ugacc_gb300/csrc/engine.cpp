@@ -155,8 +155,9 @@ Tensor Ctx::alloc(const std::string& name, const std::vector<int64_t>& dims, boo
   for (auto x : dims) n *= (size_t)x;
   auto it = store.find(name);
   if (it == store.end() || it->second->n != n) {
-    store[name].reset();
-    store[name] = std::make_unique<DeviceBuffer>(n, stream);
+    drop(name);  // a failed allocation leaves no entry
+    auto b = std::make_unique<DeviceBuffer>(n, stream);
+    store[name] = std::move(b);
   }
   shapes[name] = dims;
   if (zero && n) UCC_CUDA(cudaMemsetAsync(store[name]->p, 0, n * sizeof(double), stream));
