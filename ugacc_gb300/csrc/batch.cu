@@ -744,6 +744,7 @@ void build(ucc_batch& B) {
   for (int b = 0; b < nm; b++) {
     Ctx& c = *B.members[b];
     ccsd_alloc(c);
+    c.pair_rows = true;
     if (packed) pair_operator(c);
     const double* to = c.get("Told").p;
     double* r = c.get("R").p;

@@ -63,6 +63,27 @@ ucc_status guard(ucc_ctx* ctx, F&& f) {
   }
 }
 
+// One stage, tried again once if it runs out of memory while the packed ladder operator can give
+// some back: CCSD without the (m, b) rows, a later stage without the operator.  A stage starts
+// from what the ones before it left, so a second attempt is a first one.
+template <typename F>
+void stage(Ctx& c, bool rows, F&& f) {
+  struct Drop {  // the guess that the stage has read applies to this call only
+    Ctx& c;
+    ~Drop() {
+      if (!c.taken.empty()) c.drop(c.taken);
+      c.taken.clear();
+    }
+  } drop{c};
+  try {
+    f();
+    return;
+  } catch (const Error& e) {
+    if (e.status != UCC_OUT_OF_MEMORY || !release_pair_operator(c, rows)) throw;
+  }
+  f();
+}
+
 void reset_state(Ctx& c) {
   cudaStreamSynchronize(c.stream);
   c.tc_cache.reset();
@@ -193,7 +214,8 @@ ucc_status ucc_ccsd(ucc_ctx* ctx, double* e, int* iters) {
     const int64_t l0 = launches();
     Timer tm(c.stream);
     tm.start();
-    CCSDResult r = run_ccsd(c);
+    CCSDResult r;
+    stage(c, true, [&] { r = run_ccsd(c); });
     c.stats.ccsd_ms += tm.stop_ms();
     c.stats.ccsd_iterations = r.iterations;
     c.stats.ccsd_flops += flops_ccsd_iter(c.no, c.nv) * r.iterations;
@@ -215,7 +237,8 @@ ucc_status ucc_triples(ucc_ctx* ctx, double* et) {
     const int64_t l0 = launches();
     Timer tm(c.stream);
     tm.start();
-    const double e = run_triples(c);
+    double e = 0.0;
+    stage(c, false, [&] { e = run_triples(c); });
     c.stats.triples_ms += tm.stop_ms();
     c.stats.triples_flops += flops_triples(c.no, c.nv);
     c.stats.kernel_launches += launches() - l0;
@@ -229,7 +252,7 @@ ucc_status ucc_triples_gradient(ucc_ctx* ctx) {
     const int64_t l0 = launches();
     Timer tm(c.stream);
     tm.start();
-    run_triples_gradient(c);
+    stage(c, false, [&] { run_triples_gradient(c); });
     c.stats.triples_ms += tm.stop_ms();
     c.stats.kernel_launches += launches() - l0;
   });
@@ -241,7 +264,7 @@ ucc_status ucc_hbar(ucc_ctx* ctx) {
     const int64_t l0 = launches();
     Timer tm(c.stream);
     tm.start();
-    run_hbar(c);
+    stage(c, false, [&] { run_hbar(c); });
     c.stats.hbar_ms += tm.stop_ms();
     c.stats.kernel_launches += launches() - l0;
   });
@@ -254,7 +277,8 @@ ucc_status ucc_lambda(ucc_ctx* ctx, double* pseudo, int* iters) {
     const int64_t l0 = launches();
     Timer tm(c.stream);
     tm.start();
-    CCSDResult r = run_lambda(c);
+    CCSDResult r;
+    stage(c, false, [&] { r = run_lambda(c); });
     c.stats.lambda_ms += tm.stop_ms();
     c.stats.lambda_iterations = r.iterations;
     c.stats.kernel_launches += launches() - l0;
@@ -276,7 +300,7 @@ ucc_status ucc_density(ucc_ctx* ctx, double* e1, double* e2) {
     Timer tm(c.stream);
     tm.start();
     double a = 0, b = 0;
-    run_density(c, &a, &b);
+    stage(c, false, [&] { run_density(c, &a, &b); });
     c.stats.density_ms += tm.stop_ms();
     c.stats.kernel_launches += launches() - l0;
     if (e1) *e1 = a;
@@ -296,7 +320,7 @@ ucc_status ucc_pert_create(ucc_ctx* ctx, const double* pert, double omega, int* 
   return guard(ctx, [&](Ctx& c) {
     UCC_REQUIRE(pert && handle && std::isfinite(omega), UCC_BAD_ARGS, "need pert, handle and a finite omega");
     UCC_CUDA(cudaSetDevice(c.device));
-    *handle = pert_create(c, pert, omega);
+    stage(c, false, [&] { *handle = pert_create(c, pert, omega); });
   });
 }
 
@@ -308,7 +332,8 @@ ucc_status ucc_pert_solve(ucc_ctx* ctx, int handle, int hand, double* pseudo, in
     const int64_t l0 = launches();
     Timer tm(c.stream);
     tm.start();
-    CCSDResult r = pert_solve(c, handle, hand == 1);
+    CCSDResult r;
+    stage(c, false, [&] { r = pert_solve(c, handle, hand == 1); });
     c.stats.pert_ms += tm.stop_ms();
     c.stats.kernel_launches += launches() - l0;
     if (pseudo) *pseudo = r.e_ccsd;
@@ -327,7 +352,7 @@ ucc_status ucc_linresp(ucc_ctx* ctx, int hx, int hy, double* value) {
     UCC_REQUIRE(value, UCC_BAD_ARGS, "null output");
     UCC_CUDA(cudaSetDevice(c.device));
     const int64_t l0 = launches();
-    *value = linresp(c, hx, hy);
+    stage(c, false, [&] { *value = linresp(c, hx, hy); });
     c.stats.kernel_launches += launches() - l0;
   });
 }

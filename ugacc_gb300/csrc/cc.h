@@ -101,9 +101,17 @@ void ccsd_alloc(Ctx& c);                                         // CCSD work ar
 void ccsd_residual(Ctx& c, const double* t_old, double* r);      // R(t_old), tau/ttau current
 double ccsd_energy(Ctx& c, const double* t);                     // E from t and the stored tau
 double run_triples(Ctx& c);
-// the packed operator of the CCSD ladder ("Vpp", "Vmm": the a <= b rows of <ab|ef>, then the
-// (m, b) rows of <mb|ef>), built once per Hamiltonian
+// the packed operator of the CCSD ladder ("Vpp", "Vmm": the a <= b rows of <ab|ef>, then with
+// c.pair_rows the (m, b) rows of <mb|ef>), built once per Hamiltonian
 void pair_operator(Ctx& c);
+// Device bytes of a CCSD solve with that operator, rows included, and the share of the device's memory that it
+// may take for the rows to be built.  A choice by the sizes alone: results do not depend on
+// what else uses the device, as long as it leaves enough.
+double ccsd_bytes(int64_t no, int64_t nv);
+constexpr double kPairRowsShare = 0.8;
+// After an allocation that failed: gives the operator back, to be built again without the (m, b) rows where it
+// is needed next.  False if there is nothing to give back (rows: if it has no such rows).
+bool release_pair_operator(Ctx& c, bool rows);
 // R2 += alpha sum_ef W_abef amp_ijef on packed pairs (cc_ground.cpp), W from HBAR block src by
 // mode (1: H_efab + H_feba, 2: H_abef + H_bafe)
 void packed_ladder(Ctx& c, double alpha, const Tensor& amp, const char* src, int mode, const char* vp_name,

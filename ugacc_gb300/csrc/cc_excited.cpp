@@ -229,7 +229,10 @@ CCSDResult run_lambda(Ctx& c) {  // :93-129
   } else {  // a supplied guess applies to this solve only
     UCC_CUDA(cudaMemcpyAsync(Lam.p, c.get("Lam_guess").p, sizeof(double) * np, cudaMemcpyDeviceToDevice, c.stream));
     UCC_CUDA(cudaStreamSynchronize(c.stream));
-    c.drop("Lam_guess");
+    if (c.has("Vpp"))
+      c.taken = "Lam_guess";  // kept for a second attempt (release_pair_operator)
+    else
+      c.drop("Lam_guess");
   }
   Tensor eps = c.get("eps");
   HostBlock sums(c);  // of a sweep: sum of squares, then the DIIS overlaps

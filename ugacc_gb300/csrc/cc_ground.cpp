@@ -10,6 +10,8 @@
 
 namespace ucc {
 
+void tc_forget(Ctx& c, const double* p, size_t n);  // tc_gemm.cu
+
 // ---------------------------------------------------------------------------------------
 // Integral blocks
 // ---------------------------------------------------------------------------------------
@@ -62,6 +64,12 @@ static void build_L_blocks(Ctx& c) {
   (void)nv;
 }
 
+static void choose_pair_rows(Ctx& c) {
+  size_t free_b = 0, total_b = 0;
+  UCC_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  c.pair_rows = ccsd_bytes(c.no, c.nv) <= kPairRowsShare * (double)total_b;
+}
+
 void load_from_ints(Ctx& c, int no, int nv, const double* fock, const double* ints) {
   c.no = no;
   c.nv = nv;
@@ -88,6 +96,7 @@ void load_from_ints(Ctx& c, int no, int nv, const double* fock, const double* in
     UCC_CUDA(cudaStreamSynchronize(c.stream));
   }
   build_L_blocks(c);
+  choose_pair_rows(c);
   UCC_CUDA(cudaStreamSynchronize(c.stream));
 }
 
@@ -122,6 +131,7 @@ void load_from_df(Ctx& c, int no, int nv, int naux, const double* fock, const do
   c.force_fp64 = saved;
   c.drop("Bdf");
   build_L_blocks(c);
+  choose_pair_rows(c);
   UCC_CUDA(cudaStreamSynchronize(c.stream));
 }
 
@@ -250,11 +260,33 @@ static void build_blocks(Ctx& c, const char* p, const std::vector<int64_t>& pdim
 }
 
 void pair_operator(Ctx& c) {
-  const int64_t no = c.no, nv = c.nv, vp = nv * (nv + 1) / 2, vm = nv * (nv - 1) / 2;
-  build_blocks(c, "Vpp", {vp + no * nv, vp}, "Vmm", {vm + no * nv, vm}, [&](double* P, double* M) {
+  const int64_t no = c.no, nv = c.nv, vp = nv * (nv + 1) / 2, vm = nv * (nv - 1) / 2, mb = c.pair_rows ? no * nv : 0;
+  build_blocks(c, "Vpp", {vp + mb, vp}, "Vmm", {vm + mb, vm}, [&](double* P, double* M) {
     pack_vvvv(c, c.nv, 0, c.get("Vvvvv").p, P, M);
-    pack_ovvv(c, c.no, c.nv, c.get("Vovvv").p, P + vp * vp, M + vm * vm);
+    if (mb) pack_ovvv(c, c.no, c.nv, c.get("Vovvv").p, P + vp * vp, M + vm * vm);
   });
+}
+
+double ccsd_bytes(int64_t no, int64_t nv) {
+  const double o = (double)no, v = (double)nv;
+  // <ab|ef> and half of it packed; <ma|ef>, its L form, a gathered copy and the packed rows; vectors of the
+  // length of t2: 16 of DIIS, 6 blocks of integrals, amplitudes, residual and tau, a sweep's scratch
+  return 8.0 * (1.5 * v * v * v * v + 4.0 * o * v * v * v + 36.0 * o * o * v * v);
+}
+
+bool release_pair_operator(Ctx& c, bool rows) {
+  if (rows ? !c.pair_rows : !c.has("Vpp")) return false;
+  c.pair_rows = false;
+  UCC_CUDA(cudaStreamSynchronize(c.stream));
+  for (const char* k : {"Vpp", "Vmm"})
+    if (c.has(k)) {
+      const DeviceBuffer& b = *c.store.at(k);
+      tc_forget(c, b.p, b.n);
+      c.drop(k);
+    }
+  UCC_CUDA(cudaStreamSynchronize(c.stream));
+  trim_pool(c.device);
+  return true;
 }
 
 // R2 += alpha sum_ef W_abef amp_ijef on packed pairs (pairs.cu), W from an HBAR block: S = Tp Vp^T
@@ -298,17 +330,19 @@ void build_F(Ctx& c, const Tensor& t1, const Tensor& ttau) {
 }
 
 // Products of tau with the packed operator, one GEMM per symmetry: the particle ladder's rows
-// (a <= b) and, below them, the (m, b) rows of Zmbij = sum_ef <mb|ef> tau_ijef.  A batch whose
-// members' packed operators would not fit in memory goes without (S and A stay null).
+// (a <= b) and, with c.pair_rows, the (m, b) rows of Zmbij = sum_ef <mb|ef> tau_ijef below them.  A
+// batch whose members' packed operators would not fit in memory goes without (S and A stay null).
 struct PairProducts {
   std::unique_ptr<Temp> S, A;
+  bool rows = false;  // Zmbij is there
   PairProducts(Ctx& c, const Tensor& tau) {
     if (recorder() && !recorder()->packed) return;
     const int64_t no = c.no, nv = c.nv, op = no * (no + 1) / 2, om = no * (no - 1) / 2;
     const int64_t vp = nv * (nv + 1) / 2, vm = nv * (nv - 1) / 2;
     if (!recorder()) pair_operator(c);
-    S = std::make_unique<Temp>(c, std::vector<int64_t>{op, PairLd(no, nv).s});
-    A = std::make_unique<Temp>(c, std::vector<int64_t>{om, PairLd(no, nv).a});
+    rows = c.get("Vpp").d[0] > vp;
+    S = std::make_unique<Temp>(c, std::vector<int64_t>{op, c.get("Vpp").d[0]});
+    A = std::make_unique<Temp>(c, std::vector<int64_t>{om, c.get("Vmm").d[0]});
     Temp Tp(c, {op, vp}), Tm(c, {om, vm});
     pack_tau(c, c.no, c.nv, tau.p, Tp->p, Tm->p);
     product(c, Tp, c.get("Vpp"), S->t);
@@ -316,6 +350,8 @@ struct PairProducts {
   }
   const double* s() const { return S ? S->t.p : nullptr; }
   const double* a() const { return A ? A->t.p : nullptr; }
+  int64_t lds() const { return S ? S->t.d[1] : 0; }
+  int64_t lda() const { return A ? A->t.d[1] : 0; }
 
  private:
   // out = T Op^T; a batch records it whatever the member's size, so that all members record
@@ -396,7 +432,7 @@ void build_t2(Ctx& c, const Tensor& t1, const Tensor& t2, const Tensor& tau, con
   {
     // Za[m,b,i,j] = <mb|ij> + Zmbij + t1[i,e] <mb|ej> + t1[j,e] <mb|ie>  ->  - t1[m,a] Za[m,b,i,j]
     Temp Za(c, {no, nv, no, no});
-    if (pairs.s())
+    if (pairs.rows)
       unpack_z(c, no, nv, pairs.s(), pairs.a(), Za->p);
     else
       contract(c, "mbef,ijef->mbij", 1.0, V(c, "ovvv"), tau, 0.0, Za);
@@ -406,7 +442,7 @@ void build_t2(Ctx& c, const Tensor& t1, const Tensor& t2, const Tensor& tau, con
     contract(c, "ma,mbij->ijab", -1.0, t1, Za, 1.0, Rh);
   }
   if (!pairs.s()) contract(c, "ijef,abef->ijab", 0.5, tau, V(c, "vvvv"), 1.0, Rh);
-  assemble_r2(c, no, nv, V(c, "oovv").p, pairs.s(), pairs.a(), Rh->p, H->p, R2.p);
+  assemble_r2(c, no, nv, V(c, "oovv").p, pairs.s(), pairs.lds(), pairs.a(), pairs.lda(), Rh->p, H->p, R2.p);
 }
 
 // the unscaled residual R(t_old) into r, given tau/ttau of t_old (ccwfn.cc:311-539); ev
@@ -604,7 +640,10 @@ CCSDResult run_ccsd(Ctx& c) {
   } else {  // a supplied guess (restart file, learned guess) applies to this solve only
     UCC_CUDA(cudaMemcpyAsync(T.p, c.get("T_guess").p, sizeof(double) * np, cudaMemcpyDeviceToDevice, c.stream));
     UCC_CUDA(cudaStreamSynchronize(c.stream));
-    c.drop("T_guess");
+    if (c.pair_rows)
+      c.taken = "T_guess";  // kept for a second attempt (release_pair_operator)
+    else
+      c.drop("T_guess");
   }
   auto tau_of = [&](double* buf) {
     build_tau(c, no, nv, buf, buf + (int64_t)no * nv, 1.0, c.get("tau").p, 0.5, c.get("ttau").p);
@@ -713,9 +752,9 @@ CCSDResult run_ccsd(Ctx& c) {
     c.stats.ladder_ms += ms;
     c.stats.ladder_launches += 1;
     const double o = no, v = nv;
-    // the ladder and Zmbij as the equations have them
-    c.stats.ladder_flops += 2.0 * o * o * v * v * v * v + 2.0 * o * o * o * v * v * v;
-    c.stats.ladder_bytes += 8.0 * (v * v * v * v + 3.0 * o * o * v * v + o * v * v * v + o * o * o * v);
+    // the ladder and, with the (m, b) rows, Zmbij as the equations have them
+    c.stats.ladder_flops += 2.0 * o * o * v * v * v * v + (c.pair_rows ? 2.0 * o * o * o * v * v * v : 0.0);
+    c.stats.ladder_bytes += 8.0 * (v * v * v * v + 3.0 * o * o * v * v + (c.pair_rows ? o * v * v * v + o * o * o * v : 0.0));
     cudaEventDestroy(ev[k]);
     cudaEventDestroy(ev[k + 1]);
   }

@@ -177,6 +177,9 @@ struct Fp64Scope {
   explicit Fp64Scope(Ctx& ctx, bool on = true);
   ~Fp64Scope();
 };
+// what lies unused in the device's stream-ordered pool, given back (for cudaMalloc)
+void trim_pool(int device);
+
 // Scoped setting of the FP64 switch to a given value (false re-enables split products
 // inside an FP64 scope when the context precision is MIXED).
 struct PrecisionScope {
@@ -195,6 +198,8 @@ struct Ctx {
   int no = 0, nv = 0, naux = 0;
   bool loaded = false, have_ccsd = false, have_hbar = false, have_lambda = false;
   bool have_tgrad = false;  // (T) gradient pieces present: Lambda and the densities include them
+  std::string taken;        // the guess that the running stage has read and leaves for a second attempt
+  bool pair_rows = true;    // the packed ladder operator has the (m, b) rows of <mb|ef> (pair_operator)
   std::vector<double> eps;  // orbital energies (diagonal of the Fock matrix)
   std::vector<double> fock;  // [nact][nact]
 
@@ -465,9 +470,9 @@ struct PairLd {
 // X = t2/2 + t1 t1, P = t2(ijba) - X, S = t2 - t2(ijba)/2 in one pass
 void ring_amplitudes(Ctx& c, int no, int nv, const double* t1, const double* t2, double* X, double* P, double* S);
 // R2 = V + ladder(S, A) + Q + Q(ji,ba), Q = Rh + H/2 + H(ijba): exactly symmetric under (i,j,a,b) -> (j,i,b,a);
-// S and A may be null (no ladder)
-void assemble_r2(Ctx& c, int no, int nv, const double* V, const double* S, const double* A, const double* Rh,
-                 const double* H, double* R2);
+// S and A may be null (no ladder), ldS and ldA their row lengths (in a batch those of PairLd)
+void assemble_r2(Ctx& c, int no, int nv, const double* V, const double* S, int64_t ldS, const double* A, int64_t ldA,
+                 const double* Rh, const double* H, double* R2);
 // Z[m][b][i][j] = sum_ef <mb|ef> tau_ijef from the (m, b) columns of S and A
 void unpack_z(Ctx& c, int no, int nv, const double* S, const double* A, double* Z);
 

@@ -85,6 +85,11 @@ HostBlock::HostBlock(Ctx& ctx) : c(ctx) {
   c.host_free.pop_back();
 }
 
+void trim_pool(int device) {
+  cudaMemPool_t pool;
+  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+}
+
 Scratch::Scratch(Ctx& c, size_t bytes) : ctx(&c) {
   if (bytes == 0) bytes = 16;
   if ((rec = recorder()) != nullptr) {

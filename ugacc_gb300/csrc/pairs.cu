@@ -137,12 +137,11 @@ void ring_amplitudes(Ctx& c, int no, int nv, const double* t1, const double* t2,
   launched("ring_amplitudes");
 }
 
-void assemble_r2(Ctx& c, int no, int nv, const double* V, const double* S, const double* A, const double* Rh,
-                 const double* H, double* R2) {
+void assemble_r2(Ctx& c, int no, int nv, const double* V, const double* S, int64_t ldS, const double* A, int64_t ldA,
+                 const double* Rh, const double* H, double* R2) {
   if (recorder()) return record(RecordedOp::kAssemble, no, nv, {V, S, A, Rh, H}, {R2});
-  const PairLd ld(no, nv);
   launch_chained(assemble_kernel, tile_grid(tile_pairs(nv), (int64_t)no * (no + 1) / 2), kBlock, c.stream, 1, no, nv, V,
-                 S, ld.s, A, ld.a, Rh, H, R2);
+                 S, ldS, A, ldA, Rh, H, R2);
   launched("assemble_r2");
 }
 

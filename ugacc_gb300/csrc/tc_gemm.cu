@@ -2152,6 +2152,20 @@ void tc_check(Ctx& c) {
   throw Error(UCC_BAD_ARGS, "sliced FP64 GEMM: an operand row maximum is beyond 2^498; use PRECISION FP64");
 }
 
+// drops the cached operands made from the n doubles at p
+void tc_forget(Ctx& c, const double* p, size_t n) {
+  if (!c.tc_cache) return;
+  tc::Cache& k = *static_cast<tc::Cache*>(c.tc_cache.get());
+  auto erase = [&](auto& m) {
+    for (auto it = m.begin(); it != m.end();) {
+      const double* q = std::get<0>(it->first);
+      it = q >= p && q < p + n ? m.erase(it) : std::next(it);
+    }
+  };
+  erase(k.ops);
+  erase(k.sliced);
+}
+
 // a device-side wait of limit_ns that nothing completes: the kernel returns once it runs
 // out and the status check that follows every tensor-core launch reports
 // UCC_DEVICE_TIMEOUT; the stream and the context stay usable
