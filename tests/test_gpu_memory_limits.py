@@ -110,3 +110,23 @@ def test_later_stage_takes_the_memory_of_the_packed_operator():
         given_back.append(not _rows_packed(cc))
         H.ctx.close()
     assert given_back[0] is False and given_back[-1] is True and given_back == sorted(given_back)
+
+
+@pytest.mark.gpu
+def test_batch_where_the_packed_operators_do_not_fit():
+    """Members whose packed integrals (2 x 375 MiB) do not fit are solved by the plain contractions."""
+    members = [make_hamiltonian(4, 96, seed=k) for k in (1, 2)]
+
+    def solve(leave):
+        b = U.Batch()
+        for h in members:
+            b.add(h)
+        with Held(leave * MB):
+            out = b.ccsd({"R_CONVERGENCE": 1e-9})
+        return (*out, b.info()["grouped_ops"])
+
+    e, it, conv, ops = solve(4000)
+    for leave, plain in ((1400, False), (500, True)):
+        f, jt, conw, n = solve(leave)
+        assert conv.all() and conw.all() and (it == jt).all() and (n != ops) == plain
+        assert abs(e - f).max() < 1e-12

@@ -724,27 +724,27 @@ void group_gemm(ucc_batch& B, GroupOp& g, const std::vector<std::vector<Recorded
   B.info.shape_choice[g.plan.shape]++;
 }
 
-// record every member's residual build and group the operations
-void build(ucc_batch& B) {
+// record every member's residual build and group the operations; packed: with the members' packed operators
+void build_with(ucc_batch& B, bool packed) {
   const int nm = (int)B.members.size();
   UCC_REQUIRE(nm >= 1, UCC_BAD_STATE, "empty batch");
   std::vector<std::vector<RecordedOp>> traces(nm);
   std::vector<std::string> tape;
   B.arenas.clear();
   B.diis_store.clear();
+  for (auto& m : B.members) {
+    m->pair_rows = packed;
+    if (!packed)
+      for (const char* k : {"Vpp", "Vmm"}) m->drop(k);
+  }
+  if (!packed) {
+    UCC_CUDA(cudaStreamSynchronize(B.stream));
+    trim_pool(B.device);
+  }
   double arena_bytes = 0.0;
-  // the packed operators (half of <ab|ef> again, and <ma|ef>) as long as they leave half of the
-  // free memory to the amplitudes, the scratch and the DIIS vectors
-  double operator_bytes = 0.0;
-  for (const auto& m : B.members)
-    if (!m->has("Vpp")) operator_bytes += 4.0 * std::pow((double)m->nv, 3) * (m->nv + 2.0 * m->no);
-  size_t free_b = 0, total_b = 0;
-  UCC_CUDA(cudaMemGetInfo(&free_b, &total_b));
-  const bool packed = operator_bytes < 0.5 * (double)free_b;
   for (int b = 0; b < nm; b++) {
     Ctx& c = *B.members[b];
     ccsd_alloc(c);
-    c.pair_rows = true;
     if (packed) pair_operator(c);
     const double* to = c.get("Told").p;
     double* r = c.get("R").p;
@@ -897,6 +897,25 @@ void build(ucc_batch& B) {
   B.info.grouped_ops = (int)nops;
   B.info.arena_bytes = arena_bytes;
   B.built = true;
+}
+
+// With the packed operators (half of <ab|ef> again, and <ma|ef>) where the batch's solves with them are
+// within their share of the device's memory.  That is a choice by the sizes alone; the plain contractions also
+// take over when others hold too much of the memory.
+void build(ucc_batch& B) {
+  double bytes = 0.0;
+  for (const auto& m : B.members) bytes += ccsd_bytes(m->no, m->nv);
+  size_t free_b = 0, total_b = 0;
+  UCC_CUDA(cudaMemGetInfo(&free_b, &total_b));
+  if (bytes <= kPairRowsShare * (double)total_b) {
+    try {
+      build_with(B, true);
+      return;
+    } catch (const Error& e) {
+      if (e.status != UCC_OUT_OF_MEMORY) throw;
+    }
+  }
+  build_with(B, false);
 }
 
 void set_all_active(ucc_batch& B) {
