@@ -131,8 +131,8 @@ __device__ __forceinline__ int find_item(const int64_t* __restrict__ prefix, int
 // one cluster of zc CTAs that share K) per tile, zg K shares per tile as partial products.
 // The members come longest K share first and every tile is its own CTA, so the hardware's
 // dispatch evens out the SMs; the FP64 pipe bounds the launch.  16 members of the
-// no <= 12 / nv <= 96 family, per solve of 8 sweeps: 1111 ms with padded 32 x 32 tiles on a
-// fixed grid, one CTA per tile whatever its K and the unpacked ladder, 354 ms now.
+// no <= 12 / nv <= 96 family, per solve of 8 sweeps: 1100 to 1180 ms with padded 32 x 32 tiles on
+// a fixed grid, one CTA per tile whatever its K and the unpacked ladder, 253 to 277 ms now (four boxes).
 // ---------------------------------------------------------------------------------------
 template <class T, bool CLUSTER>
 __global__ void __launch_bounds__(T::THREADS) grouped_gemm(const GemmDesc* __restrict__ desc,

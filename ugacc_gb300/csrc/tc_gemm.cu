@@ -3,18 +3,20 @@
 // C[m][n] (FP64, strided, alpha/beta, permuting epilogue) =
 //     sum_k  Ahi[m][k] Bhi[n][k] + Ahi[m][k] Blo[n][k] + Alo[m][k] Bhi[n][k]
 // where x = hi + lo with hi = bf16(x), lo = bf16(x - hi): the two-term split product of
-// FP64 operands, accumulated in FP32 in tensor memory.  The three products are one
-// K loop over 3 * K/64 blocks that switches the TMA source between the hi and lo copies.
+// FP64 operands, accumulated in FP32 in tensor memory (gemm_kernel); and FP64-accurate
+// products of exact bf16 digits (sliced_gemm_kernel, sliced_short_kernel below).
 //
-// Kernel layout (one CTA per SM, persistent over 128 x 256 output tiles):
-//   warp 0      TMA producer (one thread): A 128x64 and B 256x64 bf16 tiles, 128B swizzle
-//   warp 1      MMA issuer (one thread): tcgen05.mma.cta_group::1.kind::f16, M=128 N=256 K=16
+// gemm_kernel (one CTA per SM, persistent over 128 x bn output tiles, bn up to 256; with two M
+// tiles or more the CTAs work in pairs, cta_group::2, on 256 rows):
+//   warp 0      TMA producer (one thread): K blocks of 64 of A (128 rows) and B (bn rows, a pair's
+//               CTA half of them), 128B swizzle; a two-part stage holds hi and lo of both
+//   warp 1      MMA issuer (one thread, rank 0 of a pair): kind::f16, M = 128 or 256, K = 16
 //   warps 2-5   epilogue: tcgen05.ld 32x32b.x32 -> FP64 alpha/beta -> global
-//   4-stage smem ring (full/empty mbarriers), two TMEM accumulators (2 x 256 columns) so
-//   the epilogue of one tile overlaps the MMAs of the next.
+//   smem ring of up to 4 stages (full/empty mbarriers), two TMEM accumulators (2 x 256 columns) so
+//   the epilogue of one tile, or of one pass over K, overlaps the MMAs of the next.
 // Every mbarrier wait is bounded (globaltimer deadline); on expiry the kernel raises a
-// device error flag, the other warps see it and leave their loops, TMEM is released and
-// the host reports UCC_DEVICE_TIMEOUT.
+// device error flag, the other warps see it and leave their loops, loads and MMAs in flight are
+// awaited, TMEM is released and the host reports UCC_DEVICE_TIMEOUT.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -47,7 +49,7 @@ inline int pick_bn(int64_t N) {
   const int64_t nt = (N + 255) / 256;
   return (int)(((N + nt - 1) / nt + 31) / 32 * 32);
 }
-// CTAs per cluster for a launch with mtiles M tiles: pairs that share the B tile whenever
+// CTAs per cluster for a launch with mtiles M tiles: pairs that work on one N tile whenever
 // there are two M tiles to pair (the B maps then have boxes of bn / 2 rows)
 inline int cluster_m(int mtiles) { return mtiles >= 2 ? 2 : 1; }
 
@@ -1180,19 +1182,6 @@ __global__ void __launch_bounds__(kShortThreads, 1)
   }
 }
 
-// element (r, k) of a two-stride operand view (r, k and the splits below 2^32: 32-bit division)
-__device__ __forceinline__ const double& mv_at(const MatView& v, int64_t r, int64_t k) {
-  int64_t ro = r * v.rs_hi, ko = k * v.ks_hi;
-  if (v.rsplit) {
-    const uint32_t q = (uint32_t)r / (uint32_t)v.rsplit;
-    ro = (int64_t)q * v.rs_hi + ((int64_t)r - (int64_t)q * v.rsplit) * v.rs_lo;
-  }
-  if (v.ksplit) {
-    const uint32_t q = (uint32_t)k / (uint32_t)v.ksplit;
-    ko = (int64_t)q * v.ks_hi + ((int64_t)k - (int64_t)q * v.ksplit) * v.ks_lo;
-  }
-  return v.p[ro + ko];
-}
 __device__ __forceinline__ bool mv_kcontig(const MatView& v) { return (v.ksplit ? v.ks_lo : v.ks_hi) == 1; }
 
 // Offsets of 32 rows and 64 columns of an operand: one division per element of the two index
@@ -2227,12 +2216,12 @@ void tc_gemm_oriented(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, con
 // form; false when the problem is too small for it or outside its exponent range
 bool sliced_gemm(Ctx& c, int64_t M, int64_t N, int64_t K, double alpha, const MatView& A, const MatView& B,
                  double beta, double* C, int64_t sCm, int64_t sCn) {
-  // a short K (a few occupied indices) leaves too little work per slice and output: routing
-  // the K = 16 contractions of a no=16/nv=160 CCSD solve here instead of the DFMA kernel
-  // (operands sliced per call, 45 padded products, the 9-order epilogue) made its sweeps
-  // slower (203 -> 220 ms per solve), and the K = 32 ones of no=32/nv=320 (outputs of 1e8,
-  // 6.7 GFLOP) made its record sweeps slower too (606 -> 625 ms at 6 digits, 877 -> 946 ms
-  // at 8): the per-order epilogue passes over the output cost more than the DFMA work
+  // K < 48 (contractions over the occupied indices of most problems) stays on the FP64 pipe.  The line was
+  // drawn when every order's sum took a pass over the output: the K = 16 contractions of no=16/nv=160 made its
+  // sweeps slower here (203 -> 220 ms per solve), and so did the K = 32 ones of no=32/nv=320.
+  // sliced_short_kernel would be the faster one now (25600 x 2560 x 16: 0.77 ms against 1.92, K = 47 0.79 against
+  // 5.16), but nine digits of the row and column maxima leave 5.7e-16 of the result at K = 16 and the
+  // FP64 multiply-adds 1.0e-16, so moving these contractions would cost accuracy
   if (K < 48 || (double)M * N * K < kSlicedMinWork || M > INT32_MAX || N > INT32_MAX) return false;
   // the output must fill at least 1/16 of its 128 x (N rounded to 32) tiles
   const int64_t lo = std::min(M, N), hi = std::max(M, N);
