@@ -2338,6 +2338,7 @@ bool mixed_triples_prepare(Ctx& c, int max_batch) {
   const int64_t no = c.no, nv = c.nv, nv2 = nv * nv, kp = (nv + no + BK - 1) / BK * BK;
   if (nv < 64) return false;  // small virtual spaces stay on the FP64 path
   Cache& k = cache(c);
+  k.triples.reset();  // of a call that ran out of memory
   auto T = std::make_shared<Triples>();
   alloc_split(T->A, no * nv2, kp, c.stream);
   alloc_split(T->A2, no * nv2, kp, c.stream);
