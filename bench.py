@@ -67,8 +67,8 @@ def select_workload(name):
 
 # DRAM bytes (read + write) per launch of the roofline kernels at no=32/nv=320, from one
 # ncu launch list of the same solve (the no=32/nv=320 launch-list summary under profiles/):
-# split GEMM 1331 launches, sliced GEMM 91, DFMA GEMM 69
-TRAFFIC_C3 = {"split": 4.68e9, "sliced": 84.2e9, "dfma": 0.28e9}
+# split GEMM 1447 launches, sliced GEMM 118 (79 at 95.1 GB, 39 with a short K at 4.8 GB), DFMA GEMM 120
+TRAFFIC_C3 = {"split": 4.10e9, "sliced": 65.2e9, "dfma": 0.16e9}
 TRAFFIC_SOURCE = ("ncu launch list of the same workload, DRAM read + write per launch averaged over the "
                   "solve (the no=32/nv=320 launch-list summary under profiles/)")
 
